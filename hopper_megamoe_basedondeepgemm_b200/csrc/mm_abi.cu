@@ -9,6 +9,7 @@
 #include "mm_kernel.cuh"
 #include "mm_frontend.cuh"
 #include "mm_prep.cuh"
+#include "mm_batch.cuh"
 
 namespace {
 
@@ -135,13 +136,14 @@ int mm_get_layout(const mm_config_t* c, mm_layout_t* out) {
     {
         // per tile: 32 row records of 16 B (token tiles only), then per streamed K unit a record of up to 32 rows x 128 B
         // and the unit's scale-word slots (16 B per (scale word, row))
-        const int64_t rec32 = mm::kWideTokens * 128 + (mm::kUnitK / (4 * vec)) * mm::kWideTokens * 16;
+        // (E4M3 tokens: 256 B per row and unit)
+        const int64_t rec32 = mm::kWideTokens * (a8 ? 256 : 128) + (mm::kUnitK / (4 * vec)) * mm::kWideTokens * 16;
         out->token_tile_bytes = mm::kWideTokens * 16 + (c->hidden / mm::kUnitK) * rec32;
         out->mid_tile_bytes = (c->intermediate / mm::kUnitK) * rec32;
     }
     out->off_token_tiles = take(out->tile_capacity * out->token_tile_bytes);
     out->off_mid_tiles = take(out->tile_capacity * out->mid_tile_bytes);
-    out->off_arrive = take(2 * 2 * out->tile_capacity * 4);
+    out->off_arrive = take(2 * 2 * out->tile_capacity * 4 + 2 * mm::kBCounts * 4);   // (then the one-rank batch kernel's counts)
     out->total_bytes = off;
     return MM_OK;
 }
@@ -350,9 +352,11 @@ static int fill_params(const mm_config_t* cfg, const mm_launch_args_t* a, mm::KP
         }
     }
     *smem_bytes = used + 1024 + 256;
-    if (static_cast<size_t>(p.T) * p.topk * 4 > p.stage_region) return MM_ERR_UNSUPPORTED;
     return MM_OK;
 }
+
+// the multi-rank kernel keeps the list of the rows it dispatches in its token staging area
+static bool dispatch_list_fits(const mm::KParams& p) { return static_cast<size_t>(p.T) * p.topk * 4 <= p.stage_region; }
 
 static bool wants_tile_images(const mm::KParams& p) {
     return (p.knobs & mm::kKnobTileImages) != 0u && p.nstage_wide >= 3u && p.nrec >= 2u && static_cast<long long>(p.T) * p.topk > mm::kTileTokens;
@@ -374,6 +378,51 @@ static int launch_variant(const mm::KParams& p, int grid, size_t smem_bytes, cud
     return MM_OK;
 }
 
+// ----------------------------------------------------------------------------- one rank, more than a handful of rows
+// The batch kernel (mm_batch.cuh) takes over from the multi-rank kernel on one rank as soon as the launch can route more
+// rows than decode mode holds in one token tile (16); up to there the other kernel's split weight tiles win (16 entries on
+// 15 experts, E4M3 tokens: 43 us there, 45 here). It reads the inputs from the buffer's views on every SM, so inputs in
+// mapped host memory stay with the other kernel, as do launches beyond its tables (4096 routing entries, 128 token tiles).
+static bool wants_batch_kernel(const mm_launch_args_t* a, const mm::KParams& p) {
+    if (p.R != 1 || a->input_region != nullptr || a->engine != MM_ENGINE_UMMA || p.T == 0) return false;
+    if ((p.knobs & mm::kKnobTileImages) == 0u) return false;
+    const long long entries = static_cast<long long>(p.T) * p.topk;
+    if (entries > mm::kBMaxRows || entries <= mm::kTileTokens) return false;
+    const long long tiles = p.e_local + entries / 64;
+    return tiles <= mm::kBMaxTiles;
+}
+
+template <int kFmt>
+static int launch_batch(const mm::KParams& k, int grid, cudaStream_t stream) {
+    auto kern = mm::batch_moe_kernel<kFmt>;
+    mm::BParams p;
+    memset(&p, 0, sizeof(p));
+    p.T = k.T; p.topk = k.topk; p.E = k.e_local; p.H = k.H; p.I = k.I;
+    p.n1 = k.n1_tiles; p.n2 = k.n2_tiles; p.k1 = k.k1_units; p.k2 = k.k2_units;
+    p.unit_bytes = k.unit_bytes;
+    p.tile_limit = kFmt == 2 ? 96u : 128u;         // (E4M3: a wider record would leave too few weight stages beside the widened units)
+    p.x_row_bytes = k.x_row_bytes; p.x_sf_row_bytes = k.x_sf_row_bytes; p.rx_row_bytes = k.rx_row_bytes;
+    p.has_clamp = k.has_clamp; p.fast_math = k.fast_math; p.clamp = k.clamp;
+    p.l1_scale = k.l1_scale; p.l2_scale = k.l2_scale; p.mid_gs = k.mid_gs; p.mid_gs_recip = 1.0f / k.mid_gs;
+    p.buf = k.peer[k.rank]; p.w1 = k.w1; p.w2 = k.w2; p.y = k.y; p.stats = k.stats;
+    p.off_ctrl = k.off_ctrl; p.off_x = k.off_x; p.off_x_sf = k.off_x_sf; p.off_topk_idx = k.off_topk_idx; p.off_topk_w = k.off_topk_w;
+    p.off_rx = k.off_rx; p.off_comb = k.off_comb; p.off_token_tiles = k.off_token_tiles; p.off_mid_tiles = k.off_mid_tiles; p.off_arrive = k.off_arrive;
+    p.rx_region = k.rx_region; p.tile_capacity = k.tile_capacity;
+    p.timeout_ns = k.timeout_ns;
+    const int dyn = 232448 - static_cast<int>((sizeof(mm::BShared) + 255) / 256 * 256);
+    p.smem_ring = static_cast<uint32_t>(dyn - 1024);
+    static bool attr_set[64] = {};
+    int dev = 0;
+    MM_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || !attr_set[dev]) {
+        MM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+        if (dev >= 0 && dev < 64) attr_set[dev] = true;
+    }
+    kern<<<grid, mm::BFmt<kFmt>::kThreadsAll, dyn, stream>>>(p);
+    MM_CUDA(cudaGetLastError());
+    return MM_OK;
+}
+
 extern "C" {
 
 int mm_mega_moe_launch(const mm_config_t* cfg, const mm_launch_args_t* a, void* stream) {
@@ -384,6 +433,11 @@ int mm_mega_moe_launch(const mm_config_t* cfg, const mm_launch_args_t* a, void* 
     if (st != MM_OK) return st;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const bool umma = a->engine == MM_ENGINE_UMMA;
+    if (wants_batch_kernel(a, p)) {
+        return cfg->act_format == MM_FMT_FP8 ? launch_batch<2>(p, grid, s)
+             : cfg->act_format == MM_FMT_NVFP4 ? launch_batch<1>(p, grid, s) : launch_batch<0>(p, grid, s);
+    }
+    if (!dispatch_list_fits(p)) return MM_ERR_UNSUPPORTED;
     if (cfg->act_format == MM_FMT_FP8)                                     // tensor-core engine only
         return umma ? launch_variant<32, true, false, true>(p, grid, smem_bytes, s) : MM_ERR_UNSUPPORTED;
 #ifdef MM_WITH_CHECK_ENGINE
@@ -560,6 +614,7 @@ int mm_mega_moe_from_hidden_launch(const mm_config_t* cfg, const mm_launch_args_
     size_t smem_bytes = 0;
     int st = fill_params(cfg, a, &p, &grid, &smem_bytes);
     if (st != MM_OK) return st;
+    if (!dispatch_list_fits(p)) return MM_ERR_UNSUPPORTED;
     if (fe == nullptr || (fe->hidden_states == nullptr && fe->num_tokens > 0) || fe->router_weight == nullptr || fe->workspace == nullptr) return MM_ERR_INVALID_ARGUMENT;
     if (fe->num_tokens != a->num_tokens) return MM_ERR_INVALID_ARGUMENT;
     if (cfg->num_topk != 8 || cfg->num_experts > 1024) return MM_ERR_UNSUPPORTED;

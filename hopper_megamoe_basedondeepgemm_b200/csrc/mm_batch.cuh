@@ -1,0 +1,973 @@
+// The layer on one rank with more than a handful of routed rows, as one persistent sm_100a kernel of its own.
+//
+// With one rank nothing crosses NVLink, every SM can work out the whole routing by itself and rows need no flagged words:
+//
+//   routing  : every SM ranks all routing entries per expert (warp-wide matches, one histogram per warp), so the token
+//              tiles and the task list follow without any exchange between SMs.
+//   tiles    : an expert's rows form ceil(rows / tile limit) token tiles of at most 128 rows (96 with E4M3 tokens). The
+//              block-scaled MMA takes the same time for 16 and 128 rows, so an expert's weights stream once per tile.
+//   images   : SM (token mod G) copies its tokens' rows into the tiles' operand images in global memory (per streamed K
+//              unit one record: the unit's 128 B of every row in the tensor core's swizzled order, then the unit's
+//              scale planes), counted per tile; a task fetches the records with bulk copies.
+//   GEMMs    : D[128 weight rows x N token rows] (N = the tile's rows, rounded up to 16), accumulators in TMEM. The epilogue
+//              turns 16 tokens at a time through shared memory, so that all 128 threads of a group work whatever the row
+//              count and a thread holds eight gate and eight up values of one token. Two groups take the tasks in turn.
+//   order    : all L1 tasks dealt round-robin, then the L2 tasks claimed one by one (no tile is split along K, a slow SM
+//              takes fewer). The weight ring runs ahead over the L1 -> L2 hand-over, so that the stream does not stop there.
+//   combine  : per (token, 128-column block) behind a count per column block; routes added in slot order in fp32.
+//
+// Bound: HBM (the weights of the live experts once) up to about 40 rows per expert; beyond that the bytes an SM takes in
+// per unit (weights + token record).
+#pragma once
+#include "mm_kernel.cuh"
+
+namespace mm {
+
+constexpr int kBMaxRows = 4096;                    // routed rows of one launch
+constexpr int kBMaxTiles = 128;                    // token tiles of one launch (64 experts + rows beyond the tile limit)
+constexpr int kBTaskRing = 64;                     // claimed tasks of one SM that some role has still to see, at most
+constexpr int kBWStages = 12, kBRSlots = 12;       // at most: weight ring stages, token record slots
+constexpr int kBServiceWarps = 4;                  // weight loader, MMA issuer, record loader, spare
+constexpr int kBEpiWarps = 8;                      // two groups of four
+constexpr int kBCombineWarps = 4;
+constexpr int kBWorkWarps = kBEpiWarps + kBCombineWarps;    // warps 4..15 place the rows and copy them into the images
+constexpr int kBRankWarps = kBServiceWarps + kBWorkWarps;   // warps 0..15 rank the routing entries
+constexpr int kBThreads = 32 * (kBServiceWarps + kBWorkWarps);
+constexpr int kBExpWarps = 8;                      // E4M3 tokens: widening warps 12..19 (they take up the combine when their role ends)
+constexpr int kBThreadsA8 = 32 * (kBServiceWarps + kBEpiWarps + kBExpWarps);
+constexpr int kBColCounters = 32;                  // column blocks of 128 (hidden <= 4096)
+constexpr int kBCounts = kBColCounters + 32;       // counters of a launch besides the tiles': the column blocks', the claimed L2 tasks
+constexpr uint32_t kBVtStride = 152;               // floats between the tokens of `vt`
+constexpr uint32_t kBBarEpi0 = 1, kBBarEpi1 = 2, kBBarWork = 3, kBBarTiles = 4;    // named barriers
+
+struct BParams {
+    int T, topk, E, H, I;
+    int n1, n2, k1, k2;                            // weight tiles and K units of the two layers
+    uint32_t unit_bytes, tile_limit;               // bytes of a streamed weight unit; rows of a token tile at most
+    uint32_t x_row_bytes, x_sf_row_bytes, rx_row_bytes;
+    int has_clamp, fast_math;
+    float clamp, l1_scale, l2_scale, mid_gs, mid_gs_recip;
+    uint8_t* buf;
+    const uint8_t* w1; const uint8_t* w2;
+    __nv_bfloat16* y; int* stats;
+    long long off_ctrl, off_x, off_x_sf, off_topk_idx, off_topk_w, off_rx, off_comb, off_token_tiles, off_mid_tiles, off_arrive;
+    long long rx_region;
+    uint32_t tile_capacity;
+    uint32_t smem_ring;                            // bytes of dynamic shared memory for the two rings (and the widened units)
+    unsigned long long timeout_ns;
+};
+
+struct BShared {
+    uint64_t wfull[kBWStages], wempty[kBWStages], rfull[kBRSlots], rempty[kBRSlots];
+    uint64_t tmem_full[2], tmem_empty[2], xfull[2], xempty[2];
+    uint32_t tmem_base, epoch, abort_flag, M, wissued, rissued, comb_next, nw, nr, slot_bytes, spu, total, start_ok;
+    uint32_t seg_shift;                            // routing entries per ranking warp: 1 << seg_shift
+    uint32_t cnt[kMaxLocalExperts], ebase[kMaxLocalExperts];
+    uint32_t tile_e[kBMaxTiles];                   // expert
+    uint32_t tile_row0[kBMaxTiles];                // first row (index into `rowf`)
+    uint32_t tile_rows[kBMaxTiles];
+    uint32_t tile_a16[kBMaxTiles];                 // 16-row groups of all tiles before this one
+    uint32_t etile[kMaxLocalExperts];              // first tile of the expert
+    uint32_t task[kBTaskRing];                     // claimed L2 tasks: turn of the ring << 16 | tile << 8 | weight tile (0xFFFF: no more)
+    alignas(16) uint16_t wcnt[kBRankWarps][kMaxLocalExperts];  // routing entries per (ranking warp, expert), then the exclusive sums over the warps
+    alignas(16) uint8_t ex[kBMaxRows];             // expert of every routing entry (0xFF: masked, 0xFE: no such expert)
+    union {
+        uint16_t rank[kBMaxRows];                  // rank of the entry among those of its expert in its ranking warp (until the rows are placed)
+        float vt[2][kTileTokens * kBVtStride];     // 16 tokens' accumulators of a task, per epilogue group (see b_role_epilogue)
+    };
+    uint16_t ef[2][128];                           // per epilogue group: routing entry and top-k weight of the task's rows
+    float ew[2][128];
+    uint16_t rowf[kBMaxRows];                      // routing entry (token * topk + slot) of every row, experts one after the other
+};
+
+__device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+// one full 32 B sector per lane
+__device__ __forceinline__ void st_global_v8(void* p, const uint32_t (&v)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+}
+
+struct BCtx {
+    const BParams& p; BShared& c;
+    uint8_t* smem;
+    uint64_t deadline;
+    uint32_t par;
+    __device__ __forceinline__ bool aborted() const { return *reinterpret_cast<volatile uint32_t*>(&c.abort_flag) != 0u; }
+    __device__ __noinline__ void fail(uint32_t code, uint32_t detail = 0) const {
+        atomicCAS(reinterpret_cast<uint32_t*>(p.buf + p.off_ctrl + kCtrlStatus), 0u, code | (blockIdx.x << 8) | (detail << 16));
+        *reinterpret_cast<volatile uint32_t*>(&c.abort_flag) = 1u;
+    }
+    __device__ __forceinline__ bool expired() const { return globaltimer_ns() > deadline; }
+    __device__ __noinline__ bool wait_slow(uint64_t* bar, uint32_t parity, uint32_t code) const {
+        uint32_t it = 0;
+        while (!mbar_try_wait(bar, parity)) {
+            if ((++it & 0xFFu) == 0u) {
+                if (aborted()) return false;
+                if (expired()) { fail(code); return false; }
+            }
+        }
+        return true;
+    }
+    __device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity, uint32_t code) const {
+        return mbar_try_wait(bar, parity) ? true : wait_slow(bar, parity, code);
+    }
+    __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, uint32_t code) const {
+        return __all_sync(0xffffffffu, wait(bar, parity, code));
+    }
+    // a count in global memory reaches `need` (one lane polls for its warp)
+    __device__ __forceinline__ bool wait_count(const uint32_t* cnt, uint32_t need, uint32_t code, uint32_t detail) const {
+        uint32_t it = 0;
+        while (ld_acquire_gpu(cnt) < need) {
+            if ((++it & 0x1Fu) == 0u) {
+                if (aborted()) return false;
+                if (expired()) { fail(code, detail); return false; }
+            }
+        }
+        return true;
+    }
+    __device__ __forceinline__ void sm_phase(int slot) const {
+        reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlSmPhase)[blockIdx.x * kSmPhaseSlots + slot] = globaltimer_ns();
+    }
+    __device__ __forceinline__ void stamp(int slot) const {
+        reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlStamps)[slot] = globaltimer_ns();
+    }
+    __device__ __forceinline__ void stamp_max(int slot) const {
+        atomicMax(reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlStamps) + slot, globaltimer_ns());
+    }
+    __device__ __forceinline__ uint32_t* arrive_set() const { return reinterpret_cast<uint32_t*>(p.buf + p.off_arrive) + par * 2u * p.tile_capacity; }
+    __device__ __forceinline__ uint32_t* col_counts(uint32_t parity) const {
+        return reinterpret_cast<uint32_t*>(p.buf + p.off_arrive) + 4u * p.tile_capacity + parity * kBCounts;
+    }
+};
+
+template <int kFmt> struct BFmt {
+    static constexpr bool kA8 = kFmt == 2;
+    static constexpr int kVec = kFmt == 1 ? 16 : 32;
+    static constexpr uint32_t kPlanes = kUnitK / (4 * kVec);
+    static constexpr uint32_t kAtoms = kA8 ? 2u : 1u;               // 128 B swizzle atoms of a token row per K unit
+    static constexpr int kThreadsAll = kA8 ? kBThreadsA8 : kBThreads;
+    // bytes of one K unit's record of a tile with `a16` groups of 16 rows
+    static __device__ __forceinline__ uint32_t rec(uint32_t a16) { return a16 * 2048u * kAtoms + kPlanes * 512u; }
+    // offset of a tile's image: `ku` K units, `before` 16-row groups and `m` tiles in front of it
+    static __device__ __forceinline__ size_t image(uint32_t ku, uint32_t before, uint32_t m) {
+        return static_cast<size_t>(ku) * (static_cast<size_t>(before) * 2048u * kAtoms + static_cast<size_t>(m) * (kPlanes * 512u));
+    }
+};
+// a row's scale word inside a plane: the 32-lane x 4-column order of the tensor-memory scale copy
+__device__ __forceinline__ uint32_t plane_off(uint32_t n) { return (n & 31u) * 16u + (n >> 5) * 4u; }
+// lane 0's value, for the compiler a warp-uniform one
+__device__ __forceinline__ uint32_t b_uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+// 1 / 2^(e - 127) for an exponent byte e in [1, 254], exact
+__device__ __forceinline__ float pow2_recip(uint32_t e) { return __uint_as_float(e == 254u ? 0x00400000u : (254u - e) << 23); }
+
+// Task `ti` of this SM: layer << 28 | tile << 8 | weight tile, ~0 past the last one (kBNoTask: the launch is being aborted). The L1 tasks are dealt round-robin;
+// the L2 tasks are claimed one by one by the weight loader (a slow SM takes fewer), which leaves them in a ring for the
+// other roles.
+constexpr uint32_t kBEnd = 0xFFFFFFFFu, kBNoTask = 0xFFFFFFFEu;
+struct BTasks {
+    const BCtx& cx;
+    uint32_t my1;
+    __device__ __forceinline__ explicit BTasks(const BCtx& c_) : cx(c_) {
+        const uint32_t nt1 = c_.c.M * c_.p.n1;
+        my1 = blockIdx.x < nt1 ? udiv_small(nt1 - 1u - blockIdx.x, gridDim.x) + 1u : 0u;
+    }
+    __device__ __forceinline__ uint32_t l1(uint32_t ti) const {
+        const uint32_t t = blockIdx.x + ti * gridDim.x, m = udiv_small(t, cx.p.n1);
+        return (m << 8) | (t - m * cx.p.n1);
+    }
+    __device__ __forceinline__ uint32_t get(uint32_t ti) const {
+        if (ti < my1) return l1(ti);
+        const uint32_t k = ti - my1, tag = (k / kBTaskRing + 1u) << 16;
+        volatile uint32_t* slot = &cx.c.task[k % kBTaskRing];
+        uint32_t v = *slot, it = 0;
+        while ((v & 0xFFFF0000u) != tag) {
+            __nanosleep(20);
+            if ((++it & 0xFFu) == 0u && (cx.aborted() || cx.expired())) { if (!cx.aborted()) cx.fail(kErrTaskCapacity); return kBNoTask; }
+            v = *slot;
+        }
+        __syncwarp();
+        return (v & 0xFFFFu) == 0xFFFFu ? kBEnd : (1u << 28) | (v & 0xFFFFu);
+    }
+};
+
+// ============================================================================================= loaders
+template <bool kA8>
+__device__ void b_role_weights(const BCtx& cx, uint32_t lane) {
+    const BParams& p = cx.p; BShared& c = cx.c;
+    const uint32_t nw = b_uniform(c.nw), step = kA8 ? 1u : b_uniform(c.spu), stage_bytes = step * p.unit_bytes, G = gridDim.x, n1 = p.n1, n2 = p.n2, M = b_uniform(c.M);
+    uint8_t* ring = cx.smem + b_uniform(c.nr * c.slot_bytes);
+    uint32_t it = 0, s = 0, ph = 0;
+    BTasks tasks(cx);
+    // Order of the L2 tasks: the SMs with one L1 task less than the others get here an L1 task earlier, when only the first
+    // tiles' L1 outputs are complete: as many tiles as those SMs can work off meanwhile come first, tile by tile; the others
+    // follow column block by column block (the combine starts on a column block when all tiles have it).
+    uint32_t mA = 0, NA = 0, NT2 = 0;
+    uint32_t* claims = cx.col_counts(cx.par) + kBColCounters;
+    uint32_t next = 0u;
+    if (tasks.my1 == 0u && lane == 0) next = atomicAdd(claims, 1u);
+    #pragma unroll 1
+    for (uint32_t ti = 0;; ++ti) {
+        uint32_t t;
+        if (ti < tasks.my1) t = tasks.l1(ti);
+        else {
+            const uint32_t k = ti - tasks.my1, q = __shfl_sync(0xffffffffu, next, 0);
+            if (k == 0u) {
+                const uint32_t r1 = M * n1 - udiv_small(M * n1, G) * G, target = udiv_small((r1 ? G - r1 : 0u) * udiv_small(p.k1, p.k2), n2);
+                mA = target < M ? target : M; NA = mA * n2; NT2 = M * n2;
+            }
+            t = 0xFFFFu;
+            if (q < NA) { const uint32_t m = udiv_small(q, n2); t = (m << 8) | (q - m * n2); }
+            else if (q < NT2) { const uint32_t j = udiv_small(q - NA, M - mA); t = ((mA + q - NA - j * (M - mA)) << 8) | j; }
+            if (lane == 0) *reinterpret_cast<volatile uint32_t*>(&c.task[k % kBTaskRing]) = ((k / kBTaskRing + 1u) << 16) | t;
+            if (t == 0xFFFFu) {                              // (the epilogue groups look at every second task: both of the next two end there)
+                if (lane == 0) *reinterpret_cast<volatile uint32_t*>(&c.task[(k + 1u) % kBTaskRing]) = (((k + 1u) / kBTaskRing + 1u) << 16) | t;
+                break;
+            }
+            t |= 1u << 28;
+        }
+        if (ti + 1u >= tasks.my1 && lane == 0) next = atomicAdd(claims, 1u);     // (needed after this task: its latency is hidden)
+        const uint32_t layer = t >> 28, e = c.tile_e[(t >> 8) & 0xFFFFu], j = t & 0xFFu;
+        const uint32_t units = layer ? p.k2 : p.k1;
+        const uint8_t* src = (layer ? p.w2 : p.w1) + (static_cast<size_t>(e) * (layer ? n2 : n1) + j) * units * p.unit_bytes;
+        #pragma unroll 1
+        for (uint32_t u = 0; u < units; u += step, ++it, src += stage_bytes) {
+            uint64_t* full = kA8 ? &c.wfull[s] : &c.rfull[s];
+            if (!cx.warp_wait(kA8 ? &c.wempty[s] : &c.rempty[s], ph ^ 1u, kErrWaitEmpty)) return;
+            if (elect_one()) {
+                const uint32_t bytes = (units - u < step ? units - u : step) * p.unit_bytes;
+                mbar_arrive_expect_tx(full, bytes);
+                bulk_g2s(ring + static_cast<size_t>(s) * stage_bytes, src, bytes, full);
+                c.wissued = it + 1u;
+                if (it == 0u) {
+                    reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlSmWFirst)[blockIdx.x] = globaltimer_ns();
+                    cx.sm_phase(kSmFirstIssue);
+                }
+            }
+            __syncwarp();
+            if (++s == nw) { s = 0; ph ^= 1u; }
+        }
+    }
+}
+
+template <int kFmt>
+__device__ void b_role_records(const BCtx& cx) {
+    using F = BFmt<kFmt>;
+    const BParams& p = cx.p; BShared& c = cx.c;
+    const uint32_t lane = threadIdx.x & 31u, nr = b_uniform(c.nr), slot_bytes = b_uniform(c.slot_bytes), step = b_uniform(c.spu);
+    const uint32_t* arrive = cx.arrive_set();
+    uint32_t it = 0, s = 0, ph = 0;
+    uint32_t ready1[kBMaxTiles / 32] = {}, ready2[kBMaxTiles / 32] = {};
+    bool seen_l2 = false;
+    BTasks tasks(cx);
+    #pragma unroll 1
+    for (uint32_t ti = 0;; ++ti) {
+        const uint32_t t = tasks.get(ti);
+        if (t >= kBNoTask) break;
+        const uint32_t layer = t >> 28, m = (t >> 8) & 0xFFFFu;
+        // the tile is complete: L1 its rows, L2 the outputs of all L1 weight tiles. Looked up for the tile only when it is
+        // not yet known: `ready` remembers the tiles seen complete, 32 of them per lookup (one lane per tile)
+        uint32_t known = 0u;
+        #pragma unroll
+        for (uint32_t w = 0; w < kBMaxTiles / 32; ++w) if (w == (m >> 5)) known = layer ? ready2[w] : ready1[w];
+        if (((known >> (m & 31u)) & 1u) == 0u) {
+            uint32_t spins = 0;
+            for (;;) {
+                const uint32_t mm_ = (m & ~31u) + lane;
+                const bool r = mm_ < c.M && ld_acquire_gpu(arrive + layer * p.tile_capacity + mm_) >= (layer ? static_cast<uint32_t>(p.n1) : c.tile_rows[mm_]);
+                const uint32_t b = __ballot_sync(0xffffffffu, r);
+                #pragma unroll
+                for (uint32_t w = 0; w < kBMaxTiles / 32; ++w)
+                    if (w == (m >> 5)) { if (layer) ready2[w] = b; else ready1[w] = b; }
+                if ((b >> (m & 31u)) & 1u) break;
+                if ((++spins & 0xFu) == 0u) {
+                    if (cx.aborted()) return;
+                    if (cx.expired()) { cx.fail(layer ? kErrWaitL1Done : kErrWaitDispatchFlag, c.tile_e[m]); return; }
+                }
+            }
+            fence_proxy_async_all();                         // rows written through the generic proxy, read by bulk copies
+        }
+        const uint32_t a16 = (c.tile_rows[m] + 15u) >> 4, rec = F::rec(a16), units = layer ? p.k2 : p.k1;
+        const uint8_t* src = p.buf + (layer ? p.off_mid_tiles : p.off_token_tiles) + F::image(units, c.tile_a16[m], m);
+        if (lane == 0u && layer != 0u && !seen_l2) { seen_l2 = true; cx.sm_phase(kSmFirstL2Staged); }
+        #pragma unroll 1
+        for (uint32_t u = 0; u < units; u += step, ++it, src += step * rec) {
+            if (!cx.warp_wait(&c.rempty[s], ph ^ 1u, kErrWaitActsEmpty)) return;
+            if (elect_one()) {
+                const uint32_t bytes = (units - u < step ? units - u : step) * rec;
+                mbar_arrive_expect_tx(&c.rfull[s], bytes);
+                bulk_g2s(cx.smem + static_cast<size_t>(s) * slot_bytes, src, bytes, &c.rfull[s]);
+                c.rissued = it + 1u;
+                if (it == 0u) cx.sm_phase(kSmFirstStaged);
+            }
+            __syncwarp();
+            if (++s == nr) { s = 0; ph ^= 1u; }
+        }
+    }
+}
+
+// ============================================================================================= MMA issuer
+template <int kFmt>
+__device__ void b_role_mma(const BCtx& cx, uint32_t lane) {
+    using F = BFmt<kFmt>;
+    constexpr bool kA8 = F::kA8;
+    constexpr uint32_t kPlanes = F::kPlanes, kStepK = kA8 ? 32u : 64u;
+    constexpr uint32_t kIdesc = kA8 ? idesc_block_scaled(kFmtF8E2M1, kFmtF8E4M3, 128u, 0u, 1u)
+                                    : idesc_block_scaled(kFmtMxf4E2M1, kFmtMxf4E2M1, 128u, 0u, kFmt == 1 ? 0u : 1u);
+    const BParams& p = cx.p; BShared& c = cx.c;
+    // Everything the instructions below take as operands is broadcast from lane 0, which tells the compiler that it is the
+    // same in all lanes: the operands then stay in uniform registers. (A unit of 4 MMAs, 4 scale copies and 2 commits takes
+    // 580 cycles to issue from per-lane registers, 313 from uniform ones; the tensor pipe needs 256 of them.)
+    const uint32_t nr = b_uniform(c.nr), slot_bytes = b_uniform(c.slot_bytes), step = b_uniform(c.spu), tm = b_uniform(c.tmem_base);
+    const uint32_t rec0 = b_uniform(smem_u32(cx.smem)), ring0 = rec0 + nr * slot_bytes, x0 = ring0 + b_uniform(c.nw) * p.unit_bytes;
+    uint32_t it = 0, rs = 0, rph = 0, wsm0 = ring0, tok0 = rec0;        // units consumed; record slot (without widening also weight stage), its phase bit
+    BTasks tasks(cx);
+    #pragma unroll 1
+    for (uint32_t ti = 0;; ++ti) {
+        const uint32_t t = b_uniform(tasks.get(ti));
+        if (t >= kBNoTask) break;
+        const uint32_t m = (t >> 8) & 0xFFFFu, units = (t >> 28) ? p.k2 : p.k1;
+        const uint32_t atom = b_uniform(((c.tile_rows[m] + 15u) >> 4) * 2048u);       // bytes of one 128 B atom of the tile's rows
+        const uint32_t idesc_n = kIdesc | ((atom >> 10) << 17);                       // N = rows, in units of 8
+        const uint32_t rec = atom * F::kAtoms + kPlanes * 512u, acc = ti & 1u, use = (ti >> 1) & 1u, d = tm + acc * 128u;
+        if (!cx.warp_wait(&c.tmem_empty[acc], use ^ 1u, kErrWaitTmemEmpty)) return;
+        tc_fence_after();
+        #pragma unroll 1
+        for (uint32_t u = 0; u < units; u += step) {
+            if (!cx.warp_wait(&c.rfull[rs], rph, kErrWaitActsFull)) return;
+            #pragma unroll
+            for (uint32_t uu = 0; uu < 2; ++uu) {
+                if (uu < step && u + uu < units) {
+                    if constexpr (kA8) { if (!cx.warp_wait(&c.xfull[it & 1u], (it >> 1) & 1u, kErrWaitFull)) return; }
+                    if (uu == 0u || kA8) tc_fence_after();
+                    if (lane == 0 && it == 0u) cx.sm_phase(kSmFirstLanded);
+                    if (elect_one()) {
+                        const uint32_t wsm = kA8 ? x0 + (it & 1u) * kXbufBytes : wsm0 + uu * p.unit_bytes, tok = tok0 + uu * rec;
+                        const uint64_t adesc = smem_desc(wsm, 1024u, kLayoutSw128), bdesc = smem_desc(tok, 1024u, kLayoutSw128);
+                        const uint64_t asf = smem_desc(wsm + (kA8 ? 2u * kUnitWBytes : static_cast<uint32_t>(kUnitWBytes)), 128u, kLayoutNone);
+                        const uint64_t bsf = smem_desc(tok + atom * F::kAtoms, 128u, kLayoutNone);
+                        const uint32_t sfa = tm + 256u + (it & 1u) * 32u, sfb = sfa + 16u;
+                        #pragma unroll
+                        for (uint32_t pl = 0; pl < kPlanes; ++pl) {
+                            utccp_32x128b_warpx4(sfa + pl * 4u, asf + pl * 32u);
+                            utccp_32x128b_warpx4(sfb + pl * 4u, bsf + pl * 32u);
+                        }
+                        #pragma unroll
+                        for (uint32_t ks = 0; ks < kUnitK / kStepK; ++ks) {
+                            const uint32_t pl = (ks * kStepK) / (4u * F::kVec), sf_id = ((ks * kStepK) % (4u * F::kVec)) / F::kVec;
+                            const uint64_t ad = adesc + (ks & 3u) * 2u + (kA8 ? (ks >> 2) * (kUnitWBytes >> 4) : 0u);
+                            const uint64_t bd = bdesc + (ks & 3u) * 2u + (kA8 ? (ks >> 2) * (atom >> 4) : 0u);
+                            const uint32_t idesc = idesc_with_sf(idesc_n, sf_id, sf_id), accum = (u | uu | ks) != 0u ? 1u : 0u;
+                            if constexpr (kA8) umma_mxf8f6f4(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
+                            else if constexpr (kFmt == 0) umma_mxf4_block32(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
+                            else umma_nvf4_block16(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
+                        }
+                        if constexpr (kA8) tc_commit(&c.xempty[it & 1u]);
+                        if (uu + 1u >= step || u + uu + 1u >= units) tc_commit(&c.rempty[rs]);
+                    }
+                    __syncwarp();
+                    ++it;
+                }
+            }
+            wsm0 += step * p.unit_bytes; tok0 += slot_bytes;
+            if (++rs == nr) { rs = 0; rph ^= 1u; wsm0 = ring0; tok0 = rec0; }
+        }
+        if (elect_one()) tc_commit(&c.tmem_full[acc]);
+        __syncwarp();
+    }
+    if (lane == 0 && it != 0u) cx.stamp_max(kStampLastWeight);
+}
+
+// ============================================================================================= weight widener (E4M3 tokens)
+// kind::mxf8f6f4 reads 4-bit operands from byte-wide slots: every 16 E2M1 values (8 bytes) sit in a 16-byte slot. Eight warps
+// turn a packed unit (128 rows x 128 B) into two atoms of 128 rows x 128 B; two buffers, so that a unit is widened while the
+// one before it is multiplied. (All eight on one unit: with two groups on alternate units a buffer's round trip - widen,
+// multiply, barriers - took twice as long and was the bound.) Eight lanes read the eight chunks of a row and store the two
+// halves of each; the lanes of the second atom store theirs in the other order, so that the eight stores of a quarter-warp
+// fall on different banks.
+__device__ void b_role_widen(const BCtx& cx, uint32_t xtid) {
+    const BParams& p = cx.p; BShared& c = cx.c;
+    const uint32_t lane = xtid & 31u, nw = c.nw, ch = xtid & 7u, at = ch >> 2;
+    uint8_t* ring = cx.smem + c.nr * c.slot_bytes;
+    uint8_t* x0 = ring + static_cast<size_t>(nw) * p.unit_bytes;
+    constexpr uint32_t kItems = kTileRows * 8 / (kBExpWarps * 32);
+    uint32_t it = 0, s = 0, ph = 0;
+    BTasks tasks(cx);
+    #pragma unroll 1
+    for (uint32_t ti = 0;; ++ti) {
+        const uint32_t t = tasks.get(ti);
+        if (t >= kBNoTask) break;
+        const uint32_t units = (t >> 28) ? p.k2 : p.k1;
+        #pragma unroll 1
+        for (uint32_t u = 0; u < units; ++u, ++it) {
+            if (!cx.warp_wait(&c.wfull[s], ph, kErrWaitFull)) return;
+            const uint8_t* wsm = ring + static_cast<size_t>(s) * p.unit_bytes;
+            uint8_t* xb = x0 + (it & 1u) * kXbufBytes;
+            uint4 v[kItems];
+            uint4 sf = make_uint4(0u, 0u, 0u, 0u);
+            #pragma unroll
+            for (uint32_t k = 0; k < kItems; ++k) {
+                const uint32_t r = k * (kBExpWarps * 4) + (xtid >> 3);
+                v[k] = *reinterpret_cast<const uint4*>(wsm + r * 128u + ((ch ^ (r & 7u)) << 4));
+            }
+            if (xtid < 64u) sf = *reinterpret_cast<const uint4*>(wsm + kUnitWBytes + xtid * 16u);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&c.wempty[s]);        // (the unit is in registers: its stage can be refilled)
+            if (!cx.warp_wait(&c.xempty[it & 1u], ((it >> 1) & 1u) ^ 1u, kErrWaitEmpty)) return;
+            #pragma unroll
+            for (uint32_t k = 0; k < kItems; ++k) {
+                const uint32_t r = k * (kBExpWarps * 4) + (xtid >> 3), j = 2u * (ch & 3u);
+                uint8_t* row = xb + at * kUnitWBytes + r * 128u;
+                const uint32_t first = (j + at) ^ (r & 7u), second = (j + 1u - at) ^ (r & 7u);
+                *reinterpret_cast<uint4*>(row + (first << 4)) = at ? make_uint4(v[k].z, v[k].w, 0u, 0u) : make_uint4(v[k].x, v[k].y, 0u, 0u);
+                *reinterpret_cast<uint4*>(row + (second << 4)) = at ? make_uint4(v[k].x, v[k].y, 0u, 0u) : make_uint4(v[k].z, v[k].w, 0u, 0u);
+            }
+            if (xtid < 64u) *reinterpret_cast<uint4*>(xb + 2 * kUnitWBytes + xtid * 16u) = sf;
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&c.xfull[it & 1u]);
+            if (++s == nw) { s = 0; ph ^= 1u; }
+        }
+    }
+}
+
+// ============================================================================================= epilogue
+// SwiGLU of 8 outputs of one token from its 8 gate and 8 up accumulators. With `fast_math` the reciprocal of 1 + exp(-gate)
+// is the hardware approximation refined by one Newton-Raphson step: straight-line code, several times faster than the
+// exact reciprocal with its range checks.
+__device__ __forceinline__ void b_swiglu(const BParams& p, const float (&a)[16], float wgt, float (&o)[8]) {
+    float g[8], u[8];
+    const bool cl = p.has_clamp != 0;
+    #pragma unroll
+    for (uint32_t i = 0; i < 8; ++i) {
+        const __nv_bfloat162 gu = __floats2bfloat162_rn(a[i] * p.l1_scale, a[i + 8] * p.l1_scale);
+        const float gate = __low2float(gu), up = __high2float(gu);
+        const float gc = fminf(gate, p.clamp), uc = fminf(fmaxf(up, -p.clamp), p.clamp);
+        g[i] = cl ? gc : gate;
+        u[i] = cl ? uc : up;
+    }
+    if (p.fast_math) {
+        #pragma unroll
+        for (uint32_t i = 0; i < 8; ++i) {
+            const float d = 1.0f + fminf(__expf(-g[i]), 1e38f);
+            float r = __fdividef(1.0f, d);
+            r = fmaf(r, fmaf(-d, r, 1.0f), r);
+            o[i] = g[i] * r * u[i] * wgt;
+        }
+    } else {
+        #pragma unroll
+        for (uint32_t i = 0; i < 8; ++i) o[i] = g[i] * (1.0f / (1.0f + expf(-g[i]))) * u[i] * wgt;
+    }
+}
+// x / b from y = RN(1 / b): one residual correction of the product x * y gives the correctly rounded quotient (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990), without a division's range checks
+__device__ __forceinline__ float div_by(float x, float b, float y) {
+    const float q = x * y;
+    return fmaf(fmaf(-q, b, x), y, q);
+}
+
+// A task's accumulators lie with weight row l in lane l and token n in column n. 16 tokens at a time go through shared
+// memory: weight row 16 q + 4 i + k of token n to vt[n * 152 + i * 40 + q * 4 + k], which neither the writes (a warp: 32
+// rows of one token) nor the 16-byte reads (thread (n, q): its i = 0..3) find bank conflicts in. Thread (n = t / 8, q = t % 8)
+// then owns the 16 weight rows of group q of token n: L1 8 gate rows and the 8 matching up rows, L2 16 output columns.
+template <int kFmt>
+__device__ void b_role_epilogue(const BCtx& cx, uint32_t grp, uint32_t etid) {
+    using F = BFmt<kFmt>;
+    constexpr bool kA8 = F::kA8;
+    constexpr int kVec = F::kVec;
+    const BParams& p = cx.p; BShared& c = cx.c;
+    const uint32_t ew = etid >> 5, q = etid & 7u, n16 = etid >> 3;
+    const float* tw = reinterpret_cast<const float*>(p.buf + p.off_topk_w);
+    const uint32_t bar = grp ? kBBarEpi1 : kBBarEpi0;
+    float* vt = c.vt[grp];
+    float* vt_w = vt + ((etid & 15u) >> 2) * 40u + (etid >> 4) * 4u + (etid & 3u);
+    const float* vt_r = vt + n16 * kBVtStride + q * 4u;
+    BTasks tasks(cx);
+    #pragma unroll 1
+    for (uint32_t ti = grp;; ti += 2) {
+        const uint32_t t = tasks.get(ti);
+        const bool task = t < kBNoTask;
+        const uint32_t layer = t >> 28, m = task ? (t >> 8) & 0xFFFFu : 0u, j = t & 0xFFu;
+        const uint32_t rows = c.tile_rows[m], a16 = (rows + 15u) >> 4, use = (ti >> 1) & 1u;
+        bool ok = t != kBNoTask;
+        if (task) {
+            if (etid < rows) {
+                const uint32_t f = c.rowf[c.tile_row0[m] + etid];
+                c.ef[grp][etid] = static_cast<uint16_t>(f);
+                if (layer == 0u) c.ew[grp][etid] = tw[f];
+            }
+            ok = cx.warp_wait(&c.tmem_full[grp], use, kErrWaitTmemFull);
+            tc_fence_after();
+        }
+        // the group leaves together (an aborted launch, or the end of the tasks); also publishes ef and ew
+        if (bar_red_or(bar, 128u, !ok)) return;
+        if (!task) break;
+        const uint32_t acc = c.tmem_base + ((ew * 32u) << 16) + grp * 128u;
+        const uint32_t rec = F::rec(a16);
+        uint8_t* img = p.buf + p.off_mid_tiles + F::image(p.k2, c.tile_a16[m], m) + static_cast<size_t>(j >> 2) * rec;
+        #pragma unroll 1
+        for (uint32_t ch = 0; ch < a16; ++ch) {
+            uint32_t raw[kTileTokens];
+            tmem_ld_32x32b_x16(acc + ch * 16u, raw);
+            tmem_ld_wait();
+            if (ch + 1u == a16) { tc_fence_before(); __syncwarp(); if ((etid & 31u) == 0u) mbar_arrive(&c.tmem_empty[grp]); }
+            if (ch != 0u) bar_sync(bar, 128u);                              // (the reads of the chunk before are over)
+            #pragma unroll
+            for (uint32_t n = 0; n < kTileTokens; ++n) vt_w[n * kBVtStride] = __uint_as_float(raw[n]);
+            bar_sync(bar, 128u);
+            float a[16];
+            #pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {
+                const float4 v = *reinterpret_cast<const float4*>(vt_r + i * 40u);
+                a[4 * i] = v.x; a[4 * i + 1] = v.y; a[4 * i + 2] = v.z; a[4 * i + 3] = v.w;
+            }
+            const uint32_t n = ch * 16u + n16;
+            const bool live = n < rows;
+            if (layer == 0u) {
+                float o[8];
+                b_swiglu(p, a, live ? c.ew[grp][n] : 0.f, o);
+                float amax = 0.f;
+                #pragma unroll
+                for (uint32_t i = 0; i < 8; ++i) {
+                    if constexpr (kVec == 16) o[i] = div_by(o[i], p.mid_gs, p.mid_gs_recip);
+                    amax = fmaxf(amax, fabsf(o[i]));
+                }
+                // a scale block is the 8 columns of two (16 per block) or four threads
+                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+                if constexpr (kVec == 32) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+                amax = fmaxf(amax, 1e-30f);
+                uint32_t sf_byte;
+                if constexpr (kVec == 32) {
+                    sf_byte = ceil_pow2_exp(__fdiv_rn(amax, kA8 ? 448.0f : 6.0f));
+                    const float inv = pow2_recip(sf_byte);                    // a power of two: the product equals the quotient
+                    #pragma unroll
+                    for (uint32_t i = 0; i < 8; ++i) o[i] *= inv;
+                } else {
+                    sf_byte = cvt_e4m3x2(__fdiv_rn(amax, 6.0f), 0.f) & 0xFFu;
+                    const float sf = e4m3_to_float(sf_byte);
+                    const bool zero = sf_byte == 0u;                          // a scale that rounds to zero: every non-zero value saturates
+                    const float inv = zero ? 0.f : __frcp_rn(sf);
+                    #pragma unroll
+                    for (uint32_t i = 0; i < 8; ++i) {
+                        const float qt = div_by(o[i], sf, inv), sat = o[i] == 0.f ? 0.f : copysignf(6.0f, o[i]);
+                        o[i] = zero ? sat : qt;
+                    }
+                }
+                // the token's scale bytes of this tile, gathered in the thread q = 0
+                uint32_t sfw = sf_byte;
+                if constexpr (kVec == 32) sfw |= __shfl_down_sync(0xffffffffu, sf_byte, 4) << 8;
+                else {
+                    sfw |= __shfl_down_sync(0xffffffffu, sf_byte, 2) << 8;
+                    sfw |= __shfl_down_sync(0xffffffffu, sfw, 4) << 16;
+                }
+                if (live) {
+                    if constexpr (kA8) {
+                        uint8_t* at = img + ((j >> 1) & 1u) * a16 * 2048u + sw128_off(n, (j & 1u) * 4u + (q >> 1)) + (q & 1u) * 8u;
+                        *reinterpret_cast<uint2*>(at) = make_uint2(cvt_e4m3x2(o[0], o[1]) | (cvt_e4m3x2(o[2], o[3]) << 16),
+                                                                   cvt_e4m3x2(o[4], o[5]) | (cvt_e4m3x2(o[6], o[7]) << 16));
+                    } else {
+                        uint8_t* at = img + sw128_off(n, (j & 3u) * 2u + (q >> 2)) + (q & 3u) * 4u;
+                        *reinterpret_cast<uint32_t*>(at) = cvt_e2m1x2(o[0], o[1]) | (cvt_e2m1x2(o[2], o[3]) << 8) |
+                                                           (cvt_e2m1x2(o[4], o[5]) << 16) | (cvt_e2m1x2(o[6], o[7]) << 24);
+                    }
+                    if (q == 0u) {
+                        uint8_t* sf = img + a16 * 2048u * F::kAtoms + plane_off(n);
+                        if constexpr (kVec == 16) *reinterpret_cast<uint32_t*>(sf + (j & 3u) * 512u) = sfw;
+                        else *reinterpret_cast<uint16_t*>(sf + ((j >> 1) & 1u) * 512u + (j & 1u) * 2u) = static_cast<uint16_t>(sfw);
+                    }
+                }
+            } else {
+                uint32_t w[8];
+                #pragma unroll
+                for (uint32_t i = 0; i < 8; ++i)
+                    w[i] = static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(a[2 * i] * p.l2_scale))) |
+                           (static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(a[2 * i + 1] * p.l2_scale))) << 16);
+                if (live) st_global_v8(p.buf + p.off_comb + (static_cast<size_t>(c.ef[grp][n]) * p.H + j * 128u + q * 16u) * 2u, w);
+            }
+        }
+        // one thread counts the finished task; its release covers the stores of the group, which the barrier orders before it
+        bar_sync(bar, 128u);
+        if (etid == 96u) {
+            if (ti < 2u) cx.sm_phase(kSmFirstEpilogue);
+            if (layer == 0u) {
+                red_release_gpu_add(cx.arrive_set() + p.tile_capacity + m, 1u);
+                cx.sm_phase(kSmLastL1Epilogue);
+            } else {
+                red_release_gpu_add(cx.col_counts(cx.par) + j, 1u);
+            }
+        }
+    }
+}
+
+// ============================================================================================= combine
+// Item i = column block * T + token: a half-warp adds the token's routes over 128 columns. SM b has the items b, b + G, ...;
+// its warps take them two by two in that order: the combine warps from the start, the others when their role has ended.
+__device__ void b_role_combine(const BCtx& cx, uint32_t lane) {
+    const BParams& p = cx.p; BShared& c = cx.c;
+    const uint32_t G = gridDim.x, nitems = static_cast<uint32_t>(p.T) * p.n2, half = lane >> 4, l16 = lane & 15u;
+    const uint32_t* cols = cx.col_counts(cx.par);
+    const uint32_t M = c.M;
+    uint32_t known = 0xFFFFFFFFu;                            // the column block this half-warp saw complete last
+    #pragma unroll 1
+    for (;;) {
+        uint32_t k = 0u;
+        if (lane == 0) k = atomicAdd(&c.comb_next, 2u);
+        k = __shfl_sync(0xffffffffu, k, 0);
+        const uint32_t first = blockIdx.x + k * G;
+        if (first >= nitems) break;
+        const uint32_t i = first + half * G;
+        const bool valid = i < nitems;
+        const uint32_t col = udiv_small(valid ? i : first, p.T), tok = (valid ? i : first) - col * p.T;
+        uint32_t mask = 0u;
+        #pragma unroll 1
+        for (int sl = 0; sl < p.topk; ++sl) mask |= (c.ex[tok * p.topk + sl] < kMaxLocalExperts ? 1u : 0u) << sl;
+        bool ok = true;
+        if (col != known && l16 == 0u) ok = cx.wait_count(cols + col, M, kErrWaitCombineFlag, tok);
+        known = col;
+        if (!__all_sync(0xffffffffu, ok)) return;
+        __syncwarp();
+        __threadfence();                                     // (the polling lanes' acquire, handed to the others)
+        const uint8_t* src = p.buf + p.off_comb + (static_cast<size_t>(tok) * p.topk * p.H + col * 128u + l16 * 8u) * 2u;
+        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        #pragma unroll 1
+        for (int s0 = 0; s0 < p.topk; s0 += 8) {
+            uint4 v[8];
+            #pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                v[u] = make_uint4(0u, 0u, 0u, 0u);
+                if ((mask >> (s0 + u)) & 1u) v[u] = ld_cg_v4(src + static_cast<size_t>(s0 + u) * p.H * 2u);
+            }
+            #pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                acc[0] += __uint_as_float(v[u].x << 16); acc[1] += __uint_as_float(v[u].x & 0xFFFF0000u);
+                acc[2] += __uint_as_float(v[u].y << 16); acc[3] += __uint_as_float(v[u].y & 0xFFFF0000u);
+                acc[4] += __uint_as_float(v[u].z << 16); acc[5] += __uint_as_float(v[u].z & 0xFFFF0000u);
+                acc[6] += __uint_as_float(v[u].w << 16); acc[7] += __uint_as_float(v[u].w & 0xFFFF0000u);
+            }
+        }
+        uint4 o;
+        uint32_t* ow = &o.x;
+        #pragma unroll
+        for (int q = 0; q < 4; ++q)
+            ow[q] = static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(acc[2 * q]))) |
+                    (static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(acc[2 * q + 1]))) << 16);
+        if (valid) *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.y) + (static_cast<size_t>(tok) * p.H + col * 128u + l16 * 8u) * 2u) = o;
+        if (lane == 0 && k == 0u) cx.sm_phase(kSmFirstCombined);
+        if (lane == 0) cx.sm_phase(kSmCombineDone);
+    }
+}
+
+// ============================================================================================= routing
+// Sums over the ranking warps, the experts' token tiles and the ring geometry (one warp; lane l takes the experts 2l and
+// 2l + 1). Everything the SM does waits for it and its code runs once, from a cold instruction cache: few instructions.
+template <int kFmt>
+__device__ __forceinline__ void b_tiles(const BCtx& cx, uint32_t lane) {
+    using F = BFmt<kFmt>;
+    const BParams& p = cx.p; BShared& c = cx.c;
+    uint32_t* w32 = reinterpret_cast<uint32_t*>(&c.wcnt[0][0]) + lane;
+    uint32_t run = 0u;                                       // two 16-bit counts, at most 4096 each
+    #pragma unroll 4
+    for (uint32_t w = 0; w < kBRankWarps; ++w) { const uint32_t v = w32[w * (kMaxLocalExperts / 2)]; w32[w * (kMaxLocalExperts / 2)] = run; run += v; }
+    const uint32_t lim = p.tile_limit;
+    uint32_t cn[2] = {run & 0xFFFFu, run >> 16}, nt[2], rpt[2];
+    #pragma unroll
+    for (uint32_t h = 0; h < 2; ++h) { nt[h] = cn[h] != 0u ? 1u : 0u; rpt[h] = (cn[h] + 15u) & ~15u; }
+    if (__any_sync(0xffffffffu, cn[0] > lim || cn[1] > lim)) {
+        #pragma unroll 1
+        for (uint32_t h = 0; h < 2; ++h) {                   // ceil(rows / limit) tiles of ceil(rows / tiles) rows, rounded up to 16
+            const uint32_t n = h ? cn[1] : cn[0];
+            uint32_t k = udiv_small(n + lim - 1u, lim), r = 0u;
+            if (k != 0u) { r = (udiv_small(n + k - 1u, k) + 15u) & ~15u; k = udiv_small(n + r - 1u, r); }
+            if (h) { nt[1] = k; rpt[1] = r; } else { nt[0] = k; rpt[0] = r; }
+        }
+    }
+    // running sums over the experts of (rows, 16-row groups, tiles), packed 13 + 9 + 10 bits (all tiles of an expert but the
+    // last are multiples of 16 rows)
+    const uint32_t v0 = cn[0] | ((cn[0] + 15u) >> 4 << 13) | (nt[0] << 22), v1 = cn[1] | ((cn[1] + 15u) >> 4 << 13) | (nt[1] << 22);
+    uint32_t incl = v0 + v1;
+    #pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const uint32_t a = __shfl_up_sync(0xffffffffu, incl, o); if (static_cast<int>(lane) >= o) incl += a; }
+    const uint32_t all = __shfl_sync(0xffffffffu, incl, 31), M = all >> 22;
+    const uint32_t max16 = __reduce_max_sync(0xffffffffu, rpt[0] > rpt[1] ? rpt[0] : rpt[1]) >> 4;
+    #pragma unroll 1
+    for (uint32_t h = 0; h < 2; ++h) {
+        const uint32_t e = 2u * lane + h, x = incl - v1 - (h ? 0u : v0), n = h ? cn[1] : cn[0], r = h ? rpt[1] : rpt[0];
+        const uint32_t r0 = x & 0x1FFFu, a0 = (x >> 13) & 0x1FFu;
+        uint32_t m = x >> 22;
+        c.cnt[e] = n; c.ebase[e] = r0; c.etile[e] = m;
+        #pragma unroll 1
+        for (uint32_t lo = 0; lo < n; lo += r, ++m) {
+            if (m >= kBMaxTiles) break;
+            c.tile_e[m] = e;
+            c.tile_row0[m] = r0 + lo;
+            c.tile_rows[m] = n - lo < r ? n - lo : r;
+            c.tile_a16[m] = a0 + (lo >> 4);
+        }
+    }
+    if (lane == 0) {
+        if (M > kBMaxTiles) cx.fail(kErrTaskCapacity, M);
+        c.M = M; c.total = all & 0x1FFFu;
+        c.start_ok = cx.aborted() ? 0u : 1u;                 // (decided once: every warp takes the same way from here)
+        // Rings. Weights and records of equal depth: a record from the L2 takes about as long as a unit from HBM while the
+        // weights stream. A stage holds two K units where four such stages fit (narrow tiles): the MMA warp's barrier waits
+        // and loop cost more than its issue, and this halves them.
+        const uint32_t rec = (max16 ? max16 : 1u) * 2048u * F::kAtoms + F::kPlanes * 512u;
+        const uint32_t room = p.smem_ring - (F::kA8 ? 2u * kXbufBytes : 0u), pair = p.unit_bytes + rec;
+        const uint32_t spu = pair * 8u <= room ? 2u : 1u;
+        uint32_t nr = udiv_small(room, pair * spu);
+        nr = nr > kBRSlots ? kBRSlots : nr;
+        uint32_t nw = nr;
+        if (F::kA8) {                                        // single-unit weight stages in what the records leave
+            nw = udiv_small(room - nr * spu * rec, p.unit_bytes);
+            nw = nw > kBWStages ? kBWStages : nw;
+        }
+        c.nr = nr; c.nw = nw; c.slot_bytes = rec * spu; c.spu = spu;
+    }
+}
+
+// ============================================================================================= the kernel
+template <int kFmt>
+__global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(const __grid_constant__ BParams p) {
+    using F = BFmt<kFmt>;
+    const unsigned long long t_first = globaltimer_ns();
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ BShared c;
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~static_cast<uintptr_t>(1023u));
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, bid = blockIdx.x, G = gridDim.x;
+    uint32_t* ctrl32 = reinterpret_cast<uint32_t*>(p.buf + p.off_ctrl);
+    const uint32_t nent = static_cast<uint32_t>(p.T) * p.topk;
+    const bool worker = warp >= kBServiceWarps && warp < kBServiceWarps + kBWorkWarps;
+    const uint32_t ww = warp - kBServiceWarps;
+    // ---- this SM's tokens (token mod G): the first row of every worker warp is fetched before the routing is known
+    const uint32_t ntok = bid < static_cast<uint32_t>(p.T) ? udiv_small(p.T - 1u - bid, G) + 1u : 0u, nrows = ntok * p.topk;
+    const uint32_t xq = p.x_row_bytes / 16u, per_row = xq + p.x_sf_row_bytes / 16u;
+    constexpr uint32_t kChunks = F::kA8 ? 9u : 5u;               // 16 B chunks of a row per lane (hidden <= 4096)
+    constexpr uint32_t kAhead = F::kA8 ? 1u : 2u;                // rows a worker warp has in flight
+    uint4 v[kAhead][kChunks];
+    auto load_row = [&](uint4 (&v)[kChunks], uint32_t k) {
+        if (k >= nrows) return;
+        const uint32_t tok = bid + udiv_small(k, p.topk) * G;
+        const uint8_t* xs = p.buf + p.off_x + static_cast<size_t>(tok) * p.x_row_bytes;
+        const uint8_t* sf = p.buf + p.off_x_sf + static_cast<size_t>(tok) * p.x_sf_row_bytes;
+        #pragma unroll
+        for (uint32_t u = 0; u < kChunks; ++u) {
+            const uint32_t ci = lane + u * 32;
+            if (ci < per_row) v[u] = ld_cg_v4(ci < xq ? xs + ci * 16u : sf + (ci - xq) * 16u);
+        }
+    };
+    if (worker) {
+        #pragma unroll
+        for (uint32_t a = 0; a < kAhead; ++a) load_row(v[a], ww + a * kBWorkWarps);
+    }
+    // ---- the routing entries' experts into shared memory
+    {
+        const long long* tk = reinterpret_cast<const long long*>(p.buf + p.off_topk_idx);
+        #pragma unroll 4
+        for (uint32_t f = tid; f < nent; f += F::kThreadsAll) {
+            const long long e = tk[f];
+            c.ex[f] = static_cast<uint8_t>(e < 0 ? 0xFF : (e < p.E ? static_cast<int>(e) : 0xFE));
+        }
+    }
+    if (tid == 0) {
+        const uint32_t ep = ctrl32[kCtrlEpoch / 4 + bid];
+        ctrl32[kCtrlEpoch / 4 + bid] = ep + 1u;
+        c.epoch = ep; c.abort_flag = 0u; c.comb_next = 0u; c.wissued = 0u; c.rissued = 0u;
+        // a run of 32, 64, 128 or 256 routing entries per ranking warp
+        const uint32_t per = (nent + kBRankWarps - 1u) / kBRankWarps;
+        c.seg_shift = per <= 32u ? 5u : 32u - __clz(per - 1u);
+        reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlSmEntry)[bid] = t_first;
+        reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlSmPhase)[bid * kSmPhaseSlots + kSmEntry] = t_first;
+        reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlSmWFirst)[bid] = ~0ull;
+    }
+    if (warp == 2) {
+        if (lane < kBWStages) { mbar_init(&c.wfull[lane], 1); mbar_init(&c.wempty[lane], F::kA8 ? kBExpWarps : 1); }
+        if (lane < kBRSlots) { mbar_init(&c.rfull[lane], F::kA8 ? 1 : 2); mbar_init(&c.rempty[lane], 1); }
+        if (lane < 2) {
+            mbar_init(&c.tmem_full[lane], 1); mbar_init(&c.tmem_empty[lane], 4);
+            mbar_init(&c.xfull[lane], kBExpWarps); mbar_init(&c.xempty[lane], 1);
+        }
+        c.task[lane] = 0u; c.task[lane + 32] = 0u;
+        mbar_fence_init();
+    }
+    if (warp == 1) { tmem_alloc(&c.tmem_base, 512); tmem_relinquish(); tc_fence_before(); }
+    if (warp < kBRankWarps) reinterpret_cast<uint32_t*>(c.wcnt[warp])[lane] = 0u;
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t epoch = c.epoch;
+    BCtx cx{p, c, smem, globaltimer_ns() + p.timeout_ns, epoch & 1u};
+    if (tid == 0) {
+        cx.sm_phase(kSmPrologue);
+        if (bid == 0) {
+            ctrl32[kCtrlStatus / 4 + 1] = epoch + 1u;
+            ctrl32[kCtrlStatus / 4 + 2] = 16u;                       // rows of an expert start on 16-row boundaries of the images
+            ctrl32[kCtrlStatus / 4 + 3] = p.tile_limit;
+            reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlStamps)[kStampEntry] = t_first;
+            cx.stamp(kStampPrologue);
+        }
+    }
+    // ---- rank of every entry among the entries of its expert in this warp's run
+    const uint32_t seg_shift = c.seg_shift;
+    if (warp < kBRankWarps) {
+        const uint32_t lo = warp << seg_shift, hi = lo + (1u << seg_shift);
+        uint16_t* cnt = c.wcnt[warp];
+        #pragma unroll 1
+        for (uint32_t f = lo + lane; f - lane < (hi < nent ? hi : nent); f += 32u) {
+            const uint32_t e = f < nent ? c.ex[f] : 0xFFu;
+            // the lanes with the same expert: one ballot per bit (several times faster than a warp-wide match)
+            uint32_t same = __ballot_sync(0xffffffffu, e < kMaxLocalExperts);
+            #pragma unroll
+            for (uint32_t b = 0; b < 6; ++b) {
+                const uint32_t v = __ballot_sync(0xffffffffu, (e >> b) & 1u);
+                same &= (e >> b) & 1u ? v : ~v;
+            }
+            const uint32_t below = same & ((1u << lane) - 1u);
+            const uint32_t base = e < kMaxLocalExperts ? cnt[e] : 0u;
+            __syncwarp();
+            if (e < kMaxLocalExperts) {
+                c.rank[f] = static_cast<uint16_t>(base + __popc(below));
+                if (below == 0u) cnt[e] = static_cast<uint16_t>(base + __popc(same));
+            } else if (e == 0xFEu) cx.fail(kErrWaitCombineFlag, 0xFFFFu);       // a route to an expert that does not exist
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    // ---- tiles. The warp that works them out is the weight loader: it starts the weight stream without waiting for the others
+    if (warp == 0) {
+        if (lane == 0) cx.sm_phase(kSmCountsKnown);
+        b_tiles<kFmt>(cx, lane);
+        __syncwarp();
+        __threadfence_block();
+        bar_arrive(kBBarTiles, F::kThreadsAll);
+        if (lane == 0) { cx.sm_phase(kSmScheduled); if (bid == 0) cx.stamp(kStampScheduled); }
+    } else {
+        bar_sync(kBBarTiles, F::kThreadsAll);
+        if (tid == 96) cx.stamp_max(kStampLastScheduled);
+    }
+
+    const bool start = c.start_ok != 0u;
+    if (warp == 3 && start) {
+        // the arrival counts of this launch's parity were cleared by the launch before it; clear the other set for the next one
+        uint32_t* other = reinterpret_cast<uint32_t*>(p.buf + p.off_arrive) + (cx.par ^ 1u) * 2u * p.tile_capacity;
+        #pragma unroll 1
+        for (uint32_t i = bid * 32u + lane; i < 2u * p.tile_capacity; i += G * 32u) other[i] = 0u;
+        if (bid == 0) {
+            cx.col_counts(cx.par ^ 1u)[lane] = 0u;
+            cx.col_counts(cx.par ^ 1u)[lane + 32] = 0u;
+            #pragma unroll 1
+            for (uint32_t e = lane; e < static_cast<uint32_t>(p.E) && p.stats != nullptr; e += 32) p.stats[e] += static_cast<int>(c.cnt[e]);
+            // header line of the receive pool, for whoever inspects it afterwards
+            if (lane == 0) st_ll_16B(p.buf + p.off_rx + static_cast<size_t>(cx.par) * p.rx_region, make_uint4(c.total, 0u, 0u, 0u), epoch + 1u);
+        }
+    }
+    if (worker && start) {
+        // ---- copy the rows of this SM's tokens into the tiles' images, one warp per row; a warp's stores are released four
+        //      rows at a time (under the weight stream a release takes microseconds)
+        uint32_t done_m[4], ndone = 0;
+        #pragma unroll 1
+        for (uint32_t k = ww; k < nrows; k += kBWorkWarps) {
+            const uint32_t kt = udiv_small(k, p.topk), tok = bid + kt * G, f = tok * p.topk + k - kt * p.topk;
+            const uint32_t e = c.ex[f];
+            uint4 row[kChunks];
+            #pragma unroll
+            for (uint32_t u = 0; u < kChunks; ++u) {
+                row[u] = v[0][u];
+                #pragma unroll
+                for (uint32_t a = 1; a < kAhead; ++a) v[a - 1][u] = v[a][u];
+            }
+            load_row(v[kAhead - 1u], k + kAhead * kBWorkWarps);
+            if (e < kMaxLocalExperts) {
+                // the expert's tile with this row
+                const uint32_t pos = c.wcnt[f >> seg_shift][e] + c.rank[f], eb = c.ebase[e];
+                uint32_t m = c.etile[e];
+                while (pos >= c.tile_row0[m] - eb + c.tile_rows[m]) ++m;
+                const uint32_t n = pos - (c.tile_row0[m] - eb), a16 = (c.tile_rows[m] + 15u) >> 4, rec = F::rec(a16);
+                uint8_t* img = p.buf + p.off_token_tiles + F::image(p.k1, c.tile_a16[m], m);
+                #pragma unroll
+                for (uint32_t u = 0; u < kChunks; ++u) {
+                    const uint32_t ci = lane + u * 32;
+                    if (ci < xq) {
+                        const uint32_t at = ci >> 3;                                          // 128 B atom of the row
+                        *reinterpret_cast<uint4*>(img + (F::kA8 ? (at >> 1) * rec + (at & 1u) * a16 * 2048u : at * rec) + sw128_off(n, ci & 7u)) = row[u];
+                    } else if (ci < per_row) {
+                        const uint32_t g = (ci - xq) * 4u;                                    // scale words g .. g + 3: unit g / planes, plane g % planes
+                        const uint32_t wv[4] = {row[u].x, row[u].y, row[u].z, row[u].w};
+                        #pragma unroll
+                        for (uint32_t q = 0; q < 4; ++q)
+                            *reinterpret_cast<uint32_t*>(img + ((g + q) / F::kPlanes) * rec + a16 * 2048u * F::kAtoms + ((g + q) % F::kPlanes) * 512u + plane_off(n)) = wv[q];
+                    }
+                }
+                #pragma unroll
+                for (uint32_t q = 0; q < 4; ++q) if (q == ndone) done_m[q] = m;
+                ++ndone;
+            }
+            if (ndone == 4u || (ndone != 0u && k + kBWorkWarps >= nrows)) {
+                __syncwarp();
+                if (lane == 0) {
+                    fence_acq_rel_gpu();             // (the reader's proxy fence after its acquire orders these stores with its bulk copies)
+                    #pragma unroll
+                    for (uint32_t q = 0; q < 4; ++q) if (q < ndone) atomicAdd(cx.arrive_set() + done_m[q], 1u);
+                }
+                ndone = 0u;
+            }
+        }
+        if (lane == 0) cx.sm_phase(kSmRowsCached);
+        // ---- the list of rows, for the epilogue
+        #pragma unroll 1
+        for (uint32_t f = tid - 32u * kBServiceWarps; f < nent; f += kBWorkWarps * 32u) {
+            const uint32_t e = c.ex[f];
+            if (e < kMaxLocalExperts) c.rowf[c.ebase[e] + c.wcnt[f >> seg_shift][e] + c.rank[f]] = static_cast<uint16_t>(f);
+        }
+        bar_sync(kBBarWork, kBWorkWarps * 32u);
+        // ---- off the critical path: the rows' records in the receive pool (a row's place: the live entries before it), for
+        //      whoever inspects the pool afterwards
+        if (warp >= kBServiceWarps + kBEpiWarps) {
+            #pragma unroll 1
+            for (uint32_t k = ww - kBEpiWarps; k < nrows; k += kBWorkWarps - kBEpiWarps) {
+                const uint32_t kt = udiv_small(k, p.topk), tok = bid + kt * G, slot = k - kt * p.topk, f = tok * p.topk + slot;
+                const uint32_t e = c.ex[f];
+                if (e >= kMaxLocalExperts) continue;
+                uint32_t li = 0u;
+                #pragma unroll 1
+                for (uint32_t i = lane * 4u; i < f; i += 128u) {
+                    const uint32_t w = *reinterpret_cast<const uint32_t*>(c.ex + i);
+                    #pragma unroll
+                    for (uint32_t b = 0; b < 4; ++b) li += (i + b < f && ((w >> (8u * b)) & 0xFFu) < kMaxLocalExperts) ? 1u : 0u;
+                }
+                li = __reduce_add_sync(0xffffffffu, li);
+                if (lane == 0)
+                    st_ll_16B(p.buf + p.off_rx + static_cast<size_t>(cx.par) * p.rx_region + 32u + static_cast<size_t>(li) * 2u * p.rx_row_bytes + 2u * (p.rx_row_bytes - 16u),
+                              make_uint4(e, tok, slot, __float_as_uint(reinterpret_cast<const float*>(p.buf + p.off_topk_w)[f])), epoch + 1u);
+            }
+        }
+    }
+
+    // ---- roles
+    if (start) {
+        if (warp == 0) b_role_weights<F::kA8>(cx, lane);
+        else if (warp == 1) b_role_mma<kFmt>(cx, lane);
+        else if (warp == 2) b_role_records<kFmt>(cx);
+        else if (warp >= kBServiceWarps && warp < kBServiceWarps + kBEpiWarps)
+            b_role_epilogue<kFmt>(cx, (warp - kBServiceWarps) >> 2, tid - 32u * kBServiceWarps - ((warp - kBServiceWarps) >> 2) * 128u);
+        else if (warp >= kBServiceWarps + kBEpiWarps) {
+            if constexpr (F::kA8) b_role_widen(cx, tid - 32u * (kBServiceWarps + kBEpiWarps));
+        }
+    }
+    if (tid == 128) { cx.stamp_max(kStampLastTasksDone); cx.sm_phase(kSmTasksDone); if (bid == 0) cx.stamp(kStampTasksDone); }
+    if (!cx.aborted()) b_role_combine(cx, lane);
+    // ---- exit: an aborted SM lets the copies in flight land (bounded waits) before its shared memory goes away
+    // (both loaders count into the stages' barriers: a stage that only one of them has filled never completes, so the
+    // wait is also bounded in time)
+    if (cx.aborted() && (warp == 0 || warp == 2)) {
+        const bool w = warp == 0;
+        const uint32_t issued = *reinterpret_cast<volatile uint32_t*>(w ? &c.wissued : &c.rissued), nst = w ? c.nw : c.nr;
+        uint64_t* bars = w && F::kA8 ? c.wfull : c.rfull;
+        #pragma unroll 1
+        for (uint32_t k = issued > nst ? issued - nst : 0u; k < issued; ++k)
+            for (uint32_t spin = 0; spin < 2000u && !mbar_try_wait(&bars[k % nst], (k / nst) & 1u); ++spin) { }
+        for (uint32_t spin = 0; spin < 2000u; ++spin) __nanosleep(100);          // (copies of some 10 KB: microseconds at most)
+    }
+    __syncthreads();
+    if (warp == 1) { tc_fence_after(); tmem_dealloc(c.tmem_base, 512); }
+    if (tid == 0) { if (bid == 0) cx.stamp(kStampExit); cx.stamp_max(kStampLastExit); cx.sm_phase(kSmExit); }
+}
+
+}  // namespace mm

@@ -1830,6 +1830,8 @@ __global__ void __launch_bounds__(kA8 ? kThreads + kNumExpThreads : kThreads, 1)
         uint32_t* other = reinterpret_cast<uint32_t*>(buf + p.off_arrive) + (par ^ 1u) * 2u * p.tile_capacity;
         #pragma unroll 1
         for (uint32_t i = bid * kO + tid; i < 2u * p.tile_capacity; i += G * kO) other[i] = 0u;
+        // (and the counts of the one-rank batch kernel, which shares the buffer and the launch numbering)
+        if (bid == 0 && tid < 64u) reinterpret_cast<uint32_t*>(buf + p.off_arrive)[4u * p.tile_capacity + (par ^ 1u) * 64u + tid] = 0u;
     }
     // The rows of this rank's own tokens never travel when `own_ok`: every SM lists them from topk_idx and reads their
     // tokens where the caller put them. The SM that would have dispatched them only leaves their header line and records
@@ -2217,7 +2219,7 @@ __global__ void __launch_bounds__(kA8 ? kThreads + kNumExpThreads : kThreads, 1)
             const uint32_t M = res >> 16, nmine = res & 0xFFFFu;
             const uint32_t nt1 = M * p.n1_tiles, nt2 = M * p.n2_tiles;
             if (lane == 0) {
-                if (bid == 0) ctrl32[kCtrlStatus / 4 + 2] = c.bulk != 0u ? c.tw : 0u;      // (for whoever inspects the intermediate rows afterwards)
+                if (bid == 0) { ctrl32[kCtrlStatus / 4 + 2] = c.bulk != 0u ? c.tw : 0u; ctrl32[kCtrlStatus / 4 + 3] = 0u; }   // (for whoever inspects the intermediate rows afterwards)
                 c.nt1 = nt1; c.nt2 = nt2;
                 if (M > kMaxMTiles || nmine > kMaxTasks) cx.fail(kErrTaskCapacity, nmine);
                 else c.ntasks = nmine;

@@ -131,8 +131,8 @@ class SymmBuffer:
         return mirror, views
 
     def tile_image_rows(self) -> int:
-        """Rows per token tile (16 or 32) if the latest launch kept its received and intermediate rows as tile images
-        (more than 16 received rows), 0 if it kept them as flagged rows. Synchronises the stream."""
+        """Row granularity of the tile images if the latest launch kept its received and intermediate rows as such: an
+        expert's rows start on a multiple of it (16 or 32). 0 if it kept them as flagged rows. Synchronises the stream."""
         return int(self.device_status()[1][2])
 
     def _rows_of_tile_images(self, tiles: torch.Tensor, row_bytes: int, tw: int, header: int):
@@ -151,9 +151,43 @@ class SymmBuffer:
         words = slots[..., :4].permute(0, 3, 1, 2, 4).reshape(nt * tw, units * planes, 4)
         return rows.contiguous(), words.contiguous()
 
+    def _rows_of_batch_images(self, limit: int):
+        """(rows uint8 [R, mid_row_bytes], scale words uint8 [R, words, 4]) of the latest launch of the one-rank batch
+        kernel (csrc/mm_batch.cuh): an expert's rows start on a 16-row boundary, experts in ascending order. An expert's
+        n rows form t = ceil(n / limit) token tiles of ceil(n / t) rows (rounded up to 16); a tile's image is one record
+        per K unit: its rows (a multiple of 16) x 128 B in the 128 B swizzle (E4M3: two such atoms), then the unit's scale
+        planes of 512 B, the word of row r at (r % 32) * 16 + (r // 32) * 4."""
+        L = self.layout
+        counts = [0] * self.num_experts
+        for (e, _, _, _) in self.received_records()[0]:
+            counts[e] += 1
+        atoms, planes = (2 if self.act_format == 'fp8' else 1), 256 // (4 * int(L.sf_vec))
+        units, row_bytes = self.intermediate_hidden // 256, int(L.mid_row_bytes)
+        raw = self.mid_tiles.reshape(-1).cpu()
+        rows_out, words_out, off = [], [], 0
+        for n in counts:
+            if n == 0:
+                continue
+            tiles = (n + limit - 1) // limit
+            per = ((n + tiles - 1) // tiles + 15) // 16 * 16
+            for lo in range(0, n, per):
+                r16 = (min(per, n - lo) + 15) // 16 * 16
+                rec = r16 * 128 * atoms + planes * 512
+                recs = raw[off:off + units * rec].reshape(units, rec)
+                off += units * rec
+                tok = recs[:, :r16 * 128 * atoms].reshape(units, atoms, r16, 8, 16)
+                r = torch.arange(r16)
+                stored = (torch.arange(8).view(1, 8) ^ (r.view(-1, 1) & 7)).view(1, 1, r16, 8, 1).expand(units, atoms, r16, 8, 16)
+                rows_out.append(torch.gather(tok, 3, stored).permute(2, 0, 1, 3, 4).reshape(r16, row_bytes))
+                slots = recs[:, r16 * 128 * atoms:].reshape(units, planes, 32, 4, 4)[:, :, r % 32, r // 32]
+                words_out.append(slots.permute(2, 0, 1, 3).reshape(r16, units * planes, 4))
+        return torch.cat(rows_out).contiguous(), torch.cat(words_out).contiguous()
+
     def l2_acts_payload(self) -> torch.Tensor:
         """The intermediate rows of the latest launch without flag words or swizzle: uint8 [mid_rows, mid_row_bytes]."""
-        tw = self.tile_image_rows()
+        tw, limit = self.device_status()[1][2:4]
+        if limit:
+            return self._rows_of_batch_images(limit)[0]
         if tw:
             return self._rows_of_tile_images(self.mid_tiles, int(self.layout.mid_row_bytes), tw, 0)[0]
         rows = self.l2_acts.size(0)
@@ -161,7 +195,10 @@ class SymmBuffer:
 
     def l2_acts_sf_payload(self) -> torch.Tensor:
         """The intermediate rows' scale bytes, K-major: uint8 [mid_rows, intermediate / vec]."""
-        tw = self.tile_image_rows()
+        tw, limit = self.device_status()[1][2:4]
+        if limit:
+            words = self._rows_of_batch_images(limit)[1]
+            return words.reshape(words.size(0), -1)[:, :self.intermediate_hidden // int(self.layout.sf_vec)].contiguous()
         if tw:
             words = self._rows_of_tile_images(self.mid_tiles, int(self.layout.mid_row_bytes), tw, 0)[1]
             return words.reshape(words.size(0), -1)[:, :self.intermediate_hidden // int(self.layout.sf_vec)].contiguous()

@@ -1,0 +1,115 @@
+"""The one-rank batch kernel (csrc/mm_batch.cuh) at the sizes where it can go wrong, against the CPU oracle: row counts around
+the 16-row groups and the tile limits (128 rows, 96 with E4M3 tokens), more tokens than SMs, masked slots, the largest
+launch, experts without rows. Tolerances are the layer's: relative RMSE 0.3 %, counts and slot maps exact."""
+import pytest
+import torch
+
+import hopper_megamoe_basedondeepgemm_b200 as mm
+from hopper_megamoe_basedondeepgemm_b200 import _lib
+from oracle import megamoe_oracle as O
+from tests import util_moe as U
+from tests.test_gpu_layer import REL_RMSE_TOL, check_against_oracle, run_layer
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize('fmt', ['mxfp4', 'nvfp4', 'fp8'])
+@pytest.mark.parametrize('e_local,topk,tokens', [
+    (8, 1, 17),           # one entry more than decode mode takes
+    (2, 2, 16), (2, 2, 17),         # exactly one 16-row group per expert, and one row beyond it
+    (2, 2, 96), (2, 2, 97),         # the E4M3 tile limit
+    (2, 2, 128), (2, 2, 129),       # the tile limit of the 4-bit formats
+    (64, 3, 31),          # the most experts, an odd number of routes, many experts with one row or none
+    (4, 3, 301),          # more tokens than SMs, several tiles per expert
+])
+def test_row_counts_around_the_tile_edges(fmt, e_local, topk, tokens):
+    y, stats, ref, buf, _ = run_layer(fmt, e_local, 512, 256, topk, tokens, 'random', 'umma', seed=tokens, std=0.02)
+    assert buf.device_status()[1][3] == (96 if fmt == 'fp8' else 128)          # the batch kernel ran
+    check_against_oracle(y, stats, ref, buf, fmt, 256)
+
+
+@pytest.mark.parametrize('num_sms', [5, 0])
+@pytest.mark.parametrize('hidden,inter', [(512, 768), (1536, 256), (4096, 256)])
+def test_shapes_and_small_grids(hidden, inter, num_sms):
+    """K units that fill no pair, an L1 task shorter than an L2 task, the largest hidden size; a grid of a few SMs."""
+    y, stats, ref, buf, _ = run_layer('mxfp4', 6, hidden, inter, 4, 23, 'random', 'umma', seed=hidden, std=0.02, num_sms=num_sms,
+                                      masked_ratio=0.3, t_max=64)
+    assert buf.device_status()[1][3] == 128
+    check_against_oracle(y, stats, ref, buf, 'mxfp4', inter)
+
+
+def _small_layer(fmt, e, hidden, inter, topk, tokens, seed, masked=0.0):
+    w, _, _ = O.make_expert_weights(e, hidden, inter, fmt, seed=seed, std=0.05)
+    l1, l2 = mm.transform_weights_for_mega_moe(*U.to_operator_weights(w, fmt, 'cuda'))
+    buf = mm.get_symm_buffer_for_mega_moe(None, e, tokens, topk, hidden, inter, act_format=fmt)
+    idx, tw = U.random_routing(tokens, e, topk, seed + 1, masked)
+    _, inp, sfb = U.make_rank_inputs(tokens, hidden, fmt, seed + 2, idx, tw)
+    U.write_inputs(buf, inp, sfb)
+    return w, l1, l2, buf, inp, sfb
+
+
+# (a clamp far inside the values' range would not do: it makes rows of equal products, and one rounding tie they share then
+# moves the whole output by 2 %, with the multi-rank kernel just as much)
+@pytest.mark.parametrize('fast_math,clamp', [(True, None), (False, 0.5)])
+def test_largest_launch_exact_math_and_clamp(fast_math, clamp):
+    """4096 routing entries, twice on one buffer (the second launch counts in the other set of arrival counters)."""
+    fmt, e, hidden, inter, topk, tokens = 'mxfp4', 64, 512, 256, 8, 512
+    w, l1, l2, buf, inp, _ = _small_layer(fmt, e, hidden, inter, topk, tokens, 900, 0.05)
+    ref = O.moe_layer_reference([inp], [w], fmt, e, clamp=clamp)
+    y = torch.empty((tokens, hidden), dtype=torch.bfloat16, device='cuda')
+    for _ in range(2):
+        mm.fp4_fp4_mega_moe(y.zero_(), l1, l2, buf, activation_clamp=clamp, fast_math=fast_math, timeout_ms=500.0)
+        assert buf.device_status()[0] == 0
+        assert O.rel_rmse(y.cpu(), ref.y[0]) <= REL_RMSE_TOL
+
+
+def test_all_slots_masked_gives_zeros():
+    _, l1, l2, buf, _, _ = _small_layer('mxfp4', 4, 512, 256, 4, 20, 910)
+    buf.topk_idx.fill_(-1)
+    y = torch.full((20, 512), 3.0, dtype=torch.bfloat16, device='cuda')
+    mm.fp4_fp4_mega_moe(y, l1, l2, buf, timeout_ms=500.0)
+    assert buf.device_status()[0] == 0 and float(y.abs().max()) == 0.0
+
+
+def test_route_to_a_missing_expert_is_reported_and_the_buffer_recovers():
+    w, l1, l2, buf, inp, sfb = _small_layer('mxfp4', 4, 512, 256, 2, 20, 920)
+    ref = O.moe_layer_reference([inp], [w], 'mxfp4', 4, clamp=None)
+    y = torch.empty((20, 512), dtype=torch.bfloat16, device='cuda')
+    buf.topk_idx[7, 1] = 4
+    mm.fp4_fp4_mega_moe(y, l1, l2, buf, timeout_ms=500.0)
+    st, words = buf.device_status()
+    assert st == 4 and (words[0] & 0xFF) == 9                  # the status a route nobody serves has always had
+    buf.reset()
+    U.write_inputs(buf, inp, sfb)
+    mm.fp4_fp4_mega_moe(y, l1, l2, buf, timeout_ms=500.0)
+    assert buf.device_status()[0] == 0 and O.rel_rmse(y.cpu(), ref.y[0]) <= REL_RMSE_TOL
+
+
+def test_decode_and_batch_launches_alternate_on_one_buffer():
+    """Both kernels share the buffer's launch numbering and clear each other's counters."""
+    fmt, e, hidden, inter, topk = 'fp8', 4, 512, 256, 2
+    w, _, _ = O.make_expert_weights(e, hidden, inter, fmt, seed=1, std=0.05)
+    l1, l2 = mm.transform_weights_for_mega_moe(*U.to_operator_weights(w, fmt, 'cuda'))
+    buf = mm.get_symm_buffer_for_mega_moe(None, e, 64, topk, hidden, inter, act_format=fmt)
+    for it, tokens in enumerate([40, 3, 40, 8, 9, 1, 2, 64]):
+        idx, tw = U.random_routing(tokens, e, topk, 930 + it)
+        _, inp, sfb = U.make_rank_inputs(tokens, hidden, fmt, 940 + it, idx, tw)
+        ref = O.moe_layer_reference([inp], [w], fmt, e, clamp=None)
+        U.write_inputs(buf, inp, sfb)
+        y = torch.empty((tokens, hidden), dtype=torch.bfloat16, device='cuda')
+        mm.fp8_fp4_mega_moe(y, l1, l2, buf, timeout_ms=500.0)
+        st, words = buf.device_status()
+        assert st == 0 and words[1] == it + 1 and (words[3] != 0) == (tokens * topk > 16)
+        assert O.rel_rmse(y.cpu(), ref.y[0]) <= REL_RMSE_TOL, (it, tokens)
+
+
+def test_layout_holds_the_packed_images():
+    """An expert's rows are rounded up to 16 in the images: the regions hold the worst case of every format."""
+    import ctypes
+    lib = _lib.load()
+    for fmt, atoms, planes in (('mxfp4', 1, 2), ('nvfp4', 1, 4), ('fp8', 2, 2)):
+        cfg, L = _lib.MMConfig(1, 0, 64, 512, 8, 3072, 1280, _lib.FMT[fmt], 148), _lib.MMLayout()
+        assert lib.mm_get_layout(ctypes.byref(cfg), ctypes.byref(L)) == 0
+        groups, tiles = (4096 + 15 * 64 + 15) // 16, 64 + 4096 // 64
+        need = lambda units: units * (groups * 2048 * atoms + tiles * planes * 512)      # noqa: E731
+        assert L.tile_capacity * L.token_tile_bytes >= need(12) and L.tile_capacity * L.mid_tile_bytes >= need(5)
