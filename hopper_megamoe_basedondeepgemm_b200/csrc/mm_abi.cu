@@ -235,6 +235,21 @@ int mm_read_phase_stamps(const mm_config_t* cfg, const void* buffer, uint64_t ou
 
 }  // extern "C"
 
+// Every kernel of the library starts with what needs no other launch's results and then waits for the grids before it by
+// itself (griddepcontrol.wait), so it may be scheduled before they have ended: on a busy stream its launch latency and its
+// prologue disappear behind the end of the previous kernel (a one-token layer: 27.0 us a pass without, see the design table).
+template <typename P>
+static int launch_early(void (*kern)(P), unsigned grid, unsigned threads, size_t smem_bytes, cudaStream_t stream, const P& params) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem_bytes; cfg.stream = stream;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    MM_CUDA(cudaLaunchKernelEx(&cfg, kern, params));
+    return MM_OK;
+}
+
 static int fill_params(const mm_config_t* cfg, const mm_launch_args_t* a, mm::KParams* P, int* grid, size_t* smem_bytes) {
     mm_layout_t L;
     int st = mm_get_layout(cfg, &L);
@@ -373,9 +388,7 @@ static int launch_variant(const mm::KParams& p, int grid, size_t smem_bytes, cud
         MM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_bytes)));
         if (dev >= 0 && dev < 64) attr_bytes[dev] = static_cast<int>(smem_bytes);
     }
-    kern<<<grid, kA8 ? mm::kThreads + mm::kNumExpThreads : mm::kThreads, smem_bytes, stream>>>(p);
-    MM_CUDA(cudaGetLastError());
-    return MM_OK;
+    return launch_early<mm::KParams>(kern, grid, kA8 ? mm::kThreads + mm::kNumExpThreads : mm::kThreads, smem_bytes, stream, p);
 }
 
 // ----------------------------------------------------------------------------- one rank, more than a handful of rows
@@ -418,9 +431,7 @@ static int launch_batch(const mm::KParams& k, int grid, cudaStream_t stream) {
         MM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
-    kern<<<grid, mm::BFmt<kFmt>::kThreadsAll, dyn, stream>>>(p);
-    MM_CUDA(cudaGetLastError());
-    return MM_OK;
+    return launch_early<mm::BParams>(kern, grid, mm::BFmt<kFmt>::kThreadsAll, dyn, stream, p);
 }
 
 extern "C" {

@@ -728,7 +728,6 @@ __device__ __forceinline__ void b_tiles(const BCtx& cx, uint32_t lane) {
 template <int kFmt>
 __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(const __grid_constant__ BParams p) {
     using F = BFmt<kFmt>;
-    const unsigned long long t_first = globaltimer_ns();
     extern __shared__ uint8_t smem_raw[];
     __shared__ BShared c;
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~static_cast<uintptr_t>(1023u));
@@ -737,6 +736,22 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
     const uint32_t nent = static_cast<uint32_t>(p.T) * p.topk;
     const bool worker = warp >= kBServiceWarps && warp < kBServiceWarps + kBWorkWarps;
     const uint32_t ww = warp - kBServiceWarps;
+    // ---- what needs nothing of the launches before this one: it overlaps the end of the previous kernel in the stream
+    if (warp == 2) {
+        if (lane < kBWStages) { mbar_init(&c.wfull[lane], 1); mbar_init(&c.wempty[lane], F::kA8 ? kBExpWarps : 1); }
+        if (lane < kBRSlots) { mbar_init(&c.rfull[lane], F::kA8 ? 1 : 2); mbar_init(&c.rempty[lane], 1); }
+        if (lane < 2) {
+            mbar_init(&c.tmem_full[lane], 1); mbar_init(&c.tmem_empty[lane], 4);
+            mbar_init(&c.xfull[lane], kBExpWarps); mbar_init(&c.xempty[lane], 1);
+        }
+        c.task[lane] = 0u; c.task[lane + 32] = 0u;
+        mbar_fence_init();
+    }
+    if (warp == 1) { tmem_alloc(&c.tmem_base, 512); tmem_relinquish(); tc_fence_before(); }
+    if (warp < kBRankWarps) reinterpret_cast<uint32_t*>(c.wcnt[warp])[lane] = 0u;
+    grid_dependency_wait();
+    grid_launch_dependents();
+    const unsigned long long t_first = globaltimer_ns();
     // ---- this SM's tokens (token mod G): the first row of every worker warp is fetched before the routing is known
     const uint32_t ntok = bid < static_cast<uint32_t>(p.T) ? udiv_small(p.T - 1u - bid, G) + 1u : 0u, nrows = ntok * p.topk;
     const uint32_t xq = p.x_row_bytes / 16u, per_row = xq + p.x_sf_row_bytes / 16u;
@@ -778,18 +793,6 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
         reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlSmPhase)[bid * kSmPhaseSlots + kSmEntry] = t_first;
         reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlSmWFirst)[bid] = ~0ull;
     }
-    if (warp == 2) {
-        if (lane < kBWStages) { mbar_init(&c.wfull[lane], 1); mbar_init(&c.wempty[lane], F::kA8 ? kBExpWarps : 1); }
-        if (lane < kBRSlots) { mbar_init(&c.rfull[lane], F::kA8 ? 1 : 2); mbar_init(&c.rempty[lane], 1); }
-        if (lane < 2) {
-            mbar_init(&c.tmem_full[lane], 1); mbar_init(&c.tmem_empty[lane], 4);
-            mbar_init(&c.xfull[lane], kBExpWarps); mbar_init(&c.xempty[lane], 1);
-        }
-        c.task[lane] = 0u; c.task[lane + 32] = 0u;
-        mbar_fence_init();
-    }
-    if (warp == 1) { tmem_alloc(&c.tmem_base, 512); tmem_relinquish(); tc_fence_before(); }
-    if (warp < kBRankWarps) reinterpret_cast<uint32_t*>(c.wcnt[warp])[lane] = 0u;
     __syncthreads();
     tc_fence_after();
     const uint32_t epoch = c.epoch;

@@ -1747,7 +1747,6 @@ __device__ __noinline__ void scout_watch_peers(const Ctx& cx, ScoutState& st, bo
 template <int kVec, bool kUmma, bool kFe, bool kA8, bool kTiles>
 __global__ void __launch_bounds__(kA8 ? kThreads + kNumExpThreads : kThreads, 1) mega_moe_kernel(const __grid_constant__ KParams p) {
     constexpr uint32_t kNT = kA8 ? kThreads + kNumExpThreads : kThreads;       // threads of this instantiation
-    const unsigned long long t_first = globaltimer_ns();
     extern __shared__ uint8_t smem_raw[];
     __shared__ Ctl c;
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~static_cast<uintptr_t>(1023u));
@@ -1766,17 +1765,8 @@ __global__ void __launch_bounds__(kA8 ? kThreads + kNumExpThreads : kThreads, 1)
     const bool is_scout = kScout && warp == kCopyWarps;
     ScoutRegs sreg;
     ScoutState sst{0ull, 0u};
-    if constexpr (kScout) {
-        if (is_scout) {
-            if (own_ok) scout_load_own(p, inp, lane, sreg);
-            if (lane == 0) reinterpret_cast<unsigned long long*>(buf + p.off_ctrl + kCtrlSmWFirst)[bid] = ~0ull;
-        }
-    }
+    // what needs nothing of the launches before this one comes first: it overlaps the end of the previous kernel in the stream
     if (tid == 0) {
-        const uint32_t ep = ctrl32[kCtrlEpoch / 4 + bid];
-        ctrl32[kCtrlEpoch / 4 + bid] = ep + 1u;
-        c.epoch = ep; c.abort_flag = 0u; c.ntasks = 0u; c.dcount = 0u; c.comb_next = 0u; c.issued = 0u; c.decode = 0u; c.bulk = 0u; c.rel_head = 0u; c.rel_tail = 0u; c.rissued = 0u;
-        if constexpr (!kScout) c.own_cnt = 0u;
         for (int s = 0; s < (p.nstage > static_cast<int>(p.nstage_wide) ? p.nstage : static_cast<int>(p.nstage_wide)); ++s) { mbar_init(&c.full[s], 1); mbar_init(&c.empty[s], kA8 ? kNumExpThreads / 64 : (kUmma ? 1 : kNumEpiThreads)); }
         #pragma unroll 1
         for (int i = 0; i < 2; ++i) {
@@ -1786,8 +1776,6 @@ __global__ void __launch_bounds__(kA8 ? kThreads + kNumExpThreads : kThreads, 1)
         }
         mbar_init(&c.tile_full, kFillWarps);
         mbar_fence_init();
-        reinterpret_cast<unsigned long long*>(buf + p.off_ctrl + kCtrlSmEntry)[bid] = t_first;
-        if constexpr (!kScout) reinterpret_cast<unsigned long long*>(buf + p.off_ctrl + kCtrlSmWFirst)[bid] = ~0ull;
     }
     if (kTiles && tid == 64) {
         // (the barriers only the tile-image roles use, set up by another thread than the one that does the rest)
@@ -1805,6 +1793,23 @@ __global__ void __launch_bounds__(kA8 ? kThreads + kNumExpThreads : kThreads, 1)
             *reinterpret_cast<uint4*>(smem + p.sm_act + off) = make_uint4(0, 0, 0, 0);
     }
     if (warp == 1) { tmem_alloc(&c.tmem_base, kTmemCols); tmem_relinquish(); tc_fence_before(); }
+    grid_dependency_wait();
+    grid_launch_dependents();
+    const unsigned long long t_first = globaltimer_ns();
+    if constexpr (kScout) {
+        if (is_scout) {
+            if (own_ok) scout_load_own(p, inp, lane, sreg);
+            if (lane == 0) reinterpret_cast<unsigned long long*>(buf + p.off_ctrl + kCtrlSmWFirst)[bid] = ~0ull;
+        }
+    }
+    if (tid == 0) {
+        const uint32_t ep = ctrl32[kCtrlEpoch / 4 + bid];
+        ctrl32[kCtrlEpoch / 4 + bid] = ep + 1u;
+        c.epoch = ep; c.abort_flag = 0u; c.ntasks = 0u; c.dcount = 0u; c.comb_next = 0u; c.issued = 0u; c.decode = 0u; c.bulk = 0u; c.rel_head = 0u; c.rel_tail = 0u; c.rissued = 0u;
+        if constexpr (!kScout) c.own_cnt = 0u;
+        reinterpret_cast<unsigned long long*>(buf + p.off_ctrl + kCtrlSmEntry)[bid] = t_first;
+        if constexpr (!kScout) reinterpret_cast<unsigned long long*>(buf + p.off_ctrl + kCtrlSmWFirst)[bid] = ~0ull;
+    }
     if (tid < kMaxLocalExperts) c.exp_count[tid] = 0u;
     // Larger batches (the build with tile images): the rows of this rank's own tokens still get their header line and
     // records in the receive pool, but their payload does not travel: whoever needs such a row reads the token where the

@@ -24,6 +24,13 @@ __device__ __forceinline__ bool elect_one() {
     return pred != 0;
 }
 
+// ----------------------------------------------------------------------------- programmatic dependent launch
+// waits until the grids this launch depends on have ended and their memory operations are visible (nothing to wait for
+// when the launch did not ask for an early start)
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// this grid no longer holds back the start of the next one in its stream (which waits for this grid's end by itself)
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ----------------------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
