@@ -75,8 +75,9 @@ _libs = {}
 def load(check: bool = False) -> ctypes.CDLL:
     """Load the compiled library; raises if it has not been built (`python -m <package>.build`). `check=True` loads the
     test build that also carries the CUDA-core cross-check engine."""
-    if check in _libs:
-        return _libs[check]
+    lib = _libs.get(check)
+    if lib is not None:
+        return lib
     path = CHECK_LIB_PATH if check else LIB_PATH
     if not os.path.exists(path):
         raise RuntimeError(f'{path} is missing: build it with `python -m hopper_megamoe_basedondeepgemm_b200.build` '

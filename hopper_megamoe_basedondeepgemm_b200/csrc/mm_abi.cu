@@ -10,6 +10,7 @@
 #include "mm_frontend.cuh"
 #include "mm_prep.cuh"
 #include "mm_batch.cuh"
+#include "mm_decode.cuh"
 
 namespace {
 
@@ -29,7 +30,7 @@ int sf_vec_of(int fmt) { return fmt == MM_FMT_NVFP4 ? 16 : 32; }
 // many experts' W1 / W2 the scout may prefetch into the L2 in one launch
 // (the L2 prefetch of live experts' weights is off by default: measured, it does not shorten the weight stream - bulk
 // copies from the L2 are barely faster than from HBM here - and its traffic delays the launch's small critical loads)
-int g_tuning[MM_TUNE_COUNT] = {mm::kKnobOwnRows | mm::kKnobEarlyCombine | mm::kKnobTileImages, 0, 14, 14, 1};
+int g_tuning[MM_TUNE_COUNT] = {mm::kKnobOwnRows | mm::kKnobEarlyCombine | mm::kKnobTileImages | mm::kKnobDecode, 0, 14, 14, 1};
 
 int check_config(const mm_config_t* c) {
     if (c == nullptr) return MM_ERR_INVALID_ARGUMENT;
@@ -143,10 +144,16 @@ int mm_get_layout(const mm_config_t* c, mm_layout_t* out) {
     }
     out->off_token_tiles = take(out->tile_capacity * out->token_tile_bytes);
     out->off_mid_tiles = take(out->tile_capacity * out->mid_tile_bytes);
-    out->off_arrive = take(2 * 2 * out->tile_capacity * 4 + 2 * mm::kBCounts * 4);   // (then the one-rank batch kernel's counts)
+    out->off_arrive = take(2 * 2 * out->tile_capacity * 4 + 2 * mm::kBCounts * 4 + mm::kFeMaxFusedTokens * 8 * 16);   // (then the one-rank batch kernel's counts and routing records)
+    take(c->num_ranks == 1 ? t_max * c->num_topk * c->hidden * 2 : 0);   // the same kernel's expert outputs (`batch_out_offset`)
     out->total_bytes = off;
     return MM_OK;
 }
+
+// Regions of the one-rank kernels behind the arrival counters, and the expert outputs at the end of the buffer. (The outputs
+// are plain bf16: they must not share memory with the flagged words of the combine buffer, which they could imitate.)
+static int64_t batch_routes_offset(const mm_layout_t& L) { return L.off_arrive + 2 * 2 * L.tile_capacity * 4 + 2 * mm::kBCounts * 4; }
+static int64_t batch_out_offset(const mm_layout_t& L) { return align_up(batch_routes_offset(L) + mm::kFeMaxFusedTokens * 8 * 16, 1024); }
 
 // ----------------------------------------------------------------------------- symmetric window without torch
 int mm_window_alloc(int64_t bytes, void** ptr_out, uint8_t handle_out[MM_WINDOW_HANDLE_BYTES]) {
@@ -377,6 +384,14 @@ static bool wants_tile_images(const mm::KParams& p) {
     return (p.knobs & mm::kKnobTileImages) != 0u && p.nstage_wide >= 3u && p.nrec >= 2u && static_cast<long long>(p.T) * p.topk > mm::kTileTokens;
 }
 
+// logits + quantisation, then the selection with as many experts per lane as the expert count needs
+static int launch_frontend(const mm::FeParams& q, int grid, cudaStream_t s) {
+    const int st = launch_early<mm::FeParams>(mm::frontend_logits_kernel, grid, mm::kFeThreads, 0, s, q);
+    if (st != MM_OK) return st;
+    auto select = q.E <= 64 ? mm::frontend_select_kernel<2> : (q.E <= 256 ? mm::frontend_select_kernel<8> : (q.E <= 384 ? mm::frontend_select_kernel<12> : mm::frontend_select_kernel<32>));
+    return launch_early<mm::FeParams>(select, q.T, 32, 0, s, q);
+}
+
 template <int kVec, bool kUmma, bool kFe = false, bool kA8 = false, bool kTiles = false>
 static int launch_variant(const mm::KParams& p, int grid, size_t smem_bytes, cudaStream_t stream) {
     auto kern = mm::mega_moe_kernel<kVec, kUmma, kFe, kA8, kTiles>;
@@ -392,10 +407,9 @@ static int launch_variant(const mm::KParams& p, int grid, size_t smem_bytes, cud
 }
 
 // ----------------------------------------------------------------------------- one rank, more than a handful of rows
-// The batch kernel (mm_batch.cuh) takes over from the multi-rank kernel on one rank as soon as the launch can route more
-// rows than decode mode holds in one token tile (16); up to there the other kernel's split weight tiles win (16 entries on
-// 15 experts, E4M3 tokens: 43 us there, 45 here). It reads the inputs from the buffer's views on every SM, so inputs in
-// mapped host memory stay with the other kernel, as do launches beyond its tables (4096 routing entries, 128 token tiles).
+// The batch kernel (mm_batch.cuh) takes the launches on one rank that route more entries than the decode kernel's token tile
+// has rows (16). It reads the inputs from the buffer's views on every SM, so inputs in mapped host memory stay with the
+// multi-rank kernel, as do launches beyond its tables (4096 routing entries, 128 token tiles).
 static bool wants_batch_kernel(const mm_launch_args_t* a, const mm::KParams& p) {
     if (p.R != 1 || a->input_region != nullptr || a->engine != MM_ENGINE_UMMA || p.T == 0) return false;
     if ((p.knobs & mm::kKnobTileImages) == 0u) return false;
@@ -405,33 +419,66 @@ static bool wants_batch_kernel(const mm_launch_args_t* a, const mm::KParams& p) 
     return tiles <= mm::kBMaxTiles;
 }
 
-template <int kFmt>
-static int launch_batch(const mm::KParams& k, int grid, cudaStream_t stream) {
-    auto kern = mm::batch_moe_kernel<kFmt>;
+// The decode kernel (mm_decode.cuh) takes the launches up to there. The token tile and, with E4M3 tokens, the widened units
+// have to leave it a ring of three weight stages; wider layers stay with the multi-rank kernel, as inputs in host memory do.
+static bool wants_decode_kernel(const mm_config_t* cfg, const mm_launch_args_t* a, const mm::KParams& p) {
+    if (p.R != 1 || a->input_region != nullptr || a->engine != MM_ENGINE_UMMA || p.T == 0) return false;
+    if ((p.knobs & mm::kKnobDecode) == 0u || static_cast<long long>(p.T) * p.topk > mm::kDEntries) return false;
+    const bool a8 = cfg->act_format == MM_FMT_FP8;
+    const int planes = mm::kUnitK / (4 * sf_vec_of(cfg->act_format));
+    const long long tiles = static_cast<long long>(p.k1_units > p.k2_units ? p.k1_units : p.k2_units) * (2048 * (a8 ? 2 : 1) + planes * 512);
+    return tiles + (a8 ? 2 * mm::kXbufBytes : 0) + 3ll * p.unit_bytes <= 232448 - static_cast<long long>(sizeof(mm::DShared)) - 256 - 1024;
+}
+
+static mm::BParams one_rank_params(const mm_config_t* cfg, const mm::KParams& k) {
+    mm_layout_t L;
+    mm_get_layout(cfg, &L);
     mm::BParams p;
     memset(&p, 0, sizeof(p));
     p.T = k.T; p.topk = k.topk; p.E = k.e_local; p.H = k.H; p.I = k.I;
     p.n1 = k.n1_tiles; p.n2 = k.n2_tiles; p.k1 = k.k1_units; p.k2 = k.k2_units;
     p.unit_bytes = k.unit_bytes;
-    p.tile_limit = kFmt == 2 ? 96u : 128u;         // (E4M3: a wider record would leave too few weight stages beside the widened units)
-    p.x_row_bytes = k.x_row_bytes; p.x_sf_row_bytes = k.x_sf_row_bytes; p.rx_row_bytes = k.rx_row_bytes;
+    p.tile_limit = cfg->act_format == MM_FMT_FP8 ? 96u : 128u;         // (E4M3: a wider record would leave too few weight stages beside the widened units)
+    p.x_row_bytes = k.x_row_bytes; p.x_sf_row_bytes = k.x_sf_row_bytes; p.rx_row_bytes = k.rx_row_bytes; p.mid_row_bytes = k.mid_row_bytes;
     p.has_clamp = k.has_clamp; p.fast_math = k.fast_math; p.clamp = k.clamp;
     p.l1_scale = k.l1_scale; p.l2_scale = k.l2_scale; p.mid_gs = k.mid_gs; p.mid_gs_recip = 1.0f / k.mid_gs;
     p.buf = k.peer[k.rank]; p.w1 = k.w1; p.w2 = k.w2; p.y = k.y; p.stats = k.stats;
     p.off_ctrl = k.off_ctrl; p.off_x = k.off_x; p.off_x_sf = k.off_x_sf; p.off_topk_idx = k.off_topk_idx; p.off_topk_w = k.off_topk_w;
     p.off_rx = k.off_rx; p.off_comb = k.off_comb; p.off_token_tiles = k.off_token_tiles; p.off_mid_tiles = k.off_mid_tiles; p.off_arrive = k.off_arrive;
+    p.off_mid = k.off_mid; p.off_mid_sf = k.off_mid_sf; p.off_red = k.off_red;
+    p.off_routes = batch_routes_offset(L); p.off_out = batch_out_offset(L);
     p.rx_region = k.rx_region; p.tile_capacity = k.tile_capacity;
+    p.fe = k.fe;
     p.timeout_ns = k.timeout_ns;
-    const int dyn = 232448 - static_cast<int>((sizeof(mm::BShared) + 255) / 256 * 256);
+    return p;
+}
+
+// shared memory: all an SM has, less the kernel's static part
+template <typename Shared>
+static int launch_one_rank(void (*kern)(mm::BParams), int threads, mm::BParams& p, int grid, bool (&attr_set)[64], cudaStream_t stream) {
+    const int dyn = 232448 - static_cast<int>((sizeof(Shared) + 255) / 256 * 256);
     p.smem_ring = static_cast<uint32_t>(dyn - 1024);
-    static bool attr_set[64] = {};
     int dev = 0;
     MM_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
         MM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
-    return launch_early<mm::BParams>(kern, grid, mm::BFmt<kFmt>::kThreadsAll, dyn, stream, p);
+    return launch_early<mm::BParams>(kern, grid, threads, dyn, stream, p);
+}
+
+template <int kFmt, bool kFe>
+static int launch_one_rank_fmt(mm::BParams& p, bool decode, int grid, cudaStream_t stream) {
+    static bool batch_attr[64] = {}, decode_attr[64] = {};
+    return decode ? launch_one_rank<mm::DShared>(mm::decode_moe_kernel<kFmt, kFe>, mm::DFmt<kFmt>::kThreads, p, grid, decode_attr, stream)
+                  : launch_one_rank<mm::BShared>(mm::batch_moe_kernel<kFmt, kFe>, mm::BFmt<kFmt>::kThreadsAll, p, grid, batch_attr, stream);
+}
+
+template <bool kFe>
+static int launch_one_rank_kernel(const mm_config_t* cfg, const mm::KParams& k, bool decode, int grid, cudaStream_t s) {
+    mm::BParams p = one_rank_params(cfg, k);
+    return cfg->act_format == MM_FMT_FP8 ? launch_one_rank_fmt<2, kFe>(p, decode, grid, s)
+         : cfg->act_format == MM_FMT_NVFP4 ? launch_one_rank_fmt<1, kFe>(p, decode, grid, s) : launch_one_rank_fmt<0, kFe>(p, decode, grid, s);
 }
 
 extern "C" {
@@ -444,10 +491,8 @@ int mm_mega_moe_launch(const mm_config_t* cfg, const mm_launch_args_t* a, void* 
     if (st != MM_OK) return st;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const bool umma = a->engine == MM_ENGINE_UMMA;
-    if (wants_batch_kernel(a, p)) {
-        return cfg->act_format == MM_FMT_FP8 ? launch_batch<2>(p, grid, s)
-             : cfg->act_format == MM_FMT_NVFP4 ? launch_batch<1>(p, grid, s) : launch_batch<0>(p, grid, s);
-    }
+    const bool decode = wants_decode_kernel(cfg, a, p);
+    if (decode || wants_batch_kernel(a, p)) return launch_one_rank_kernel<false>(cfg, p, decode, grid, s);
     if (!dispatch_list_fits(p)) return MM_ERR_UNSUPPORTED;
     if (cfg->act_format == MM_FMT_FP8)                                     // tensor-core engine only
         return umma ? launch_variant<32, true, false, true>(p, grid, smem_bytes, s) : MM_ERR_UNSUPPORTED;
@@ -511,12 +556,7 @@ int mm_frontend_launch(const mm_config_t* cfg, void* buffer, const mm_frontend_a
     q.topk_w = reinterpret_cast<float*>(b + L.off_topk_weights);
     q.x_row_bytes = static_cast<int>(L.x_row_bytes); q.x_sf_row_bytes = static_cast<int>(L.x_sf_row_bytes);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    mm::frontend_logits_kernel<<<grid, 256, 0, s>>>(q);
-    MM_CUDA(cudaGetLastError());
-    const int sel_blocks = (q.T + 3) / 4;
-    mm::frontend_select_quant_kernel<<<sel_blocks, 128, q.E * 2 * 4 * 4, s>>>(q);
-    MM_CUDA(cudaGetLastError());
-    return MM_OK;
+    return launch_frontend(q, grid, s);
 }
 
 int mm_transform_weights(const void* w_packed, const void* sf, int32_t sf_is_fp32, int64_t sf_stride_e, int64_t sf_stride_n,
@@ -612,11 +652,7 @@ int mm_fe_forward(const void* hidden, const void* router_weight, void* x, void* 
     q.x_row_bytes = fmt == MM_FMT_FP8 ? h : h / 2;
     q.x_sf_row_bytes = h / sf_vec_of(fmt);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    mm::frontend_logits_kernel<<<grid, 256, 0, s>>>(q);
-    MM_CUDA(cudaGetLastError());
-    mm::frontend_select_quant_kernel<<<(m + 3) / 4, 128, q.E * 2 * 4 * 4, s>>>(q);
-    MM_CUDA(cudaGetLastError());
-    return MM_OK;
+    return launch_frontend(q, grid, s);
 }
 
 int mm_mega_moe_from_hidden_launch(const mm_config_t* cfg, const mm_launch_args_t* a, const mm_frontend_args_t* fe, void* stream) {
@@ -625,14 +661,15 @@ int mm_mega_moe_from_hidden_launch(const mm_config_t* cfg, const mm_launch_args_
     size_t smem_bytes = 0;
     int st = fill_params(cfg, a, &p, &grid, &smem_bytes);
     if (st != MM_OK) return st;
-    if (!dispatch_list_fits(p)) return MM_ERR_UNSUPPORTED;
     if (fe == nullptr || (fe->hidden_states == nullptr && fe->num_tokens > 0) || fe->router_weight == nullptr || fe->workspace == nullptr) return MM_ERR_INVALID_ARGUMENT;
     if (fe->num_tokens != a->num_tokens) return MM_ERR_INVALID_ARGUMENT;
     if (cfg->num_topk != 8 || cfg->num_experts > 1024) return MM_ERR_UNSUPPORTED;
     if (cfg->num_experts < cfg->num_topk) return MM_ERR_INVALID_ARGUMENT;      // fewer experts than routes per token
     if (fe->score_mode == 1 && fe->expert_bias == nullptr) return MM_ERR_INVALID_ARGUMENT;
     const bool a8 = cfg->act_format == MM_FMT_FP8;
-    if (static_cast<size_t>(cfg->num_experts) * 2 * 4 * ((mm::kThreads + (a8 ? mm::kNumExpThreads : 0)) / 32) > p.stage_region) return MM_ERR_UNSUPPORTED;
+    const bool decode = wants_decode_kernel(cfg, a, p), one_rank = decode || wants_batch_kernel(a, p);
+    if (!one_rank && (!dispatch_list_fits(p) ||
+        static_cast<size_t>(cfg->num_experts) * 2 * 4 * ((mm::kThreads + (a8 ? mm::kNumExpThreads : 0)) / 32) > p.stage_region)) return MM_ERR_UNSUPPORTED;
     if (fe->num_tokens > mm::kFeMaxFusedTokens) return MM_ERR_UNSUPPORTED;
     mm_layout_t L;
     mm_get_layout(cfg, &L);
@@ -654,6 +691,7 @@ int mm_mega_moe_from_hidden_launch(const mm_config_t* cfg, const mm_launch_args_
     // (the dispatching SMs also select the routes, each of them for all tokens: `fill_params` chose one SM per eight rows)
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (a->engine != MM_ENGINE_UMMA) return MM_ERR_UNSUPPORTED;     // the cross-check engine takes pre-routed inputs only
+    if (one_rank) return launch_one_rank_kernel<true>(cfg, p, decode, grid, s);
     if (a8) return fe->num_tokens == 0 ? launch_variant<32, true, false, true>(p, grid, smem_bytes, s)
                                        : launch_variant<32, true, true, true>(p, grid, smem_bytes, s);
     if (fe->num_tokens == 0) return cfg->act_format == MM_FMT_MXFP4 ? launch_variant<32, true>(p, grid, smem_bytes, s)

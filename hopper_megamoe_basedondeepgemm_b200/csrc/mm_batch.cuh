@@ -53,6 +53,10 @@ struct BParams {
     long long off_ctrl, off_x, off_x_sf, off_topk_idx, off_topk_w, off_rx, off_comb, off_token_tiles, off_mid_tiles, off_arrive;
     long long rx_region;
     uint32_t tile_capacity;
+    long long off_routes, off_out;                 // [tokens][8] flagged routing records (launches from hidden states); [entries][H] bf16 expert outputs
+    long long off_mid, off_mid_sf, off_red;        // flagged words of the decode kernel: intermediate rows, their scale bytes, partial sums
+    uint32_t mid_row_bytes;
+    FeParams fe;
     uint32_t smem_ring;                            // bytes of dynamic shared memory for the two rings (and the widened units)
     unsigned long long timeout_ns;
 };
@@ -60,7 +64,7 @@ struct BParams {
 struct BShared {
     uint64_t wfull[kBWStages], wempty[kBWStages], rfull[kBRSlots], rempty[kBRSlots];
     uint64_t tmem_full[2], tmem_empty[2], xfull[2], xempty[2];
-    uint32_t tmem_base, epoch, abort_flag, M, wissued, rissued, comb_next, nw, nr, slot_bytes, spu, total, start_ok;
+    uint32_t tmem_base, abort_flag, M, wissued, rissued, comb_next, nw, nr, slot_bytes, spu, total, start_ok;
     uint32_t seg_shift;                            // routing entries per ranking warp: 1 << seg_shift
     uint32_t cnt[kMaxLocalExperts], ebase[kMaxLocalExperts];
     uint32_t tile_e[kBMaxTiles];                   // expert
@@ -75,6 +79,7 @@ struct BShared {
         uint16_t rank[kBMaxRows];                  // rank of the entry among those of its expert in its ranking warp (until the rows are placed)
         float vt[2][kTileTokens * kBVtStride];     // 16 tokens' accumulators of a task, per epilogue group (see b_role_epilogue)
     };
+    uint8_t nonzero[kFeMaxFusedTokens];            // launches from hidden states: is this SM's k-th token all zeros (1) or not (2)
     uint16_t ef[2][128];                           // per epilogue group: routing entry and top-k weight of the task's rows
     float ew[2][128];
     uint16_t rowf[kBMaxRows];                      // routing entry (token * topk + slot) of every row, experts one after the other
@@ -87,17 +92,26 @@ __device__ __forceinline__ void st_global_v8(void* p, const uint32_t (&v)[8]) {
                  ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
 }
 
-struct BCtx {
-    const BParams& p; BShared& c;
+// What the one-rank kernels share: abort flag, deadline, bounded waits, time records.
+struct BCore {
+    const BParams& p;
+    uint32_t* abort_flag;
     uint8_t* smem;
     uint64_t deadline;
     uint32_t par;
-    __device__ __forceinline__ bool aborted() const { return *reinterpret_cast<volatile uint32_t*>(&c.abort_flag) != 0u; }
+    __device__ __forceinline__ bool aborted() const { return *reinterpret_cast<volatile uint32_t*>(abort_flag) != 0u; }
     __device__ __noinline__ void fail(uint32_t code, uint32_t detail = 0) const {
         atomicCAS(reinterpret_cast<uint32_t*>(p.buf + p.off_ctrl + kCtrlStatus), 0u, code | (blockIdx.x << 8) | (detail << 16));
-        *reinterpret_cast<volatile uint32_t*>(&c.abort_flag) = 1u;
+        *reinterpret_cast<volatile uint32_t*>(abort_flag) = 1u;
     }
     __device__ __forceinline__ bool expired() const { return globaltimer_ns() > deadline; }
+    // for polling loops: give up when the launch is aborted or its time has run out (looked at every 64th time)
+    __device__ __forceinline__ bool give_up(uint32_t& spins, uint32_t code, uint32_t detail) const {
+        if ((++spins & 0x3Fu) != 0u) return false;
+        if (aborted()) return true;
+        if (expired()) { fail(code, detail); return true; }
+        return false;
+    }
     __device__ __noinline__ bool wait_slow(uint64_t* bar, uint32_t parity, uint32_t code) const {
         uint32_t it = 0;
         while (!mbar_try_wait(bar, parity)) {
@@ -138,6 +152,11 @@ struct BCtx {
     __device__ __forceinline__ uint32_t* col_counts(uint32_t parity) const {
         return reinterpret_cast<uint32_t*>(p.buf + p.off_arrive) + 4u * p.tile_capacity + parity * kBCounts;
     }
+};
+struct BCtx : BCore {
+    BShared& c;
+    __device__ __forceinline__ BCtx(const BParams& p_, BShared& c_, uint8_t* smem_, uint64_t deadline_, uint32_t par_)
+        : BCore{p_, &c_.abort_flag, smem_, deadline_, par_}, c(c_) {}
 };
 
 template <int kFmt> struct BFmt {
@@ -384,12 +403,37 @@ __device__ void b_role_mma(const BCtx& cx, uint32_t lane) {
 // multiply, barriers - took twice as long and was the bound.) Eight lanes read the eight chunks of a row and store the two
 // halves of each; the lanes of the second atom store theirs in the other order, so that the eight stores of a quarter-warp
 // fall on different banks.
+struct BWiden {
+    static constexpr uint32_t kItems = kTileRows * 8 / (kBExpWarps * 32);
+    uint4 v[kItems], sf;
+    __device__ __forceinline__ void load(const uint8_t* wsm, uint32_t xtid) {
+        const uint32_t ch = xtid & 7u;
+        #pragma unroll
+        for (uint32_t k = 0; k < kItems; ++k) {
+            const uint32_t r = k * (kBExpWarps * 4) + (xtid >> 3);
+            v[k] = *reinterpret_cast<const uint4*>(wsm + r * 128u + ((ch ^ (r & 7u)) << 4));
+        }
+        if (xtid < 64u) sf = *reinterpret_cast<const uint4*>(wsm + kUnitWBytes + xtid * 16u);
+    }
+    __device__ __forceinline__ void store(uint8_t* xb, uint32_t xtid) const {
+        const uint32_t ch = xtid & 7u, at = ch >> 2, j = 2u * (ch & 3u);
+        #pragma unroll
+        for (uint32_t k = 0; k < kItems; ++k) {
+            const uint32_t r = k * (kBExpWarps * 4) + (xtid >> 3);
+            uint8_t* row = xb + at * kUnitWBytes + r * 128u;
+            const uint32_t first = (j + at) ^ (r & 7u), second = (j + 1u - at) ^ (r & 7u);
+            *reinterpret_cast<uint4*>(row + (first << 4)) = at ? make_uint4(v[k].z, v[k].w, 0u, 0u) : make_uint4(v[k].x, v[k].y, 0u, 0u);
+            *reinterpret_cast<uint4*>(row + (second << 4)) = at ? make_uint4(v[k].x, v[k].y, 0u, 0u) : make_uint4(v[k].z, v[k].w, 0u, 0u);
+        }
+        if (xtid < 64u) *reinterpret_cast<uint4*>(xb + 2 * kUnitWBytes + xtid * 16u) = sf;
+    }
+};
+
 __device__ void b_role_widen(const BCtx& cx, uint32_t xtid) {
     const BParams& p = cx.p; BShared& c = cx.c;
-    const uint32_t lane = xtid & 31u, nw = c.nw, ch = xtid & 7u, at = ch >> 2;
+    const uint32_t lane = xtid & 31u, nw = c.nw;
     uint8_t* ring = cx.smem + c.nr * c.slot_bytes;
     uint8_t* x0 = ring + static_cast<size_t>(nw) * p.unit_bytes;
-    constexpr uint32_t kItems = kTileRows * 8 / (kBExpWarps * 32);
     uint32_t it = 0, s = 0, ph = 0;
     BTasks tasks(cx);
     #pragma unroll 1
@@ -400,28 +444,12 @@ __device__ void b_role_widen(const BCtx& cx, uint32_t xtid) {
         #pragma unroll 1
         for (uint32_t u = 0; u < units; ++u, ++it) {
             if (!cx.warp_wait(&c.wfull[s], ph, kErrWaitFull)) return;
-            const uint8_t* wsm = ring + static_cast<size_t>(s) * p.unit_bytes;
-            uint8_t* xb = x0 + (it & 1u) * kXbufBytes;
-            uint4 v[kItems];
-            uint4 sf = make_uint4(0u, 0u, 0u, 0u);
-            #pragma unroll
-            for (uint32_t k = 0; k < kItems; ++k) {
-                const uint32_t r = k * (kBExpWarps * 4) + (xtid >> 3);
-                v[k] = *reinterpret_cast<const uint4*>(wsm + r * 128u + ((ch ^ (r & 7u)) << 4));
-            }
-            if (xtid < 64u) sf = *reinterpret_cast<const uint4*>(wsm + kUnitWBytes + xtid * 16u);
+            BWiden w;
+            w.load(ring + static_cast<size_t>(s) * p.unit_bytes, xtid);
             __syncwarp();
             if (lane == 0) mbar_arrive(&c.wempty[s]);        // (the unit is in registers: its stage can be refilled)
             if (!cx.warp_wait(&c.xempty[it & 1u], ((it >> 1) & 1u) ^ 1u, kErrWaitEmpty)) return;
-            #pragma unroll
-            for (uint32_t k = 0; k < kItems; ++k) {
-                const uint32_t r = k * (kBExpWarps * 4) + (xtid >> 3), j = 2u * (ch & 3u);
-                uint8_t* row = xb + at * kUnitWBytes + r * 128u;
-                const uint32_t first = (j + at) ^ (r & 7u), second = (j + 1u - at) ^ (r & 7u);
-                *reinterpret_cast<uint4*>(row + (first << 4)) = at ? make_uint4(v[k].z, v[k].w, 0u, 0u) : make_uint4(v[k].x, v[k].y, 0u, 0u);
-                *reinterpret_cast<uint4*>(row + (second << 4)) = at ? make_uint4(v[k].x, v[k].y, 0u, 0u) : make_uint4(v[k].z, v[k].w, 0u, 0u);
-            }
-            if (xtid < 64u) *reinterpret_cast<uint4*>(xb + 2 * kUnitWBytes + xtid * 16u) = sf;
+            w.store(x0 + (it & 1u) * kXbufBytes, xtid);
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(&c.xfull[it & 1u]);
@@ -465,18 +493,61 @@ __device__ __forceinline__ float div_by(float x, float b, float y) {
     return fmaf(fmaf(-q, b, x), y, q);
 }
 
+// Requantises the 8 outputs of thread (n, q): o becomes the scaled values, the thread q = 0 gets the scale bytes of the
+// token's 64 columns in sfw (two bytes, one per 32 columns, or four). All lanes of the warp call it.
+template <int kFmt>
+__device__ __forceinline__ void b_requantise(const BParams& p, float (&o)[8], uint32_t& sfw) {
+    constexpr bool kA8 = BFmt<kFmt>::kA8;
+    constexpr int kVec = BFmt<kFmt>::kVec;
+    float amax = 0.f;
+    #pragma unroll
+    for (uint32_t i = 0; i < 8; ++i) {
+        if constexpr (kVec == 16) o[i] = div_by(o[i], p.mid_gs, p.mid_gs_recip);
+        amax = fmaxf(amax, fabsf(o[i]));
+    }
+    // a scale block is the 8 columns of two (16 per block) or four threads
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    if constexpr (kVec == 32) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    amax = fmaxf(amax, 1e-30f);
+    uint32_t sf_byte;
+    if constexpr (kVec == 32) {
+        sf_byte = ceil_pow2_exp(__fdiv_rn(amax, kA8 ? 448.0f : 6.0f));
+        const float inv = pow2_recip(sf_byte);                    // a power of two: the product equals the quotient
+        #pragma unroll
+        for (uint32_t i = 0; i < 8; ++i) o[i] *= inv;
+    } else {
+        sf_byte = cvt_e4m3x2(__fdiv_rn(amax, 6.0f), 0.f) & 0xFFu;
+        const float sf = e4m3_to_float(sf_byte);
+        const bool zero = sf_byte == 0u;                          // a scale that rounds to zero: every non-zero value saturates
+        const float inv = zero ? 0.f : __frcp_rn(sf);
+        #pragma unroll
+        for (uint32_t i = 0; i < 8; ++i) {
+            const float qt = div_by(o[i], sf, inv), sat = o[i] == 0.f ? 0.f : copysignf(6.0f, o[i]);
+            o[i] = zero ? sat : qt;
+        }
+    }
+    // the token's scale bytes of this tile, gathered in the thread q = 0
+    sfw = sf_byte;
+    if constexpr (kVec == 32) sfw |= __shfl_down_sync(0xffffffffu, sf_byte, 4) << 8;
+    else {
+        sfw |= __shfl_down_sync(0xffffffffu, sf_byte, 2) << 8;
+        sfw |= __shfl_down_sync(0xffffffffu, sfw, 4) << 16;
+    }
+}
 // A task's accumulators lie with weight row l in lane l and token n in column n. 16 tokens at a time go through shared
 // memory: weight row 16 q + 4 i + k of token n to vt[n * 152 + i * 40 + q * 4 + k], which neither the writes (a warp: 32
 // rows of one token) nor the 16-byte reads (thread (n, q): its i = 0..3) find bank conflicts in. Thread (n = t / 8, q = t % 8)
 // then owns the 16 weight rows of group q of token n: L1 8 gate rows and the 8 matching up rows, L2 16 output columns.
-template <int kFmt>
+template <int kFmt, bool kFe>
 __device__ void b_role_epilogue(const BCtx& cx, uint32_t grp, uint32_t etid) {
     using F = BFmt<kFmt>;
     constexpr bool kA8 = F::kA8;
     constexpr int kVec = F::kVec;
     const BParams& p = cx.p; BShared& c = cx.c;
     const uint32_t ew = etid >> 5, q = etid & 7u, n16 = etid >> 3;
-    const float* tw = reinterpret_cast<const float*>(p.buf + p.off_topk_w);
+    // the rows' top-k weights: the caller's view, or the routing records this launch's own frontend wrote
+    const uint8_t* tw = kFe ? p.buf + p.off_routes + 8 : p.buf + p.off_topk_w;
+    constexpr uint32_t kTwStride = kFe ? 16u : 4u;
     const uint32_t bar = grp ? kBBarEpi1 : kBBarEpi0;
     float* vt = c.vt[grp];
     float* vt_w = vt + ((etid & 15u) >> 2) * 40u + (etid >> 4) * 4u + (etid & 3u);
@@ -493,7 +564,7 @@ __device__ void b_role_epilogue(const BCtx& cx, uint32_t grp, uint32_t etid) {
             if (etid < rows) {
                 const uint32_t f = c.rowf[c.tile_row0[m] + etid];
                 c.ef[grp][etid] = static_cast<uint16_t>(f);
-                if (layer == 0u) c.ew[grp][etid] = tw[f];
+                if (layer == 0u) c.ew[grp][etid] = __uint_as_float(ld_cg_u32(tw + static_cast<size_t>(f) * kTwStride));
             }
             ok = cx.warp_wait(&c.tmem_full[grp], use, kErrWaitTmemFull);
             tc_fence_after();
@@ -525,40 +596,8 @@ __device__ void b_role_epilogue(const BCtx& cx, uint32_t grp, uint32_t etid) {
             if (layer == 0u) {
                 float o[8];
                 b_swiglu(p, a, live ? c.ew[grp][n] : 0.f, o);
-                float amax = 0.f;
-                #pragma unroll
-                for (uint32_t i = 0; i < 8; ++i) {
-                    if constexpr (kVec == 16) o[i] = div_by(o[i], p.mid_gs, p.mid_gs_recip);
-                    amax = fmaxf(amax, fabsf(o[i]));
-                }
-                // a scale block is the 8 columns of two (16 per block) or four threads
-                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-                if constexpr (kVec == 32) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-                amax = fmaxf(amax, 1e-30f);
-                uint32_t sf_byte;
-                if constexpr (kVec == 32) {
-                    sf_byte = ceil_pow2_exp(__fdiv_rn(amax, kA8 ? 448.0f : 6.0f));
-                    const float inv = pow2_recip(sf_byte);                    // a power of two: the product equals the quotient
-                    #pragma unroll
-                    for (uint32_t i = 0; i < 8; ++i) o[i] *= inv;
-                } else {
-                    sf_byte = cvt_e4m3x2(__fdiv_rn(amax, 6.0f), 0.f) & 0xFFu;
-                    const float sf = e4m3_to_float(sf_byte);
-                    const bool zero = sf_byte == 0u;                          // a scale that rounds to zero: every non-zero value saturates
-                    const float inv = zero ? 0.f : __frcp_rn(sf);
-                    #pragma unroll
-                    for (uint32_t i = 0; i < 8; ++i) {
-                        const float qt = div_by(o[i], sf, inv), sat = o[i] == 0.f ? 0.f : copysignf(6.0f, o[i]);
-                        o[i] = zero ? sat : qt;
-                    }
-                }
-                // the token's scale bytes of this tile, gathered in the thread q = 0
-                uint32_t sfw = sf_byte;
-                if constexpr (kVec == 32) sfw |= __shfl_down_sync(0xffffffffu, sf_byte, 4) << 8;
-                else {
-                    sfw |= __shfl_down_sync(0xffffffffu, sf_byte, 2) << 8;
-                    sfw |= __shfl_down_sync(0xffffffffu, sfw, 4) << 16;
-                }
+                uint32_t sfw;
+                b_requantise<kFmt>(p, o, sfw);
                 if (live) {
                     if constexpr (kA8) {
                         uint8_t* at = img + ((j >> 1) & 1u) * a16 * 2048u + sw128_off(n, (j & 1u) * 4u + (q >> 1)) + (q & 1u) * 8u;
@@ -581,7 +620,7 @@ __device__ void b_role_epilogue(const BCtx& cx, uint32_t grp, uint32_t etid) {
                 for (uint32_t i = 0; i < 8; ++i)
                     w[i] = static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(a[2 * i] * p.l2_scale))) |
                            (static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(a[2 * i + 1] * p.l2_scale))) << 16);
-                if (live) st_global_v8(p.buf + p.off_comb + (static_cast<size_t>(c.ef[grp][n]) * p.H + j * 128u + q * 16u) * 2u, w);
+                if (live) st_global_v8(p.buf + p.off_out + (static_cast<size_t>(c.ef[grp][n]) * p.H + j * 128u + q * 16u) * 2u, w);
             }
         }
         // one thread counts the finished task; its release covers the stores of the group, which the barrier orders before it
@@ -626,7 +665,7 @@ __device__ void b_role_combine(const BCtx& cx, uint32_t lane) {
         if (!__all_sync(0xffffffffu, ok)) return;
         __syncwarp();
         __threadfence();                                     // (the polling lanes' acquire, handed to the others)
-        const uint8_t* src = p.buf + p.off_comb + (static_cast<size_t>(tok) * p.topk * p.H + col * 128u + l16 * 8u) * 2u;
+        const uint8_t* src = p.buf + p.off_out + (static_cast<size_t>(tok) * p.topk * p.H + col * 128u + l16 * 8u) * 2u;
         float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         #pragma unroll 1
         for (int s0 = 0; s0 < p.topk; s0 += 8) {
@@ -725,7 +764,7 @@ __device__ __forceinline__ void b_tiles(const BCtx& cx, uint32_t lane) {
 }
 
 // ============================================================================================= the kernel
-template <int kFmt>
+template <int kFmt, bool kFe>
 __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(const __grid_constant__ BParams p) {
     using F = BFmt<kFmt>;
     extern __shared__ uint8_t smem_raw[];
@@ -749,10 +788,11 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
     }
     if (warp == 1) { tmem_alloc(&c.tmem_base, 512); tmem_relinquish(); tc_fence_before(); }
     if (warp < kBRankWarps) reinterpret_cast<uint32_t*>(c.wcnt[warp])[lane] = 0u;
+    if (kFe && tid < kFeMaxFusedTokens) c.nonzero[tid] = 0;
     grid_dependency_wait();
     grid_launch_dependents();
     const unsigned long long t_first = globaltimer_ns();
-    // ---- this SM's tokens (token mod G): the first row of every worker warp is fetched before the routing is known
+    const uint32_t epoch = ld_volatile_u32(ctrl32 + kCtrlEpoch / 4 + bid);         // (tid 0 counts on after the barrier below)
     const uint32_t ntok = bid < static_cast<uint32_t>(p.T) ? udiv_small(p.T - 1u - bid, G) + 1u : 0u, nrows = ntok * p.topk;
     const uint32_t xq = p.x_row_bytes / 16u, per_row = xq + p.x_sf_row_bytes / 16u;
     constexpr uint32_t kChunks = F::kA8 ? 9u : 5u;               // 16 B chunks of a row per lane (hidden <= 4096)
@@ -769,12 +809,14 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
             if (ci < per_row) v[u] = ld_cg_v4(ci < xq ? xs + ci * 16u : sf + (ci - xq) * 16u);
         }
     };
-    if (worker) {
-        #pragma unroll
-        for (uint32_t a = 0; a < kAhead; ++a) load_row(v[a], ww + a * kBWorkWarps);
-    }
-    // ---- the routing entries' experts into shared memory
-    {
+    const BCtx cx(p, c, smem, globaltimer_ns() + p.timeout_ns, epoch & 1u);
+    if constexpr (!kFe) {
+        // ---- this SM's tokens (token mod G): the first rows of every worker warp are fetched before the routing is known
+        if (worker) {
+            #pragma unroll
+            for (uint32_t a = 0; a < kAhead; ++a) load_row(v[a], ww + a * kBWorkWarps);
+        }
+        // ---- the routing entries' experts into shared memory
         const long long* tk = reinterpret_cast<const long long*>(p.buf + p.off_topk_idx);
         #pragma unroll 4
         for (uint32_t f = tid; f < nent; f += F::kThreadsAll) {
@@ -783,9 +825,7 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
         }
     }
     if (tid == 0) {
-        const uint32_t ep = ctrl32[kCtrlEpoch / 4 + bid];
-        ctrl32[kCtrlEpoch / 4 + bid] = ep + 1u;
-        c.epoch = ep; c.abort_flag = 0u; c.comb_next = 0u; c.wissued = 0u; c.rissued = 0u;
+        c.abort_flag = 0u; c.comb_next = 0u; c.wissued = 0u; c.rissued = 0u;
         // a run of 32, 64, 128 or 256 routing entries per ranking warp
         const uint32_t per = (nent + kBRankWarps - 1u) / kBRankWarps;
         c.seg_shift = per <= 32u ? 5u : 32u - __clz(per - 1u);
@@ -795,9 +835,71 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
     }
     __syncthreads();
     tc_fence_after();
-    const uint32_t epoch = c.epoch;
-    BCtx cx{p, c, smem, globaltimer_ns() + p.timeout_ns, epoch & 1u};
+    if constexpr (kFe) {
+        // ---- router frontend. All warps of all SMs work out partial logits (flagged records); SM (token mod G) then selects
+        //      the token's experts as its records arrive and publishes the routing, while other warps quantise the token;
+        //      every SM polls all routing records. No barrier between SMs, two exchanges through memory.
+        const uint32_t flag = epoch + 1u, gw = warp * G + bid, nw = G * (F::kThreadsAll / 32);   // (consecutive items on different SMs)
+        auto give_up = [&]() -> bool {
+            if (cx.aborted()) return true;
+            if (cx.expired()) { cx.fail(kErrWaitFrontend); return true; }
+            return false;
+        };
+        // the upper warps, which have the fewest logits to work out, quantise this SM's tokens first
+        const uint32_t half_warps = kBRankWarps / 2;
+        if (warp >= half_warps && warp < kBRankWarps) {
+            #pragma unroll 1
+            for (uint32_t k = warp - half_warps; k < ntok; k += half_warps) {
+                const uint32_t tok = bid + k * G;
+                const bool nz = fe_quant_token(p.fe.hidden + static_cast<size_t>(tok) * p.H, p.H, kFmt, p.fe.x_gs, p.buf + p.off_x + static_cast<size_t>(tok) * p.x_row_bytes,
+                                               p.buf + p.off_x_sf + static_cast<size_t>(tok) * p.x_sf_row_bytes, lane);
+                if (lane == 0) *reinterpret_cast<volatile uint8_t*>(&c.nonzero[k]) = nz ? 2 : 1;
+            }
+        }
+        const uint32_t eb = fe_expert_block(p.fe, G);
+        if (eb == 1u) fe_logits_blocks<1, 3>(p.fe, gw, nw, lane, flag);
+        else if (F::kA8 || eb == 2u) fe_logits_blocks<2, 2>(p.fe, gw, nw, lane, flag);
+        else fe_logits_blocks<4, F::kA8 ? 1 : 2>(p.fe, gw, nw, lane, flag);
+        if (warp < half_warps) {
+            #pragma unroll 1
+            for (uint32_t k = warp; k < ntok; k += half_warps) {
+                uint32_t spins = 0;
+                uint8_t nz;
+                while ((nz = *reinterpret_cast<volatile uint8_t*>(&c.nonzero[k])) == 0 && !((++spins & 0x3Fu) == 0u && give_up())) { }
+                if (!fe_select_token_regs<2>(p.fe, bid + k * G, nz == 2, lane, flag, p.buf + p.off_routes, give_up)) break;
+            }
+        }
+        #pragma unroll 1
+        for (uint32_t f0 = tid; f0 < nent; f0 += 4u * F::kThreadsAll) {            // (four records per thread in flight)
+            uint4 r[4];
+            bool ok;
+            uint32_t spins = 0;
+            do {
+                ok = true;
+                #pragma unroll
+                for (uint32_t u = 0; u < 4; ++u) {
+                    const uint32_t f = f0 + u * F::kThreadsAll;
+                    if (f < nent) {
+                        r[u] = ld_volatile_v4(p.buf + p.off_routes + static_cast<size_t>(f) * 16u);
+                        ok = ok && r[u].y == flag && r[u].w == flag;
+                    }
+                }
+            } while (!ok && !((++spins & 0x3Fu) == 0u && give_up()));
+            #pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) {
+                const uint32_t f = f0 + u * F::kThreadsAll;
+                if (f < nent) c.ex[f] = static_cast<uint8_t>(ok && r[u].x < static_cast<uint32_t>(p.E) ? r[u].x : 0xFFu);
+            }
+        }
+        __syncthreads();
+        if (bid == 0 && tid == 0) cx.stamp(kStampFrontend);
+        if (worker) {
+            #pragma unroll
+            for (uint32_t a = 0; a < kAhead; ++a) load_row(v[a], ww + a * kBWorkWarps);
+        }
+    }
     if (tid == 0) {
+        ctrl32[kCtrlEpoch / 4 + bid] = epoch + 1u;
         cx.sm_phase(kSmPrologue);
         if (bid == 0) {
             ctrl32[kCtrlStatus / 4 + 1] = epoch + 1u;
@@ -938,7 +1040,8 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
                 li = __reduce_add_sync(0xffffffffu, li);
                 if (lane == 0)
                     st_ll_16B(p.buf + p.off_rx + static_cast<size_t>(cx.par) * p.rx_region + 32u + static_cast<size_t>(li) * 2u * p.rx_row_bytes + 2u * (p.rx_row_bytes - 16u),
-                              make_uint4(e, tok, slot, __float_as_uint(reinterpret_cast<const float*>(p.buf + p.off_topk_w)[f])), epoch + 1u);
+                              make_uint4(e, tok, slot, kFe ? ld_cg_u32(p.buf + p.off_routes + static_cast<size_t>(f) * 16u + 8u)
+                                                   : __float_as_uint(reinterpret_cast<const float*>(p.buf + p.off_topk_w)[f])), epoch + 1u);
             }
         }
     }
@@ -949,7 +1052,7 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
         else if (warp == 1) b_role_mma<kFmt>(cx, lane);
         else if (warp == 2) b_role_records<kFmt>(cx);
         else if (warp >= kBServiceWarps && warp < kBServiceWarps + kBEpiWarps)
-            b_role_epilogue<kFmt>(cx, (warp - kBServiceWarps) >> 2, tid - 32u * kBServiceWarps - ((warp - kBServiceWarps) >> 2) * 128u);
+            b_role_epilogue<kFmt, kFe>(cx, (warp - kBServiceWarps) >> 2, tid - 32u * kBServiceWarps - ((warp - kBServiceWarps) >> 2) * 128u);
         else if (warp >= kBServiceWarps + kBEpiWarps) {
             if constexpr (F::kA8) b_role_widen(cx, tid - 32u * (kBServiceWarps + kBEpiWarps));
         }

@@ -1,0 +1,689 @@
+// The layer on one rank with at most 16 routing entries (decode), as one persistent sm_100a kernel of its own.
+//
+// The launch is a chain of short steps around 50 MB of weights (8 us of HBM time for one token and eight experts), so what
+// counts is the number of steps and what one costs:
+//   * Every SM reads the routing entries and sorts them itself (one warp, registers), starts its weight stream right away,
+//     and builds ONE token tile of all 16 rows in shared memory (rows grouped by expert), which every task multiplies with:
+//     D[128 weight rows x 16 rows]; a task's epilogue looks at its expert's columns.
+//   * L1 weight tiles are dealt round-robin; the remainder tiles are cut along K between fixed groups of SMs, so that every SM
+//     streams the same number of units. The parts come first; the group's first SM adds the others' sums in SM order.
+//   * What one SM hands to another (parts, intermediate rows, expert outputs) are flagged 8-byte words {data, launch number}
+//     that the consumer polls: one trip through the L2, no fence, no counter. All SMs gather all intermediate rows (a few KB)
+//     into the L2 tasks' token tile while the L2 weights are already in the ring.
+//   * From hidden states: the router's partial logits are spread over the SMs as flagged records, then every SM selects and
+//     quantises the (one or two) tokens by itself: one exchange instead of two.
+// Bound: latency. Of the 8-expert launch's time about half is the weight stream.
+#pragma once
+#include "mm_batch.cuh"
+
+namespace mm {
+
+constexpr uint32_t kDEntries = 16;                 // routing entries (= rows) of a launch at most
+constexpr int kDEpiWarps = 8;                      // warps 4..11: build the token tiles, two epilogue groups
+constexpr int kDThreads = 32 * (4 + kDEpiWarps);
+constexpr int kDThreadsA8 = kDThreads + 32 * kBExpWarps;     // E4M3 tokens: widening warps 12..19
+constexpr int kDStages = 12;
+constexpr uint32_t kDBarGroups = 5, kDBarRouted = 6;
+
+struct DShared {
+    uint64_t wfull[kDStages], wempty[kDStages];
+    uint64_t tmem_full[2], tmem_empty[2], xfull[2], xempty[2], tile_full[2];
+    uint32_t tmem_base, abort_flag, comb_next, wissued, M, nlive, live_mask, start_ok;
+    uint32_t split_t, split_range, split_first, split_parts;      // this SM's part of a remainder tile: tile, first unit | end unit << 8, first SM of the group, parts (0: none)
+    uint32_t exp_e[kDEntries], exp_c0[kDEntries], exp_n[kDEntries];    // active experts, ascending: id, first column, rows
+    uint32_t ent_e[kDEntries]; float ent_w[kDEntries];               // per routing entry: expert (>= 64: none), weight
+    uint32_t ent_col[kDEntries];                                    // column of the entry's row in the token tile
+    uint32_t col_f[kDEntries], col_mid[kDEntries]; float col_w[kDEntries];   // per column: entry, row of the intermediate pool, weight
+    float vt[2][kTileTokens * kBVtStride];
+};
+
+struct DCtx : BCore {
+    DShared& c;
+    __device__ __forceinline__ DCtx(const BParams& p_, DShared& c_, uint8_t* smem_, uint64_t deadline_, uint32_t par_)
+        : BCore{p_, &c_.abort_flag, smem_, deadline_, par_}, c(c_) {}
+};
+
+template <int kFmt> struct DFmt : BFmt<kFmt> {
+    static constexpr int kThreads = BFmt<kFmt>::kA8 ? kDThreadsA8 : kDThreads;
+    static constexpr uint32_t kRec = 2048u * BFmt<kFmt>::kAtoms + BFmt<kFmt>::kPlanes * 512u;     // one K unit of the 16-row tile
+};
+
+// task `ti` of this SM: its part of a remainder L1 tile, its whole L1 tiles, its L2 tiles
+struct DTask { uint32_t layer, a, j, ub, ue, parts; bool valid; };
+struct DTasks {
+    const DCtx& cx;
+    uint32_t has_split, my1, r1;
+    __device__ __forceinline__ explicit DTasks(const DCtx& c_) : cx(c_) {
+        const uint32_t NT1 = c_.c.M * c_.p.n1, G = gridDim.x;
+        r1 = NT1 - udiv_small(NT1, G) * G;
+        has_split = c_.c.split_parts != 0u ? 1u : 0u;
+        my1 = r1 + blockIdx.x < NT1 ? udiv_small(NT1 - 1u - r1 - blockIdx.x, G) + 1u : 0u;
+    }
+    __device__ __forceinline__ DTask get(uint32_t ti) const {
+        DTask t;
+        const uint32_t G = gridDim.x;
+        t.layer = 0u; t.ub = 0u; t.ue = cx.p.k1; t.parts = 1u; t.valid = true;
+        uint32_t x;
+        if (ti < has_split) { x = cx.c.split_t; t.ub = cx.c.split_range & 0xFFu; t.ue = cx.c.split_range >> 8; t.parts = cx.c.split_parts; }
+        else if (ti < has_split + my1) x = r1 + blockIdx.x + (ti - has_split) * G;
+        else {
+            x = blockIdx.x + (ti - has_split - my1) * G;
+            t.layer = 1u; t.ue = cx.p.k2;
+            t.valid = x < cx.c.M * cx.p.n2;
+        }
+        const uint32_t n = t.layer ? cx.p.n2 : cx.p.n1;
+        t.a = t.valid ? udiv_small(x, n) : 0u;
+        t.j = x - t.a * n;
+        return t;
+    }
+};
+
+__device__ void d_role_weights(const DCtx& cx, uint32_t nw, uint8_t* ring) {
+    const BParams& p = cx.p; DShared& c = cx.c;
+    uint32_t it = 0, s = 0, ph = 0;
+    DTasks tasks(cx);
+    #pragma unroll 1
+    for (uint32_t ti = 0;; ++ti) {
+        const DTask t = tasks.get(ti);
+        if (!t.valid) break;
+        const uint8_t* src = (t.layer ? p.w2 : p.w1) +
+            ((static_cast<size_t>(c.exp_e[t.a]) * (t.layer ? p.n2 : p.n1) + t.j) * (t.layer ? p.k2 : p.k1) + t.ub) * p.unit_bytes;
+        #pragma unroll 1
+        for (uint32_t u = t.ub; u < t.ue; ++u, ++it, src += p.unit_bytes) {
+            if (!cx.warp_wait(&c.wempty[s], ph ^ 1u, kErrWaitEmpty)) return;
+            if (elect_one()) {
+                mbar_arrive_expect_tx(&c.wfull[s], p.unit_bytes);
+                bulk_g2s(ring + static_cast<size_t>(s) * p.unit_bytes, src, p.unit_bytes, &c.wfull[s]);
+                c.wissued = it + 1u;
+                if (it == 0u) {
+                    reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlSmWFirst)[blockIdx.x] = globaltimer_ns();
+                    cx.sm_phase(kSmFirstIssue);
+                }
+            }
+            __syncwarp();
+            if (++s == nw) { s = 0; ph ^= 1u; }
+        }
+    }
+}
+
+template <int kFmt>
+__device__ void d_role_mma(const DCtx& cx, uint32_t lane, uint32_t nw_, uint32_t ring_off) {
+    using F = DFmt<kFmt>;
+    constexpr bool kA8 = F::kA8;
+    constexpr uint32_t kPlanes = F::kPlanes, kStepK = kA8 ? 32u : 64u;
+    constexpr uint32_t kIdesc = kA8 ? idesc_block_scaled(kFmtF8E2M1, kFmtF8E4M3, 128u, kTileTokens, 1u)
+                                    : idesc_block_scaled(kFmtMxf4E2M1, kFmtMxf4E2M1, 128u, kTileTokens, kFmt == 1 ? 0u : 1u);
+    const BParams& p = cx.p; DShared& c = cx.c;
+    // (operands broadcast from lane 0: uniform registers, see the batch kernel's issuer)
+    const uint32_t nw = b_uniform(nw_), tm = b_uniform(c.tmem_base);
+    const uint32_t s0 = b_uniform(smem_u32(cx.smem)), ring0 = s0 + b_uniform(ring_off), x0 = ring0 + nw * p.unit_bytes;
+    uint32_t it = 0, s = 0, ph = 0, wsm0 = ring0;
+    bool have1 = false, have2 = false;
+    DTasks tasks(cx);
+    #pragma unroll 1
+    for (uint32_t ti = 0;; ++ti) {
+        const DTask t = tasks.get(ti);
+        if (!b_uniform(t.valid ? 1u : 0u)) break;
+        const uint32_t layer = b_uniform(t.layer), ub = b_uniform(t.ub), ue = b_uniform(t.ue);
+        const uint32_t acc = ti & 1u, use = (ti >> 1) & 1u, d = tm + acc * 16u;
+        if (!cx.warp_wait(&c.tmem_empty[acc], use ^ 1u, kErrWaitTmemEmpty)) return;
+        if (layer == 0u && !have1) { if (!cx.warp_wait(&c.tile_full[0], 0u, kErrWaitActsFull)) return; have1 = true; }
+        if (layer != 0u && !have2) { if (!cx.warp_wait(&c.tile_full[1], 0u, kErrWaitL1Done)) return; have2 = true; }
+        tc_fence_after();
+        uint32_t tok = s0 + ub * F::kRec;
+        #pragma unroll 1
+        for (uint32_t u = ub; u < ue; ++u, ++it, tok += F::kRec) {
+            if (!cx.warp_wait(kA8 ? &c.xfull[it & 1u] : &c.wfull[s], kA8 ? (it >> 1) & 1u : ph, kErrWaitFull)) return;
+            tc_fence_after();
+            if (lane == 0 && it == 0u) cx.sm_phase(kSmFirstLanded);
+            if (elect_one()) {
+                const uint32_t wsm = kA8 ? x0 + (it & 1u) * kXbufBytes : wsm0;
+                const uint64_t adesc = smem_desc(wsm, 1024u, kLayoutSw128), bdesc = smem_desc(tok, 1024u, kLayoutSw128);
+                const uint64_t asf = smem_desc(wsm + (kA8 ? 2u * kUnitWBytes : static_cast<uint32_t>(kUnitWBytes)), 128u, kLayoutNone);
+                const uint64_t bsf = smem_desc(tok + 2048u * F::kAtoms, 128u, kLayoutNone);
+                const uint32_t sfa = tm + 32u + (it & 1u) * 32u, sfb = sfa + 16u;
+                #pragma unroll
+                for (uint32_t pl = 0; pl < kPlanes; ++pl) {
+                    utccp_32x128b_warpx4(sfa + pl * 4u, asf + pl * 32u);
+                    utccp_32x128b_warpx4(sfb + pl * 4u, bsf + pl * 32u);
+                }
+                #pragma unroll
+                for (uint32_t ks = 0; ks < kUnitK / kStepK; ++ks) {
+                    const uint32_t pl = (ks * kStepK) / (4u * F::kVec), sf_id = ((ks * kStepK) % (4u * F::kVec)) / F::kVec;
+                    const uint64_t ad = adesc + (ks & 3u) * 2u + (kA8 ? (ks >> 2) * (kUnitWBytes >> 4) : 0u);
+                    const uint64_t bd = bdesc + (ks & 3u) * 2u + (kA8 ? (ks >> 2) * (2048u >> 4) : 0u);
+                    const uint32_t idesc = idesc_with_sf(kIdesc, sf_id, sf_id), accum = (u != ub || ks != 0u) ? 1u : 0u;
+                    if constexpr (kA8) umma_mxf8f6f4(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
+                    else if constexpr (kFmt == 0) umma_mxf4_block32(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
+                    else umma_nvf4_block16(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
+                }
+                tc_commit(kA8 ? &c.xempty[it & 1u] : &c.wempty[s]);
+            }
+            __syncwarp();
+            wsm0 += p.unit_bytes;
+            if (++s == nw) { s = 0; ph ^= 1u; wsm0 = ring0; }
+        }
+        if (elect_one()) tc_commit(&c.tmem_full[acc]);
+        __syncwarp();
+    }
+    if (lane == 0 && it != 0u) cx.stamp_max(kStampLastWeight);
+}
+
+// the widening warps' loop (E4M3 tokens) over this kernel's tasks; the unit's work is the batch kernel's
+__device__ void d_role_widen(const DCtx& cx, uint32_t xtid, uint32_t nw, const uint8_t* ring) {
+    const BParams& p = cx.p; DShared& c = cx.c;
+    const uint32_t lane = xtid & 31u;
+    uint8_t* x0 = const_cast<uint8_t*>(ring) + static_cast<size_t>(nw) * p.unit_bytes;
+    uint32_t it = 0, s = 0, ph = 0;
+    DTasks tasks(cx);
+    #pragma unroll 1
+    for (uint32_t ti = 0;; ++ti) {
+        const DTask t = tasks.get(ti);
+        if (!t.valid) break;
+        #pragma unroll 1
+        for (uint32_t u = t.ub; u < t.ue; ++u, ++it) {
+            if (!cx.warp_wait(&c.wfull[s], ph, kErrWaitFull)) return;
+            BWiden w;
+            w.load(ring + static_cast<size_t>(s) * p.unit_bytes, xtid);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&c.wempty[s]);
+            if (!cx.warp_wait(&c.xempty[it & 1u], ((it >> 1) & 1u) ^ 1u, kErrWaitEmpty)) return;
+            w.store(x0 + (it & 1u) * kXbufBytes, xtid);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&c.xfull[it & 1u]);
+            if (++s == nw) { s = 0; ph ^= 1u; }
+        }
+    }
+}
+
+// Intermediate rows of all experts -> the token tile of the L2 tasks (both epilogue groups, after the SM's last L1 task: its
+// MMAs on the tokens' tile, whose place this one takes, are over). Payload in 8-byte pieces (one 16 B load of two flagged words), then the scale words.
+template <int kFmt>
+__device__ __forceinline__ bool d_gather(const DCtx& cx, uint8_t* tile, uint32_t gtid) {
+    using F = DFmt<kFmt>;
+    const BParams& p = cx.p; DShared& c = cx.c;
+    constexpr uint32_t kThreads = kDEpiWarps * 32, kFly = 3;
+    const uint32_t flag = *reinterpret_cast<volatile uint32_t*>(&c.start_ok), pieces = p.mid_row_bytes / 8u, n = c.nlive * pieces;   // (start_ok holds the launch's flag)
+    uint32_t spins = 0;
+    #pragma unroll 1
+    for (uint32_t i0 = gtid; i0 < n; i0 += kThreads * kFly) {
+        uint4 v[kFly];
+        bool ok;
+        do {
+            ok = true;
+            #pragma unroll
+            for (uint32_t u = 0; u < kFly; ++u) {
+                const uint32_t i = i0 + u * kThreads;
+                if (i < n) {
+                    const uint32_t col = udiv_small(i, pieces), pc = i - col * pieces;
+                    v[u] = ld_volatile_v4(p.buf + p.off_mid + static_cast<size_t>(c.col_mid[col]) * 2u * p.mid_row_bytes + pc * 16u);
+                    ok = ok && v[u].y == flag && v[u].w == flag;
+                }
+            }
+            if (!ok && cx.give_up(spins, kErrWaitL1Done, 0u)) return false;
+        } while (!ok);
+        #pragma unroll
+        for (uint32_t u = 0; u < kFly; ++u) {
+            const uint32_t i = i0 + u * kThreads;
+            if (i < n) {
+                const uint32_t col = udiv_small(i, pieces), pc = i - col * pieces, ci = pc >> 1, at = ci >> 3;       // 16 B chunk, 128 B atom of the row
+                uint8_t* dst = tile + (F::kA8 ? (at >> 1) * F::kRec + (at & 1u) * 2048u : at * F::kRec) + sw128_off(col, ci & 7u) + (pc & 1u) * 8u;
+                *reinterpret_cast<uint2*>(dst) = make_uint2(v[u].x, v[u].z);
+            }
+        }
+    }
+    #pragma unroll 1
+    for (uint32_t i = gtid; i < c.nlive * p.n1; i += kThreads) {
+        const uint32_t col = udiv_small(i, p.n1), j = i - col * p.n1;
+        const uint8_t* src = p.buf + p.off_mid_sf + (static_cast<size_t>(c.col_mid[col]) * p.n1 + j) * 8u;
+        uint2 q = ld_volatile_v2(src);
+        while (q.y != flag) {
+            if (cx.give_up(spins, kErrWaitL1Done, 0u)) return false;
+            q = ld_volatile_v2(src);
+        }
+        uint8_t* sf = tile + (j >> 2) * F::kRec + 2048u * F::kAtoms + plane_off(col);
+        if constexpr (F::kVec == 16) *reinterpret_cast<uint32_t*>(sf + (j & 3u) * 512u) = q.x;
+        else *reinterpret_cast<uint16_t*>(sf + ((j >> 1) & 1u) * 512u + (j & 1u) * 2u) = static_cast<uint16_t>(q.x);
+    }
+    return true;
+}
+
+template <int kFmt>
+__device__ void d_role_epilogue(const DCtx& cx, uint32_t grp, uint32_t etid, uint8_t* tile, uint32_t flag) {
+    using F = DFmt<kFmt>;
+    constexpr bool kA8 = F::kA8;
+    constexpr int kVec = F::kVec;
+    const BParams& p = cx.p; DShared& c = cx.c;
+    const uint32_t ew = etid >> 5, q = etid & 7u, n = etid >> 3, bar = grp ? kBBarEpi1 : kBBarEpi0;
+    float* vt = c.vt[grp];
+    float* vt_w = vt + ((etid & 15u) >> 2) * 40u + (etid >> 4) * 4u + (etid & 3u);
+    const float* vt_r = vt + n * kBVtStride + q * 4u;
+    DTasks tasks(cx);
+    bool gathered = false, bad = false;
+    // the second token tile, when this group meets its first L2 task (or has no further task): the other group does the same
+    auto second_tile = [&]() -> bool {
+        gathered = true;
+        // (both groups are past their L1 tasks: nothing reads the first tile any more; they leave together if one has failed)
+        if (bar_red_or(kDBarGroups, kDEpiWarps * 32u, bad)) return false;
+        const bool ok = d_gather<kFmt>(cx, tile, grp * 128u + etid);
+        fence_proxy_async_smem();
+        const bool all_ok = __all_sync(0xffffffffu, ok);
+        if ((etid & 31u) == 0u && all_ok) mbar_arrive(&c.tile_full[1]);
+        if (grp == 0u && etid == 0u) cx.sm_phase(kSmFirstL2Staged);
+        return !bar_red_or(bar, 128u, !all_ok);
+    };
+    #pragma unroll 1
+    for (uint32_t ti = grp;; ti += 2) {
+        const DTask t = tasks.get(ti);
+        if ((!t.valid || t.layer != 0u) && !gathered) { if (!second_tile()) return; }
+        if (!t.valid) break;
+        const uint32_t use = (ti >> 1) & 1u, c0 = c.exp_c0[t.a], nv = c.exp_n[t.a];
+        const bool ok = cx.warp_wait(&c.tmem_full[grp], use, kErrWaitTmemFull);
+        tc_fence_after();
+        uint32_t raw[kTileTokens];
+        if (ok) {
+            tmem_ld_32x32b_x16(c.tmem_base + ((ew * 32u) << 16) + grp * 16u, raw);
+            tmem_ld_wait();
+            tc_fence_before();
+        }
+        __syncwarp();
+        if ((etid & 31u) == 0u) mbar_arrive(&c.tmem_empty[grp]);
+        if (bar_red_or(bar, 128u, !ok)) { bad = true; if (!gathered) second_tile(); return; }
+        #pragma unroll
+        for (uint32_t i = 0; i < kTileTokens; ++i) vt_w[i * kBVtStride] = __uint_as_float(raw[i]);
+        if (ti < 2u && etid == 0u) cx.sm_phase(kSmFirstMmaDone);
+        if (t.parts > 1u) {
+            // a part of a remainder tile: [part SM][row of the expert][weight row] flagged fp32 words; the group's first SM adds
+            const uint32_t first = c.split_first;
+            auto part_word = [&](uint32_t sm, uint32_t i) { return p.buf + p.off_red + ((static_cast<size_t>(sm) * kDEntries + i) * kTileRows + etid) * 8u; };
+            if (blockIdx.x != first) {
+                #pragma unroll 1
+                for (uint32_t i = 0; i < nv; ++i) st_volatile_v2(part_word(blockIdx.x, i), __float_as_uint(vt_w[(c0 + i) * kBVtStride]), flag);
+                continue;                                            // (each thread wrote and read its own words of vt)
+            }
+            bool got = true;
+            uint32_t spins = 0;
+            #pragma unroll 1
+            for (uint32_t i = 0; i < nv && got; ++i) {
+                float sum = 0.f + vt_w[(c0 + i) * kBVtStride];
+                #pragma unroll 1
+                for (uint32_t p0 = 1; p0 < t.parts && got; p0 += 8) {        // eight parts' words in flight, added in SM order
+                    uint2 w[8];
+                    bool all;
+                    do {
+                        all = true;
+                        #pragma unroll
+                        for (uint32_t u = 0; u < 8; ++u)
+                            if (p0 + u < t.parts) { w[u] = ld_volatile_v2(part_word(first + p0 + u, i)); all = all && w[u].y == flag; }
+                        if (!all && cx.give_up(spins, kErrWaitL1Done, 1u)) got = false;
+                    } while (!all && got);
+                    #pragma unroll
+                    for (uint32_t u = 0; u < 8; ++u) if (p0 + u < t.parts) sum += __uint_as_float(w[u].x);
+                }
+                vt_w[(c0 + i) * kBVtStride] = sum;
+            }
+            if (bar_red_or(bar, 128u, !got)) { bad = true; if (!gathered) second_tile(); return; }
+        } else bar_sync(bar, 128u);
+        float a[16];
+        #pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) {
+            const float4 v = *reinterpret_cast<const float4*>(vt_r + i * 40u);
+            a[4 * i] = v.x; a[4 * i + 1] = v.y; a[4 * i + 2] = v.z; a[4 * i + 3] = v.w;
+        }
+        const bool live = n - c0 < nv;
+        if (t.layer == 0u) {
+            float o[8];
+            uint32_t sfw;
+            b_swiglu(p, a, live ? c.col_w[n] : 0.f, o);
+            b_requantise<kFmt>(p, o, sfw);
+            if (live) {
+                const size_t row = c.col_mid[n];
+                uint8_t* dst = p.buf + p.off_mid + row * 2u * p.mid_row_bytes + (t.j * 8u + q) * (kA8 ? 16u : 8u);
+                if constexpr (kA8) {
+                    const uint32_t w0 = cvt_e4m3x2(o[0], o[1]) | (cvt_e4m3x2(o[2], o[3]) << 16), w1 = cvt_e4m3x2(o[4], o[5]) | (cvt_e4m3x2(o[6], o[7]) << 16);
+                    st_ll_half(dst, make_uint4(w0, w1, 0u, 0u), flag, 0u);
+                } else {
+                    st_volatile_v2(dst, cvt_e2m1x2(o[0], o[1]) | (cvt_e2m1x2(o[2], o[3]) << 8) | (cvt_e2m1x2(o[4], o[5]) << 16) | (cvt_e2m1x2(o[6], o[7]) << 24), flag);
+                }
+                if (q == 0u) st_volatile_v2(p.buf + p.off_mid_sf + (row * p.n1 + t.j) * 8u, kVec == 16 ? sfw : sfw & 0xFFFFu, flag);
+            }
+            if (etid == 0u) cx.sm_phase(kSmLastL1Epilogue);
+        } else if (live) {
+            uint32_t w[8];
+            #pragma unroll
+            for (uint32_t i = 0; i < 8; ++i)
+                w[i] = static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(a[2 * i] * p.l2_scale))) |
+                       (static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(a[2 * i + 1] * p.l2_scale))) << 16);
+            uint8_t* dst = p.buf + p.off_comb + (static_cast<size_t>(c.col_f[n]) * p.H + t.j * 128u + q * 16u) * 4u;
+            const uint32_t lo[8] = {w[0], flag, w[1], flag, w[2], flag, w[3], flag}, hi[8] = {w[4], flag, w[5], flag, w[6], flag, w[7], flag};
+            st_global_v8(dst, lo);
+            st_global_v8(dst + 32, hi);
+        }
+        if (ti < 2u && etid == 0u) cx.sm_phase(kSmFirstEpilogue);
+        bar_sync(bar, 128u);                                         // (the reads of vt are over)
+    }
+}
+
+// Items (token, eight columns): a thread adds the token's live routes in slot order as their flagged words arrive.
+__device__ void d_role_combine(const DCtx& cx, uint32_t flag) {
+    const BParams& p = cx.p; DShared& c = cx.c;
+    const uint32_t G = gridDim.x, per = p.H / 8u, nitems = static_cast<uint32_t>(p.T) * per;
+    uint32_t spins = 0;
+    #pragma unroll 1
+    for (;;) {
+        const uint32_t k = atomicAdd(&c.comb_next, 1u), idx = blockIdx.x + k * G;
+        if (idx >= nitems) return;
+        const uint32_t tok = udiv_small(idx, per), ch = idx - tok * per;
+        const uint32_t mask = (c.live_mask >> (tok * p.topk)) & ((1u << p.topk) - 1u);
+        const uint8_t* base = p.buf + p.off_comb + (static_cast<size_t>(tok) * p.topk * p.H + ch * 8u) * 4u;
+        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        #pragma unroll 1
+        for (int s0 = 0; s0 < p.topk; s0 += 8) {
+            uint4 v[8];
+            bool ok;
+            do {
+                ok = true;
+                #pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    v[u] = make_uint4(0u, 0u, 0u, 0u);
+                    if ((mask >> (s0 + u)) & 1u) {
+                        const uint8_t* src = base + static_cast<size_t>(s0 + u) * p.H * 4u;
+                        const uint4 a = ld_volatile_v4(src), b = ld_volatile_v4(src + 16);
+                        ok = ok && ll_valid(a, b, flag);
+                        v[u] = ll_data(a, b);
+                    }
+                }
+                if (!ok && cx.give_up(spins, kErrWaitCombineFlag, tok)) return;
+            } while (!ok);
+            #pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                acc[0] += __uint_as_float(v[u].x << 16); acc[1] += __uint_as_float(v[u].x & 0xFFFF0000u);
+                acc[2] += __uint_as_float(v[u].y << 16); acc[3] += __uint_as_float(v[u].y & 0xFFFF0000u);
+                acc[4] += __uint_as_float(v[u].z << 16); acc[5] += __uint_as_float(v[u].z & 0xFFFF0000u);
+                acc[6] += __uint_as_float(v[u].w << 16); acc[7] += __uint_as_float(v[u].w & 0xFFFF0000u);
+            }
+        }
+        uint4 o;
+        uint32_t* ow = &o.x;
+        #pragma unroll
+        for (int i = 0; i < 4; ++i)
+            ow[i] = static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(acc[2 * i]))) |
+                    (static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(acc[2 * i + 1]))) << 16);
+        *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.y) + (static_cast<size_t>(tok) * p.H + ch * 8u) * 2u) = o;
+        if (k == 0u) cx.sm_phase(kSmFirstCombined);
+        cx.sm_phase(kSmCombineDone);
+    }
+}
+
+// Sorts the routing entries by (expert, entry) and derives this SM's part of a remainder tile (one warp; lane i holds entry i).
+__device__ __forceinline__ void d_route(const DCtx& cx, uint32_t e, float w, uint32_t n, uint32_t lane) {
+    const BParams& p = cx.p; DShared& c = cx.c;
+    const bool live = lane < n && e < kMaxLocalExperts;
+    if (__any_sync(0xffffffffu, lane < n && e == 0xFEu)) { if (lane == 0) cx.fail(kErrWaitCombineFlag, 0xFFFFu); }   // a route to an expert that does not exist
+    const uint32_t key = live ? e : 0xFFu;
+    uint32_t below = 0u, pos = 0u, group = 0u;                       // rows of smaller experts, earlier rows of this one, smaller experts
+    #pragma unroll
+    for (uint32_t i = 0; i < kDEntries; ++i) {
+        const uint32_t ei = __shfl_sync(0xffffffffu, key, i);
+        const bool head = (__ballot_sync(0xffffffffu, key == ei) & ((1u << i) - 1u)) == 0u;      // entry i is its expert's first
+        below += ei < key ? 1u : 0u;
+        pos += (ei == key && i < lane) ? 1u : 0u;
+        group += (head && ei < key) ? 1u : 0u;
+    }
+    const uint32_t live_mask = __ballot_sync(0xffffffffu, live), firsts = __ballot_sync(0xffffffffu, live && pos == 0u), M = __popc(firsts);
+    if (live) {
+        const uint32_t col = below + pos;
+        c.ent_col[lane] = col;
+        c.col_f[col] = lane; c.col_mid[col] = group * kTileTokens + pos; c.col_w[col] = w;
+        if (pos == 0u) { c.exp_e[group] = e; c.exp_c0[group] = below; }
+    }
+    __syncwarp();
+    if (live) atomicMax(&c.exp_n[group], pos + 1u);
+    if (lane < kDEntries) c.ent_e[lane] = live ? e : 0xFFu;
+    const uint32_t G = gridDim.x, bid = blockIdx.x, NT1 = M * p.n1, r = NT1 - udiv_small(NT1, G) * G, k = p.k1;
+    if (lane == 0) {
+        c.M = M; c.nlive = __popc(live_mask); c.live_mask = live_mask;
+        c.split_parts = 0u;
+        if (r != 0u) {
+            // the first r tiles are the remainder: tile t is shared by the SMs [ceil(t G / r), ceil((t + 1) G / r))
+            const uint32_t t = udiv_small(bid * r, G), gs = udiv_small(t * G + r - 1u, r), ge = udiv_small((t + 1u) * G + r - 1u, r);
+            const uint32_t S = ge - gs, li = bid - gs, base = udiv_small(k, S), extra = k - base * S;
+            const uint32_t ub = li * base + (li < extra ? li : extra), ue = ub + base + (li < extra ? 1u : 0u);
+            if (ue > ub) { c.split_t = t; c.split_range = ub | (ue << 8); c.split_first = gs; c.split_parts = S < k ? S : k; }
+        }
+    }
+}
+
+template <int kFmt, bool kFe>
+__global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(const __grid_constant__ BParams p) {
+    using F = DFmt<kFmt>;
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ DShared c;
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~static_cast<uintptr_t>(1023u));
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, bid = blockIdx.x, G = gridDim.x;
+    uint32_t* ctrl32 = reinterpret_cast<uint32_t*>(p.buf + p.off_ctrl);
+    const uint32_t n = static_cast<uint32_t>(p.T) * p.topk;
+    // shared memory: token tile (the intermediate rows' tile takes the place of the tokens'), weight ring, widened units
+    const uint32_t ring_off = (p.k1 > p.k2 ? p.k1 : p.k2) * F::kRec;
+    uint32_t nw = udiv_small(p.smem_ring - ring_off - (F::kA8 ? 2u * kXbufBytes : 0u), p.unit_bytes);
+    nw = nw > kDStages ? kDStages : nw;
+    // ---- what needs nothing of the launches before this one: it overlaps the end of the previous kernel in the stream
+    if (warp == 2) {
+        if (lane < kDStages) { mbar_init(&c.wfull[lane], 1); mbar_init(&c.wempty[lane], F::kA8 ? kBExpWarps : 1); }
+        if (lane < 2) {
+            mbar_init(&c.tmem_full[lane], 1); mbar_init(&c.tmem_empty[lane], 4);
+            mbar_init(&c.xfull[lane], kBExpWarps); mbar_init(&c.xempty[lane], 1);
+            mbar_init(&c.tile_full[lane], kDEpiWarps);
+        }
+        mbar_fence_init();
+        if (lane < kDEntries) c.exp_n[lane] = 0u;
+        if (lane == 0) { c.abort_flag = 0u; c.comb_next = 0u; c.wissued = 0u; c.start_ok = 0u; }
+    }
+    if (warp == 1) { tmem_alloc(&c.tmem_base, 128); tmem_relinquish(); tc_fence_before(); }
+    __syncthreads();
+    tc_fence_after();
+    grid_dependency_wait();
+    grid_launch_dependents();
+    const unsigned long long t_first = globaltimer_ns();
+    const uint32_t epoch = ld_volatile_u32(ctrl32 + kCtrlEpoch / 4 + bid), flag = epoch + 1u;      // (tid 64 counts on after the barrier below)
+    const DCtx cx(p, c, smem, globaltimer_ns() + p.timeout_ns, epoch & 1u);
+    constexpr uint32_t kEW = 4;                                       // the first of the warps that build the token tile
+    const bool builder = warp >= kEW && warp < kEW + kDEpiWarps;
+    constexpr uint32_t kPerWarp = kDEntries / kDEpiWarps;             // entries a builder warp writes: 2
+    // Rows of entries bw and bw + 8 in registers before the routing is known: the 16 B chunks of the packed row and its scale
+    // bytes (lane, lane + 32, ...), or, from hidden states, the quantised pieces of this lane (8 elements of every unit).
+    constexpr uint32_t kChunks = F::kA8 ? 9u : 5u;
+    const uint32_t xq = p.x_row_bytes / 16u, per_row = xq + p.x_sf_row_bytes / 16u;
+    uint4 v[kPerWarp][kChunks];
+    uint2 hb[kPerWarp][kFe ? 16 : 1];
+    uint32_t hsf[kPerWarp][kFe ? 4 : 1];                              // scale bytes of four units to a word
+    uint32_t e = 0xFFu;
+    float w = 0.f;
+    if constexpr (!kFe) {
+        if (warp == 0 && lane < n) {
+            const long long ex = reinterpret_cast<const long long*>(p.buf + p.off_topk_idx)[lane];
+            w = reinterpret_cast<const float*>(p.buf + p.off_topk_w)[lane];
+            e = ex < 0 ? 0xFFu : (ex < p.E ? static_cast<uint32_t>(ex) : 0xFEu);
+        }
+        if (builder) {
+            #pragma unroll
+            for (uint32_t a = 0; a < kPerWarp; ++a) {
+                const uint32_t f = warp - kEW + a * kDEpiWarps;
+                if (f < n) {
+                    const uint32_t tok = udiv_small(f, p.topk);
+                    const uint8_t* xs = p.buf + p.off_x + static_cast<size_t>(tok) * p.x_row_bytes;
+                    const uint8_t* sf = p.buf + p.off_x_sf + static_cast<size_t>(tok) * p.x_sf_row_bytes;
+                    #pragma unroll
+                    for (uint32_t u = 0; u < kChunks; ++u) {
+                        const uint32_t ci = lane + u * 32;
+                        if (ci < per_row) v[a][u] = ld_cg_v4(ci < xq ? xs + ci * 16u : sf + (ci - xq) * 16u);
+                    }
+                }
+            }
+        }
+    } else {
+        // ---- router frontend: partial logits spread over the SMs; selection and quantisation on every SM
+        fe_logits_blocks<1, 3>(p.fe, warp * G + bid, G * (F::kThreads / 32), lane, flag);
+        if (builder) {
+            #pragma unroll
+            for (uint32_t a = 0; a < kPerWarp; ++a) {
+                const uint32_t f = warp - kEW + a * kDEpiWarps;
+                if (f < n) {
+                    const uint32_t tok = f >> 3;                      // (eight routes per token)
+                    const uint4* xrow = reinterpret_cast<const uint4*>(p.fe.hidden + static_cast<size_t>(tok) * p.H);
+                    const bool out = bid == tok && (f & 7u) == 0u;    // the token's row of the x / x_sf views
+                    bool nz = false;
+                    #pragma unroll
+                    for (uint32_t u0 = 0; u0 < 16; u0 += 4) {
+                        uint4 raw[4];
+                        #pragma unroll
+                        for (uint32_t u = 0; u < 4; ++u) if (u0 + u < static_cast<uint32_t>(p.k1)) raw[u] = __ldg(xrow + (u0 + u) * 32u + lane);
+                        hsf[a][u0 / 4] = 0u;
+                        #pragma unroll
+                        for (uint32_t u = 0; u < 4; ++u) {
+                            if (u0 + u < static_cast<uint32_t>(p.k1)) {
+                                uint32_t sfb;
+                                const uint2 b = fe_quant8(raw[u], kFmt, p.fe.x_gs, nz, sfb);
+                                hb[a][u0 + u] = b;
+                                hsf[a][u0 / 4] |= sfb << (8u * u);
+                                if (out) {
+                                    uint8_t* xr = p.buf + p.off_x + static_cast<size_t>(tok) * p.x_row_bytes;
+                                    if constexpr (F::kA8) *reinterpret_cast<uint2*>(xr + (u0 + u) * 256u + lane * 8u) = b;
+                                    else *reinterpret_cast<uint32_t*>(xr + (u0 + u) * 128u + lane * 4u) = b.x;
+                                    constexpr uint32_t kLanes = F::kVec / 8;         // lanes that share a scale block
+                                    if (lane % kLanes == 0u) p.buf[p.off_x_sf + static_cast<size_t>(tok) * p.x_sf_row_bytes + (u0 + u) * (256u / F::kVec) + lane / kLanes] = static_cast<uint8_t>(sfb);
+                                }
+                            }
+                        }
+                    }
+                }
+            }
+        }
+        if (warp == 2 || warp == 3) {
+            auto give_up = [&]() -> bool {
+                if (cx.aborted()) return true;
+                if (cx.expired()) { cx.fail(kErrWaitFrontend); return true; }
+                return false;
+            };
+            const uint32_t tok = warp - 2u;
+            if (tok < static_cast<uint32_t>(p.T)) {
+                const bool nz = fe_row_nonzero(p.fe.hidden + static_cast<size_t>(tok) * p.H, p.H, lane);
+                FeParams q = p.fe;
+                if (bid != tok) { q.topk_idx = nullptr; q.topk_w = nullptr; }          // one SM writes the token's routing views
+                uint32_t ce; float cw;
+                const bool ok = fe_select_token_regs<2>(q, tok, nz, lane, flag, nullptr, give_up, &ce, &cw);
+                if (lane < 8u) { c.ent_e[tok * 8u + lane] = ok ? ce : 0xFFu; c.ent_w[tok * 8u + lane] = ok ? cw : 0.f; }
+            }
+        }
+        __syncthreads();
+        if (bid == 0 && tid == 0) cx.stamp(kStampFrontend);
+        if (warp == 0 && lane < n) { e = c.ent_e[lane]; w = c.ent_w[lane]; e = e < static_cast<uint32_t>(p.E) ? e : 0xFFu; }
+    }
+    // ---- routing. The warp that sorts the entries is the weight loader: it does not wait for the others
+    if (warp == 0) {
+        d_route(cx, e, w, n, lane);
+        __syncwarp();
+        if (lane == 0) c.start_ok = cx.aborted() ? 0u : flag;        // (decided once: every warp takes the same way from here)
+        __threadfence_block();
+        __syncwarp();
+        bar_arrive(kDBarRouted, F::kThreads);
+        if (lane == 0) { cx.sm_phase(kSmScheduled); cx.stamp_max(kStampLastScheduled); if (bid == 0) cx.stamp(kStampScheduled); }
+    } else bar_sync(kDBarRouted, F::kThreads);
+    const bool start = *reinterpret_cast<volatile uint32_t*>(&c.start_ok) != 0u;
+    if (start) {
+        if (warp == 0) {
+            d_role_weights(cx, nw, smem + ring_off);
+        } else if (warp == 1) {
+            d_role_mma<kFmt>(cx, lane, nw, ring_off);
+        } else if (builder) {
+            // ---- the token tile
+            #pragma unroll
+            for (uint32_t a = 0; a < kPerWarp; ++a) {
+                const uint32_t f = warp - kEW + a * kDEpiWarps;
+                if (f < n && ((c.live_mask >> f) & 1u) != 0u) {
+                    const uint32_t col = c.ent_col[f];
+                    if constexpr (!kFe) {
+                        #pragma unroll
+                        for (uint32_t u = 0; u < kChunks; ++u) {
+                            const uint32_t ci = lane + u * 32;
+                            if (ci < xq) {
+                                const uint32_t at = ci >> 3;
+                                *reinterpret_cast<uint4*>(smem + (F::kA8 ? (at >> 1) * F::kRec + (at & 1u) * 2048u : at * F::kRec) + sw128_off(col, ci & 7u)) = v[a][u];
+                            } else if (ci < per_row) {
+                                const uint32_t g = (ci - xq) * 4u;
+                                const uint32_t wv[4] = {v[a][u].x, v[a][u].y, v[a][u].z, v[a][u].w};
+                                #pragma unroll
+                                for (uint32_t k = 0; k < 4; ++k)
+                                    *reinterpret_cast<uint32_t*>(smem + ((g + k) / F::kPlanes) * F::kRec + 2048u * F::kAtoms + ((g + k) % F::kPlanes) * 512u + plane_off(col)) = wv[k];
+                            }
+                        }
+                    } else {
+                        constexpr uint32_t kLanes = F::kVec / 8;
+                        #pragma unroll
+                        for (uint32_t u = 0; u < 16; ++u) {
+                            if (u < static_cast<uint32_t>(p.k1)) {
+                                uint8_t* rec = smem + u * F::kRec;
+                                if constexpr (F::kA8) *reinterpret_cast<uint2*>(rec + (lane >> 4) * 2048u + sw128_off(col, (lane >> 1) & 7u) + (lane & 1u) * 8u) = hb[a][u];
+                                else *reinterpret_cast<uint32_t*>(rec + sw128_off(col, lane >> 2) + (lane & 3u) * 4u) = hb[a][u].x;
+                                const uint32_t blk = lane / kLanes;
+                                if (lane % kLanes == 0u)
+                                    rec[2048u * F::kAtoms + (blk >> 2) * 512u + plane_off(col) + (blk & 3u)] = static_cast<uint8_t>(hsf[a][u / 4] >> (8u * (u & 3u)));
+                            }
+                        }
+                    }
+                }
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) { mbar_arrive(&c.tile_full[0]); cx.sm_phase(kSmRowsCached); }
+            d_role_epilogue<kFmt>(cx, (warp - kEW) >> 2, (tid - 32u * kEW) & 127u, smem, flag);
+        } else if (warp >= kEW + kDEpiWarps) {
+            if constexpr (F::kA8) d_role_widen(cx, tid - 32u * (kEW + kDEpiWarps), nw, smem + ring_off);
+        }
+    }
+    // ---- off the critical path: launch number, counters, stamps, and what others may inspect afterwards
+    if (warp == 3) {
+        if (lane == 0) {
+            ctrl32[kCtrlEpoch / 4 + bid] = epoch + 1u;
+            reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlSmEntry)[bid] = t_first;
+            reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlSmPhase)[bid * kSmPhaseSlots + kSmEntry] = t_first;
+            if (bid == 0) {
+                ctrl32[kCtrlStatus / 4 + 1] = epoch + 1u; ctrl32[kCtrlStatus / 4 + 2] = 0u; ctrl32[kCtrlStatus / 4 + 3] = 0u;
+                reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlStamps)[kStampEntry] = t_first;
+                reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlStamps)[kStampPrologue] = t_first;   // (set-up precedes the first stamp)
+            }
+        }
+        // the batch kernel's arrival counts of the other parity
+        uint32_t* other = reinterpret_cast<uint32_t*>(p.buf + p.off_arrive) + (cx.par ^ 1u) * 2u * p.tile_capacity;
+        #pragma unroll 1
+        for (uint32_t i = bid * 32u + lane; i < 2u * p.tile_capacity; i += G * 32u) other[i] = 0u;
+        if (bid == 0 && start) {
+            cx.col_counts(cx.par ^ 1u)[lane] = 0u;
+            cx.col_counts(cx.par ^ 1u)[lane + 32] = 0u;
+            if (p.stats != nullptr && lane < c.M) p.stats[c.exp_e[lane]] += static_cast<int>(c.exp_n[lane]);
+            uint8_t* region = p.buf + p.off_rx + static_cast<size_t>(cx.par) * p.rx_region;
+            if (lane == 0) st_ll_16B(region, make_uint4(c.nlive, 0u, 0u, 0u), flag);
+            if (lane < n && ((c.live_mask >> lane) & 1u) != 0u) {
+                const uint32_t li = __popc(c.live_mask & ((1u << lane) - 1u)), tok = udiv_small(lane, p.topk);
+                st_ll_16B(region + 32u + static_cast<size_t>(li) * 2u * p.rx_row_bytes + 2u * (p.rx_row_bytes - 16u),
+                          make_uint4(c.ent_e[lane], tok, lane - tok * p.topk, __float_as_uint(c.col_w[c.ent_col[lane]])), flag);
+            }
+        }
+    }
+    if (tid == 128) { cx.stamp_max(kStampLastTasksDone); cx.sm_phase(kSmTasksDone); if (bid == 0) cx.stamp(kStampTasksDone); }
+    if (start) d_role_combine(cx, flag);
+    // ---- exit: an aborted SM lets the copies in flight land (bounded waits) before its shared memory goes away
+    if (cx.aborted() && warp == 0) {
+        const uint32_t issued = *reinterpret_cast<volatile uint32_t*>(&c.wissued);
+        #pragma unroll 1
+        for (uint32_t k = issued > nw ? issued - nw : 0u; k < issued; ++k)
+            for (uint32_t spin = 0; spin < 2000u && !mbar_try_wait(&c.wfull[k % nw], (k / nw) & 1u); ++spin) { }
+        for (uint32_t spin = 0; spin < 2000u; ++spin) __nanosleep(100);
+    }
+    __syncthreads();
+    if (warp == 1) { tc_fence_after(); tmem_dealloc(c.tmem_base, 128); }
+    if (tid == 0) { if (bid == 0) cx.stamp(kStampExit); cx.stamp_max(kStampLastExit); cx.sm_phase(kSmExit); }
+}
+
+}  // namespace mm

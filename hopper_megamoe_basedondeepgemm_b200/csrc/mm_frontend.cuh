@@ -87,6 +87,79 @@ __device__ __forceinline__ void fe_logits_items(const FeParams& q, uint32_t warp
     }
 }
 
+// The same partial logits (the same sums in the same order) with blocks of kEb experts x 4 tokens per warp and kAhead chunks
+// per lane in flight: per multiply-add a block of 4 x 4 reads 0.5 operand chunks instead of 1.25. The loads run at what an
+// SM takes in from the L2 (about 50 GB/s), so that is the time of a large batch; a small one needs every (expert, half) as
+// an item of its own to have enough of them. `fe_expert_block` draws the line at four items per SM.
+template <int kEb, int kAhead>
+__device__ __forceinline__ void fe_logits_blocks(const FeParams& q, uint32_t warp, uint32_t nwarps, uint32_t lane, uint32_t flag) {
+    const uint32_t tblocks = (q.T + 3) / 4, eblocks = (q.E + kEb - 1) / kEb, nchunk = q.H / 8, half = (nchunk + kFeParts - 1) / kFeParts;
+    const uint32_t nitems = eblocks * kFeParts * tblocks;
+    #pragma unroll 1
+    for (uint32_t item = warp; item < nitems; item += nwarps) {
+        const uint32_t part = item % kFeParts, r = item / kFeParts, tb = udiv_small(r, eblocks), e0 = (r - tb * eblocks) * kEb, t0 = tb * 4u;
+        const uint32_t nt = min(4u, static_cast<uint32_t>(q.T) - t0), ne = min(static_cast<uint32_t>(kEb), static_cast<uint32_t>(q.E) - e0);
+        const uint32_t c_lo = part * half, c_hi = min(nchunk, c_lo + half);
+        float acc[kEb][4];
+        #pragma unroll
+        for (int e = 0; e < kEb; ++e) { acc[e][0] = 0.f; acc[e][1] = 0.f; acc[e][2] = 0.f; acc[e][3] = 0.f; }
+        // (rows beyond the last expert or token repeat the last one: their sums are not stored)
+        const uint4 *wrow[kEb], *xrow[4];
+        #pragma unroll
+        for (uint32_t e = 0; e < kEb; ++e) wrow[e] = reinterpret_cast<const uint4*>(q.router_w + static_cast<size_t>(e0 + (e < ne ? e : ne - 1u)) * q.H);
+        #pragma unroll
+        for (uint32_t t = 0; t < 4; ++t) xrow[t] = reinterpret_cast<const uint4*>(q.hidden + static_cast<size_t>(t0 + (t < nt ? t : nt - 1u)) * q.H);
+        #pragma unroll 1
+        for (uint32_t ch0 = c_lo + lane; ch0 < c_hi; ch0 += 32 * kAhead) {
+            uint4 wq[kEb][kAhead], xq[4][kAhead];
+            #pragma unroll
+            for (uint32_t b = 0; b < kAhead; ++b) {
+                const uint32_t ch = ch0 + 32 * b;
+                if (ch < c_hi) {
+                    #pragma unroll
+                    for (uint32_t e = 0; e < kEb; ++e) wq[e][b] = __ldg(wrow[e] + ch);
+                    #pragma unroll
+                    for (uint32_t t = 0; t < 4; ++t) if (t < nt) xq[t][b] = __ldg(xrow[t] + ch);
+                }
+            }
+            #pragma unroll
+            for (uint32_t b = 0; b < kAhead; ++b) {
+                if (ch0 + 32 * b < c_hi) {
+                    #pragma unroll
+                    for (uint32_t t = 0; t < 4; ++t) {
+                        if (t < nt) {
+                            float x[8];
+                            unpack_bf16x8(xq[t][b], x);
+                            #pragma unroll
+                            for (uint32_t e = 0; e < kEb; ++e) {
+                                float w[8];
+                                unpack_bf16x8(wq[e][b], w);
+                                #pragma unroll
+                                for (int k = 0; k < 8; ++k) acc[e][t] = fmaf(x[k], w[k], acc[e][t]);
+                            }
+                        }
+                    }
+                }
+            }
+        }
+        #pragma unroll
+        for (uint32_t e = 0; e < kEb; ++e) {
+            #pragma unroll
+            for (uint32_t t = 0; t < 4; ++t) {
+                #pragma unroll
+                for (int o = 16; o > 0; o >>= 1) acc[e][t] += __shfl_xor_sync(0xffffffffu, acc[e][t], o);
+                if (lane == 0 && t < nt && e < ne)
+                    st_volatile_v2(reinterpret_cast<uint8_t*>(q.logits) + (static_cast<size_t>(t0 + t) * q.E + e0 + e) * 16u + part * 8u,
+                                   __float_as_uint(acc[e][t]), flag);
+            }
+        }
+    }
+}
+__device__ __forceinline__ uint32_t fe_expert_block(const FeParams& q, uint32_t grid) {
+    const uint32_t per = static_cast<uint32_t>(q.E) * kFeParts * ((q.T + 3) / 4);     // items of one expert each
+    return per >= 16u * grid ? 4u : (per >= 8u * grid ? 2u : 1u);
+}
+
 // logit of (token t, expert e) from its two halves; `flag` != 0: poll until both halves carry it (`ok` = false if `give_up`
 // says so first)
 template <typename GiveUp>
@@ -98,10 +171,6 @@ __device__ __forceinline__ float fe_read_logit(const FeParams& q, uint32_t t, ui
         if (flag == 0u || (v.y == flag && v.w == flag)) return bf16_round(__uint_as_float(v.x) + __uint_as_float(v.z)) + 0.0f;
         if ((++spins & 0x3Fu) == 0u && give_up()) { ok = false; return 0.f; }
     }
-}
-
-__global__ void __launch_bounds__(256) frontend_logits_kernel(const FeParams q) {
-    fe_logits_items(q, blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), gridDim.x * (blockDim.x >> 5), threadIdx.x & 31u, 1u);
 }
 
 __device__ __forceinline__ uint32_t orderable_f32(float v) {
@@ -117,6 +186,42 @@ __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v)
     return v;
 }
 
+// Eight consecutive elements per lane -> 4 bytes of E2M1 codes (formats 0, 1; in .x) or 8 bytes of E4M3 (format 2), and the
+// byte of the lane's scale block, which two (format 1) or four neighbouring lanes share. Every lane of the warp calls it.
+__device__ __forceinline__ uint2 fe_quant8(const uint4& raw, int fmt, float x_gs, bool& nonzero, uint32_t& sf_byte) {
+    float x[8];
+    unpack_bf16x8(raw, x);
+    float local = 0.f;
+    #pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        nonzero |= x[j] != 0.f;
+        if (fmt == 1) x[j] = __fdiv_rn(x[j], x_gs);
+        local = fmaxf(local, fabsf(x[j]));
+    }
+    local = fmaxf(local, __shfl_xor_sync(0xffffffffu, local, 1));
+    if (fmt != 1) local = fmaxf(local, __shfl_xor_sync(0xffffffffu, local, 2));
+    const float v = fmt == 2 ? fmaxf(local, 1.0e-4f) * (1.0f / 448.0f) : fmaxf(local, 1.0e-30f) * (1.0f / 6.0f);
+    float sf;
+    if (fmt == 1) {
+        sf_byte = cvt_e4m3x2(v, 0.f) & 0xFFu;
+        if (sf_byte == 0u) sf_byte = 1u;
+        sf = e4m3_to_float(sf_byte);
+    } else {
+        sf_byte = ceil_pow2_exp(v);
+        sf = __uint_as_float(sf_byte << 23);
+    }
+    const float inv = 1.0f / sf;
+    uint2 bytes = make_uint2(0u, 0u);
+    if (fmt == 2) {
+        bytes.x = cvt_e4m3x2(x[0] * inv, x[1] * inv) | (cvt_e4m3x2(x[2] * inv, x[3] * inv) << 16);
+        bytes.y = cvt_e4m3x2(x[4] * inv, x[5] * inv) | (cvt_e4m3x2(x[6] * inv, x[7] * inv) << 16);
+    } else {
+        #pragma unroll
+        for (int j = 0; j < 4; ++j) bytes.x |= cvt_e2m1x2(x[2 * j] * inv, x[2 * j + 1] * inv) << (8 * j);
+    }
+    return bytes;
+}
+
 // One warp quantises token row `xrow` (bf16 [H]) to packed E2M1 (formats 0, 1) or E4M3 bytes (format 2) + scale bytes;
 // returns whether any element is non-zero. With `pool_row` != nullptr the same bytes are also stored there as a row of
 // the receive pool (packed row, then the scale bytes; every 4 data bytes followed by `flag`): the dispatch of the fused
@@ -126,45 +231,26 @@ __device__ __forceinline__ bool fe_quant_token(const __nv_bfloat16* xrow, int H,
                                                uint8_t* pool_row = nullptr, uint32_t flag = 0u, uint32_t x_row_bytes = 0u) {
     const int vec = fmt == 1 ? 16 : 32, lanes_per_group = vec / 8;
     bool nonzero = false;
+    uint4 ahead[4];                                              // (four slices of the row in flight)
+    #pragma unroll 4
     for (int k0 = lane * 8; k0 < H; k0 += 256) {
-        float x[8];
-        unpack_bf16x8(*reinterpret_cast<const uint4*>(xrow + k0), x);
-        float local = 0.f;
-        #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            nonzero |= x[j] != 0.f;
-            if (fmt == 1) x[j] = __fdiv_rn(x[j], x_gs);
-            local = fmaxf(local, fabsf(x[j]));
+        if (((k0 >> 8) & 3) == 0) {
+            #pragma unroll
+            for (int b = 0; b < 4; ++b) if (k0 + 256 * b < H) ahead[b] = *reinterpret_cast<const uint4*>(xrow + k0 + 256 * b);
         }
-        local = fmaxf(local, __shfl_xor_sync(0xffffffffu, local, 1));
-        if (lanes_per_group == 4) local = fmaxf(local, __shfl_xor_sync(0xffffffffu, local, 2));
-        const float v = fmt == 2 ? fmaxf(local, 1.0e-4f) * (1.0f / 448.0f) : fmaxf(local, 1.0e-30f) * (1.0f / 6.0f);
-        uint32_t sf_byte; float sf;
-        if (fmt == 1) {
-            sf_byte = cvt_e4m3x2(v, 0.f) & 0xFFu;
-            if (sf_byte == 0u) sf_byte = 1u;
-            sf = e4m3_to_float(sf_byte);
-        } else {
-            sf_byte = ceil_pow2_exp(v);
-            sf = __uint_as_float(sf_byte << 23);
-        }
+        const int slice = (k0 >> 8) & 3;
+        uint32_t sf_byte;
+        const uint2 bytes = fe_quant8(slice == 0 ? ahead[0] : (slice == 1 ? ahead[1] : (slice == 2 ? ahead[2] : ahead[3])), fmt, x_gs, nonzero, sf_byte);
         if ((lane % lanes_per_group) == 0) sfrow[k0 / vec] = static_cast<uint8_t>(sf_byte);
-        const float inv = 1.0f / sf;
         const int it = k0 >> 8;                                  // which 256-element slice of the row
         if (fmt == 2) {
-            uint2 bytes;
-            bytes.x = cvt_e4m3x2(x[0] * inv, x[1] * inv) | (cvt_e4m3x2(x[2] * inv, x[3] * inv) << 16);
-            bytes.y = cvt_e4m3x2(x[4] * inv, x[5] * inv) | (cvt_e4m3x2(x[6] * inv, x[7] * inv) << 16);
             *reinterpret_cast<uint2*>(qrow + k0) = bytes;
             if (pool_row != nullptr) {
                 asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %4};" :: "l"(pool_row + 2 * k0), "r"(bytes.x), "r"(flag), "r"(bytes.y), "r"(flag) : "memory");
             }
         } else {
-            uint32_t packed = 0u;
-            #pragma unroll
-            for (int j = 0; j < 4; ++j) packed |= cvt_e2m1x2(x[2 * j] * inv, x[2 * j + 1] * inv) << (8 * j);
-            *reinterpret_cast<uint32_t*>(qrow + k0 / 2) = packed;
-            if (pool_row != nullptr) st_volatile_v2(pool_row + k0, packed, flag);          // 2 * (k0 / 2)
+            *reinterpret_cast<uint32_t*>(qrow + k0 / 2) = bytes.x;
+            if (pool_row != nullptr) st_volatile_v2(pool_row + k0, bytes.x, flag);         // 2 * (k0 / 2)
         }
         if (pool_row != nullptr) {
             // four scale bytes make one word: every lane of a group holds its group's byte; the first lane of four groups stores
@@ -273,15 +359,124 @@ __device__ __forceinline__ bool fe_select_token(const FeParams& q, uint32_t t, f
     return true;
 }
 
-// one warp per token: the token's quantisation, then top-8 + weights
-__global__ void __launch_bounds__(128) frontend_select_quant_kernel(const FeParams q) {
-    extern __shared__ float fe_scores[];                 // [4 warps][2 E]
-    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-    const uint32_t t = blockIdx.x * 4 + w;
-    if (t >= static_cast<uint32_t>(q.T)) return;
-    const bool nonzero = fe_quant_token(q.hidden + static_cast<size_t>(t) * q.H, q.H, q.fmt, q.x_gs,
-                                        q.x + static_cast<size_t>(t) * q.x_row_bytes, q.x_sf + static_cast<size_t>(t) * q.x_sf_row_bytes, lane);
-    fe_select_token(q, t, fe_scores + w * 2 * q.E, nonzero, lane, 0u, [] { return false; });
+// One warp selects the top-8 of token t among at most 32 kPer experts, kPer per lane, in registers: the same keys, weights
+// and order of additions as `fe_select_token` (maximum of the scores, then the smallest expert with it, eight times); a lane
+// keeps its best score at hand, so that a round is two warp reductions and a rescan by one lane. The routing goes into
+// topk_idx / topk_weights and, with `records`, as flagged 16 B records {expert (~0: none), flag, weight, flag} to where the
+// launch's other SMs poll it; `e_out` / `w_out` get lane k's route k (a null topk_idx: only those). `flag` 0: the logits are complete. Returns false if `give_up` ended a poll.
+template <int kPer, typename GiveUp>
+__device__ __forceinline__ bool fe_select_token_regs(const FeParams& q, uint32_t t, bool nonzero, uint32_t lane, uint32_t flag, uint8_t* records, GiveUp give_up,
+                                                     uint32_t* e_out = nullptr, float* w_out = nullptr) {
+    bool ok = true;
+    float lg[kPer];
+    uint32_t key[kPer];                                           // orderable score, 0: not selectable
+    constexpr int kFly = kPer < 8 ? kPer : 4;                     // records in flight
+    #pragma unroll
+    for (int h0 = 0; h0 < kPer; h0 += kFly) {
+        uint4 rec[kFly];
+        #pragma unroll
+        for (int h = 0; h < kFly; ++h) {
+            const uint32_t e = lane + 32u * (h0 + h);
+            if (e < static_cast<uint32_t>(q.E)) rec[h] = ld_volatile_v4(reinterpret_cast<const uint8_t*>(q.logits) + (static_cast<size_t>(t) * q.E + e) * 16u);
+        }
+        #pragma unroll
+        for (int h = 0; h < kFly; ++h) {
+            const uint32_t e = lane + 32u * (h0 + h);
+            lg[h0 + h] = 0.f; key[h0 + h] = 0u;
+            if (e < static_cast<uint32_t>(q.E)) {
+                float v;
+                if (flag == 0u || (rec[h].y == flag && rec[h].w == flag)) v = bf16_round(__uint_as_float(rec[h].x) + __uint_as_float(rec[h].z)) + 0.0f;
+                else v = fe_read_logit(q, t, e, flag, ok, give_up);
+                const float s = (q.score_mode == 1 ? (1.0f / (1.0f + expf(-v))) + q.bias[e] : v) + 0.0f;
+                lg[h0 + h] = v;
+                if (s != -INFINITY) key[h0 + h] = orderable_f32(s);
+            }
+        }
+    }
+    if (!__all_sync(0xffffffffu, ok)) return false;
+    uint32_t top = 0u, top_h = 0u;                                // this lane's best score and the first of its experts that has it
+    float top_v = 0.f;
+    auto rescan = [&]() {
+        top = 0u;
+        #pragma unroll
+        for (uint32_t h = 0; h < kPer; ++h) if (key[h] > top) { top = key[h]; top_h = h; top_v = lg[h]; }
+    };
+    rescan();
+    uint32_t chosen = 0xFFFFFFFFu;
+    float v_sel = -INFINITY;
+    #pragma unroll 1
+    for (uint32_t k = 0; k < 8; ++k) {
+        const uint32_t best = __reduce_max_sync(0xffffffffu, top);
+        const uint32_t e = __reduce_min_sync(0xffffffffu, best != 0u && top == best ? lane + 32u * top_h : 0xFFFFFFFFu);
+        const float v = __shfl_sync(0xffffffffu, top_v, e & 31u);
+        if (e != 0xFFFFFFFFu) {
+            if (lane == k) { chosen = e; v_sel = v; }
+            if ((e & 31u) == lane) {
+                #pragma unroll
+                for (uint32_t h = 0; h < kPer; ++h) if (h == (e >> 5)) key[h] = 0u;
+                rescan();
+            }
+        }
+        __syncwarp();
+    }
+    const bool empty_slot = chosen == 0xFFFFFFFFu;
+    float wgt;
+    if (q.score_mode == 1) {
+        const float s = lane < 8 ? 1.0f / (1.0f + expf(-v_sel)) : 0.f;
+        float sum = 0.f;
+        #pragma unroll
+        for (int k = 0; k < 8; ++k) sum += __shfl_sync(0xffffffffu, s, k);
+        wgt = s / sum;
+    } else {
+        float mx = v_sel;
+        #pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const float ex = lane < 8 ? expf(v_sel - mx) : 0.f;
+        float sum = 0.f;
+        #pragma unroll
+        for (int k = 0; k < 8; ++k) sum += __shfl_sync(0xffffffffu, ex, k);
+        wgt = ex / sum;
+    }
+    if (lane < 8) {
+        const bool live = nonzero && !empty_slot;
+        const float w = live ? wgt : 0.f;
+        if (records != nullptr)
+            asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %4};"
+                     :: "l"(records + (static_cast<size_t>(t) * 8u + lane) * 16u), "r"(live ? chosen : 0xFFFFFFFFu), "r"(flag), "r"(__float_as_uint(w)), "r"(flag) : "memory");
+        if (e_out != nullptr) { *e_out = live ? chosen : 0xFFFFFFFFu; *w_out = w; }
+        if (q.topk_idx != nullptr) {
+            q.topk_idx[static_cast<size_t>(t) * 8 + lane] = live ? static_cast<long long>(chosen) : -1ll;
+            q.topk_w[static_cast<size_t>(t) * 8 + lane] = w;
+        }
+    }
+    return true;
+}
+
+// The stand-alone frontend, two launches. First the partial logits and, by the last warps of the grid, the tokens'
+// quantisation (it needs no logits); then one warp per token for the selection. The second launch starts early and waits on
+// the device, so its launch latency is hidden behind the first.
+constexpr int kFeThreads = 512;
+__global__ void __launch_bounds__(kFeThreads, 1) frontend_logits_kernel(const __grid_constant__ FeParams q) {
+    const uint32_t lane = threadIdx.x & 31u, nwarps = gridDim.x * (kFeThreads / 32), w = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;   // (consecutive items on different SMs)
+    grid_dependency_wait();
+    grid_launch_dependents();
+    #pragma unroll 1
+    for (uint32_t t = nwarps - 1u - w; t < static_cast<uint32_t>(q.T); t += nwarps)
+        fe_quant_token(q.hidden + static_cast<size_t>(t) * q.H, q.H, q.fmt, q.x_gs, q.x + static_cast<size_t>(t) * q.x_row_bytes,
+                       q.x_sf + static_cast<size_t>(t) * q.x_sf_row_bytes, lane);
+    const uint32_t eb = fe_expert_block(q, gridDim.x);
+    if (eb == 1u) fe_logits_blocks<1, 3>(q, w, nwarps, lane, 1u);
+    else if (eb == 2u) fe_logits_blocks<2, 2>(q, w, nwarps, lane, 1u);
+    else fe_logits_blocks<4, 2>(q, w, nwarps, lane, 1u);
+}
+
+template <int kPer>
+__global__ void __launch_bounds__(32) frontend_select_kernel(const __grid_constant__ FeParams q) {
+    const uint32_t lane = threadIdx.x, t = blockIdx.x;
+    grid_dependency_wait();
+    grid_launch_dependents();
+    const bool nonzero = fe_row_nonzero(q.hidden + static_cast<size_t>(t) * q.H, q.H, lane);
+    fe_select_token_regs<kPer>(q, t, nonzero, lane, 0u, nullptr, [] { return false; });
 }
 
 }  // namespace mm

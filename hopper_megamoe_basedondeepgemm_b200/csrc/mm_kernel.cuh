@@ -85,6 +85,7 @@ enum : uint32_t {
     kKnobEarlyCombine = 4u,             // warps start on the combine as soon as their role ends
     kKnobRehearse = 8u,                 // idle role warps run their code once on made-up tasks before the roles start
     kKnobWaitProfile = 32u,             // the roles add up the cycles they spend waiting; totals replace the per-unit landing times in the SM records
+    kKnobDecode = 64u,                  // one rank, at most 16 routing entries: the decode kernel (csrc/mm_decode.cuh)
     kKnobTileImages = 16u               // launches with more than 16 received rows: operand tiles prepared in global memory, fetched by bulk copies
 };
 
@@ -1900,7 +1901,7 @@ __global__ void __launch_bounds__(kA8 ? kThreads + kNumExpThreads : kThreads, 1)
     //      and no arrival counter in between: the selecting warps wait for exactly the values they read.
     if constexpr (kFe) {
         const uint32_t fe_flag = epoch + 1u;
-        fe_logits_items(p.fe, bid * (kNT / 32) + warp, G * (kNT / 32), lane, fe_flag);
+        fe_logits_items(p.fe, warp * G + bid, G * (kNT / 32), lane, fe_flag);            // (consecutive items on different SMs)
         if (dispatching) {                       // (every dispatching SM selects all tokens: it needs the whole routing for its row list)
             float* sc = reinterpret_cast<float*>(smem + p.sm_act) + warp * 2 * p.fe.E;
             auto give_up = [&]() -> bool {

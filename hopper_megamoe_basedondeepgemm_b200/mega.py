@@ -5,6 +5,7 @@ sm_100a library behind the C ABI of `include/megamoe_b200.h`. PyTorch supplies d
 the symmetric-memory rendezvous only.
 """
 import ctypes
+import weakref
 from types import SimpleNamespace
 from typing import Optional, Tuple
 
@@ -16,6 +17,12 @@ from .quant import SF_VEC, interleave_gate_up, pretile_weights
 
 def _align(x: int, y: int) -> int:
     return (x + y - 1) // y * y
+
+
+def _current_stream() -> int:
+    """Raw handle of the current device's current stream (what `torch.cuda.current_stream().cuda_stream` gives, without
+    building the stream object: a call of the layer pays for it every time)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def get_token_alignment_for_mega_moe() -> int:
@@ -82,6 +89,12 @@ class SymmBuffer:
             self.group.barrier()
         torch.cuda.synchronize()
         self._peer_array = (ctypes.c_void_p * self.num_ranks)(*self.buffer_ptrs)
+        # launch arguments with everything that is the same in every call; a call copies them and fills in the rest
+        self._args_template = bytes(_lib.MMLaunchArgs(self.buffer.data_ptr(), self._peer_array, None, None, None, 0, _lib.ENGINE['umma'],
+                                                      None, -1.0, 1, 1.0, 1.0, 1.0, 1.0, 0.0, None))
+        self._cfg_ref = ctypes.byref(self.cfg)
+        self._fe_workspace_bytes = fe_workspace_bytes(self)
+        self._weights_seen = None                      # weak references to the weight tensors checked last
         L, t = self.layout, num_max_tokens_per_rank
         vec = int(L.sf_vec)
 
@@ -242,7 +255,7 @@ class SymmBuffer:
         if self.num_ranks > 1:
             self.group.barrier()
         _lib.check(lib.mm_reset(ctypes.byref(self.cfg), self.buffer.data_ptr(),
-                                torch.cuda.current_stream().cuda_stream), 'reset')
+                                _current_stream()), 'reset')
         torch.cuda.synchronize()
         if self.num_ranks > 1:
             self.group.barrier()
@@ -252,14 +265,14 @@ class SymmBuffer:
         lib = _lib.load()
         words = (ctypes.c_uint32 * 16)()
         st = lib.mm_read_device_status(ctypes.byref(self.cfg), self.buffer.data_ptr(), words,
-                                       torch.cuda.current_stream().cuda_stream)
+                                       _current_stream())
         return st, list(words)
 
     def phase_stamps(self):
         lib = _lib.load()
         stamps = (ctypes.c_uint64 * 32)()
         _lib.check(lib.mm_read_phase_stamps(ctypes.byref(self.cfg), self.buffer.data_ptr(), stamps,
-                                            torch.cuda.current_stream().cuda_stream), 'phase_stamps')
+                                            _current_stream()), 'phase_stamps')
         return list(stamps)
 
     def sm_phases(self):
@@ -268,7 +281,7 @@ class SymmBuffer:
         lib = _lib.load()
         out = (ctypes.c_uint64 * (256 * 32))()
         _lib.check(lib.mm_read_sm_phases(ctypes.byref(self.cfg), self.buffer.data_ptr(), out,
-                                         torch.cuda.current_stream().cuda_stream), 'sm_phases')
+                                         _current_stream()), 'sm_phases')
         return torch.tensor(list(out), dtype=torch.int64).view(256, 32)
 
     def destroy(self):
@@ -318,7 +331,7 @@ def nvfp4_global_scale(t: torch.Tensor) -> float:
         t = t.clone()                                     # (a view that starts inside a 16 B word: the kernel loads 16 B at a time)
     out = torch.zeros(1, dtype=torch.float32, device=t.device)
     _lib.check(_lib.load().mm_tensor_absmax(t.data_ptr(), 1 if t.dtype == torch.bfloat16 else 0, t.numel(), out.data_ptr(),
-                                            torch.cuda.current_stream().cuda_stream), 'nvfp4_global_scale')
+                                            _current_stream()), 'nvfp4_global_scale')
     return float(out.item()) / (6.0 * 448.0)
 
 
@@ -355,7 +368,7 @@ def transform_weights_for_mega_moe(l1_weights: Tuple[torch.Tensor, torch.Tensor]
         out = torch.empty((e, n // 128, (kh * 2) // 256, int(geo.unit_bytes)), dtype=torch.uint8, device=w.device)
         _lib.check(lib.mm_transform_weights(w.data_ptr(), sf.data_ptr(), int(sf.dtype == torch.float32), sf.stride(0),
                                             sf.stride(1), sf.stride(2), e, n, kh * 2, vec, int(interleave), out.data_ptr(),
-                                            torch.cuda.current_stream().cuda_stream), 'transform_weights_for_mega_moe')
+                                            _current_stream()), 'transform_weights_for_mega_moe')
         return out, shape
     return one(l1_weights, True), one(l2_weights, False)
 
@@ -371,37 +384,68 @@ def _input_region_ptr(sym_buffer: 'SymmBuffer', host_inputs):
     return host_inputs.data_ptr()
 
 
-def _launch(y, l1_weights, l2_weights, sym_buffer: SymmBuffer, stats, recipe, activation, activation_clamp, fast_math,
-            engine='umma', global_scales=(1.0, 1.0, 1.0, 1.0), timeout_ms=0.0, host_inputs=None):
-    lib = _lib.load(check=(engine == 'check'))          # the cross-check engine lives in the test build of the library
-    if activation != 'swiglu':
-        raise RuntimeError('only the swiglu activation is supported')
-    b = sym_buffer
+def _check_weights(b: SymmBuffer, w1, s1, w2, s2) -> None:
+    """The weight streams fit the buffer. Their tensors are remembered (weakly), so that the calls of a layer whose
+    weights stay the same compare four references."""
     vec = b.act_sf_vec_size or 32        # FP8 tokens carry one UE8M0 scale per 32 elements, like the MXFP4 weights
-    if tuple(recipe) != (1, 1, vec):
-        raise RuntimeError(f'recipe {recipe} does not match the buffer format {b.act_format}')
-    if y.dtype != torch.bfloat16 or y.dim() != 2 or y.size(1) != b.hidden or not y.is_contiguous() or \
-            not (y.is_cuda or y.is_pinned()):
-        raise RuntimeError('y must be a contiguous bf16 [num_tokens, hidden] tensor')
-    if y.size(0) > b.num_max_tokens_per_rank:
-        raise RuntimeError('more tokens than the buffer was created for')
     e_local = b.num_experts // b.num_ranks
-    (w1, s1), (w2, s2) = l1_weights, l2_weights
     if w1.dtype != torch.uint8 or w1.dim() != 4 or w2.dtype != torch.uint8 or w2.dim() != 4:
         raise RuntimeError('weights must come from transform_weights_for_mega_moe')
     if s1.tolist() != [2 * b.intermediate_hidden, b.hidden, vec] or s2.tolist() != [b.hidden, b.intermediate_hidden, vec]:
         raise RuntimeError('weight shapes do not match the buffer')
     if w1.size(0) != e_local or w2.size(0) != e_local or not (w1.is_contiguous() and w2.is_contiguous()):
         raise RuntimeError('expected one contiguous weight stream per local expert')
-    if stats is not None and (stats.dtype != torch.int32 or stats.numel() != e_local):
+    b._weights_seen = tuple(weakref.ref(t) for t in (w1, s1, w2, s2))
+
+
+def _launch_args(b: SymmBuffer, y, w1, w2, stats, activation_clamp, fast_math, timeout_ms):
+    args = _lib.MMLaunchArgs.from_buffer_copy(b._args_template)
+    args.l1_weights, args.l2_weights = w1.data_ptr(), w2.data_ptr()
+    args.num_tokens = y.shape[0]
+    if args.num_tokens:
+        args.y = y.data_ptr()
+    if stats is not None:
+        args.cumulative_local_expert_recv_stats = stats.data_ptr()
+    if activation_clamp is not None:
+        args.activation_clamp = activation_clamp
+    if not fast_math:
+        args.fast_math = 0
+    if timeout_ms:
+        args.timeout_ms = timeout_ms
+    return args
+
+
+def _launch(y, l1_weights, l2_weights, sym_buffer: SymmBuffer, stats, recipe, activation, activation_clamp, fast_math,
+            engine='umma', global_scales=None, timeout_ms=0.0, host_inputs=None):
+    b = sym_buffer
+    if activation != 'swiglu':
+        raise RuntimeError('only the swiglu activation is supported')
+    if recipe is not None and tuple(recipe) != (1, 1, b.act_sf_vec_size or 32):
+        raise RuntimeError(f'recipe {recipe} does not match the buffer format {b.act_format}')
+    shape = y.shape
+    if y.dtype != torch.bfloat16 or len(shape) != 2 or shape[1] != b.hidden or not y.is_contiguous() or \
+            not (y.is_cuda or y.is_pinned()):
+        raise RuntimeError('y must be a contiguous bf16 [num_tokens, hidden] tensor')
+    if shape[0] > b.num_max_tokens_per_rank:
+        raise RuntimeError('more tokens than the buffer was created for')
+    (w1, s1), (w2, s2) = l1_weights, l2_weights
+    seen = b._weights_seen
+    if seen is None or seen[0]() is not w1 or seen[1]() is not s1 or seen[2]() is not w2 or seen[3]() is not s2:
+        _check_weights(b, w1, s1, w2, s2)
+    if stats is not None and (stats.dtype != torch.int32 or stats.numel() != b.num_experts // b.num_ranks):
         raise RuntimeError('cumulative_local_expert_recv_stats must be int32 [num_local_experts]')
-    args = _lib.MMLaunchArgs(
-        b.buffer.data_ptr(), b._peer_array, w1.data_ptr(), w2.data_ptr(), y.data_ptr() if y.numel() else None,
-        y.size(0), _lib.ENGINE[engine], stats.data_ptr() if stats is not None else None,
-        float(activation_clamp) if activation_clamp is not None else -1.0, int(bool(fast_math)),
-        *[float(g) for g in global_scales], float(timeout_ms), _input_region_ptr(b, host_inputs))
-    _lib.check(lib.mm_mega_moe_launch(ctypes.byref(b.cfg), ctypes.byref(args), torch.cuda.current_stream().cuda_stream),
-               'mega_moe launch')
+    args = _launch_args(b, y, w1, w2, stats, activation_clamp, fast_math, timeout_ms)
+    lib = _lib.load()
+    if engine != 'umma':
+        args.engine = _lib.ENGINE[engine]
+        lib = _lib.load(check=(engine == 'check'))      # the cross-check engine lives in the test build of the library
+    if global_scales is not None:
+        args.x_global_scale, args.l1_global_scale, args.l2_global_scale, args.mid_global_scale = global_scales
+    if host_inputs is not None:
+        args.input_region = _input_region_ptr(b, host_inputs)
+    status = lib.mm_mega_moe_launch(b._cfg_ref, args, _current_stream())
+    if status:
+        _lib.check(status, 'mega_moe launch')
 
 
 def fp4_fp4_mega_moe(y: torch.Tensor, l1_weights, l2_weights, sym_buffer: SymmBuffer,
@@ -422,9 +466,7 @@ def fp4_fp4_mega_moe(y: torch.Tensor, l1_weights, l2_weights, sym_buffer: SymmBu
     host tensor).
     """
     assert sym_buffer.act_format in ('mxfp4', 'nvfp4'), 'buffer must be created with act_format mxfp4/nvfp4'
-    if recipe is None:
-        recipe = (1, 1, sym_buffer.act_sf_vec_size)
-    assert recipe[2] == sym_buffer.act_sf_vec_size
+    assert recipe is None or recipe[2] == sym_buffer.act_sf_vec_size
     _launch(y, l1_weights, l2_weights, sym_buffer, cumulative_local_expert_recv_stats, recipe, activation,
             activation_clamp, fast_math, engine, (x_global_scale, l1_global_scale, l2_global_scale, mid_global_scale),
             timeout_ms, host_inputs)
@@ -444,7 +486,7 @@ def fp8_fp4_mega_moe(y: torch.Tensor, l1_weights, l2_weights, sym_buffer: SymmBu
     """
     assert sym_buffer.act_format == 'fp8', 'buffer must be created with act_format fp8'
     _launch(y, l1_weights, l2_weights, sym_buffer, cumulative_local_expert_recv_stats, recipe, activation,
-            activation_clamp, fast_math, engine, (1.0, 1.0, 1.0, 1.0), timeout_ms, host_inputs)
+            activation_clamp, fast_math, engine, None, timeout_ms, host_inputs)
 
 
 def mega_moe_from_hidden(y: torch.Tensor, hidden: torch.Tensor, router_weight: torch.Tensor, l1_weights, l2_weights,
@@ -462,23 +504,21 @@ def mega_moe_from_hidden(y: torch.Tensor, hidden: torch.Tensor, router_weight: t
     b = sym_buffer
     if hidden.dtype != torch.bfloat16 or router_weight.dtype != torch.bfloat16 or not hidden.is_contiguous():
         raise RuntimeError('hidden states and router weight must be contiguous bf16')
-    if hidden.size(0) != y.size(0) or hidden.size(1) != b.hidden or tuple(router_weight.shape) != (b.num_experts, b.hidden):
+    if hidden.shape != y.shape or hidden.shape[1] != b.hidden or router_weight.shape != (b.num_experts, b.hidden):
         raise RuntimeError('router shapes do not match the buffer')
-    if workspace.numel() * workspace.element_size() < fe_workspace_bytes(b):
+    if workspace.nbytes < b._fe_workspace_bytes:
         raise RuntimeError('frontend workspace too small')
     (w1, _), (w2, _) = l1_weights, l2_weights
-    stats = cumulative_local_expert_recv_stats
-    args = _lib.MMLaunchArgs(
-        b.buffer.data_ptr(), b._peer_array, w1.data_ptr(), w2.data_ptr(), y.data_ptr() if y.numel() else None,
-        y.size(0), _lib.ENGINE[engine], stats.data_ptr() if stats is not None else None,
-        float(activation_clamp) if activation_clamp is not None else -1.0, int(bool(fast_math)),
-        float(x_global_scale), float(l1_global_scale), float(l2_global_scale), float(mid_global_scale),
-        float(timeout_ms), None)
+    args = _launch_args(b, y, w1, w2, cumulative_local_expert_recv_stats, activation_clamp, fast_math, timeout_ms)
+    args.engine = _lib.ENGINE[engine]
+    args.x_global_scale, args.l1_global_scale, args.l2_global_scale, args.mid_global_scale = \
+        x_global_scale, l1_global_scale, l2_global_scale, mid_global_scale
     fe = _lib.MMFrontendArgs(hidden.data_ptr(), router_weight.data_ptr(),
                              expert_bias.data_ptr() if expert_bias is not None else None,
-                             hidden.size(0), score_mode, workspace.data_ptr(), float(x_global_scale))
-    _lib.check(lib.mm_mega_moe_from_hidden_launch(ctypes.byref(b.cfg), ctypes.byref(args), ctypes.byref(fe),
-                                                  torch.cuda.current_stream().cuda_stream), 'mega_moe_from_hidden')
+                             args.num_tokens, score_mode, workspace.data_ptr(), x_global_scale)
+    status = lib.mm_mega_moe_from_hidden_launch(b._cfg_ref, args, fe, _current_stream())
+    if status:
+        _lib.check(status, 'mega_moe_from_hidden')
 
 
 def set_tuning(**kwargs) -> None:
@@ -508,28 +548,32 @@ def fe_forward(hidden: torch.Tensor, router_weight: torch.Tensor, x: torch.Tenso
     """Router frontend with the reference's argument list (`sm100_b200/fe_sm100/fe_binding.cpp:8-28`): router GEMM,
     top-8 + softmax over the selected logits, and the token quantisation (mode 2 FP8 / 3 MXFP4 / 4 NVFP4), written into
     the given views (normally `sym_buffer.x / x_sf / topk_idx / topk_weights`). The checks are the reference's."""
-    lib = _lib.load()
     if hidden.dim() != 2 or hidden.dtype != torch.bfloat16 or not hidden.is_contiguous():
         raise RuntimeError('hidden must be a contiguous bf16 [m, h] tensor')
     if router_weight.dim() != 2 or router_weight.dtype != torch.bfloat16 or not router_weight.is_contiguous():
         raise RuntimeError('router_weight must be a contiguous bf16 [e, h] tensor')
     m, h = hidden.shape
-    e, topk = router_weight.size(0), topk_idx.size(1)
-    if router_weight.size(1) != h or not (1 <= m <= 64):
+    e, rh = router_weight.shape
+    ti, tw = topk_idx.shape, topk_weights.shape
+    topk = ti[1]
+    if rh != h or not (1 <= m <= 64):
         raise RuntimeError('router shapes do not match (1 <= m <= 64)')
     if topk_idx.dtype != torch.int64 or topk_weights.dtype != torch.float32:
         raise RuntimeError('topk_idx must be int64 and topk_weights float32')
-    if topk_idx.size(0) < m or topk_weights.size(0) < m or x.size(0) < m or x_sf.size(0) < m:
+    if ti[0] < m or tw[0] < m or x.shape[0] < m or x_sf.shape[0] < m:
         raise RuntimeError('output views hold fewer than m rows')
     row = h if mode == 2 else h // 2
     sf_row = h // (16 if mode == 4 else 32)
+    # (m rows of the routing views without gaps: as a whole they have none, or their rows are packed)
     if x.stride(0) * x.element_size() != row or x_sf.stride(0) * x_sf.element_size() != sf_row or \
-            not (topk_idx[:m].is_contiguous() and topk_weights[:m].is_contiguous()):
+            not ((topk_idx.is_contiguous() or topk_idx[:m].is_contiguous()) and
+                 (topk_weights.is_contiguous() or topk_weights[:m].is_contiguous())):
         raise RuntimeError('output views do not have the row strides of the activation format')
-    nbytes = workspace.numel() * workspace.element_size()
-    _lib.check(lib.mm_fe_forward(hidden.data_ptr(), router_weight.data_ptr(), x.data_ptr(), x_sf.data_ptr(),
-                                 topk_idx.data_ptr(), topk_weights.data_ptr(), workspace.data_ptr(), nbytes, m, h, e, topk,
-                                 int(mode), int(l2_persist), torch.cuda.current_stream().cuda_stream), 'fe_forward')
+    status = _lib.load().mm_fe_forward(hidden.data_ptr(), router_weight.data_ptr(), x.data_ptr(), x_sf.data_ptr(),
+                                       topk_idx.data_ptr(), topk_weights.data_ptr(), workspace.data_ptr(), workspace.nbytes,
+                                       m, h, e, topk, mode, l2_persist, _current_stream())
+    if status:
+        _lib.check(status, 'fe_forward')
 
 
 def fe_forward_into_buffer(hidden: torch.Tensor, router_weight: torch.Tensor, sym_buffer: SymmBuffer, workspace: torch.Tensor,
@@ -548,4 +592,4 @@ def fe_forward_into_buffer(hidden: torch.Tensor, router_weight: torch.Tensor, sy
                                expert_bias.data_ptr() if expert_bias is not None else None,
                                hidden.size(0), score_mode, workspace.data_ptr(), float(x_global_scale))
     _lib.check(lib.mm_frontend_launch(ctypes.byref(b.cfg), b.buffer.data_ptr(), ctypes.byref(args),
-                                      torch.cuda.current_stream().cuda_stream), 'fe_forward_into_buffer')
+                                      _current_stream()), 'fe_forward_into_buffer')

@@ -196,7 +196,8 @@ int mm_read_sm_phases(const mm_config_t* cfg, const void* buffer, uint64_t* out_
  * live expert's weights (L2 prefetch) as soon as it learns of the expert, 2 every SM lists the rows of this rank's own
  * tokens from topk_idx instead of waiting for the own-rank header line, 4 warps start the combine when their role ends,
  * 8 the token-staging warps rehearse their code on made-up tasks while the dispatch is in flight, 16 launches with more
- * than 16 received rows sort them into ready-made operand tiles in global memory and fetch a task's tokens by bulk copies. */
+ * than 16 received rows sort them into ready-made operand tiles in global memory and fetch a task's tokens by bulk copies
+ * (on one rank: by a kernel of their own), 32 wait profile, 64 launches of at most 16 routing entries on one rank take the decode kernel. */
 enum mm_tuning_key { MM_TUNE_KNOBS = 0, MM_TUNE_STAGES = 1 /* ring depth, 0 = default */,
                      MM_TUNE_PREFETCH_W1_EXPERTS = 2, MM_TUNE_PREFETCH_W2_EXPERTS = 3 /* experts prefetched per launch at most */,
                      MM_TUNE_ROW_CACHE = 4 /* 1: received rows are fetched into shared memory before the weight stream starts */,

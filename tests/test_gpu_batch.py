@@ -1,4 +1,4 @@
-"""The one-rank batch kernel (csrc/mm_batch.cuh) at the sizes where it can go wrong, against the CPU oracle: row counts around
+"""The one-rank kernels, batch (csrc/mm_batch.cuh) and decode (csrc/mm_decode.cuh), at the sizes where it can go wrong, against the CPU oracle: row counts around
 the 16-row groups and the tile limits (128 rows, 96 with E4M3 tokens), more tokens than SMs, masked slots, the largest
 launch, experts without rows. Tolerances are the layer's: relative RMSE 0.3 %, counts and slot maps exact."""
 import pytest
@@ -113,3 +113,86 @@ def test_layout_holds_the_packed_images():
         groups, tiles = (4096 + 15 * 64 + 15) // 16, 64 + 4096 // 64
         need = lambda units: units * (groups * 2048 * atoms + tiles * planes * 512)      # noqa: E731
         assert L.tile_capacity * L.token_tile_bytes >= need(12) and L.tile_capacity * L.mid_tile_bytes >= need(5)
+
+
+@pytest.mark.parametrize('fmt', ['mxfp4', 'nvfp4', 'fp8'])
+@pytest.mark.parametrize('e_local,topk,tokens,hidden,inter', [
+    (1, 1, 1, 512, 256),            # one row, one expert
+    (64, 8, 2, 1024, 256),          # sixteen rows, (almost) all on experts of their own
+    (16, 1, 16, 512, 512),          # one route per token
+    (2, 2, 8, 1536, 256),           # eight rows per expert
+    (20, 5, 3, 512, 2048),          # an odd entry count; an L2 task longer than an L1 task
+    (48, 8, 1, 3072, 1280),         # the benchmark's layer: remainder tiles split over the SMs
+])
+def test_decode_kernel(fmt, e_local, topk, tokens, hidden, inter):
+    """At most 16 routing entries on one rank (csrc/mm_decode.cuh), a few slots masked."""
+    y, stats, ref, buf, _ = run_layer(fmt, e_local, hidden, inter, topk, tokens, 'random', 'umma', seed=7 * tokens, std=0.02,
+                                      masked_ratio=0.15 if tokens > 1 else 0.0)
+    check_against_oracle(y, stats, ref, buf, fmt, inter)
+
+
+@pytest.mark.parametrize('num_sms', [3, 0])
+def test_decode_kernel_small_grid_masked_and_missing_expert(num_sms):
+    fmt, e, hidden, inter, topk, tokens = 'mxfp4', 6, 1024, 512, 4, 4
+    w, _, _ = O.make_expert_weights(e, hidden, inter, fmt, seed=50, std=0.05)
+    l1, l2 = mm.transform_weights_for_mega_moe(*U.to_operator_weights(w, fmt, 'cuda'))
+    buf = mm.get_symm_buffer_for_mega_moe(None, e, 16, topk, hidden, inter, act_format=fmt, num_sms=num_sms)
+    y = torch.empty((tokens, hidden), dtype=torch.bfloat16, device='cuda')
+    idx, tw = U.random_routing(tokens, e, topk, 51)
+    _, inp, sfb = U.make_rank_inputs(tokens, hidden, fmt, 52, idx, tw)
+    ref = O.moe_layer_reference([inp], [w], fmt, e, clamp=10.0)
+    for case in ('plain', 'masked', 'missing', 'plain'):
+        U.write_inputs(buf, inp, sfb)
+        if case == 'masked':
+            buf.topk_idx.fill_(-1)
+        if case == 'missing':
+            buf.topk_idx[1, 2] = e
+        mm.fp4_fp4_mega_moe(y.fill_(1.0), l1, l2, buf, activation_clamp=10.0, timeout_ms=300.0)
+        st, words = buf.device_status()
+        if case == 'missing':
+            assert st == 4 and (words[0] & 0xFF) == 9
+            buf.reset()
+        else:
+            assert st == 0
+        if case == 'plain':
+            assert O.rel_rmse(y.cpu(), ref.y[0]) <= REL_RMSE_TOL
+        if case == 'masked':
+            assert float(y.abs().max()) == 0.0
+
+
+@pytest.mark.parametrize('fmt', ['mxfp4', 'nvfp4', 'fp8'])
+@pytest.mark.parametrize('tokens', [1, 2, 3, 160])
+@pytest.mark.parametrize('score_mode', [0, 1])
+def test_from_hidden_states_in_the_decode_and_batch_kernels(fmt, tokens, score_mode):
+    """One and two tokens (decode kernel), three, and more tokens than SMs with four experts per logit block: routing exact,
+    the quantised views as the stand-alone frontend writes them, the layer's output against the oracle."""
+    e, hidden, inter = 64, 1024, 256
+    g = torch.Generator().manual_seed(60 + tokens)
+    x = torch.randn((tokens, hidden), generator=g).to(torch.bfloat16)
+    if tokens > 1:
+        x[1] = 0
+    wr = (torch.randn((e, hidden), generator=g) / hidden ** 0.5).to(torch.bfloat16)
+    bias = (0.3 * torch.rand(e, generator=g)) if score_mode else None
+    w, gs1, gs2 = O.make_expert_weights(e, hidden, inter, fmt, seed=61, std=0.02)
+    x_gs, mid_gs = (1.0 / 64.0, 1.0 / 512.0) if fmt == 'nvfp4' else (1.0, 1.0)
+    buf = mm.get_symm_buffer_for_mega_moe(None, e, tokens, 8, hidden, inter, act_format=fmt)
+    l1, l2 = mm.transform_weights_for_mega_moe(*U.to_operator_weights(w, fmt, 'cuda'))
+    ws = torch.zeros(mm.fe_workspace_bytes(buf), dtype=torch.uint8, device='cuda')
+    y = torch.empty((tokens, hidden), dtype=torch.bfloat16, device='cuda')
+    stats = torch.zeros(e, dtype=torch.int32, device='cuda')
+    bias_d = bias.cuda() if bias is not None else None
+    mm.mega_moe_from_hidden(y, x.cuda(), wr.cuda(), l1, l2, buf, ws, cumulative_local_expert_recv_stats=stats, activation_clamp=10.0,
+                            score_mode=score_mode, expert_bias=bias_d, x_global_scale=x_gs, l1_global_scale=gs1, l2_global_scale=gs2,
+                            mid_global_scale=mid_gs, timeout_ms=500.0)
+    st, words = buf.device_status()
+    assert st == 0, [hex(v) for v in words[:4]]
+    idx, tw = O.route_from_logits(O.router_logits_device_order(x, wr), x, 8, 'sigmoid_bias' if score_mode else 'softmax', bias)
+    assert torch.equal(buf.topk_idx[:tokens].cpu(), idx) and torch.allclose(buf.topk_weights[:tokens].cpu(), tw, rtol=2e-6, atol=1e-7)
+    fused = [t[:tokens].view(torch.uint8).clone() for t in (buf.x, buf.x_sf, buf.topk_weights)]
+    mm.fe_forward_into_buffer(x.cuda(), wr.cuda(), buf, ws, score_mode=score_mode, expert_bias=bias_d, x_global_scale=x_gs)
+    assert all(torch.equal(a, t[:tokens].view(torch.uint8)) for a, t in zip(fused, (buf.x, buf.x_sf, buf.topk_weights)))
+    q, sf, _ = O.quantise_tokens(x, fmt, rounding='rne', sf_rule='mul', global_scale=x_gs)
+    ref = O.moe_layer_reference([O.RankInput(q, sf, idx, tw)], [w], fmt, e, clamp=10.0, x_global_scale=x_gs, w1_global_scale=gs1,
+                                w2_global_scale=gs2, mid_global_scale=mid_gs)
+    assert torch.equal(stats.cpu(), ref.counts[0])
+    assert O.rel_rmse(y.cpu(), ref.y[0]) <= REL_RMSE_TOL
