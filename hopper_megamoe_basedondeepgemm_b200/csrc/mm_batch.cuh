@@ -25,6 +25,7 @@ namespace mm {
 
 constexpr int kBMaxRows = 4096;                    // routed rows of one launch
 constexpr int kBMaxTiles = 128;                    // token tiles of one launch (64 experts + rows beyond the tile limit)
+constexpr uint32_t kBColumnTasks = 4;              // L2 tasks per SM that are claimed column block by column block
 constexpr int kBTaskRing = 64;                     // claimed tasks of one SM that some role has still to see, at most
 constexpr int kBWStages = 12, kBRSlots = 12;       // at most: weight ring stages, token record slots
 constexpr int kBServiceWarps = 4;                  // weight loader, MMA issuer, record loader, spare
@@ -72,7 +73,7 @@ struct BShared {
     uint32_t tile_rows[kBMaxTiles];
     uint32_t tile_a16[kBMaxTiles];                 // 16-row groups of all tiles before this one
     uint32_t etile[kMaxLocalExperts];              // first tile of the expert
-    uint32_t task[kBTaskRing];                     // claimed L2 tasks: turn of the ring << 16 | tile << 8 | weight tile (0xFFFF: no more)
+    uint32_t task[kBTaskRing];                     // claimed tasks: turn of the ring << 16 | L2 << 15 | tile << 8 | weight tile (0xFFFF: no more)
     alignas(16) uint16_t wcnt[kBRankWarps][kMaxLocalExperts];  // routing entries per (ranking warp, expert), then the exclusive sums over the warps
     alignas(16) uint8_t ex[kBMaxRows];             // expert of every routing entry (0xFF: masked, 0xFE: no such expert)
     union {
@@ -179,23 +180,24 @@ __device__ __forceinline__ uint32_t b_uniform(uint32_t v) { return __shfl_sync(0
 // 1 / 2^(e - 127) for an exponent byte e in [1, 254], exact
 __device__ __forceinline__ float pow2_recip(uint32_t e) { return __uint_as_float(e == 254u ? 0x00400000u : (254u - e) << 23); }
 
-// Task `ti` of this SM: layer << 28 | tile << 8 | weight tile, ~0 past the last one (kBNoTask: the launch is being aborted). The L1 tasks are dealt round-robin;
-// the L2 tasks are claimed one by one by the weight loader (a slow SM takes fewer), which leaves them in a ring for the
-// other roles.
+// Task `ti` of this SM: layer << 28 | tile << 8 | weight tile, ~0 past the last one (kBNoTask: the launch is being aborted).
+// The L1 tasks are dealt round-robin up to the last full round but one; the others and the L2 tasks are claimed one by one
+// by the weight loader (a slow SM takes fewer), which leaves them in a ring for the other roles.
 constexpr uint32_t kBEnd = 0xFFFFFFFFu, kBNoTask = 0xFFFFFFFEu;
 struct BTasks {
     const BCtx& cx;
-    uint32_t my1;
+    uint32_t my1, dealt;                             // dealt tasks of this SM, and of all SMs
     __device__ __forceinline__ explicit BTasks(const BCtx& c_) : cx(c_) {
-        const uint32_t nt1 = c_.c.M * c_.p.n1;
-        my1 = blockIdx.x < nt1 ? udiv_small(nt1 - 1u - blockIdx.x, gridDim.x) + 1u : 0u;
+        const uint32_t G = gridDim.x, nt1 = c_.c.M * c_.p.n1, full = udiv_small(nt1, G);
+        my1 = full > 2u ? full - 1u : (blockIdx.x < nt1 ? 1u : 0u);
+        dealt = full > 2u ? (full - 1u) * G : (nt1 < G ? nt1 : G);
     }
-    __device__ __forceinline__ uint32_t l1(uint32_t ti) const {
-        const uint32_t t = blockIdx.x + ti * gridDim.x, m = udiv_small(t, cx.p.n1);
+    __device__ __forceinline__ uint32_t l1(uint32_t t) const {
+        const uint32_t m = udiv_small(t, cx.p.n1);
         return (m << 8) | (t - m * cx.p.n1);
     }
     __device__ __forceinline__ uint32_t get(uint32_t ti) const {
-        if (ti < my1) return l1(ti);
+        if (ti < my1) return l1(blockIdx.x + ti * gridDim.x);
         const uint32_t k = ti - my1, tag = (k / kBTaskRing + 1u) << 16;
         volatile uint32_t* slot = &cx.c.task[k % kBTaskRing];
         uint32_t v = *slot, it = 0;
@@ -205,7 +207,7 @@ struct BTasks {
             v = *slot;
         }
         __syncwarp();
-        return (v & 0xFFFFu) == 0xFFFFu ? kBEnd : (1u << 28) | (v & 0xFFFFu);
+        return (v & 0xFFFFu) == 0xFFFFu ? kBEnd : ((v & 0x8000u) << 13) | (v & 0x7FFFu);
     }
 };
 
@@ -217,32 +219,33 @@ __device__ void b_role_weights(const BCtx& cx, uint32_t lane) {
     uint8_t* ring = cx.smem + b_uniform(c.nr * c.slot_bytes);
     uint32_t it = 0, s = 0, ph = 0;
     BTasks tasks(cx);
-    // Order of the L2 tasks: the SMs with one L1 task less than the others get here an L1 task earlier, when only the first
-    // tiles' L1 outputs are complete: as many tiles as those SMs can work off meanwhile come first, tile by tile; the others
-    // follow column block by column block (the combine starts on a column block when all tiles have it).
-    uint32_t mA = 0, NA = 0, NT2 = 0;
+    // Order of the L2 tasks: tile by tile (the first tiles' L1 outputs are complete long before the last ones'), but the last
+    // tiles, kBColumnTasks tasks per SM of them, column block by column block: the combine starts on a column block when all
+    // tiles have it, beside the remaining ones.
+    const uint32_t NT1 = M * n1, NT2 = M * n2, tail = udiv_small(kBColumnTasks * G + n2 - 1u, n2), mA = tail < M ? M - tail : 0u, NA = mA * n2;
     uint32_t* claims = cx.col_counts(cx.par) + kBColCounters;
     uint32_t next = 0u;
     if (tasks.my1 == 0u && lane == 0) next = atomicAdd(claims, 1u);
     #pragma unroll 1
     for (uint32_t ti = 0;; ++ti) {
         uint32_t t;
-        if (ti < tasks.my1) t = tasks.l1(ti);
+        if (ti < tasks.my1) t = tasks.l1(blockIdx.x + ti * G);
         else {
-            const uint32_t k = ti - tasks.my1, q = __shfl_sync(0xffffffffu, next, 0);
-            if (k == 0u) {
-                const uint32_t r1 = M * n1 - udiv_small(M * n1, G) * G, target = udiv_small((r1 ? G - r1 : 0u) * udiv_small(p.k1, p.k2), n2);
-                mA = target < M ? target : M; NA = mA * n2; NT2 = M * n2;
+            const uint32_t k = ti - tasks.my1;
+            uint32_t q = __shfl_sync(0xffffffffu, next, 0) + tasks.dealt;
+            if (q < NT1) t = tasks.l1(q);
+            else {
+                q -= NT1;
+                t = 0xFFFFu;
+                if (q < NA) { const uint32_t m = udiv_small(q, n2); t = 0x8000u | (m << 8) | (q - m * n2); }
+                else if (q < NT2) { const uint32_t j = udiv_small(q - NA, M - mA); t = 0x8000u | ((mA + q - NA - j * (M - mA)) << 8) | j; }
             }
-            t = 0xFFFFu;
-            if (q < NA) { const uint32_t m = udiv_small(q, n2); t = (m << 8) | (q - m * n2); }
-            else if (q < NT2) { const uint32_t j = udiv_small(q - NA, M - mA); t = ((mA + q - NA - j * (M - mA)) << 8) | j; }
             if (lane == 0) *reinterpret_cast<volatile uint32_t*>(&c.task[k % kBTaskRing]) = ((k / kBTaskRing + 1u) << 16) | t;
             if (t == 0xFFFFu) {                              // (the epilogue groups look at every second task: both of the next two end there)
                 if (lane == 0) *reinterpret_cast<volatile uint32_t*>(&c.task[(k + 1u) % kBTaskRing]) = (((k + 1u) / kBTaskRing + 1u) << 16) | t;
                 break;
             }
-            t |= 1u << 28;
+            t = ((t & 0x8000u) << 13) | (t & 0x7FFFu);
         }
         if (ti + 1u >= tasks.my1 && lane == 0) next = atomicAdd(claims, 1u);     // (needed after this task: its latency is hidden)
         const uint32_t layer = t >> 28, e = c.tile_e[(t >> 8) & 0xFFFFu], j = t & 0xFFu;
