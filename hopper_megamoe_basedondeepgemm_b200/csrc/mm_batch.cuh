@@ -217,6 +217,7 @@ __device__ void b_role_weights(const BCtx& cx, uint32_t lane) {
     const BParams& p = cx.p; BShared& c = cx.c;
     const uint32_t nw = b_uniform(c.nw), step = kA8 ? 1u : b_uniform(c.spu), stage_bytes = step * p.unit_bytes, G = gridDim.x, n1 = p.n1, n2 = p.n2, M = b_uniform(c.M);
     uint8_t* ring = cx.smem + b_uniform(c.nr * c.slot_bytes);
+    const uint64_t policy = l2_evict_first_policy();
     uint32_t it = 0, s = 0, ph = 0;
     BTasks tasks(cx);
     // Order of the L2 tasks: tile by tile (the first tiles' L1 outputs are complete long before the last ones'), but the last
@@ -258,7 +259,7 @@ __device__ void b_role_weights(const BCtx& cx, uint32_t lane) {
             if (elect_one()) {
                 const uint32_t bytes = (units - u < step ? units - u : step) * p.unit_bytes;
                 mbar_arrive_expect_tx(full, bytes);
-                bulk_g2s(ring + static_cast<size_t>(s) * stage_bytes, src, bytes, full);
+                bulk_g2s_hint(ring + static_cast<size_t>(s) * stage_bytes, src, bytes, full, policy);
                 c.wissued = it + 1u;
                 if (it == 0u) {
                     reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlSmWFirst)[blockIdx.x] = globaltimer_ns();

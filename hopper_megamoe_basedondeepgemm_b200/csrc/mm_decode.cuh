@@ -80,6 +80,7 @@ struct DTasks {
 
 __device__ void d_role_weights(const DCtx& cx, uint32_t nw, uint8_t* ring) {
     const BParams& p = cx.p; DShared& c = cx.c;
+    const uint64_t policy = l2_evict_first_policy();
     uint32_t it = 0, s = 0, ph = 0;
     DTasks tasks(cx);
     #pragma unroll 1
@@ -93,7 +94,7 @@ __device__ void d_role_weights(const DCtx& cx, uint32_t nw, uint8_t* ring) {
             if (!cx.warp_wait(&c.wempty[s], ph ^ 1u, kErrWaitEmpty)) return;
             if (elect_one()) {
                 mbar_arrive_expect_tx(&c.wfull[s], p.unit_bytes);
-                bulk_g2s(ring + static_cast<size_t>(s) * p.unit_bytes, src, p.unit_bytes, &c.wfull[s]);
+                bulk_g2s_hint(ring + static_cast<size_t>(s) * p.unit_bytes, src, p.unit_bytes, &c.wfull[s], policy);
                 c.wissued = it + 1u;
                 if (it == 0u) {
                     reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlSmWFirst)[blockIdx.x] = globaltimer_ns();
