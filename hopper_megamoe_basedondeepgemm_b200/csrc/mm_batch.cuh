@@ -93,6 +93,23 @@ __device__ __forceinline__ void st_global_v8(void* p, const uint32_t (&v)[8]) {
                  ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
 }
 
+// The cold parts of failing and waiting are out of line and get what they need by value: were they members, the context would
+// have to live in memory, and every access through it after a barrier or a volatile access would go there again.
+__device__ __noinline__ void b_fail(uint8_t* ctrl, uint32_t* abort_flag, uint32_t code, uint32_t detail) {
+    atomicCAS(reinterpret_cast<uint32_t*>(ctrl + kCtrlStatus), 0u, code | (blockIdx.x << 8) | (detail << 16));
+    *reinterpret_cast<volatile uint32_t*>(abort_flag) = 1u;
+}
+__device__ __noinline__ bool b_wait_slow(uint64_t* bar, uint32_t parity, uint32_t code, uint32_t* abort_flag, uint64_t deadline, uint8_t* ctrl) {
+    uint32_t it = 0;
+    while (!mbar_try_wait(bar, parity)) {
+        if ((++it & 0xFFu) == 0u) {
+            if (*reinterpret_cast<volatile uint32_t*>(abort_flag) != 0u) return false;
+            if (globaltimer_ns() > deadline) { b_fail(ctrl, abort_flag, code, 0u); return false; }
+        }
+    }
+    return true;
+}
+
 // What the one-rank kernels share: abort flag, deadline, bounded waits, time records.
 struct BCore {
     const BParams& p;
@@ -101,10 +118,7 @@ struct BCore {
     uint64_t deadline;
     uint32_t par;
     __device__ __forceinline__ bool aborted() const { return *reinterpret_cast<volatile uint32_t*>(abort_flag) != 0u; }
-    __device__ __noinline__ void fail(uint32_t code, uint32_t detail = 0) const {
-        atomicCAS(reinterpret_cast<uint32_t*>(p.buf + p.off_ctrl + kCtrlStatus), 0u, code | (blockIdx.x << 8) | (detail << 16));
-        *reinterpret_cast<volatile uint32_t*>(abort_flag) = 1u;
-    }
+    __device__ __forceinline__ void fail(uint32_t code, uint32_t detail = 0) const { b_fail(p.buf + p.off_ctrl, abort_flag, code, detail); }
     __device__ __forceinline__ bool expired() const { return globaltimer_ns() > deadline; }
     // for polling loops: give up when the launch is aborted or its time has run out (looked at every 64th time)
     __device__ __forceinline__ bool give_up(uint32_t& spins, uint32_t code, uint32_t detail) const {
@@ -113,18 +127,8 @@ struct BCore {
         if (expired()) { fail(code, detail); return true; }
         return false;
     }
-    __device__ __noinline__ bool wait_slow(uint64_t* bar, uint32_t parity, uint32_t code) const {
-        uint32_t it = 0;
-        while (!mbar_try_wait(bar, parity)) {
-            if ((++it & 0xFFu) == 0u) {
-                if (aborted()) return false;
-                if (expired()) { fail(code); return false; }
-            }
-        }
-        return true;
-    }
     __device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity, uint32_t code) const {
-        return mbar_try_wait(bar, parity) ? true : wait_slow(bar, parity, code);
+        return mbar_try_wait(bar, parity) ? true : b_wait_slow(bar, parity, code, abort_flag, deadline, p.buf + p.off_ctrl);
     }
     __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, uint32_t code) const {
         return __all_sync(0xffffffffu, wait(bar, parity, code));
@@ -279,7 +283,7 @@ __device__ void b_role_records(const BCtx& cx) {
     const uint32_t lane = threadIdx.x & 31u, nr = b_uniform(c.nr), slot_bytes = b_uniform(c.slot_bytes), step = b_uniform(c.spu);
     const uint32_t* arrive = cx.arrive_set();
     uint32_t it = 0, s = 0, ph = 0;
-    uint32_t ready1[kBMaxTiles / 32] = {}, ready2[kBMaxTiles / 32] = {};
+    uint32_t ready = 0u, seen = ~0u;
     bool seen_l2 = false;
     BTasks tasks(cx);
     #pragma unroll 1
@@ -287,26 +291,22 @@ __device__ void b_role_records(const BCtx& cx) {
         const uint32_t t = tasks.get(ti);
         if (t >= kBNoTask) break;
         const uint32_t layer = t >> 28, m = (t >> 8) & 0xFFFFu;
-        // the tile is complete: L1 its rows, L2 the outputs of all L1 weight tiles. Looked up for the tile only when it is
-        // not yet known: `ready` remembers the tiles seen complete, 32 of them per lookup (one lane per tile)
-        uint32_t known = 0u;
-        #pragma unroll
-        for (uint32_t w = 0; w < kBMaxTiles / 32; ++w) if (w == (m >> 5)) known = layer ? ready2[w] : ready1[w];
-        if (((known >> (m & 31u)) & 1u) == 0u) {
+        // The tile is complete: L1 its rows, L2 the outputs of all L1 weight tiles. Looked up 32 tiles at a time, one lane per
+        // tile; the latest answer is kept, so that following tasks of the same tiles ask only while theirs is incomplete.
+        const uint32_t window = (m >> 5) | (layer << 8);
+        if (window != seen || ((ready >> (m & 31u)) & 1u) == 0u) {
             uint32_t spins = 0;
             for (;;) {
                 const uint32_t mm_ = (m & ~31u) + lane;
                 const bool r = mm_ < c.M && ld_acquire_gpu(arrive + layer * p.tile_capacity + mm_) >= (layer ? static_cast<uint32_t>(p.n1) : c.tile_rows[mm_]);
-                const uint32_t b = __ballot_sync(0xffffffffu, r);
-                #pragma unroll
-                for (uint32_t w = 0; w < kBMaxTiles / 32; ++w)
-                    if (w == (m >> 5)) { if (layer) ready2[w] = b; else ready1[w] = b; }
-                if ((b >> (m & 31u)) & 1u) break;
+                ready = __ballot_sync(0xffffffffu, r);
+                if ((ready >> (m & 31u)) & 1u) break;
                 if ((++spins & 0xFu) == 0u) {
                     if (cx.aborted()) return;
                     if (cx.expired()) { cx.fail(layer ? kErrWaitL1Done : kErrWaitDispatchFlag, c.tile_e[m]); return; }
                 }
             }
+            seen = window;
             fence_proxy_async_all();                         // rows written through the generic proxy, read by bulk copies
         }
         const uint32_t a16 = (c.tile_rows[m] + 15u) >> 4, rec = F::rec(a16), units = layer ? p.k2 : p.k1;
