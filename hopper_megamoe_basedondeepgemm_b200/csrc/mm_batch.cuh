@@ -342,7 +342,7 @@ __device__ void b_role_mma(const BCtx& cx, uint32_t lane) {
     // 580 cycles to issue from per-lane registers, 313 from uniform ones; the tensor pipe needs 256 of them.)
     const uint32_t nr = b_uniform(c.nr), slot_bytes = b_uniform(c.slot_bytes), step = b_uniform(c.spu), tm = b_uniform(c.tmem_base);
     const uint32_t rec0 = b_uniform(smem_u32(cx.smem)), ring0 = rec0 + nr * slot_bytes, x0 = ring0 + b_uniform(c.nw) * p.unit_bytes;
-    uint32_t it = 0, rs = 0, rph = 0, wsm0 = ring0, tok0 = rec0;        // units consumed; record slot (without widening also weight stage), its phase bit
+    uint32_t it = 0, rs = 0, rph = 0;                                   // units consumed; record slot (without widening also weight stage), its phase bit
     BTasks tasks(cx);
     #pragma unroll 1
     for (uint32_t ti = 0;; ++ti) {
@@ -353,46 +353,57 @@ __device__ void b_role_mma(const BCtx& cx, uint32_t lane) {
         const uint32_t idesc_n = kIdesc | ((atom >> 10) << 17);                       // N = rows, in units of 8
         const uint32_t rec = atom * F::kAtoms + kPlanes * 512u, acc = ti & 1u, use = (ti >> 1) & 1u, d = tm + acc * 128u;
         if (!cx.warp_wait(&c.tmem_empty[acc], use ^ 1u, kErrWaitTmemEmpty)) return;
-        tc_fence_after();
         #pragma unroll 1
-        for (uint32_t u = 0; u < units; u += step) {
+        for (uint32_t u = 0; u < units;) {
+            // Every turn of this loop costs about 450 cycles beside the 130 a unit takes to issue (barrier wait, fence, election,
+            // reconvergence), a unit 256 on the tensor pipe: a stage that is there already when the first is goes with it.
             if (!cx.warp_wait(&c.rfull[rs], rph, kErrWaitActsFull)) return;
-            #pragma unroll
-            for (uint32_t uu = 0; uu < 2; ++uu) {
-                if (uu < step && u + uu < units) {
-                    if constexpr (kA8) { if (!cx.warp_wait(&c.xfull[it & 1u], (it >> 1) & 1u, kErrWaitFull)) return; }
-                    if (uu == 0u || kA8) tc_fence_after();
-                    if (lane == 0 && it == 0u) cx.sm_phase(kSmFirstLanded);
-                    if (elect_one()) {
-                        const uint32_t wsm = kA8 ? x0 + (it & 1u) * kXbufBytes : wsm0 + uu * p.unit_bytes, tok = tok0 + uu * rec;
-                        const uint64_t adesc = smem_desc(wsm, 1024u, kLayoutSw128), bdesc = smem_desc(tok, 1024u, kLayoutSw128);
-                        const uint64_t asf = smem_desc(wsm + (kA8 ? 2u * kUnitWBytes : static_cast<uint32_t>(kUnitWBytes)), 128u, kLayoutNone);
-                        const uint64_t bsf = smem_desc(tok + atom * F::kAtoms, 128u, kLayoutNone);
-                        const uint32_t sfa = tm + 256u + (it & 1u) * 32u, sfb = sfa + 16u;
-                        #pragma unroll
-                        for (uint32_t pl = 0; pl < kPlanes; ++pl) {
-                            utccp_32x128b_warpx4(sfa + pl * 4u, asf + pl * 32u);
-                            utccp_32x128b_warpx4(sfb + pl * 4u, bsf + pl * 32u);
+            if constexpr (kA8) { if (!cx.warp_wait(&c.xfull[it & 1u], (it >> 1) & 1u, kErrWaitFull)) return; }
+            const uint32_t rs1 = rs + 1u == nr ? 0u : rs + 1u, rph1 = rs1 == 0u ? rph ^ 1u : rph;
+            bool more = u + step < units && mbar_test(&c.rfull[rs1], rph1);
+            if constexpr (kA8) more = more && mbar_test(&c.xfull[(it + 1u) & 1u], ((it + 1u) >> 1) & 1u);
+            const uint32_t n = __all_sync(0xffffffffu, more) ? 2u : 1u;
+            tc_fence_after();
+            if (lane == 0 && it == 0u) cx.sm_phase(kSmFirstLanded);
+            if (elect_one()) {
+                #pragma unroll 1
+                for (uint32_t b = 0; b < n; ++b) {
+                    const uint32_t slot = b ? rs1 : rs, tok0 = rec0 + slot * slot_bytes, wsm0 = ring0 + slot * (step * p.unit_bytes), u0 = u + b * step;
+                    #pragma unroll
+                    for (uint32_t uu = 0; uu < (kA8 ? 1u : 2u); ++uu) {
+                        if (uu < step && u0 + uu < units) {
+                            const uint32_t i = it + b * step + uu;
+                            const uint32_t wsm = kA8 ? x0 + (i & 1u) * kXbufBytes : wsm0 + uu * p.unit_bytes, tok = tok0 + uu * rec;
+                            const uint64_t adesc = smem_desc(wsm, 1024u, kLayoutSw128), bdesc = smem_desc(tok, 1024u, kLayoutSw128);
+                            const uint64_t asf = smem_desc(wsm + (kA8 ? 2u * kUnitWBytes : static_cast<uint32_t>(kUnitWBytes)), 128u, kLayoutNone);
+                            const uint64_t bsf = smem_desc(tok + atom * F::kAtoms, 128u, kLayoutNone);
+                            const uint32_t sfa = tm + 256u + (i & 1u) * 32u, sfb = sfa + 16u;
+                            #pragma unroll
+                            for (uint32_t pl = 0; pl < kPlanes; ++pl) {
+                                utccp_32x128b_warpx4(sfa + pl * 4u, asf + pl * 32u);
+                                utccp_32x128b_warpx4(sfb + pl * 4u, bsf + pl * 32u);
+                            }
+                            #pragma unroll
+                            for (uint32_t ks = 0; ks < kUnitK / kStepK; ++ks) {
+                                const uint32_t pl = (ks * kStepK) / (4u * F::kVec), sf_id = ((ks * kStepK) % (4u * F::kVec)) / F::kVec;
+                                const uint64_t ad = adesc + (ks & 3u) * 2u + (kA8 ? (ks >> 2) * (kUnitWBytes >> 4) : 0u);
+                                const uint64_t bd = bdesc + (ks & 3u) * 2u + (kA8 ? (ks >> 2) * (atom >> 4) : 0u);
+                                const uint32_t idesc = idesc_with_sf(idesc_n, sf_id, sf_id), accum = (u0 | uu | ks) != 0u ? 1u : 0u;
+                                if constexpr (kA8) umma_mxf8f6f4(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
+                                else if constexpr (kFmt == 0) umma_mxf4_block32(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
+                                else umma_nvf4_block16(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
+                            }
+                            if constexpr (kA8) tc_commit(&c.xempty[i & 1u]);
                         }
-                        #pragma unroll
-                        for (uint32_t ks = 0; ks < kUnitK / kStepK; ++ks) {
-                            const uint32_t pl = (ks * kStepK) / (4u * F::kVec), sf_id = ((ks * kStepK) % (4u * F::kVec)) / F::kVec;
-                            const uint64_t ad = adesc + (ks & 3u) * 2u + (kA8 ? (ks >> 2) * (kUnitWBytes >> 4) : 0u);
-                            const uint64_t bd = bdesc + (ks & 3u) * 2u + (kA8 ? (ks >> 2) * (atom >> 4) : 0u);
-                            const uint32_t idesc = idesc_with_sf(idesc_n, sf_id, sf_id), accum = (u | uu | ks) != 0u ? 1u : 0u;
-                            if constexpr (kA8) umma_mxf8f6f4(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
-                            else if constexpr (kFmt == 0) umma_mxf4_block32(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
-                            else umma_nvf4_block16(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
-                        }
-                        if constexpr (kA8) tc_commit(&c.xempty[it & 1u]);
-                        if (uu + 1u >= step || u + uu + 1u >= units) tc_commit(&c.rempty[rs]);
                     }
-                    __syncwarp();
-                    ++it;
+                    tc_commit(&c.rempty[slot]);
                 }
             }
-            wsm0 += step * p.unit_bytes; tok0 += slot_bytes;
-            if (++rs == nr) { rs = 0; rph ^= 1u; wsm0 = ring0; tok0 = rec0; }
+            __syncwarp();
+            const uint32_t done = n * step < units - u ? n * step : units - u;
+            u += n * step; it += done;
+            if (n == 2u) { rs = rs1; rph = rph1; }
+            if (++rs == nr) { rs = 0; rph ^= 1u; }
         }
         if (elect_one()) tc_commit(&c.tmem_full[acc]);
         __syncwarp();
