@@ -412,20 +412,20 @@ __device__ void b_role_mma(const BCtx& cx, uint32_t lane) {
 }
 
 // ============================================================================================= weight widener (E4M3 tokens)
-// kind::mxf8f6f4 reads 4-bit operands from byte-wide slots: every 16 E2M1 values (8 bytes) sit in a 16-byte slot. Eight warps
-// turn a packed unit (128 rows x 128 B) into two atoms of 128 rows x 128 B; two buffers, so that a unit is widened while the
-// one before it is multiplied. (All eight on one unit: with two groups on alternate units a buffer's round trip - widen,
-// multiply, barriers - took twice as long and was the bound.) Eight lanes read the eight chunks of a row and store the two
-// halves of each; the lanes of the second atom store theirs in the other order, so that the eight stores of a quarter-warp
-// fall on different banks.
+// kind::mxf8f6f4 reads 4-bit operands from byte-wide slots: every 16 E2M1 values (8 bytes) sit in a 16-byte slot. Two groups
+// of four warps take the units in turn and turn a packed unit (128 rows x 128 B) into two atoms of 128 rows x 128 B, each in a
+// buffer of its own: a group's barrier waits and its proxy fence (400 cycles of a unit's 1200) lie beside the other's copying.
+// Eight lanes read the eight chunks of a row and store the two halves of each; the lanes of the second atom store theirs in
+// the other order, so that the eight stores of a quarter-warp fall on different banks.
+constexpr uint32_t kBWidenThreads = kBExpWarps * 16;      // of one group
 struct BWiden {
-    static constexpr uint32_t kItems = kTileRows * 8 / (kBExpWarps * 32);
+    static constexpr uint32_t kItems = kTileRows * 8 / kBWidenThreads;
     uint4 v[kItems], sf;
     __device__ __forceinline__ void load(const uint8_t* wsm, uint32_t xtid) {
         const uint32_t ch = xtid & 7u;
         #pragma unroll
         for (uint32_t k = 0; k < kItems; ++k) {
-            const uint32_t r = k * (kBExpWarps * 4) + (xtid >> 3);
+            const uint32_t r = k * (kBWidenThreads / 8) + (xtid >> 3);
             v[k] = *reinterpret_cast<const uint4*>(wsm + r * 128u + ((ch ^ (r & 7u)) << 4));
         }
         if (xtid < 64u) sf = *reinterpret_cast<const uint4*>(wsm + kUnitWBytes + xtid * 16u);
@@ -434,7 +434,7 @@ struct BWiden {
         const uint32_t ch = xtid & 7u, at = ch >> 2, j = 2u * (ch & 3u);
         #pragma unroll
         for (uint32_t k = 0; k < kItems; ++k) {
-            const uint32_t r = k * (kBExpWarps * 4) + (xtid >> 3);
+            const uint32_t r = k * (kBWidenThreads / 8) + (xtid >> 3);
             uint8_t* row = xb + at * kUnitWBytes + r * 128u;
             const uint32_t first = (j + at) ^ (r & 7u), second = (j + 1u - at) ^ (r & 7u);
             *reinterpret_cast<uint4*>(row + (first << 4)) = at ? make_uint4(v[k].z, v[k].w, 0u, 0u) : make_uint4(v[k].x, v[k].y, 0u, 0u);
@@ -444,11 +444,11 @@ struct BWiden {
     }
 };
 
-__device__ void b_role_widen(const BCtx& cx, uint32_t xtid) {
+__device__ void b_role_widen(const BCtx& cx, uint32_t grp, uint32_t xtid) {
     const BParams& p = cx.p; BShared& c = cx.c;
     const uint32_t lane = xtid & 31u, nw = c.nw;
     uint8_t* ring = cx.smem + c.nr * c.slot_bytes;
-    uint8_t* x0 = ring + static_cast<size_t>(nw) * p.unit_bytes;
+    uint8_t* xb = ring + static_cast<size_t>(nw) * p.unit_bytes + grp * kXbufBytes;
     uint32_t it = 0, s = 0, ph = 0;
     BTasks tasks(cx);
     #pragma unroll 1
@@ -458,16 +458,19 @@ __device__ void b_role_widen(const BCtx& cx, uint32_t xtid) {
         const uint32_t units = (t >> 28) ? p.k2 : p.k1;
         #pragma unroll 1
         for (uint32_t u = 0; u < units; ++u, ++it) {
-            if (!cx.warp_wait(&c.wfull[s], ph, kErrWaitFull)) return;
-            BWiden w;
-            w.load(ring + static_cast<size_t>(s) * p.unit_bytes, xtid);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&c.wempty[s]);        // (the unit is in registers: its stage can be refilled)
-            if (!cx.warp_wait(&c.xempty[it & 1u], ((it >> 1) & 1u) ^ 1u, kErrWaitEmpty)) return;
-            w.store(x0 + (it & 1u) * kXbufBytes, xtid);
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&c.xfull[it & 1u]);
+            if ((it & 1u) == grp) {
+                // (the ring's depth is even: a stage always belongs to the same group, which sees every phase of its barrier)
+                if (!cx.warp_wait(&c.wfull[s], ph, kErrWaitFull)) return;
+                BWiden w;
+                w.load(ring + static_cast<size_t>(s) * p.unit_bytes, xtid);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&c.wempty[s]);    // (the unit is in registers: its stage can be refilled)
+                if (!cx.warp_wait(&c.xempty[grp], ((it >> 1) & 1u) ^ 1u, kErrWaitEmpty)) return;
+                w.store(xb, xtid);
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&c.xfull[grp]);
+            }
             if (++s == nw) { s = 0; ph ^= 1u; }
         }
     }
@@ -767,13 +770,13 @@ __device__ __forceinline__ void b_tiles(const BCtx& cx, uint32_t lane) {
         const uint32_t rec = (max16 ? max16 : 1u) * 2048u * F::kAtoms + F::kPlanes * 512u;
         const uint32_t room = p.smem_ring - (F::kA8 ? 2u * kXbufBytes : 0u), pair = p.unit_bytes + rec;
         const uint32_t spu = pair * 8u <= room ? 2u : 1u;
-        uint32_t nr = udiv_small(room, pair * spu);
-        nr = nr > kBRSlots ? kBRSlots : nr;
-        uint32_t nw = nr;
-        if (F::kA8) {                                        // single-unit weight stages in what the records leave
-            nw = udiv_small(room - nr * spu * rec, p.unit_bytes);
-            nw = nw > kBWStages ? kBWStages : nw;
+        uint32_t nr = udiv_small(room, pair * spu), nw = nr;
+        if (F::kA8) {                                        // single-unit weight stages (an even number) beside two or three records at least
+            nw = udiv_small(room - (rec > 12288u ? 2u : 3u) * rec, p.unit_bytes) & ~1u;
+            nr = udiv_small(room - nw * p.unit_bytes, rec);
         }
+        nr = nr > kBRSlots ? kBRSlots : nr;
+        if (!F::kA8) nw = nr;
         c.nr = nr; c.nw = nw; c.slot_bytes = rec * spu; c.spu = spu;
     }
 }
@@ -792,11 +795,11 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
     const uint32_t ww = warp - kBServiceWarps;
     // ---- what needs nothing of the launches before this one: it overlaps the end of the previous kernel in the stream
     if (warp == 2) {
-        if (lane < kBWStages) { mbar_init(&c.wfull[lane], 1); mbar_init(&c.wempty[lane], F::kA8 ? kBExpWarps : 1); }
+        if (lane < kBWStages) { mbar_init(&c.wfull[lane], 1); mbar_init(&c.wempty[lane], F::kA8 ? kBExpWarps / 2 : 1); }
         if (lane < kBRSlots) { mbar_init(&c.rfull[lane], F::kA8 ? 1 : 2); mbar_init(&c.rempty[lane], 1); }
         if (lane < 2) {
             mbar_init(&c.tmem_full[lane], 1); mbar_init(&c.tmem_empty[lane], 4);
-            mbar_init(&c.xfull[lane], kBExpWarps); mbar_init(&c.xempty[lane], 1);
+            mbar_init(&c.xfull[lane], kBExpWarps / 2); mbar_init(&c.xempty[lane], 1);
         }
         c.task[lane] = 0u; c.task[lane + 32] = 0u;
         mbar_fence_init();
@@ -1069,7 +1072,7 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
         else if (warp >= kBServiceWarps && warp < kBServiceWarps + kBEpiWarps)
             b_role_epilogue<kFmt, kFe>(cx, (warp - kBServiceWarps) >> 2, tid - 32u * kBServiceWarps - ((warp - kBServiceWarps) >> 2) * 128u);
         else if (warp >= kBServiceWarps + kBEpiWarps) {
-            if constexpr (F::kA8) b_role_widen(cx, tid - 32u * (kBServiceWarps + kBEpiWarps));
+            if constexpr (F::kA8) { const uint32_t x = tid - 32u * (kBServiceWarps + kBEpiWarps); b_role_widen(cx, x / kBWidenThreads, x % kBWidenThreads); }
         }
     }
     if (tid == 128) { cx.stamp_max(kStampLastTasksDone); cx.sm_phase(kSmTasksDone); if (bid == 0) cx.stamp(kStampTasksDone); }

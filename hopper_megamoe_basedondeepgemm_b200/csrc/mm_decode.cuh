@@ -170,11 +170,11 @@ __device__ void d_role_mma(const DCtx& cx, uint32_t lane, uint32_t nw_, uint32_t
     if (lane == 0 && it != 0u) cx.stamp_max(kStampLastWeight);
 }
 
-// the widening warps' loop (E4M3 tokens) over this kernel's tasks; the unit's work is the batch kernel's
-__device__ void d_role_widen(const DCtx& cx, uint32_t xtid, uint32_t nw, const uint8_t* ring) {
+// the widening warps' loop (E4M3 tokens) over this kernel's tasks; the unit's work and the two groups are the batch kernel's
+__device__ void d_role_widen(const DCtx& cx, uint32_t grp, uint32_t xtid, uint32_t nw, uint8_t* ring) {
     const BParams& p = cx.p; DShared& c = cx.c;
     const uint32_t lane = xtid & 31u;
-    uint8_t* x0 = const_cast<uint8_t*>(ring) + static_cast<size_t>(nw) * p.unit_bytes;
+    uint8_t* xb = ring + static_cast<size_t>(nw) * p.unit_bytes + grp * kXbufBytes;
     uint32_t it = 0, s = 0, ph = 0;
     DTasks tasks(cx);
     #pragma unroll 1
@@ -183,16 +183,18 @@ __device__ void d_role_widen(const DCtx& cx, uint32_t xtid, uint32_t nw, const u
         if (!t.valid) break;
         #pragma unroll 1
         for (uint32_t u = t.ub; u < t.ue; ++u, ++it) {
-            if (!cx.warp_wait(&c.wfull[s], ph, kErrWaitFull)) return;
-            BWiden w;
-            w.load(ring + static_cast<size_t>(s) * p.unit_bytes, xtid);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&c.wempty[s]);
-            if (!cx.warp_wait(&c.xempty[it & 1u], ((it >> 1) & 1u) ^ 1u, kErrWaitEmpty)) return;
-            w.store(x0 + (it & 1u) * kXbufBytes, xtid);
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&c.xfull[it & 1u]);
+            if ((it & 1u) == grp) {
+                if (!cx.warp_wait(&c.xempty[grp], ((it >> 1) & 1u) ^ 1u, kErrWaitEmpty)) return;
+                if (!cx.warp_wait(&c.wfull[s], ph, kErrWaitFull)) return;
+                BWiden w;
+                w.load(ring + static_cast<size_t>(s) * p.unit_bytes, xtid);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&c.wempty[s]);
+                w.store(xb, xtid);
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&c.xfull[grp]);
+            }
             if (++s == nw) { s = 0; ph ^= 1u; }
         }
     }
@@ -295,7 +297,9 @@ __device__ void d_role_epilogue(const DCtx& cx, uint32_t grp, uint32_t etid, uin
         for (uint32_t i = 0; i < kTileTokens; ++i) vt_w[i * kBVtStride] = __uint_as_float(raw[i]);
         if (ti < 2u && etid == 0u) cx.sm_phase(kSmFirstMmaDone);
         if (t.parts > 1u) {
-            // a part of a remainder tile: [part SM][row of the expert][weight row] flagged fp32 words; the group's first SM adds
+            // A part of a remainder tile: [part SM][row of the expert][weight row] flagged fp32 words; the group's first SM adds.
+            // (The multi-rank kernel leaves plain partial sums in this region. Read as a float a launch number is a denormal,
+            // which a sum of block-scaled products is only where the scales themselves have underflowed.)
             const uint32_t first = c.split_first;
             auto part_word = [&](uint32_t sm, uint32_t i) { return p.buf + p.off_red + ((static_cast<size_t>(sm) * kDEntries + i) * kTileRows + etid) * 8u; };
             if (blockIdx.x != first) {
@@ -471,10 +475,10 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
     nw = nw > kDStages ? kDStages : nw;
     // ---- what needs nothing of the launches before this one: it overlaps the end of the previous kernel in the stream
     if (warp == 2) {
-        if (lane < kDStages) { mbar_init(&c.wfull[lane], 1); mbar_init(&c.wempty[lane], F::kA8 ? kBExpWarps : 1); }
+        if (lane < kDStages) { mbar_init(&c.wfull[lane], 1); mbar_init(&c.wempty[lane], F::kA8 ? kBExpWarps / 2 : 1); }
         if (lane < 2) {
             mbar_init(&c.tmem_full[lane], 1); mbar_init(&c.tmem_empty[lane], 4);
-            mbar_init(&c.xfull[lane], kBExpWarps); mbar_init(&c.xempty[lane], 1);
+            mbar_init(&c.xfull[lane], kBExpWarps / 2); mbar_init(&c.xempty[lane], 1);
             mbar_init(&c.tile_full[lane], kDEpiWarps);
         }
         mbar_fence_init();
@@ -640,7 +644,7 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
             if (lane == 0) { mbar_arrive(&c.tile_full[0]); cx.sm_phase(kSmRowsCached); }
             d_role_epilogue<kFmt>(cx, (warp - kEW) >> 2, (tid - 32u * kEW) & 127u, smem, flag);
         } else if (warp >= kEW + kDEpiWarps) {
-            if constexpr (F::kA8) d_role_widen(cx, tid - 32u * (kEW + kDEpiWarps), nw, smem + ring_off);
+            if constexpr (F::kA8) { const uint32_t x = tid - 32u * (kEW + kDEpiWarps); d_role_widen(cx, x / kBWidenThreads, x % kBWidenThreads, nw, smem + ring_off); }
         }
     }
     // ---- off the critical path: launch number, counters, stamps, and what others may inspect afterwards
