@@ -749,7 +749,7 @@ int mm_mega_moe_launch_static_scratch(const mm_config_t* cfg, const mm_static_ar
     MM_CUDA(cudaMemsetAsync(scratch + L.off_ctrl, 0, L.off_x - L.off_ctrl, s));
     MM_CUDA(cudaMemsetAsync(scratch + L.off_rx, 0, L.off_red - L.off_rx, s));
     MM_CUDA(cudaMemsetAsync(scratch + L.off_cnt, 0, L.off_token_tiles - L.off_cnt, s));
-    MM_CUDA(cudaMemsetAsync(scratch + L.off_arrive, 0, L.total_bytes - L.off_arrive, s));      // (the tile images need no clearing)
+    MM_CUDA(cudaMemsetAsync(scratch + L.off_arrive, 0, batch_out_offset(L) - L.off_arrive, s));      // (the tile images and the batch kernel's outputs need no clearing)
     const size_t t = static_cast<size_t>(a->num_tokens);
     if (t > 0) {
         MM_CUDA(cudaMemcpyAsync(scratch + L.off_x, a->x, t * L.x_row_bytes, cudaMemcpyDeviceToDevice, s));

@@ -206,7 +206,7 @@ int mm_set_tuning(int32_t key, int32_t value);
 int32_t mm_get_tuning(int32_t key);
 
 /* Bytes of the library's built-in working memory (one array per GPU, resident from library load to process exit). */
-#define MM_STATIC_SCRATCH_BYTES (16ll * 1024 * 1024)
+#define MM_STATIC_SCRATCH_BYTES (24ll * 1024 * 1024)
 
 typedef struct mm_static_args {
     const void* x;                   /* packed tokens [num_tokens][hidden / 2] (device) */
