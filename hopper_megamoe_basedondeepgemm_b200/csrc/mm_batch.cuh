@@ -80,7 +80,6 @@ struct BShared {
         uint16_t rank[kBMaxRows];                  // rank of the entry among those of its expert in its ranking warp (until the rows are placed)
         float vt[2][kTileTokens * kBVtStride];     // 16 tokens' accumulators of a task, per epilogue group (see b_role_epilogue)
     };
-    uint8_t nonzero[kFeMaxFusedTokens];            // launches from hidden states: is this SM's k-th token all zeros (1) or not (2)
     uint16_t ef[2][128];                           // per epilogue group: routing entry and top-k weight of the task's rows
     float ew[2][128];
     uint16_t rowf[kBMaxRows];                      // routing entry (token * topk + slot) of every row, experts one after the other
@@ -806,7 +805,6 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
     }
     if (warp == 1) { tmem_alloc(&c.tmem_base, 512); tmem_relinquish(); tc_fence_before(); }
     if (warp < kBRankWarps) reinterpret_cast<uint32_t*>(c.wcnt[warp])[lane] = 0u;
-    if (kFe && tid < kFeMaxFusedTokens) c.nonzero[tid] = 0;
     grid_dependency_wait();
     grid_launch_dependents();
     const unsigned long long t_first = globaltimer_ns();
@@ -869,9 +867,8 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
             #pragma unroll 1
             for (uint32_t k = warp - half_warps; k < ntok; k += half_warps) {
                 const uint32_t tok = bid + k * G;
-                const bool nz = fe_quant_token(p.fe.hidden + static_cast<size_t>(tok) * p.H, p.H, kFmt, p.fe.x_gs, p.buf + p.off_x + static_cast<size_t>(tok) * p.x_row_bytes,
-                                               p.buf + p.off_x_sf + static_cast<size_t>(tok) * p.x_sf_row_bytes, lane);
-                if (lane == 0) *reinterpret_cast<volatile uint8_t*>(&c.nonzero[k]) = nz ? 2 : 1;
+                fe_quant_token(p.fe.hidden + static_cast<size_t>(tok) * p.H, p.H, kFmt, p.fe.x_gs, p.buf + p.off_x + static_cast<size_t>(tok) * p.x_row_bytes,
+                               p.buf + p.off_x_sf + static_cast<size_t>(tok) * p.x_sf_row_bytes, lane);
             }
         }
         const uint32_t eb = fe_expert_block(p.fe, G);
@@ -881,10 +878,10 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
         if (warp < half_warps) {
             #pragma unroll 1
             for (uint32_t k = warp; k < ntok; k += half_warps) {
-                uint32_t spins = 0;
-                uint8_t nz;
-                while ((nz = *reinterpret_cast<volatile uint8_t*>(&c.nonzero[k])) == 0 && !((++spins & 0x3Fu) == 0u && give_up())) { }
-                if (!fe_select_token_regs<2>(p.fe, bid + k * G, nz == 2, lane, flag, p.buf + p.off_routes, give_up)) break;
+                // the row is looked at here once more: the quantising warp would know 1.6 us
+                // later (96 tokens of 3072, 128 experts: 77.3 -> 75.7 us a pass)
+                const bool nz = fe_row_nonzero(p.fe.hidden + static_cast<size_t>(bid + k * G) * p.H, p.H, lane);
+                if (!fe_select_token_regs<2>(p.fe, bid + k * G, nz, lane, flag, p.buf + p.off_routes, give_up)) break;
             }
         }
         #pragma unroll 1

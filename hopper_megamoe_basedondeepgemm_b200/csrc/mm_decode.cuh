@@ -565,20 +565,21 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
                 }
             }
         }
-        if (warp == 2 || warp == 3) {
+        // (warp 1, which has nothing to do yet, runs the selection once on whatever records lie there and drops the result: the
+        // SM then has the code in its instruction cache when the records arrive)
+        if (warp >= 1u && warp <= 3u) {
             auto give_up = [&]() -> bool {
                 if (cx.aborted()) return true;
                 if (cx.expired()) { cx.fail(kErrWaitFrontend); return true; }
                 return false;
             };
-            const uint32_t tok = warp - 2u;
+            const bool dry = warp == 1u;
+            const uint32_t tok = dry ? 0u : warp - 2u;
             if (tok < static_cast<uint32_t>(p.T)) {
                 const bool nz = fe_row_nonzero(p.fe.hidden + static_cast<size_t>(tok) * p.H, p.H, lane);
-                FeParams q = p.fe;
-                if (bid != tok) { q.topk_idx = nullptr; q.topk_w = nullptr; }          // one SM writes the token's routing views
                 uint32_t ce; float cw;
-                const bool ok = fe_select_token_regs<2>(q, tok, nz, lane, flag, nullptr, give_up, &ce, &cw);
-                if (lane < 8u) { c.ent_e[tok * 8u + lane] = ok ? ce : 0xFFu; c.ent_w[tok * 8u + lane] = ok ? cw : 0.f; }
+                const bool ok = fe_select_token_regs<2>(p.fe, tok, nz, lane, dry ? 0u : flag, nullptr, give_up, !dry && bid == tok, &ce, &cw);   // (one SM writes the token's routing views)
+                if (lane < 8u && !dry) { c.ent_e[tok * 8u + lane] = ok ? ce : 0xFFu; c.ent_w[tok * 8u + lane] = ok ? cw : 0.f; }
             }
         }
         __syncthreads();

@@ -363,14 +363,20 @@ __device__ __forceinline__ bool fe_select_token(const FeParams& q, uint32_t t, f
 // and order of additions as `fe_select_token` (maximum of the scores, then the smallest expert with it, eight times); a lane
 // keeps its best score at hand, so that a round is two warp reductions and a rescan by one lane. The routing goes into
 // topk_idx / topk_weights and, with `records`, as flagged 16 B records {expert (~0: none), flag, weight, flag} to where the
-// launch's other SMs poll it; `e_out` / `w_out` get lane k's route k (a null topk_idx: only those). `flag` 0: the logits are complete. Returns false if `give_up` ended a poll.
+// launch's other SMs poll it; `e_out` / `w_out` get lane k's route k (`publish` false: only those). `flag` 0: the logits are complete. Returns false if `give_up` ended a poll.
 template <int kPer, typename GiveUp>
 __device__ __forceinline__ bool fe_select_token_regs(const FeParams& q, uint32_t t, bool nonzero, uint32_t lane, uint32_t flag, uint8_t* records, GiveUp give_up,
-                                                     uint32_t* e_out = nullptr, float* w_out = nullptr) {
+                                                     bool publish = true, uint32_t* e_out = nullptr, float* w_out = nullptr) {
     bool ok = true;
     float lg[kPer];
     uint32_t key[kPer];                                           // orderable score, 0: not selectable
     constexpr int kFly = kPer < 8 ? kPer : 4;                     // records in flight
+    float bias[kPer];                                             // (fetched before the records are awaited: the load may come from HBM)
+    #pragma unroll
+    for (int h = 0; h < kPer; ++h) {
+        const uint32_t e = lane + 32u * h;
+        bias[h] = q.score_mode == 1 && e < static_cast<uint32_t>(q.E) ? __ldg(q.bias + e) : 0.f;
+    }
     #pragma unroll
     for (int h0 = 0; h0 < kPer; h0 += kFly) {
         uint4 rec[kFly];
@@ -387,7 +393,7 @@ __device__ __forceinline__ bool fe_select_token_regs(const FeParams& q, uint32_t
                 float v;
                 if (flag == 0u || (rec[h].y == flag && rec[h].w == flag)) v = bf16_round(__uint_as_float(rec[h].x) + __uint_as_float(rec[h].z)) + 0.0f;
                 else v = fe_read_logit(q, t, e, flag, ok, give_up);
-                const float s = (q.score_mode == 1 ? (1.0f / (1.0f + expf(-v))) + q.bias[e] : v) + 0.0f;
+                const float s = (q.score_mode == 1 ? (1.0f / (1.0f + expf(-v))) + bias[h0 + h] : v) + 0.0f;
                 lg[h0 + h] = v;
                 if (s != -INFINITY) key[h0 + h] = orderable_f32(s);
             }
@@ -440,11 +446,11 @@ __device__ __forceinline__ bool fe_select_token_regs(const FeParams& q, uint32_t
     if (lane < 8) {
         const bool live = nonzero && !empty_slot;
         const float w = live ? wgt : 0.f;
-        if (records != nullptr)
+        if (records != nullptr && publish)
             asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %4};"
                      :: "l"(records + (static_cast<size_t>(t) * 8u + lane) * 16u), "r"(live ? chosen : 0xFFFFFFFFu), "r"(flag), "r"(__float_as_uint(w)), "r"(flag) : "memory");
         if (e_out != nullptr) { *e_out = live ? chosen : 0xFFFFFFFFu; *w_out = w; }
-        if (q.topk_idx != nullptr) {
+        if (publish) {
             q.topk_idx[static_cast<size_t>(t) * 8 + lane] = live ? static_cast<long long>(chosen) : -1ll;
             q.topk_w[static_cast<size_t>(t) * 8 + lane] = w;
         }
