@@ -206,9 +206,6 @@ __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ void st_release_gpu(uint32_t* p, uint32_t v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 __device__ __forceinline__ uint32_t ld_volatile_u32(const void* p) {
     uint32_t v;
     asm volatile("ld.volatile.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -269,9 +266,6 @@ __device__ __forceinline__ bool ll_valid(const uint4& a, const uint4& b, uint32_
 }
 __device__ __forceinline__ uint4 ll_data(const uint4& a, const uint4& b) { return make_uint4(a.x, a.z, b.x, b.z); }
 
-__device__ __forceinline__ void st_global_v4(void* p, uint4 v) {
-    asm volatile("st.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
-}
 
 // ----------------------------------------------------------------------------- small integer division
 // a / b for a < 2^24, b > 0 and a / b < 2^21 (tile, unit, SM, token and chunk indices are far below that) through one
