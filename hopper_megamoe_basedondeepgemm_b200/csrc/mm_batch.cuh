@@ -416,20 +416,19 @@ __device__ void b_role_mma(const BCtx& cx, uint32_t lane) {
 }
 
 // ============================================================================================= weight widener (E4M3 tokens)
-// kind::mxf8f6f4 reads 4-bit operands from byte-wide slots: every 16 E2M1 values (8 bytes) sit in a 16-byte slot. Two groups
-// of four warps take the units in turn and turn a packed unit (128 rows x 128 B) into two atoms of 128 rows x 128 B, each in a
-// buffer of its own: a group's barrier waits and its proxy fence (400 cycles of a unit's 1200) lie beside the other's copying.
+// kind::mxf8f6f4 reads 4-bit operands from byte-wide slots: every 16 E2M1 values (8 bytes) sit in a 16-byte slot. kThreads
+// threads turn a packed unit (128 rows x 128 B) into two atoms of 128 rows x 128 B.
 // Eight lanes read the eight chunks of a row and store the two halves of each; the lanes of the second atom store theirs in
 // the other order, so that the eight stores of a quarter-warp fall on different banks.
-constexpr uint32_t kBWidenThreads = kBExpWarps * 16;      // of one group
+template <uint32_t kThreads>
 struct BWiden {
-    static constexpr uint32_t kItems = kTileRows * 8 / kBWidenThreads;
+    static constexpr uint32_t kItems = kTileRows * 8 / kThreads;
     uint4 v[kItems], sf;
     __device__ __forceinline__ void load(const uint8_t* wsm, uint32_t xtid) {
         const uint32_t ch = xtid & 7u;
         #pragma unroll
         for (uint32_t k = 0; k < kItems; ++k) {
-            const uint32_t r = k * (kBWidenThreads / 8) + (xtid >> 3);
+            const uint32_t r = k * (kThreads / 8) + (xtid >> 3);
             v[k] = *reinterpret_cast<const uint4*>(wsm + r * 128u + ((ch ^ (r & 7u)) << 4));
         }
         if (xtid < 64u) sf = *reinterpret_cast<const uint4*>(wsm + kUnitWBytes + xtid * 16u);
@@ -438,7 +437,7 @@ struct BWiden {
         const uint32_t ch = xtid & 7u, at = ch >> 2, j = 2u * (ch & 3u);
         #pragma unroll
         for (uint32_t k = 0; k < kItems; ++k) {
-            const uint32_t r = k * (kBWidenThreads / 8) + (xtid >> 3);
+            const uint32_t r = k * (kThreads / 8) + (xtid >> 3);
             uint8_t* row = xb + at * kUnitWBytes + r * 128u;
             const uint32_t first = (j + at) ^ (r & 7u), second = (j + 1u - at) ^ (r & 7u);
             *reinterpret_cast<uint4*>(row + (first << 4)) = at ? make_uint4(v[k].z, v[k].w, 0u, 0u) : make_uint4(v[k].x, v[k].y, 0u, 0u);
@@ -448,11 +447,14 @@ struct BWiden {
     }
 };
 
-__device__ void b_role_widen(const BCtx& cx, uint32_t grp, uint32_t xtid) {
+// All eight warps on one unit after the other: the next one is read from the ring while the tensor core has this one. (Two
+// groups of four on alternate units, which the decode kernel prefers, keep more of a unit in registers here and want an even
+// ring: 100 tokens 91.8 us, this way 90.9.)
+__device__ void b_role_widen(const BCtx& cx, uint32_t xtid) {
     const BParams& p = cx.p; BShared& c = cx.c;
     const uint32_t lane = xtid & 31u, nw = c.nw;
     uint8_t* ring = cx.smem + c.nr * c.slot_bytes;
-    uint8_t* xb = ring + static_cast<size_t>(nw) * p.unit_bytes + grp * kXbufBytes;
+    uint8_t* xb = ring + static_cast<size_t>(nw) * p.unit_bytes;
     uint32_t it = 0, s = 0, ph = 0;
     BTasks tasks(cx);
     #pragma unroll 1
@@ -462,19 +464,17 @@ __device__ void b_role_widen(const BCtx& cx, uint32_t grp, uint32_t xtid) {
         const uint32_t units = (t >> 28) ? p.k2 : p.k1;
         #pragma unroll 1
         for (uint32_t u = 0; u < units; ++u, ++it) {
-            if ((it & 1u) == grp) {
-                // (the ring's depth is even: a stage always belongs to the same group, which sees every phase of its barrier)
-                if (!cx.warp_wait(&c.wfull[s], ph, kErrWaitFull)) return;
-                BWiden w;
-                w.load(ring + static_cast<size_t>(s) * p.unit_bytes, xtid);
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&c.wempty[s]);    // (the unit is in registers: its stage can be refilled)
-                if (!cx.warp_wait(&c.xempty[grp], ((it >> 1) & 1u) ^ 1u, kErrWaitEmpty)) return;
-                w.store(xb, xtid);
-                fence_proxy_async_smem();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&c.xfull[grp]);
-            }
+            if (!cx.warp_wait(&c.wfull[s], ph, kErrWaitFull)) return;
+            BWiden<32 * kBExpWarps> w;
+            w.load(ring + static_cast<size_t>(s) * p.unit_bytes, xtid);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&c.wempty[s]);        // (the unit is in registers: its stage can be refilled)
+            const uint32_t b = it & 1u;
+            if (!cx.warp_wait(&c.xempty[b], ((it >> 1) & 1u) ^ 1u, kErrWaitEmpty)) return;
+            w.store(xb + b * kXbufBytes, xtid);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&c.xfull[b]);
             if (++s == nw) { s = 0; ph ^= 1u; }
         }
     }
@@ -775,8 +775,8 @@ __device__ __forceinline__ void b_tiles(const BCtx& cx, uint32_t lane) {
         const uint32_t room = p.smem_ring - (F::kA8 ? 2u * kXbufBytes : 0u), pair = p.unit_bytes + rec;
         const uint32_t spu = pair * 8u <= room ? 2u : 1u;
         uint32_t nr = udiv_small(room, pair * spu), nw = nr;
-        if (F::kA8) {                                        // single-unit weight stages (an even number) beside two or three records at least
-            nw = udiv_small(room - (rec > 12288u ? 2u : 3u) * rec, p.unit_bytes) & ~1u;
+        if (F::kA8) {                                        // single-unit weight stages beside two or three records at least
+            nw = udiv_small(room - (rec > 12288u ? 2u : 3u) * rec, p.unit_bytes);
             nr = udiv_small(room - nw * p.unit_bytes, rec);
         }
         nr = nr > kBRSlots ? kBRSlots : nr;
@@ -799,11 +799,11 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
     const uint32_t ww = warp - kBServiceWarps;
     // ---- what needs nothing of the launches before this one: it overlaps the end of the previous kernel in the stream
     if (warp == 2) {
-        if (lane < kBWStages) { mbar_init(&c.wfull[lane], 1); mbar_init(&c.wempty[lane], F::kA8 ? kBExpWarps / 2 : 1); }
+        if (lane < kBWStages) { mbar_init(&c.wfull[lane], 1); mbar_init(&c.wempty[lane], F::kA8 ? kBExpWarps : 1); }
         if (lane < kBRSlots) { mbar_init(&c.rfull[lane], F::kA8 ? 1 : 2); mbar_init(&c.rempty[lane], 1); }
         if (lane < 2) {
             mbar_init(&c.tmem_full[lane], 1); mbar_init(&c.tmem_empty[lane], 4);
-            mbar_init(&c.xfull[lane], kBExpWarps / 2); mbar_init(&c.xempty[lane], 1);
+            mbar_init(&c.xfull[lane], kBExpWarps); mbar_init(&c.xempty[lane], 1);
         }
         c.task[lane] = 0u; c.task[lane + 32] = 0u;
         mbar_fence_init();
@@ -1074,7 +1074,7 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
         else if (warp >= kBServiceWarps && warp < kBServiceWarps + kBEpiWarps)
             b_role_epilogue<kFmt, kFe>(cx, (warp - kBServiceWarps) >> 2, tid - 32u * kBServiceWarps - ((warp - kBServiceWarps) >> 2) * 128u);
         else if (warp >= kBServiceWarps + kBEpiWarps) {
-            if constexpr (F::kA8) { const uint32_t x = tid - 32u * (kBServiceWarps + kBEpiWarps); b_role_widen(cx, x / kBWidenThreads, x % kBWidenThreads); }
+            if constexpr (F::kA8) b_role_widen(cx, tid - 32u * (kBServiceWarps + kBEpiWarps));
         }
     }
     if (tid == 128) { cx.stamp_max(kStampLastTasksDone); cx.sm_phase(kSmTasksDone); if (bid == 0) cx.stamp(kStampTasksDone); }

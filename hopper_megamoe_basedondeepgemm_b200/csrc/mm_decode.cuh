@@ -22,6 +22,7 @@ constexpr uint32_t kDEntries = 16;                 // routing entries (= rows) o
 constexpr int kDEpiWarps = 8;                      // warps 4..11: build the token tiles, two epilogue groups
 constexpr int kDThreads = 32 * (4 + kDEpiWarps);
 constexpr int kDThreadsA8 = kDThreads + 32 * kBExpWarps;     // E4M3 tokens: widening warps 12..19
+constexpr uint32_t kDWidenThreads = kBExpWarps * 16;         // of one of their two groups
 constexpr int kDStages = 12;
 constexpr uint32_t kDBarGroups = 5, kDBarRouted = 6;
 
@@ -170,7 +171,10 @@ __device__ void d_role_mma(const DCtx& cx, uint32_t lane, uint32_t nw_, uint32_t
     if (lane == 0 && it != 0u) cx.stamp_max(kStampLastWeight);
 }
 
-// the widening warps' loop (E4M3 tokens) over this kernel's tasks; the unit's work and the two groups are the batch kernel's
+// The widening warps' loop (E4M3 tokens) over this kernel's tasks. Two groups of four warps take the units in turn, each into a
+// buffer of its own: a group's barrier waits and its proxy fence (400 cycles of a unit's 1200) lie beside the other's copying
+// (two tokens: 37.0 us a pass, 38.7 with all eight warps on one unit). The ring's depth is even: a stage always belongs to the
+// same group, which sees every phase of its barrier.
 __device__ void d_role_widen(const DCtx& cx, uint32_t grp, uint32_t xtid, uint32_t nw, uint8_t* ring) {
     const BParams& p = cx.p; DShared& c = cx.c;
     const uint32_t lane = xtid & 31u;
@@ -186,7 +190,7 @@ __device__ void d_role_widen(const DCtx& cx, uint32_t grp, uint32_t xtid, uint32
             if ((it & 1u) == grp) {
                 if (!cx.warp_wait(&c.xempty[grp], ((it >> 1) & 1u) ^ 1u, kErrWaitEmpty)) return;
                 if (!cx.warp_wait(&c.wfull[s], ph, kErrWaitFull)) return;
-                BWiden w;
+                BWiden<kDWidenThreads> w;
                 w.load(ring + static_cast<size_t>(s) * p.unit_bytes, xtid);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&c.wempty[s]);
@@ -645,7 +649,7 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
             if (lane == 0) { mbar_arrive(&c.tile_full[0]); cx.sm_phase(kSmRowsCached); }
             d_role_epilogue<kFmt>(cx, (warp - kEW) >> 2, (tid - 32u * kEW) & 127u, smem, flag);
         } else if (warp >= kEW + kDEpiWarps) {
-            if constexpr (F::kA8) { const uint32_t x = tid - 32u * (kEW + kDEpiWarps); d_role_widen(cx, x / kBWidenThreads, x % kBWidenThreads, nw, smem + ring_off); }
+            if constexpr (F::kA8) { const uint32_t x = tid - 32u * (kEW + kDEpiWarps); d_role_widen(cx, x / kDWidenThreads, x % kDWidenThreads, nw, smem + ring_off); }
         }
     }
     // ---- off the critical path: launch number, counters, stamps, and what others may inspect afterwards
