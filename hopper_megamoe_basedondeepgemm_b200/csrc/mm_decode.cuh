@@ -173,8 +173,9 @@ __device__ void d_role_mma(const DCtx& cx, uint32_t lane, uint32_t nw_, uint32_t
 
 // The widening warps' loop (E4M3 tokens) over this kernel's tasks. Two groups of four warps take the units in turn, each into a
 // buffer of its own: a group's barrier waits and its proxy fence (400 cycles of a unit's 1200) lie beside the other's copying
-// (two tokens: 37.0 us a pass, 38.7 with all eight warps on one unit). The ring's depth is even: a stage always belongs to the
-// same group, which sees every phase of its barrier.
+// (two tokens: 37.0 us a pass, 38.7 with all eight warps on one unit). A free buffer is awaited before the unit: it
+// says that the MMAs of the unit two before are over, so every earlier use of the stage (three or more units back) has landed
+// and been read. Whatever the depth of the ring, a group therefore never takes an older phase of the barrier for its own.
 __device__ void d_role_widen(const DCtx& cx, uint32_t grp, uint32_t xtid, uint32_t nw, uint8_t* ring) {
     const BParams& p = cx.p; DShared& c = cx.c;
     const uint32_t lane = xtid & 31u;
