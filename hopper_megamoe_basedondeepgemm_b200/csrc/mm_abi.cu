@@ -746,9 +746,18 @@ int mm_mega_moe_launch_static_scratch(const mm_config_t* cfg, const mm_static_ar
     // the array keeps the previous call's contents: the control block, the arrival flags and the split-tile counters
     // must start from zero (the launch counters restart with them, so every call runs as the buffer's first launch),
     // and with the counters every flagged word of the receive pool and the combine buffer
-    // (the split-tile partial sums between them are always written before they are read: not cleared)
+    // The multi-rank kernel always writes its split-tile partial sums between them before it reads them. The decode kernel polls
+    // its own there, flagged like the rest: [SM][row of the expert][weight row], rows below the number of routing entries.
     MM_CUDA(cudaMemsetAsync(scratch + L.off_ctrl, 0, L.off_x - L.off_ctrl, s));
     MM_CUDA(cudaMemsetAsync(scratch + L.off_rx, 0, L.off_red - L.off_rx, s));
+    const int64_t entries = static_cast<int64_t>(a->num_tokens) * cfg->num_topk;
+    if (entries > 0 && entries <= mm::kDEntries) {
+        int grid = 0;
+        st = grid_size(cfg, &grid);
+        if (st != MM_OK) return st;
+        constexpr size_t kRowBytes = mm::kTileRows * 8;
+        MM_CUDA(cudaMemset2DAsync(scratch + L.off_red, mm::kDEntries * kRowBytes, 0, static_cast<size_t>(entries) * kRowBytes, grid, s));
+    }
     MM_CUDA(cudaMemsetAsync(scratch + L.off_cnt, 0, L.off_token_tiles - L.off_cnt, s));
     MM_CUDA(cudaMemsetAsync(scratch + L.off_arrive, 0, batch_out_offset(L) - L.off_arrive, s));      // (the tile images and the batch kernel's outputs need no clearing)
     const size_t t = static_cast<size_t>(a->num_tokens);

@@ -60,6 +60,34 @@ def test_static_scratch_entry_matches_regular_entry_twice():
         assert O.rel_rmse(y.cpu(), ref.y[0]) <= 3e-3
 
 
+@pytest.mark.parametrize('fmt', ['mxfp4', 'nvfp4', 'fp8'])
+@pytest.mark.parametrize('e_local,topk,sizes', [(48, 8, [2, 1, 2, 1, 2]), (6, 3, [5, 1, 5, 3, 5])])
+def test_static_scratch_decode_launches_in_a_row(fmt, e_local, topk, sizes):
+    """Every call starts as the first launch of its memory, so nothing a call before it left there may carry that launch's
+    number: consecutive launches of the decode kernel (at most 16 routing entries), whose remainder tiles are shared by groups of
+    SMs, with other inputs, routings and magnitudes each time. Two layouts take turns in the array."""
+    lib = _lib.load()
+    hidden, inter, t_max = 1024, 512, 16
+    w, gs1, gs2 = O.make_expert_weights(e_local, hidden, inter, fmt, seed=72, std=0.05)
+    l1, l2 = mm.transform_weights_for_mega_moe(*U.to_operator_weights(w, fmt, 'cuda'))
+    stream = torch.cuda.current_stream().cuda_stream
+    for call, tokens in enumerate(sizes * 4):
+        cfg = _lib.MMConfig(1, 0, e_local, t_max + 16 * (call % 3 == 2), topk, hidden, inter, _lib.FMT[fmt], 0)
+        idx, tw = U.random_routing(tokens, e_local, topk, 500 + call)
+        x = (torch.randn((tokens, hidden), generator=torch.Generator().manual_seed(600 + call)) * (0.25, 1.0, 2.0)[call % 3]).to(torch.bfloat16)
+        q, sf, sfb = O.quantise_tokens(x, fmt, rounding='rne', sf_rule='mul', global_scale=1.0)
+        ref = O.moe_layer_reference([O.RankInput(q, sf, idx, tw)], [w], fmt, e_local, clamp=10.0, w1_global_scale=gs1, w2_global_scale=gs2)
+        x_d, sf_d, idx_d, tw_d = q.view(torch.int8).cuda(), sfb.contiguous().cuda(), idx.cuda(), tw.cuda()
+        y = torch.empty((tokens, hidden), dtype=torch.bfloat16, device='cuda')
+        status = torch.full((16,), 0xFFFF, dtype=torch.int32, device='cuda')
+        args = _lib.MMStaticArgs(x_d.data_ptr(), sf_d.data_ptr(), idx_d.data_ptr(), tw_d.data_ptr(), l1[0].data_ptr(), l2[0].data_ptr(),
+                                 y.data_ptr(), tokens, 1, None, 10.0, 1.0, gs1, gs2, 1.0, 500.0, status.data_ptr())
+        assert lib.mm_mega_moe_launch_static_scratch(ctypes.byref(cfg), ctypes.byref(args), stream) == 0, lib.mm_last_cuda_error().decode()
+        torch.cuda.synchronize()
+        assert int(status[0]) == 0, hex(int(status[0]))
+        assert O.rel_rmse(y.cpu(), ref.y[0]) <= 3e-3, (call, O.rel_rmse(y.cpu(), ref.y[0]))
+
+
 def test_static_scratch_entry_rejects_what_it_cannot_hold():
     lib = _lib.load()
     stream = torch.cuda.current_stream().cuda_stream
