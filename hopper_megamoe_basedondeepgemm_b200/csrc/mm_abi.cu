@@ -448,7 +448,7 @@ static mm::BParams one_rank_params(const mm_config_t* cfg, const mm::KParams& k)
     p.off_rx = k.off_rx; p.off_comb = k.off_comb; p.off_token_tiles = k.off_token_tiles; p.off_mid_tiles = k.off_mid_tiles; p.off_arrive = k.off_arrive;
     p.off_mid = k.off_mid; p.off_mid_sf = k.off_mid_sf; p.off_red = k.off_red;
     p.off_routes = batch_routes_offset(L); p.off_out = batch_out_offset(L);
-    p.rx_region = k.rx_region; p.tile_capacity = k.tile_capacity;
+    p.rx_region = k.rx_region; p.tile_capacity = k.tile_capacity; p.cap_rows = static_cast<uint32_t>(k.cap);
     p.fe = k.fe;
     p.timeout_ns = k.timeout_ns;
     return p;

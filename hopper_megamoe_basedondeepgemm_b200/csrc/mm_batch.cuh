@@ -58,7 +58,7 @@ struct BParams {
     __nv_bfloat16* y; int* stats;
     long long off_ctrl, off_x, off_x_sf, off_topk_idx, off_topk_w, off_rx, off_comb, off_token_tiles, off_mid_tiles, off_arrive;
     long long rx_region;
-    uint32_t tile_capacity;
+    uint32_t tile_capacity, cap_rows;              // token tiles the images, rows the receive pool and the images have room for
     long long off_routes, off_out;                 // [tokens][8] flagged routing records (launches from hidden states); [entries][H] bf16 expert outputs
     long long off_mid, off_mid_sf, off_red;        // flagged words of the decode kernel: intermediate rows, their scale bytes, partial sums
     uint32_t mid_row_bytes;
@@ -765,8 +765,10 @@ __device__ __forceinline__ void b_tiles(const BCtx& cx, uint32_t lane) {
         }
     }
     if (lane == 0) {
-        if (M > kBMaxTiles) cx.fail(kErrTaskCapacity, M);
         c.M = M; c.total = all & 0x1FFFu;
+        if (M > kBMaxTiles) cx.fail(kErrTaskCapacity, M);
+        // (a token that names an expert more than once: more rows than tokens x experts, for which there is no room)
+        if ((all & 0x1FFFu) > p.cap_rows) cx.fail(kErrMetaCapacity, (all & 0x1FFFu) >> 4);
         c.start_ok = cx.aborted() ? 0u : 1u;                 // (decided once: every warp takes the same way from here)
         // Rings. Weights and records of equal depth: a record from the L2 takes about as long as a unit from HBM while the
         // weights stream. A stage holds two K units where four such stages fit (narrow tiles): the MMA warp's barrier waits

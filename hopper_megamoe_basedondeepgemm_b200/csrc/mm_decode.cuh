@@ -431,6 +431,7 @@ __device__ __forceinline__ void d_route(const DCtx& cx, uint32_t e, float w, uin
     const BParams& p = cx.p; DShared& c = cx.c;
     const bool live = lane < n && e < kMaxLocalExperts;
     if (__any_sync(0xffffffffu, lane < n && e == 0xFEu)) { if (lane == 0) cx.fail(kErrWaitCombineFlag, 0xFFFFu); }   // a route to an expert that does not exist
+    if (static_cast<uint32_t>(__popc(__ballot_sync(0xffffffffu, live))) > p.cap_rows) { if (lane == 0) cx.fail(kErrMetaCapacity, 0u); }     // (more rows than the receive pool has room for)
     const uint32_t key = live ? e : 0xFFu;
     uint32_t below = 0u, pos = 0u, group = 0u;                       // rows of smaller experts, earlier rows of this one, smaller experts
     #pragma unroll

@@ -196,3 +196,35 @@ def test_from_hidden_states_in_the_decode_and_batch_kernels(fmt, tokens, score_m
                                 w2_global_scale=gs2, mid_global_scale=mid_gs)
     assert torch.equal(stats.cpu(), ref.counts[0])
     assert O.rel_rmse(y.cpu(), ref.y[0]) <= REL_RMSE_TOL
+
+
+@pytest.mark.parametrize('tokens,t_max', [(512, 512), (3, 16), (1, 1)])
+def test_more_rows_than_the_buffer_has_room_for_is_reported(tokens, t_max):
+    """A buffer has room for tokens x min(routes, experts) rows. Two experts, eight routes each of which names one of them: four
+    times as many rows (batch kernel; with one token of a buffer for one token the decode kernel) are refused on the device, as many
+    as there is room for (24 rows of 32 here) are served, and the buffer recovers."""
+    fmt, e, hidden, inter, topk = 'mxfp4', 2, 512, 256, 8
+    w, _, _ = O.make_expert_weights(e, hidden, inter, fmt, seed=71, std=0.05)
+    l1, l2 = mm.transform_weights_for_mega_moe(*U.to_operator_weights(w, fmt, 'cuda'))
+    buf = mm.SymmBuffer(None, e, t_max, topk, hidden, inter, act_format=fmt)
+    assert int(buf.layout.rx_cap_rows) == 2 * t_max
+    full = torch.arange(tokens * topk).reshape(tokens, topk) % e
+    weights = torch.full((tokens, topk), 0.125)
+    _, inp, sfb = U.make_rank_inputs(tokens, hidden, fmt, 72, full, weights)
+    y = torch.zeros((tokens, hidden), dtype=torch.bfloat16, device='cuda')
+    U.write_inputs(buf, inp, sfb)
+    before = buf.inputs.clone()
+    mm.fp4_fp4_mega_moe(y, l1, l2, buf, timeout_ms=500.0)
+    st, words = buf.device_status()
+    if tokens * topk <= 2 * t_max:
+        ref = O.moe_layer_reference([inp], [w], fmt, e, clamp=None)
+        assert st == 0 and O.rel_rmse(y.cpu(), ref.y[0]) <= REL_RMSE_TOL
+        return
+    assert st == 5 and (words[0] & 0xFF) == 10 and torch.equal(buf.inputs, before)
+    buf.reset()
+    inp.topk_idx[:, 2:] = -1                                       # one row per token and expert
+    ref = O.moe_layer_reference([inp], [w], fmt, e, clamp=None)
+    U.write_inputs(buf, inp, sfb)
+    for _ in range(2):
+        mm.fp4_fp4_mega_moe(y, l1, l2, buf, timeout_ms=500.0)
+        assert buf.device_status()[0] == 0 and O.rel_rmse(y.cpu(), ref.y[0]) <= REL_RMSE_TOL
