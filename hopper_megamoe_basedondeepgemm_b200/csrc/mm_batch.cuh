@@ -971,18 +971,21 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
     }
 
     const bool start = c.start_ok != 0u;
-    if (warp == 3 && start) {
+    if (warp == 3) {
         // the arrival counts of this launch's parity were cleared by the launch before it; clear the other set for the next one
+        // (also when this launch has failed: the set holds the counts of the launch before)
         uint32_t* other = reinterpret_cast<uint32_t*>(p.buf + p.off_arrive) + (cx.par ^ 1u) * 2u * p.tile_capacity;
         #pragma unroll 1
         for (uint32_t i = bid * 32u + lane; i < 2u * p.tile_capacity; i += G * 32u) other[i] = 0u;
         if (bid == 0) {
             cx.col_counts(cx.par ^ 1u)[lane] = 0u;
             cx.col_counts(cx.par ^ 1u)[lane + 32] = 0u;
-            #pragma unroll 1
-            for (uint32_t e = lane; e < static_cast<uint32_t>(p.E) && p.stats != nullptr; e += 32) p.stats[e] += static_cast<int>(c.cnt[e]);
-            // header line of the receive pool, for whoever inspects it afterwards
-            if (lane == 0) st_ll_16B(p.buf + p.off_rx + static_cast<size_t>(cx.par) * p.rx_region, make_uint4(c.total, 0u, 0u, 0u), epoch + 1u);
+            if (start) {
+                #pragma unroll 1
+                for (uint32_t e = lane; e < static_cast<uint32_t>(p.E) && p.stats != nullptr; e += 32) p.stats[e] += static_cast<int>(c.cnt[e]);
+                // header line of the receive pool, for whoever inspects it afterwards
+                if (lane == 0) st_ll_16B(p.buf + p.off_rx + static_cast<size_t>(cx.par) * p.rx_region, make_uint4(c.total, 0u, 0u, 0u), epoch + 1u);
+            }
         }
     }
     if (worker && start) {

@@ -228,3 +228,24 @@ def test_more_rows_than_the_buffer_has_room_for_is_reported(tokens, t_max):
     for _ in range(2):
         mm.fp4_fp4_mega_moe(y, l1, l2, buf, timeout_ms=500.0)
         assert buf.device_status()[0] == 0 and O.rel_rmse(y.cpu(), ref.y[0]) <= REL_RMSE_TOL
+
+
+@pytest.mark.parametrize('between', [20, 3])
+def test_a_launch_that_fails_at_routing_leaves_clean_counters(between):
+    """The launch after one that failed (a route to a missing expert, in a batch-size and in a decode-size launch) counts in the set
+    that the failed launch had to clear: its results are right without a reset. The status keeps the first failure."""
+    fmt, e, hidden, inter, topk, tokens = 'mxfp4', 4, 512, 256, 2, 20
+    w, l1, l2, buf, inp, sfb = _small_layer(fmt, e, hidden, inter, topk, tokens, 925)
+    y = torch.empty((tokens, hidden), dtype=torch.bfloat16, device='cuda')
+    for it in range(4):
+        idx, tw = U.random_routing(tokens, e, topk, 926 + it)
+        _, inp, sfb = U.make_rank_inputs(tokens, hidden, fmt, 930 + it, idx, tw)
+        ref = O.moe_layer_reference([inp], [w], fmt, e, clamp=None)
+        U.write_inputs(buf, inp, sfb)
+        mm.fp4_fp4_mega_moe(y, l1, l2, buf, timeout_ms=500.0)
+        torch.cuda.synchronize()
+        assert O.rel_rmse(y.cpu(), ref.y[0]) <= REL_RMSE_TOL, it
+        buf.topk_idx[1, 1] = e
+        mm.fp4_fp4_mega_moe(torch.empty((between, hidden), dtype=torch.bfloat16, device='cuda'), l1, l2, buf, timeout_ms=500.0)
+        st, words = buf.device_status()
+        assert st == 4 and (words[0] & 0xFF) == 9
