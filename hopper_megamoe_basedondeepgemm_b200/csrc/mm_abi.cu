@@ -442,7 +442,7 @@ static mm::BParams one_rank_params(const mm_config_t* cfg, const mm::KParams& k)
     p.tile_limit = cfg->act_format == MM_FMT_FP8 ? 96u : 128u;         // (E4M3: a wider record would leave too few weight stages beside the widened units)
     p.x_row_bytes = k.x_row_bytes; p.x_sf_row_bytes = k.x_sf_row_bytes; p.rx_row_bytes = k.rx_row_bytes; p.mid_row_bytes = k.mid_row_bytes;
     p.has_clamp = k.has_clamp; p.fast_math = k.fast_math; p.clamp = k.clamp;
-    p.l1_scale = k.l1_scale; p.l2_scale = k.l2_scale; p.mid_gs = k.mid_gs; p.mid_gs_recip = 1.0f / k.mid_gs;
+    p.l1_scale = k.l1_scale; p.l2_scale = k.l2_scale; p.mid_gs = k.mid_gs; p.mid_gs_recip = k.mid_gs >= 0x1p-40f && k.mid_gs <= 0x1p40f ? 1.0f / k.mid_gs : 0.f;
     p.buf = k.peer[k.rank]; p.w1 = k.w1; p.w2 = k.w2; p.y = k.y; p.stats = k.stats;
     p.off_ctrl = k.off_ctrl; p.off_x = k.off_x; p.off_x_sf = k.off_x_sf; p.off_topk_idx = k.off_topk_idx; p.off_topk_w = k.off_topk_w;
     p.off_rx = k.off_rx; p.off_comb = k.off_comb; p.off_token_tiles = k.off_token_tiles; p.off_mid_tiles = k.off_mid_tiles; p.off_arrive = k.off_arrive;

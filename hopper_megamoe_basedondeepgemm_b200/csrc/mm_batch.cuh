@@ -52,7 +52,7 @@ struct BParams {
     uint32_t unit_bytes, tile_limit;               // bytes of a streamed weight unit; rows of a token tile at most
     uint32_t x_row_bytes, x_sf_row_bytes, rx_row_bytes;
     int has_clamp, fast_math;
-    float clamp, l1_scale, l2_scale, mid_gs, mid_gs_recip;
+    float clamp, l1_scale, l2_scale, mid_gs, mid_gs_recip;         // (the reciprocal is 0 where `divide8` would not be exact)
     uint8_t* buf;
     const uint8_t* w1; const uint8_t* w2;
     __nv_bfloat16* y; int* stats;
@@ -483,8 +483,9 @@ __device__ void b_role_widen(const BCtx& cx, uint32_t xtid) {
 // ============================================================================================= epilogue
 // SwiGLU of 8 outputs of one token from its 8 gate and 8 up accumulators. With `fast_math` the reciprocal of 1 + exp(-gate)
 // is the hardware approximation refined by one Newton-Raphson step: straight-line code, several times faster than the
-// exact reciprocal with its range checks.
-__device__ __forceinline__ void b_swiglu(const BParams& p, const float (&a)[16], float wgt, float (&o)[8]) {
+// exact reciprocal with its range checks. (Compared with the correctly rounded reciprocal for every mantissa and the
+// exponents 0 to 125: no difference. Beyond, from a gate of -87.3 on, the approximation is zero: those take the other way.)
+__device__ __forceinline__ void b_swiglu(const BParams& p, const float (&a)[16], float wgt, bool live, float (&o)[8]) {
     float g[8], u[8];
     const bool cl = p.has_clamp != 0;
     #pragma unroll
@@ -495,10 +496,13 @@ __device__ __forceinline__ void b_swiglu(const BParams& p, const float (&a)[16],
         g[i] = cl ? gc : gate;
         u[i] = cl ? uc : up;
     }
-    if (p.fast_math) {
+    float least = 0.f;
+    #pragma unroll
+    for (uint32_t i = 0; i < 8; ++i) least = fminf(least, g[i]);
+    if (p.fast_math && (least >= -87.0f || !live)) {              // (the columns beyond the tile's rows hold anything)
         #pragma unroll
         for (uint32_t i = 0; i < 8; ++i) {
-            const float d = 1.0f + fminf(__expf(-g[i]), 1e38f);
+            const float d = 1.0f + __expf(-g[i]);
             float r = __fdividef(1.0f, d);
             r = fmaf(r, fmaf(-d, r, 1.0f), r);
             o[i] = g[i] * r * u[i] * wgt;
@@ -509,24 +513,36 @@ __device__ __forceinline__ void b_swiglu(const BParams& p, const float (&a)[16],
     }
 }
 // x / b from y = RN(1 / b): one residual correction of the product x * y gives the correctly rounded quotient (Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990), without a division's range checks
-__device__ __forceinline__ float div_by(float x, float b, float y) {
-    const float q = x * y;
-    return fmaf(fmaf(-q, b, x), y, q);
+// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990), without a division's range checks.
+// Its condition is that the residual is exact: with 2^-40 <= b <= 2^40 for quotients from 2^-40 up to the largest finite one.
+// Where one of the eight is something else - a zero, whose sign the residual loses, or an infinity - `divide8` divides them all.
+__device__ __forceinline__ void divide8(float (&o)[8], float b, float y) {
+    float lo = INFINITY, hi = 0.f, d[8];
+    #pragma unroll
+    for (uint32_t i = 0; i < 8; ++i) {
+        const float q = o[i] * y;
+        d[i] = fmaf(fmaf(-q, b, o[i]), y, q);
+        lo = fminf(lo, fabsf(q));
+        hi = fmaxf(hi, fabsf(q));
+    }
+    if (__builtin_expect(!(lo >= 0x1p-40f && hi < INFINITY), 0)) {
+        #pragma unroll
+        for (uint32_t i = 0; i < 8; ++i) d[i] = __fdiv_rn(o[i], b);
+    }
+    #pragma unroll
+    for (uint32_t i = 0; i < 8; ++i) o[i] = d[i];
 }
 
 // Requantises the 8 outputs of thread (n, q): o becomes the scaled values, the thread q = 0 gets the scale bytes of the
-// token's 64 columns in sfw (two bytes, one per 32 columns, or four). All lanes of the warp call it.
+// token's 64 columns in sfw (two bytes, one per 32 columns, or four). All lanes of the warp call it; `live`: the token is one.
 template <int kFmt>
-__device__ __forceinline__ void b_requantise(const BParams& p, float (&o)[8], uint32_t& sfw) {
+__device__ __forceinline__ void b_requantise(const BParams& p, float (&o)[8], bool live, uint32_t& sfw) {
     constexpr bool kA8 = BFmt<kFmt>::kA8;
     constexpr int kVec = BFmt<kFmt>::kVec;
     float amax = 0.f;
+    if constexpr (kVec == 16) { if (live) divide8(o, p.mid_gs, p.mid_gs_recip); }
     #pragma unroll
-    for (uint32_t i = 0; i < 8; ++i) {
-        if constexpr (kVec == 16) o[i] = div_by(o[i], p.mid_gs, p.mid_gs_recip);
-        amax = fmaxf(amax, fabsf(o[i]));
-    }
+    for (uint32_t i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(o[i]));
     // a scale block is the 8 columns of two (16 per block) or four threads
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
     if constexpr (kVec == 32) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
@@ -539,13 +555,11 @@ __device__ __forceinline__ void b_requantise(const BParams& p, float (&o)[8], ui
         for (uint32_t i = 0; i < 8; ++i) o[i] *= inv;
     } else {
         sf_byte = cvt_e4m3x2(__fdiv_rn(amax, 6.0f), 0.f) & 0xFFu;
-        const float sf = e4m3_to_float(sf_byte);
-        const bool zero = sf_byte == 0u;                          // a scale that rounds to zero: every non-zero value saturates
-        const float inv = zero ? 0.f : __frcp_rn(sf);
-        #pragma unroll
-        for (uint32_t i = 0; i < 8; ++i) {
-            const float qt = div_by(o[i], sf, inv), sat = o[i] == 0.f ? 0.f : copysignf(6.0f, o[i]);
-            o[i] = zero ? sat : qt;
+        if (sf_byte != 0u) {
+            if (live) { const float sf = e4m3_to_float(sf_byte); divide8(o, sf, __frcp_rn(sf)); }
+        } else {                                                  // a scale that rounds to zero: every non-zero value saturates
+            #pragma unroll
+            for (uint32_t i = 0; i < 8; ++i) o[i] = o[i] == 0.f ? 0.f : copysignf(6.0f, o[i]);
         }
     }
     // the token's scale bytes of this tile, gathered in the thread q = 0
@@ -617,9 +631,9 @@ __device__ void b_role_epilogue(const BCtx& cx, uint32_t grp, uint32_t etid) {
             const bool live = n < rows;
             if (layer == 0u) {
                 float o[8];
-                b_swiglu(p, a, live ? c.ew[grp][n] : 0.f, o);
+                b_swiglu(p, a, live ? c.ew[grp][n] : 0.f, live, o);
                 uint32_t sfw;
-                b_requantise<kFmt>(p, o, sfw);
+                b_requantise<kFmt>(p, o, live, sfw);
                 if (live) {
                     if constexpr (kA8) {
                         uint8_t* at = img + ((j >> 1) & 1u) * a16 * 2048u + sw128_off(n, (j & 1u) * 4u + (q >> 1)) + (q & 1u) * 8u;

@@ -345,8 +345,8 @@ __device__ void d_role_epilogue(const DCtx& cx, uint32_t grp, uint32_t etid, uin
         if (t.layer == 0u) {
             float o[8];
             uint32_t sfw;
-            b_swiglu(p, a, live ? c.col_w[n] : 0.f, o);
-            b_requantise<kFmt>(p, o, sfw);
+            b_swiglu(p, a, live ? c.col_w[n] : 0.f, live, o);
+            b_requantise<kFmt>(p, o, live, sfw);
             if (live) {
                 const size_t row = c.col_mid[n];
                 uint8_t* dst = p.buf + p.off_mid + row * 2u * p.mid_row_bytes + (t.j * 8u + q) * (kA8 ? 16u : 8u);

@@ -249,3 +249,72 @@ def test_a_launch_that_fails_at_routing_leaves_clean_counters(between):
         mm.fp4_fp4_mega_moe(torch.empty((between, hidden), dtype=torch.bfloat16, device='cuda'), l1, l2, buf, timeout_ms=500.0)
         st, words = buf.device_status()
         assert st == 4 and (words[0] & 0xFF) == 9
+
+
+def _exact_sum_weights(e, n, k, fmt, g):
+    """Random E2M1 codes under scales that are powers of two close together: every sum of products is exact, in any order."""
+    q = torch.randint(0, 256, (e, n, k // 2), generator=g).to(torch.uint8)
+    vec = 16 if fmt == 'nvfp4' else 32
+    sf = torch.randint(0, 3, (e, n, k // vec), generator=g)
+    words = (((sf + 5) * 8) if fmt == 'nvfp4' else sf + 120).to(torch.uint8).view(torch.int32)
+    sf_mn = torch.empty((e, words.shape[-1], n), dtype=torch.int32).permute(0, 2, 1)
+    sf_mn.copy_(words)
+    return q.view(torch.int8).cuda(), sf_mn.cuda()
+
+
+@pytest.mark.parametrize('tokens', [2, 23])                     # the decode and the batch kernel
+@pytest.mark.parametrize('fmt,weights,scales', [
+    ('mxfp4', 'plain', (1.0, 1.0, 1.0, 1.0)), ('mxfp4', 'odd', (1.0, 1.0, 1.0, 1.0)), ('fp8', 'plain', None), ('fp8', 'odd', None),
+    ('nvfp4', 'plain', (1.0 / 64, 1.0 / 64, 1.0, 1.0 / 512)),
+    ('nvfp4', 'plain', (1.0 / 64, 1.0 / 64, 1.0, 0.0123)),       # a divisor that is no power of two
+    ('nvfp4', 'plain', (1.0 / 64, 1.0 / 8, 1.0, 1e-3)),          # gates far below zero: outputs that are zeros of either sign
+    ('nvfp4', 'plain', (1.0 / 64, 0.22, 1.0, 1.0 / 512)),        # ... and about where exp(-gate) leaves fp32
+    ('nvfp4', 'plain', (1e10, 1e9, 1e-9, 1.0)),                  # outputs beyond fp32
+    ('nvfp4', 'plain', (1.0, 1e15, 1.0, 1e-15)),                 # quotients beyond fp32
+    ('nvfp4', 'plain', (1.0, 1.0, 1.0, 3e-39)), ('nvfp4', 'plain', (1.0, 1.0, 1.0, 1e38)),         # divisors without a normal reciprocal
+    ('nvfp4', 'plain', (1e-12, 1e-10, 1.0, 1e-20)),              # quotients around the smallest ones that are corrected
+    ('nvfp4', 'odd', (1.0 / 64, 1.0 / 64, 1.0, 1.0 / 512)),
+])
+@pytest.mark.parametrize('fast_math', [True, False])
+def test_intermediate_rows_equal_those_of_the_multi_rank_kernel(fmt, weights, scales, tokens, fast_math):
+    """The one-rank kernels' SwiGLU and requantisation take other instructions than the general kernel (a refined reciprocal, division by
+    a known divisor). From the same accumulators they give the same bytes, also for zeros, infinities and NaN."""
+    e, topk, hidden, inter = 8, 4, 512, 256
+    g = torch.Generator().manual_seed(80 + tokens)
+    l1, l2 = mm.transform_weights_for_mega_moe(_exact_sum_weights(e, 2 * inter, hidden, fmt, g), _exact_sum_weights(e, hidden, inter, fmt, g))
+    buf = mm.get_symm_buffer_for_mega_moe(None, e, 32, topk, hidden, inter, act_format=fmt)
+    idx, tw = U.random_routing(tokens, e, topk, 81)
+    if weights == 'odd':
+        special = torch.tensor([float('nan'), float('inf'), -float('inf'), 0.0, -0.0, -1e20, 1e-36, -1.0])
+        tw = special[torch.randint(0, len(special), tw.shape, generator=g)]
+    if fmt == 'fp8':
+        xq = torch.randint(-4, 5, (tokens, hidden), generator=g).float().to(torch.float8_e4m3fn).view(torch.uint8)
+        sfb = torch.full((tokens, hidden // 32), 127)
+    else:
+        xq = torch.randint(0, 256, (tokens, hidden // 2), generator=g).to(torch.uint8)
+        sfb = torch.full((tokens, hidden // 32), 121) if fmt == 'mxfp4' else torch.full((tokens, hidden // 16), 5 * 8)
+    lib, got = _lib.load(), []
+    knobs = lib.mm_get_tuning(_lib.TUNE['knobs'])
+    kw = dict(zip(('x_global_scale', 'l1_global_scale', 'l2_global_scale', 'mid_global_scale'), scales)) if scales else {}
+    try:
+        for k in (knobs, knobs & ~(16 | 64)):                    # (without the tile images and the decode kernel: the multi-rank kernel)
+            mm.set_tuning(knobs=k)
+            buf.x[:tokens].view(torch.uint8).copy_(xq)
+            buf.x_sf[:tokens].view(torch.uint8).copy_(sfb.to(torch.uint8))
+            buf.topk_idx[:tokens].copy_(idx)
+            buf.topk_weights[:tokens].copy_(tw)
+            y = torch.empty((tokens, hidden), dtype=torch.bfloat16, device='cuda')
+            (mm.fp8_fp4_mega_moe if fmt == 'fp8' else mm.fp4_fp4_mega_moe)(y, l1, l2, buf, fast_math=fast_math, timeout_ms=500.0, **kw)
+            assert buf.device_status()[0] == 0
+            recs = buf.received_records()[0]
+            rows, sf = buf.l2_acts_payload().cpu(), buf.l2_acts_sf_payload().cpu()[:, :inter // (16 if fmt == 'nvfp4' else 32)]
+            live, base = [], 0
+            for ex in range(e):
+                n = sum(1 for r in recs if r[0] == ex)
+                live += range(base, base + n)
+                base += (n + 15) // 16 * 16
+            got.append((y.view(torch.int16).cpu(), rows[live], sf[live]))
+    finally:
+        mm.set_tuning(knobs=knobs)
+    for a, b, what in zip(got[0], got[1], ('y', 'codes', 'scale bytes')):
+        assert a.shape == b.shape and torch.equal(a, b), (what, int((a != b).sum()), a.numel())
