@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
                 if (f < n) {
                     const uint32_t tok = f >> 3;                      // (eight routes per token)
                     const uint4* xrow = reinterpret_cast<const uint4*>(p.fe.hidden + static_cast<size_t>(tok) * p.H);
-                    const bool out = bid == tok && (f & 7u) == 0u;    // the token's row of the x / x_sf views
+                    const bool out = bid == (tok < G ? tok : 0u) && (f & 7u) == 0u;    // the token's row of the x / x_sf views (two tokens at most)
                     bool nz = false;
                     #pragma unroll
                     for (uint32_t u0 = 0; u0 < 16; u0 += 4) {
@@ -584,7 +584,7 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
             if (tok < static_cast<uint32_t>(p.T)) {
                 const bool nz = fe_row_nonzero(p.fe.hidden + static_cast<size_t>(tok) * p.H, p.H, lane);
                 uint32_t ce; float cw;
-                const bool ok = fe_select_token_regs<2>(p.fe, tok, nz, lane, dry ? 0u : flag, nullptr, give_up, !dry && bid == tok, &ce, &cw);   // (one SM writes the token's routing views)
+                const bool ok = fe_select_token_regs<2>(p.fe, tok, nz, lane, dry ? 0u : flag, nullptr, give_up, !dry && bid == (tok < G ? tok : 0u), &ce, &cw);   // (one SM writes the token's routing views)
                 if (lane < 8u && !dry) { c.ent_e[tok * 8u + lane] = ok ? ce : 0xFFu; c.ent_w[tok * 8u + lane] = ok ? cw : 0.f; }
             }
         }

@@ -318,3 +318,27 @@ def test_intermediate_rows_equal_those_of_the_multi_rank_kernel(fmt, weights, sc
         mm.set_tuning(knobs=knobs)
     for a, b, what in zip(got[0], got[1], ('y', 'codes', 'scale bytes')):
         assert a.shape == b.shape and torch.equal(a, b), (what, int((a != b).sum()), a.numel())
+
+
+@pytest.mark.parametrize('fmt', ['mxfp4', 'fp8'])
+@pytest.mark.parametrize('num_sms,tokens', [(1, 1), (1, 2), (2, 2), (1, 3)])
+def test_from_hidden_states_on_one_or_two_sms_fills_every_view(fmt, num_sms, tokens):
+    """The routing and the quantised tokens land in the buffer's views whatever the grid: fewer SMs than tokens, in both kernels."""
+    e, hidden, inter = 8, 512, 256
+    g = torch.Generator().manual_seed(90)
+    x = torch.randn((tokens, hidden), generator=g).to(torch.bfloat16).cuda()
+    wr = (torch.randn((e, hidden), generator=g) / hidden ** 0.5).to(torch.bfloat16).cuda()
+    w, _, _ = O.make_expert_weights(e, hidden, inter, fmt, seed=91, std=0.02)
+    l1, l2 = mm.transform_weights_for_mega_moe(*U.to_operator_weights(w, fmt, 'cuda'))
+    buf = mm.get_symm_buffer_for_mega_moe(None, e, 16, 8, hidden, inter, act_format=fmt, num_sms=num_sms)
+    ws = torch.zeros(mm.fe_workspace_bytes(buf), dtype=torch.uint8, device='cuda')
+    y = torch.empty((tokens, hidden), dtype=torch.bfloat16, device='cuda')
+    views = (buf.x, buf.x_sf, buf.topk_idx, buf.topk_weights)
+    for v in views:
+        v.view(torch.uint8).fill_(0x55)
+    mm.mega_moe_from_hidden(y, x, wr, l1, l2, buf, ws, timeout_ms=500.0)
+    assert buf.device_status()[0] == 0
+    got = [v[:tokens].view(torch.uint8).clone() for v in views]
+    mm.fe_forward_into_buffer(x, wr, buf, ws)
+    for a, v in zip(got, views):
+        assert torch.equal(a, v[:tokens].view(torch.uint8))
