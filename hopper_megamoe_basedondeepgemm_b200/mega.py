@@ -400,6 +400,7 @@ def _check_weights(b: SymmBuffer, w1, s1, w2, s2) -> None:
 
 def _launch_args(b: SymmBuffer, y, w1, w2, stats, activation_clamp, fast_math, timeout_ms):
     args = _lib.MMLaunchArgs.from_buffer_copy(b._args_template)
+    args.buffer = b.buffer.data_ptr()                    # (asked for in every call: a buffer that has been destroyed has none)
     args.l1_weights, args.l2_weights = w1.data_ptr(), w2.data_ptr()
     args.num_tokens = y.shape[0]
     if args.num_tokens:

@@ -260,3 +260,67 @@ def test_global_scale_helper_refuses_host_tensors():
         mm.nvfp4_global_scale(torch.ones(8))
     lib = _lib.load()
     assert lib.mm_tensor_absmax(None, 1, 8, None, None) == 1        # invalid argument: null pointers
+
+
+class _RecordingLibrary:
+    """Stands in for the C library behind the launch functions: remembers what it was called with."""
+    def __init__(self):
+        self.calls = []
+
+    def mm_mega_moe_launch(self, cfg, args, stream):
+        self.calls.append(('layer', args))
+        return 0
+
+    def mm_mega_moe_from_hidden_launch(self, cfg, args, fe, stream):
+        self.calls.append(('hidden', args, fe))
+        return 0
+
+    def mm_fe_forward(self, *a):
+        self.calls.append(('frontend', a))
+        return 0
+
+
+@pytest.fixture
+def launches(monkeypatch):
+    """A factory of small one-rank buffers in host memory, and the launches made on them (recorded, not run)."""
+    from types import SimpleNamespace
+    from hopper_megamoe_basedondeepgemm_b200 import mega
+    lib = _RecordingLibrary()
+    real_load = _lib.load
+    monkeypatch.setattr(torch.Tensor, 'cuda', lambda self, *a, **k: self)
+    monkeypatch.setattr(torch.cuda, 'synchronize', lambda *a, **k: None)
+    monkeypatch.setattr(torch.Tensor, 'is_pinned', lambda self, *a, **k: True)
+    monkeypatch.setattr(mega, '_current_stream', lambda: 0)
+    real_empty = torch.empty
+    monkeypatch.setattr(torch, 'empty', lambda *a, **k: real_empty(*a, **{x: v for x, v in k.items() if x != 'device'}))
+
+    def make(fmt='mxfp4', experts=8, topk=8, hidden=512, inter=256):
+        monkeypatch.setattr(_lib, 'load', real_load)
+        buf = mega.SymmBuffer(None, experts, 16, topk, hidden, inter, act_format=fmt, num_sms=148)
+        unit = 18432 if fmt == 'nvfp4' else 17408
+        vec = 16 if fmt == 'nvfp4' else 32
+        w = lambda n, k: (torch.zeros((experts, n // 128, k // 256, unit), dtype=torch.uint8), torch.tensor([n, k, vec]))      # noqa: E731
+        monkeypatch.setattr(_lib, 'load', lambda check=False: lib)
+        return buf, w(2 * inter, hidden), w(hidden, inter), torch.zeros((4, hidden), dtype=torch.bfloat16)
+    return SimpleNamespace(make=make, calls=lib.calls)
+
+
+def test_a_destroyed_buffer_is_not_launched_on(launches):
+    """`destroy` gives the memory back: no call may hand its address to a kernel afterwards."""
+    for fmt, call in (('mxfp4', mm.fp4_fp4_mega_moe), ('fp8', mm.fp8_fp4_mega_moe)):
+        buf, l1, l2, y = launches.make(fmt)
+        call(y, l1, l2, buf)
+        assert launches.calls[-1][1].buffer == buf.buffer.data_ptr()
+        n = len(launches.calls)
+        buf.destroy()
+        with pytest.raises((AttributeError, RuntimeError)):
+            call(y, l1, l2, buf)
+        assert len(launches.calls) == n
+    buf, l1, l2, y = launches.make()
+    router, ws = torch.zeros((8, 512), dtype=torch.bfloat16), torch.zeros(buf._fe_workspace_bytes, dtype=torch.uint8)
+    mm.mega_moe_from_hidden(y, y.clone(), router, l1, l2, buf, ws)
+    n = len(launches.calls)
+    buf.destroy()
+    with pytest.raises((AttributeError, RuntimeError)):
+        mm.mega_moe_from_hidden(y, y.clone(), router, l1, l2, buf, ws)
+    assert len(launches.calls) == n
