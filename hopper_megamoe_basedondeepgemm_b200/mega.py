@@ -5,7 +5,6 @@ sm_100a library behind the C ABI of `include/megamoe_b200.h`. PyTorch supplies d
 the symmetric-memory rendezvous only.
 """
 import ctypes
-import weakref
 from types import SimpleNamespace
 from typing import Optional, Tuple
 
@@ -94,7 +93,6 @@ class SymmBuffer:
                                                       None, -1.0, 1, 1.0, 1.0, 1.0, 1.0, 0.0, None))
         self._cfg_ref = ctypes.byref(self.cfg)
         self._fe_workspace_bytes = fe_workspace_bytes(self)
-        self._weights_seen = None                      # weak references to the weight tensors checked last
         L, t = self.layout, num_max_tokens_per_rank
         vec = int(L.sf_vec)
 
@@ -385,17 +383,15 @@ def _input_region_ptr(sym_buffer: 'SymmBuffer', host_inputs):
 
 
 def _check_weights(b: SymmBuffer, w1, s1, w2, s2) -> None:
-    """The weight streams fit the buffer. Their tensors are remembered (weakly), so that the calls of a layer whose
-    weights stay the same compare four references."""
+    """The weight streams fit the buffer. Looked at in every call: a tensor can get other memory and another shape in place."""
     vec = b.act_sf_vec_size or 32        # FP8 tokens carry one UE8M0 scale per 32 elements, like the MXFP4 weights
     e_local = b.num_experts // b.num_ranks
     if w1.dtype != torch.uint8 or w1.dim() != 4 or w2.dtype != torch.uint8 or w2.dim() != 4:
         raise RuntimeError('weights must come from transform_weights_for_mega_moe')
     if s1.tolist() != [2 * b.intermediate_hidden, b.hidden, vec] or s2.tolist() != [b.hidden, b.intermediate_hidden, vec]:
         raise RuntimeError('weight shapes do not match the buffer')
-    if w1.size(0) != e_local or w2.size(0) != e_local or not (w1.is_contiguous() and w2.is_contiguous()):
+    if w1.shape[0] != e_local or w2.shape[0] != e_local or not (w1.is_contiguous() and w2.is_contiguous()):
         raise RuntimeError('expected one contiguous weight stream per local expert')
-    b._weights_seen = tuple(weakref.ref(t) for t in (w1, s1, w2, s2))
 
 
 def _launch_args(b: SymmBuffer, y, w1, w2, stats, activation_clamp, fast_math, timeout_ms):
@@ -430,9 +426,7 @@ def _launch(y, l1_weights, l2_weights, sym_buffer: SymmBuffer, stats, recipe, ac
     if shape[0] > b.num_max_tokens_per_rank:
         raise RuntimeError('more tokens than the buffer was created for')
     (w1, s1), (w2, s2) = l1_weights, l2_weights
-    seen = b._weights_seen
-    if seen is None or seen[0]() is not w1 or seen[1]() is not s1 or seen[2]() is not w2 or seen[3]() is not s2:
-        _check_weights(b, w1, s1, w2, s2)
+    _check_weights(b, w1, s1, w2, s2)
     if stats is not None and (stats.dtype != torch.int32 or stats.numel() != b.num_experts // b.num_ranks):
         raise RuntimeError('cumulative_local_expert_recv_stats must be int32 [num_local_experts]')
     args = _launch_args(b, y, w1, w2, stats, activation_clamp, fast_math, timeout_ms)

@@ -324,3 +324,21 @@ def test_a_destroyed_buffer_is_not_launched_on(launches):
     with pytest.raises((AttributeError, RuntimeError)):
         mm.mega_moe_from_hidden(y, y.clone(), router, l1, l2, buf, ws)
     assert len(launches.calls) == n
+
+
+def test_weights_are_checked_in_every_call(launches):
+    """The same tensors with other contents: what a first call would refuse, a later one refuses too."""
+    def changed(change):
+        buf, l1, l2, y = launches.make()
+        mm.fp4_fp4_mega_moe(y, l1, l2, buf)
+        n = len(launches.calls)
+        change(l1[0], l1[1], l2[0], l2[1])
+        with pytest.raises(RuntimeError):
+            mm.fp4_fp4_mega_moe(y, l1, l2, buf)
+        assert len(launches.calls) == n
+    changed(lambda w1, s1, w2, s2: w1.resize_(7, *w1.shape[1:]))
+    changed(lambda w1, s1, w2, s2: w2.set_(w2[:4].clone()))
+    changed(lambda w1, s1, w2, s2: w1.transpose_(0, 1))
+    changed(lambda w1, s1, w2, s2: setattr(w1, 'data', torch.zeros(w1.shape, dtype=torch.int8)))
+    changed(lambda w1, s1, w2, s2: s1.fill_(1))
+    changed(lambda w1, s1, w2, s2: s2[0].add_(128))
