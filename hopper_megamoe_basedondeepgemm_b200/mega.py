@@ -417,7 +417,7 @@ def _launch(y, l1_weights, l2_weights, sym_buffer: SymmBuffer, stats, recipe, ac
     b = sym_buffer
     if activation != 'swiglu':
         raise RuntimeError('only the swiglu activation is supported')
-    if recipe is not None and tuple(recipe) != (1, 1, b.act_sf_vec_size or 32):
+    if tuple(recipe) != (1, 1, b.act_sf_vec_size or 32):
         raise RuntimeError(f'recipe {recipe} does not match the buffer format {b.act_format}')
     shape = y.shape
     if y.dtype != torch.bfloat16 or len(shape) != 2 or shape[1] != b.hidden or not y.is_contiguous() or \
@@ -461,7 +461,9 @@ def fp4_fp4_mega_moe(y: torch.Tensor, l1_weights, l2_weights, sym_buffer: SymmBu
     host tensor).
     """
     assert sym_buffer.act_format in ('mxfp4', 'nvfp4'), 'buffer must be created with act_format mxfp4/nvfp4'
-    assert recipe is None or recipe[2] == sym_buffer.act_sf_vec_size
+    if recipe is None:
+        recipe = (1, 1, sym_buffer.act_sf_vec_size)
+    assert recipe[2] == sym_buffer.act_sf_vec_size
     _launch(y, l1_weights, l2_weights, sym_buffer, cumulative_local_expert_recv_stats, recipe, activation,
             activation_clamp, fast_math, engine, (x_global_scale, l1_global_scale, l2_global_scale, mid_global_scale),
             timeout_ms, host_inputs)

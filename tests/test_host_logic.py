@@ -342,3 +342,16 @@ def test_weights_are_checked_in_every_call(launches):
     changed(lambda w1, s1, w2, s2: setattr(w1, 'data', torch.zeros(w1.shape, dtype=torch.int8)))
     changed(lambda w1, s1, w2, s2: s1.fill_(1))
     changed(lambda w1, s1, w2, s2: s2[0].add_(128))
+
+
+def test_recipes_that_are_taken_and_refused(launches):
+    """None stands for the format's own recipe in the W4A4 call; the A-FP8 call has a default and takes no None."""
+    for fmt, call, vec in (('mxfp4', mm.fp4_fp4_mega_moe, 32), ('nvfp4', mm.fp4_fp4_mega_moe, 16), ('fp8', mm.fp8_fp4_mega_moe, 32)):
+        buf, l1, l2, y = launches.make(fmt)
+        call(y, l1, l2, buf)
+        call(y, l1, l2, buf, recipe=[1, 1, vec])
+        n = len(launches.calls)
+        for wrong in ((1, 1, 64), (2, 1, vec), (1, 1)) + ((None,) if fmt == 'fp8' else ()):
+            with pytest.raises((RuntimeError, AssertionError, TypeError, IndexError)):
+                call(y, l1, l2, buf, recipe=wrong)
+        assert len(launches.calls) == n
