@@ -501,7 +501,8 @@ def mega_moe_from_hidden(y: torch.Tensor, hidden: torch.Tensor, router_weight: t
     b = sym_buffer
     if hidden.dtype != torch.bfloat16 or router_weight.dtype != torch.bfloat16 or not hidden.is_contiguous():
         raise RuntimeError('hidden states and router weight must be contiguous bf16')
-    if hidden.shape != y.shape or hidden.shape[1] != b.hidden or router_weight.shape != (b.num_experts, b.hidden):
+    if hidden.shape[0] != y.shape[0] or hidden.shape[1] != b.hidden or y.numel() < hidden.numel() or \
+            router_weight.shape != (b.num_experts, b.hidden):
         raise RuntimeError('router shapes do not match the buffer')
     if workspace.nbytes < b._fe_workspace_bytes:
         raise RuntimeError('frontend workspace too small')

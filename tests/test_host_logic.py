@@ -355,3 +355,18 @@ def test_recipes_that_are_taken_and_refused(launches):
             with pytest.raises((RuntimeError, AssertionError, TypeError, IndexError)):
                 call(y, l1, l2, buf, recipe=wrong)
         assert len(launches.calls) == n
+
+
+def test_from_hidden_states_takes_outputs_of_any_shape_with_a_row_per_token(launches):
+    """The output of the from-hidden call is asked for its rows and its size, not for the shape of the hidden states; one with no room
+    for every row is refused."""
+    buf, l1, l2, y = launches.make()
+    hidden, router, ws = y.clone(), torch.zeros((8, 512), dtype=torch.bfloat16), torch.zeros(buf._fe_workspace_bytes, dtype=torch.uint8)
+    for out in (y, y.view(4, 1, 512), y.view(4, 8, 64), torch.zeros((4, 520), dtype=torch.bfloat16)):
+        mm.mega_moe_from_hidden(out, hidden, router, l1, l2, buf, ws)
+        assert launches.calls[-1][1].y == out.data_ptr() and launches.calls[-1][1].num_tokens == 4
+    n = len(launches.calls)
+    for out in (y[:3], torch.zeros((4, 256), dtype=torch.bfloat16)):
+        with pytest.raises(RuntimeError):
+            mm.mega_moe_from_hidden(out, hidden, router, l1, l2, buf, ws)
+    assert len(launches.calls) == n
