@@ -404,11 +404,11 @@ def _launch_args(b: SymmBuffer, y, w1, w2, stats, activation_clamp, fast_math, t
     if stats is not None:
         args.cumulative_local_expert_recv_stats = stats.data_ptr()
     if activation_clamp is not None:
-        args.activation_clamp = activation_clamp
+        args.activation_clamp = float(activation_clamp)
     if not fast_math:
         args.fast_math = 0
     if timeout_ms:
-        args.timeout_ms = timeout_ms
+        args.timeout_ms = float(timeout_ms)
     return args
 
 
@@ -435,7 +435,7 @@ def _launch(y, l1_weights, l2_weights, sym_buffer: SymmBuffer, stats, recipe, ac
         args.engine = _lib.ENGINE[engine]
         lib = _lib.load(check=(engine == 'check'))      # the cross-check engine lives in the test build of the library
     if global_scales is not None:
-        args.x_global_scale, args.l1_global_scale, args.l2_global_scale, args.mid_global_scale = global_scales
+        args.x_global_scale, args.l1_global_scale, args.l2_global_scale, args.mid_global_scale = map(float, global_scales)
     if host_inputs is not None:
         args.input_region = _input_region_ptr(b, host_inputs)
     status = lib.mm_mega_moe_launch(b._cfg_ref, args, _current_stream())
@@ -510,10 +510,10 @@ def mega_moe_from_hidden(y: torch.Tensor, hidden: torch.Tensor, router_weight: t
     args = _launch_args(b, y, w1, w2, cumulative_local_expert_recv_stats, activation_clamp, fast_math, timeout_ms)
     args.engine = _lib.ENGINE[engine]
     args.x_global_scale, args.l1_global_scale, args.l2_global_scale, args.mid_global_scale = \
-        x_global_scale, l1_global_scale, l2_global_scale, mid_global_scale
+        float(x_global_scale), float(l1_global_scale), float(l2_global_scale), float(mid_global_scale)
     fe = _lib.MMFrontendArgs(hidden.data_ptr(), router_weight.data_ptr(),
                              expert_bias.data_ptr() if expert_bias is not None else None,
-                             args.num_tokens, score_mode, workspace.data_ptr(), x_global_scale)
+                             args.num_tokens, score_mode, workspace.data_ptr(), args.x_global_scale)
     status = lib.mm_mega_moe_from_hidden_launch(b._cfg_ref, args, fe, _current_stream())
     if status:
         _lib.check(status, 'mega_moe_from_hidden')
@@ -569,7 +569,7 @@ def fe_forward(hidden: torch.Tensor, router_weight: torch.Tensor, x: torch.Tenso
         raise RuntimeError('output views do not have the row strides of the activation format')
     status = _lib.load().mm_fe_forward(hidden.data_ptr(), router_weight.data_ptr(), x.data_ptr(), x_sf.data_ptr(),
                                        topk_idx.data_ptr(), topk_weights.data_ptr(), workspace.data_ptr(), workspace.nbytes,
-                                       m, h, e, topk, mode, l2_persist, _current_stream())
+                                       m, h, e, topk, int(mode), int(l2_persist), _current_stream())
     if status:
         _lib.check(status, 'fe_forward')
 

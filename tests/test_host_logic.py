@@ -370,3 +370,21 @@ def test_from_hidden_states_takes_outputs_of_any_shape_with_a_row_per_token(laun
         with pytest.raises(RuntimeError):
             mm.mega_moe_from_hidden(out, hidden, router, l1, l2, buf, ws)
     assert len(launches.calls) == n
+
+
+@pytest.mark.parametrize('number', [lambda v: v, str, lambda v: torch.tensor(v)])
+def test_numbers_are_taken_in_every_form_that_converts(launches, number):
+    """Scales, clamp and time limit in whatever float() takes; the frontend's mode and cache hint in whatever int() does."""
+    buf, l1, l2, y = launches.make('nvfp4')
+    scales = dict(x_global_scale=number(0.25), l1_global_scale=number(0.5), l2_global_scale=number(2.0), mid_global_scale=number(4.0))
+    router, ws = torch.zeros((8, 512), dtype=torch.bfloat16), torch.zeros(buf._fe_workspace_bytes, dtype=torch.uint8)
+    mm.fp4_fp4_mega_moe(y, l1, l2, buf, activation_clamp=number(8.0), timeout_ms=number(100.0), **scales)
+    mm.mega_moe_from_hidden(y, y.clone(), router, l1, l2, buf, ws, activation_clamp=number(8.0), timeout_ms=number(100.0), **scales)
+    for c in launches.calls:
+        a = c[1]
+        assert (a.x_global_scale, a.l1_global_scale, a.l2_global_scale, a.mid_global_scale) == (0.25, 0.5, 2.0, 4.0)
+        assert a.activation_clamp == 8.0 and a.timeout_ms == 100.0
+    assert launches.calls[1][2].x_global_scale == 0.25
+    sf, idx, tw = torch.zeros((4, 8), dtype=torch.int32), torch.zeros((4, 8), dtype=torch.int64), torch.zeros((4, 8))
+    mm.fe_forward(y, router, torch.zeros((4, 256), dtype=torch.int8), sf, idx, tw, ws, torch.tensor(4.0), number(1.0) if number is not str else '1')
+    assert launches.calls[-1][1][12:14] == (4, 1) and all(type(v) is int for v in launches.calls[-1][1][12:14])
