@@ -167,15 +167,16 @@ class SymmBuffer:
         kernel (csrc/mm_batch.cuh): an expert's rows start on a 16-row boundary, experts in ascending order. An expert's
         n rows form t = ceil(n / limit) token tiles of ceil(n / t) rows (rounded up to 16); a tile's image is one record
         per K unit: its rows (a multiple of 16) x 128 B in the 128 B swizzle (E4M3: two such atoms), then the unit's scale
-        planes of 512 B, the word of row r at (r % 32) * 16 + (r // 32) * 4."""
+        planes of 512 B, the word of row r at (r % 32) * 16 + (r // 32) * 4. No rows for a launch that had none or has failed."""
         L = self.layout
         counts = [0] * self.num_experts
-        for (e, _, _, _) in self.received_records()[0]:
-            counts[e] += 1
+        for rec in self.received_records()[0] or ():
+            if rec is not None:
+                counts[rec[0]] += 1
         atoms, planes = (2 if self.act_format == 'fp8' else 1), 256 // (4 * int(L.sf_vec))
         units, row_bytes = self.intermediate_hidden // 256, int(L.mid_row_bytes)
         raw = self.mid_tiles.reshape(-1).cpu()
-        rows_out, words_out, off = [], [], 0
+        rows_out, words_out, off = [raw.new_zeros((0, row_bytes))], [raw.new_zeros((0, units * planes, 4))], 0
         for n in counts:
             if n == 0:
                 continue
@@ -209,7 +210,7 @@ class SymmBuffer:
         tw, limit = self.device_status()[1][2:4]
         if limit:
             words = self._rows_of_batch_images(limit)[1]
-            return words.reshape(words.size(0), -1)[:, :self.intermediate_hidden // int(self.layout.sf_vec)].contiguous()
+            return words.flatten(1)[:, :self.intermediate_hidden // int(self.layout.sf_vec)].contiguous()
         if tw:
             words = self._rows_of_tile_images(self.mid_tiles, int(self.layout.mid_row_bytes), tw, 0)[1]
             return words.reshape(words.size(0), -1)[:, :self.intermediate_hidden // int(self.layout.sf_vec)].contiguous()

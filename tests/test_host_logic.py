@@ -388,3 +388,16 @@ def test_numbers_are_taken_in_every_form_that_converts(launches, number):
     sf, idx, tw = torch.zeros((4, 8), dtype=torch.int32), torch.zeros((4, 8), dtype=torch.int64), torch.zeros((4, 8))
     mm.fe_forward(y, router, torch.zeros((4, 256), dtype=torch.int8), sf, idx, tw, ws, torch.tensor(4.0), number(1.0) if number is not str else '1')
     assert launches.calls[-1][1][12:14] == (4, 1) and all(type(v) is int for v in launches.calls[-1][1][12:14])
+
+
+@pytest.mark.parametrize('fmt', ['mxfp4', 'nvfp4', 'fp8'])
+@pytest.mark.parametrize('records', [[], None])
+def test_intermediate_rows_of_a_batch_launch_without_rows(launches, fmt, records):
+    """A launch of the one-rank batch kernel in which every slot is masked (its header line says 0 rows), or one that failed before it
+    left a header line: no rows, in the shapes of the others."""
+    buf = launches.make(fmt)[0]
+    buf.device_status = lambda: (0, [0, 1, 16, 128] + [0] * 12)
+    buf.received_records = lambda: [records]
+    row = 256 if fmt == 'fp8' else 128
+    assert buf.l2_acts_payload().shape == (0, row) and buf.l2_acts_payload().dtype == torch.uint8
+    assert buf.l2_acts_sf_payload().shape == (0, 256 // (16 if fmt == 'nvfp4' else 32))
