@@ -145,7 +145,9 @@ int mm_get_layout(const mm_config_t* c, mm_layout_t* out) {
     out->off_token_tiles = take(out->tile_capacity * out->token_tile_bytes);
     out->off_mid_tiles = take(out->tile_capacity * out->mid_tile_bytes);
     out->off_arrive = take(2 * 2 * out->tile_capacity * 4 + 2 * mm::kBCounts * 4 + mm::kFeMaxFusedTokens * 8 * 16);   // (then the one-rank batch kernel's counts and routing records)
-    take(c->num_ranks == 1 ? t_max * c->num_topk * c->hidden * 2 : 0);   // the same kernel's expert outputs (`batch_out_offset`)
+    // the same kernel's expert outputs, of as many routing entries as it takes (`batch_out_offset`)
+    const int64_t out_rows = t_max * c->num_topk < mm::kBMaxRows ? t_max * c->num_topk : mm::kBMaxRows;
+    take(c->num_ranks == 1 ? out_rows * c->hidden * 2 : 0);
     out->total_bytes = off;
     return MM_OK;
 }

@@ -401,3 +401,14 @@ def test_intermediate_rows_of_a_batch_launch_without_rows(launches, fmt, records
     row = 256 if fmt == 'fp8' else 128
     assert buf.l2_acts_payload().shape == (0, row) and buf.l2_acts_payload().dtype == torch.uint8
     assert buf.l2_acts_sf_payload().shape == (0, 256 // (16 if fmt == 'nvfp4' else 32))
+
+
+def test_large_buffers_hold_the_one_rank_kernels_regions_for_their_largest_launch_only():
+    """The one-rank batch kernel takes at most 4096 routing entries: its expert outputs at the end of the buffer stop growing there, and
+    hold every entry of a smaller buffer."""
+    for tmax, rows in ((16, 128), (512, 4096), (4096, 4096), (32768, 4096)):
+        st, L = _layout(ranks=1, experts=48, tmax=tmax)
+        behind = L.total_bytes - (L.off_arrive + 4 * 4 * L.tile_capacity)        # (arrival counts, then other counts and the routing records)
+        assert st == 0 and rows * 3072 * 2 <= behind - (2 * 64 * 4 + 256 * 8 * 16) <= rows * 3072 * 2 + 2048
+    st, L = _layout(ranks=8)
+    assert L.total_bytes - (L.off_arrive + 4 * 4 * L.tile_capacity) <= 2 * 64 * 4 + 256 * 8 * 16 + 2048
