@@ -133,12 +133,14 @@ int mm_get_layout(const mm_config_t* c, mm_layout_t* out) {
     // partial router logits of the fused frontend: 16 B per (token, expert), flagged with the launch number
     out->off_logits = take((t_max < mm::kFeMaxFusedTokens ? t_max : mm::kFeMaxFusedTokens) * c->num_experts * 16);
     // tile images of the launches with more than 16 received rows: token bytes of 16 rows, then one 16 B slot per (scale word, row)
+    // (E4M3 tokens: only the one-rank batch kernel works from images, with 256 B per row and unit and 4096 rows at most)
+    const bool a8_images = a8 && c->num_ranks == 1;
     out->tile_capacity = out->mid_rows / mm::kTileTokens;
+    if (a8_images && out->tile_capacity > mm::kBMaxRows / mm::kTileTokens + e_local) out->tile_capacity = mm::kBMaxRows / mm::kTileTokens + e_local;
     {
         // per tile: 32 row records of 16 B (token tiles only), then per streamed K unit a record of up to 32 rows x 128 B
         // and the unit's scale-word slots (16 B per (scale word, row))
-        // (E4M3 tokens: 256 B per row and unit)
-        const int64_t rec32 = mm::kWideTokens * (a8 ? 256 : 128) + (mm::kUnitK / (4 * vec)) * mm::kWideTokens * 16;
+        const int64_t rec32 = mm::kWideTokens * (a8_images ? 256 : 128) + (mm::kUnitK / (4 * vec)) * mm::kWideTokens * 16;
         out->token_tile_bytes = mm::kWideTokens * 16 + (c->hidden / mm::kUnitK) * rec32;
         out->mid_tile_bytes = (c->intermediate / mm::kUnitK) * rec32;
     }

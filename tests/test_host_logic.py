@@ -412,3 +412,19 @@ def test_large_buffers_hold_the_one_rank_kernels_regions_for_their_largest_launc
         assert st == 0 and rows * 3072 * 2 <= behind - (2 * 64 * 4 + 256 * 8 * 16) <= rows * 3072 * 2 + 2048
     st, L = _layout(ranks=8)
     assert L.total_bytes - (L.off_arrive + 4 * 4 * L.tile_capacity) <= 2 * 64 * 4 + 256 * 8 * 16 + 2048
+
+
+def test_tile_images_of_e4m3_tokens_take_the_room_their_one_user_needs():
+    """Images with 256 B per E4M3 row and K unit are the one-rank batch kernel's, which takes at most 4096 rows (of 64 experts: 4096 / 16
+    groups and one begun group per expert). Several ranks never write images of E4M3 tokens: their buffers keep the 128 B records."""
+    rec32 = 32 * 128 + 2 * 32 * 16
+    st, L = _layout(ranks=8, fmt='fp8')
+    assert st == 0 and L.tile_capacity == L.mid_rows // 16
+    assert L.token_tile_bytes == 32 * 16 + 12 * rec32 and L.mid_tile_bytes == 5 * rec32
+    for experts, tmax in ((48, 512), (48, 4096), (64, 32768), (3, 1000), (1, 1)):
+        st, L = _layout(ranks=1, experts=experts, tmax=tmax, fmt='fp8')
+        rows = min(4096, tmax * min(8, experts))
+        groups, tiles = rows // 16 + experts, min(128, experts + rows // 64)
+        assert st == 0 and L.tile_capacity >= groups and L.tile_capacity <= 4096 // 16 + experts
+        assert L.tile_capacity * L.token_tile_bytes >= 12 * (groups * 2 * 2048 + tiles * 2 * 512)
+        assert L.tile_capacity * L.mid_tile_bytes >= 5 * (groups * 2 * 2048 + tiles * 2 * 512)
