@@ -941,6 +941,7 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
             ctrl32[kCtrlStatus / 4 + 1] = epoch + 1u;
             ctrl32[kCtrlStatus / 4 + 2] = 16u;                       // rows of an expert start on 16-row boundaries of the images
             ctrl32[kCtrlStatus / 4 + 3] = p.tile_limit;
+            ctrl32[kCtrlStatus / 4 + 4] = kRanBatch;
             reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlStamps)[kStampEntry] = t_first;
             cx.stamp(kStampPrologue);
         }

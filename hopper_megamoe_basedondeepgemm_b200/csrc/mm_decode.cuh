@@ -662,6 +662,7 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
             reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlSmPhase)[bid * kSmPhaseSlots + kSmEntry] = t_first;
             if (bid == 0) {
                 ctrl32[kCtrlStatus / 4 + 1] = epoch + 1u; ctrl32[kCtrlStatus / 4 + 2] = 0u; ctrl32[kCtrlStatus / 4 + 3] = 0u;
+                ctrl32[kCtrlStatus / 4 + 4] = kRanDecode;
                 reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlStamps)[kStampEntry] = t_first;
                 reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlStamps)[kStampPrologue] = t_first;   // (set-up precedes the first stamp)
             }

@@ -96,6 +96,8 @@ enum : uint32_t {
     kErrWaitCombineFlag = 9 /* expert outputs */,
     kErrMetaCapacity = 10, kErrTaskCapacity = 11, kErrWaitFrontend = 12
 };
+// the kernel that ran last (status word 4)
+enum : uint32_t { kRanMultiRank = 1, kRanBatch = 2, kRanDecode = 3 };
 // phase stamp slots (SM 0 unless noted)
 enum : int {
     kStampEntry = 0, kStampDispatched = 1, kStampFlagsSeen = 2, kStampScheduled = 3, kStampTasksDone = 4, kStampPrologue = 5 /* SM 0: shared memory, barriers and TMEM are set up */,
@@ -2227,7 +2229,7 @@ __global__ void __launch_bounds__(kA8 ? kThreads + kNumExpThreads : kThreads, 1)
             const uint32_t M = res >> 16, nmine = res & 0xFFFFu;
             const uint32_t nt1 = M * p.n1_tiles, nt2 = M * p.n2_tiles;
             if (lane == 0) {
-                if (bid == 0) { ctrl32[kCtrlStatus / 4 + 2] = c.bulk != 0u ? c.tw : 0u; ctrl32[kCtrlStatus / 4 + 3] = 0u; }   // (for whoever inspects the intermediate rows afterwards)
+                if (bid == 0) { ctrl32[kCtrlStatus / 4 + 2] = c.bulk != 0u ? c.tw : 0u; ctrl32[kCtrlStatus / 4 + 3] = 0u; ctrl32[kCtrlStatus / 4 + 4] = kRanMultiRank; }   // (for whoever inspects the intermediate rows afterwards)
                 c.nt1 = nt1; c.nt2 = nt2;
                 if (M > kMaxMTiles || nmine > kMaxTasks) cx.fail(kErrTaskCapacity, nmine);
                 else c.ntasks = nmine;

@@ -175,7 +175,7 @@ int mm_reset(const mm_config_t* cfg, void* buffer, void* stream);
 /* Synchronises `stream`, then copies the 16 device status words: [0] first failure (0 = none; code | sm << 8 |
  * detail << 16), [1] launches seen, [2] row granularity of the tile images (16 or 32) when the latest launch kept its rows as such (more
  * than 16 received rows), else 0, [3] row limit of a token tile when that launch was one of the one-rank batch kernel (its images are
- * packed: see csrc/mm_batch.cuh), else 0, [4..] diagnostics. The reference traps instead (sm100_b200/layout_mega_moe.cuh:13-19). */
+ * packed: see csrc/mm_batch.cuh), else 0, [4] kernel of the latest launch (1 multi-rank, 2 one-rank batch, 3 one-rank decode), [5..] diagnostics. The reference traps instead (sm100_b200/layout_mega_moe.cuh:13-19). */
 int mm_read_device_status(const mm_config_t* cfg, const void* buffer, uint32_t out_words[16], void* stream);
 /* Synchronises `stream`, then copies the 32 phase stamps (globaltimer ns) of the last launch. Slots, SM 0 unless
  * noted: 0 first instruction, 1 dispatched, 2 header lines of all ranks seen, 3 scheduled, 4 tasks done, 5 prologue

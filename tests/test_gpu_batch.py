@@ -342,3 +342,59 @@ def test_from_hidden_states_on_one_or_two_sms_fills_every_view(fmt, num_sms, tok
     mm.fe_forward_into_buffer(x, wr, buf, ws)
     for a, v in zip(got, views):
         assert torch.equal(a, v[:tokens].view(torch.uint8))
+
+
+MULTI_RANK, BATCH, DECODE = 1, 2, 3             # status word 4
+
+
+@pytest.mark.parametrize('fmt', ['mxfp4', 'nvfp4', 'fp8'])
+@pytest.mark.parametrize('topk,tokens,hidden,inter,kernel', [
+    (1, 1, 512, 256, DECODE), (1, 16, 512, 512, DECODE), (8, 2, 1024, 256, DECODE), (5, 3, 512, 2048, DECODE), (8, 1, 3072, 1280, DECODE),
+    (2, 8, 1536, 256, DECODE), (1, 17, 512, 256, BATCH), (8, 3, 1024, 256, BATCH), (16, 256, 2048, 256, BATCH),
+])
+def test_which_kernel_a_launch_takes(fmt, topk, tokens, hidden, inter, kernel):
+    """The dispatch rule at its line (16 routing entries), over the shapes of the decode tests, and with inputs in host memory, which
+    stay with the multi-rank kernel; a launch without tokens does too."""
+    e = 16
+    stream = lambda n, k: (torch.zeros((e, n // 128, k // 256, 18432 if fmt == 'nvfp4' else 17408), dtype=torch.uint8, device='cuda'),      # noqa: E731
+                           torch.tensor([n, k, 16 if fmt == 'nvfp4' else 32]))
+    l1, l2 = stream(2 * inter, hidden), stream(hidden, inter)
+    buf = mm.get_symm_buffer_for_mega_moe(None, e, tokens, topk, hidden, inter, act_format=fmt)
+    buf.topk_idx[:tokens].copy_(U.random_routing(tokens, e, topk, 100)[0])
+    call = mm.fp8_fp4_mega_moe if fmt == 'fp8' else mm.fp4_fp4_mega_moe
+    y = torch.empty((tokens, hidden), dtype=torch.bfloat16, device='cuda')
+    call(y, l1, l2, buf, timeout_ms=500.0)
+    st, words = buf.device_status()
+    assert st == 0 and words[4] == kernel
+    mirror, views = buf.host_inputs()
+    views['topk_idx'].fill_(-1)
+    for out, kw in ((y, dict(host_inputs=mirror)), (y[:0], {})):
+        call(out, l1, l2, buf, timeout_ms=500.0, **kw)
+        st, words = buf.device_status()
+        assert st == 0 and words[4] == MULTI_RANK
+
+
+@pytest.mark.parametrize('fmt', ['mxfp4', 'fp8'])
+def test_launches_with_mapped_inputs_alternate_with_the_one_rank_kernels(fmt):
+    """Inputs in host memory stay with the multi-rank kernel, which shares buffer, launch numbers and counters with the other two."""
+    e, hidden, inter, topk = 4, 512, 256, 2
+    w, _, _ = O.make_expert_weights(e, hidden, inter, fmt, seed=110, std=0.05)
+    l1, l2 = mm.transform_weights_for_mega_moe(*U.to_operator_weights(w, fmt, 'cuda'))
+    buf = mm.get_symm_buffer_for_mega_moe(None, e, 64, topk, hidden, inter, act_format=fmt)
+    call = mm.fp8_fp4_mega_moe if fmt == 'fp8' else mm.fp4_fp4_mega_moe
+    mirror, views = buf.host_inputs()
+    order = [(40, 0), (40, 1), (40, 0), (3, 1), (3, 0), (64, 1), (64, 0), (5, 0), (5, 1), (40, 0), (40, 1), (64, 0), (33, 0), (2, 1), (50, 0)]
+    for it, (tokens, mapped) in enumerate(order):
+        idx, tw = U.random_routing(tokens, e, topk, 111 + it)
+        _, inp, sfb = U.make_rank_inputs(tokens, hidden, fmt, 130 + it, idx, tw)
+        ref = O.moe_layer_reference([inp], [w], fmt, e, clamp=None)
+        if mapped:
+            for name, v in (('x', inp.x_q.view(buf.x.dtype)), ('x_sf', sfb.contiguous().view(torch.int32)), ('topk_idx', idx), ('topk_weights', tw)):
+                views[name].view(torch.uint8)[:tokens].copy_(v.contiguous().view(torch.uint8))
+        else:
+            U.write_inputs(buf, inp, sfb)
+        y = torch.empty((tokens, hidden), dtype=torch.bfloat16, device='cuda')
+        call(y, l1, l2, buf, timeout_ms=500.0, **(dict(host_inputs=mirror) if mapped else {}))
+        st, words = buf.device_status()
+        assert st == 0 and words[1] == it + 1 and words[4] == (MULTI_RANK if mapped else (BATCH if tokens * topk > 16 else DECODE))
+        assert O.rel_rmse(y.cpu(), ref.y[0]) <= REL_RMSE_TOL, (it, tokens, mapped)
