@@ -39,6 +39,20 @@ def peaks():
     return 6650.0, 'fallback'
 
 
+def token_tile_rows(buf):
+    """Rows of the widest token tile of the latest launch: the batch kernel's (an expert's rows in as few tiles as its limit allows,
+    rounded up to 16), or the fixed width of the multi-rank kernel's images; 0 if rows travelled as flagged words."""
+    granularity, limit = buf.device_status()[1][2:4]
+    if not limit:
+        return granularity
+    counts = {}
+    for rec in buf.received_records()[0]:
+        counts[rec[0]] = counts.get(rec[0], 0) + 1
+    n = max(counts.values(), default=0)
+    tiles = max(1, -(-n // limit))
+    return -(-n // (tiles * 16)) * 16
+
+
 def recorded_traffic(fmt, n):
     """DRAM bytes per algorithmic byte from the committed ncu summary of this workload, if one exists: (ratio, source)."""
     path = os.path.join(ROOT, 'profiles', 'dram_traffic.txt')
@@ -620,7 +634,7 @@ def main():
                 alg = max(case.active) * W.weight_bytes_per_expert(HIDDEN, INTER, fmt)
                 ev_mean = sum(ev) / len(ev)
                 tokens_sweep[f'T{t}'] = {'tokens': t, 'rows': t * TOPK, 'event_us': ev_mean, 'span_us': sp, 'active_experts': max(case.active),
-                                         'token_tile_rows': buf.tile_image_rows(),
+                                         'token_tile_rows': token_tile_rows(buf),
                                          'frac_of_hbm_roofline_events': alg / (ev_mean * 1e-6) / 1e9 / peaks()[0],
                                          'frac_of_hbm_roofline_span': alg / (sp * 1e-6) / 1e9 / peaks()[0],
                                          'parity_ok': None if pr is None else pr['ok'],
