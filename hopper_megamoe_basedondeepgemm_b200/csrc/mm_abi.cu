@@ -414,7 +414,8 @@ static int launch_variant(const mm::KParams& p, int grid, size_t smem_bytes, cud
 // ----------------------------------------------------------------------------- one rank, more than a handful of rows
 // The batch kernel (mm_batch.cuh) takes the launches on one rank that route more entries than the decode kernel's token tile
 // has rows (16). It reads the inputs from the buffer's views on every SM, so inputs in mapped host memory stay with the
-// multi-rank kernel, as do launches beyond its tables (4096 routing entries, 128 token tiles).
+// multi-rank kernel, as do launches of more than 4096 routing entries. (The multi-rank kernel's tables end there too: it takes such a launch
+// while no more than 4096 of the entries are live, as with many masked slots, and reports a capacity error otherwise.)
 static bool wants_batch_kernel(const mm_launch_args_t* a, const mm::KParams& p) {
     if (p.R != 1 || a->input_region != nullptr || a->engine != MM_ENGINE_UMMA || p.T == 0) return false;
     if ((p.knobs & mm::kKnobTileImages) == 0u) return false;
@@ -551,7 +552,6 @@ int mm_frontend_launch(const mm_config_t* cfg, void* buffer, const mm_frontend_a
     q.router_w = static_cast<const __nv_bfloat16*>(fe->router_weight);
     q.bias = fe->expert_bias;
     q.logits = reinterpret_cast<float*>(static_cast<uint8_t*>(fe->workspace) + 256);
-    q.arrive = reinterpret_cast<uint32_t*>(fe->workspace);
     q.T = fe->num_tokens; q.H = cfg->hidden; q.E = cfg->num_experts; q.topk = cfg->num_topk;
     q.score_mode = fe->score_mode; q.fmt = cfg->act_format;
     q.x_gs = fe->x_global_scale > 0.f ? fe->x_global_scale : 1.f;
@@ -650,7 +650,6 @@ int mm_fe_forward(const void* hidden, const void* router_weight, void* x, void* 
     q.hidden = static_cast<const __nv_bfloat16*>(hidden);
     q.router_w = static_cast<const __nv_bfloat16*>(router_weight);
     q.logits = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + 256);
-    q.arrive = reinterpret_cast<uint32_t*>(workspace);
     q.T = m; q.H = h; q.E = e; q.topk = topk; q.score_mode = 0; q.fmt = fmt; q.x_gs = 1.f;
     q.x = static_cast<uint8_t*>(x); q.x_sf = static_cast<uint8_t*>(x_sf);
     q.topk_idx = static_cast<long long*>(topk_idx); q.topk_w = static_cast<float*>(topk_weights);
@@ -684,7 +683,6 @@ int mm_mega_moe_from_hidden_launch(const mm_config_t* cfg, const mm_launch_args_
     q.router_w = static_cast<const __nv_bfloat16*>(fe->router_weight);
     q.bias = fe->expert_bias;
     q.logits = reinterpret_cast<float*>(b + L.off_logits);       // inside the buffer: `mm_reset` clears the flagged records with it
-    q.arrive = nullptr;
     q.T = fe->num_tokens; q.H = cfg->hidden; q.E = cfg->num_experts; q.topk = cfg->num_topk;
     q.score_mode = fe->score_mode; q.fmt = cfg->act_format;
     q.x_gs = fe->x_global_scale > 0.f ? fe->x_global_scale : 1.f;

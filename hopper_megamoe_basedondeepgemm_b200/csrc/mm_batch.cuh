@@ -5,7 +5,8 @@
 //   routing  : every SM ranks all routing entries per expert (warp-wide matches, one histogram per warp), so the token
 //              tiles and the task list follow without any exchange between SMs.
 //   tiles    : an expert's rows form ceil(rows / tile limit) token tiles of at most 128 rows (96 with E4M3 tokens). The
-//              block-scaled MMA takes the same time for 16 and 128 rows, so an expert's weights stream once per tile.
+//              block-scaled MMAs of a weight unit take 199 cycles for 16 rows and 288 for 128, so wide tiles are nearly free and an
+//              expert's weights stream once per tile.
 //   images   : SM (token mod G) copies its tokens' rows into the tiles' operand images in global memory (per streamed K
 //              unit one record: the unit's 128 B of every row in the tensor core's swizzled order, then the unit's
 //              scale planes), counted per tile; a task fetches the records with bulk copies.
@@ -342,8 +343,8 @@ __device__ void b_role_mma(const BCtx& cx, uint32_t lane) {
                                     : idesc_block_scaled(kFmtMxf4E2M1, kFmtMxf4E2M1, 128u, 0u, kFmt == 1 ? 0u : 1u);
     const BParams& p = cx.p; BShared& c = cx.c;
     // Everything the instructions below take as operands is broadcast from lane 0, which tells the compiler that it is the
-    // same in all lanes: the operands then stay in uniform registers. (A unit of 4 MMAs, 4 scale copies and 2 commits takes
-    // 580 cycles to issue from per-lane registers, 313 from uniform ones; the tensor pipe needs 256 of them.)
+    // same in all lanes: the operands then stay in uniform registers. (A unit of 4 MMAs, 4 scale copies and a commit goes out in
+    // 210 cycles with 16 rows and 257 with 96: the tensor pipe itself needs 199 and 256. E4M3 tokens, 16 to 32 rows: 525, the pipe 345 to 365.)
     const uint32_t nr = b_uniform(c.nr), slot_bytes = b_uniform(c.slot_bytes), step = b_uniform(c.spu), tm = b_uniform(c.tmem_base);
     const uint32_t rec0 = b_uniform(smem_u32(cx.smem)), ring0 = rec0 + nr * slot_bytes, x0 = ring0 + b_uniform(c.nw) * p.unit_bytes;
     uint32_t it = 0, rs = 0, rph = 0;                                   // units consumed; record slot (without widening also weight stage), its phase bit
@@ -359,8 +360,8 @@ __device__ void b_role_mma(const BCtx& cx, uint32_t lane) {
         if (!cx.warp_wait(&c.tmem_empty[acc], use ^ 1u, kErrWaitTmemEmpty)) return;
         #pragma unroll 1
         for (uint32_t u = 0; u < units;) {
-            // Every turn of this loop costs about 450 cycles beside the 130 a unit takes to issue (barrier wait, fence, election,
-            // reconvergence), a unit 256 on the tensor pipe: a stage that is there already when the first is goes with it.
+            // A turn of this loop is a barrier wait, a fence, an election and a reconvergence beside the issue itself: a stage that is
+            // there already when the first is goes with it (300 tokens 72.9 us with one stage a turn, 71.4 this way; 512: 79.7, 77.0).
             if (!cx.warp_wait(&c.rfull[rs], rph, kErrWaitActsFull)) return;
             if constexpr (kA8) { if (!cx.warp_wait(&c.xfull[it & 1u], (it >> 1) & 1u, kErrWaitFull)) return; }
             const uint32_t rs1 = rs + 1u == nr ? 0u : rs + 1u, rph1 = rs1 == 0u ? rph ^ 1u : rph;
@@ -895,7 +896,7 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
         const uint32_t eb = fe_expert_block(p.fe, G);
         if (eb == 1u) fe_logits_blocks<1, 3>(p.fe, gw, nw, lane, flag);
         else if (F::kA8 || eb == 2u) fe_logits_blocks<2, 2>(p.fe, gw, nw, lane, flag);
-        else fe_logits_blocks<4, F::kA8 ? 1 : 2>(p.fe, gw, nw, lane, flag);
+        else fe_logits_blocks<4, 2>(p.fe, gw, nw, lane, flag);
         if (warp < half_warps) {
             #pragma unroll 1
             for (uint32_t k = warp; k < ntok; k += half_warps) {

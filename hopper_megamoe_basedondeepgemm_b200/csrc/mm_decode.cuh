@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
     grid_dependency_wait();
     grid_launch_dependents();
     const unsigned long long t_first = globaltimer_ns();
-    const uint32_t epoch = ld_volatile_u32(ctrl32 + kCtrlEpoch / 4 + bid), flag = epoch + 1u;      // (tid 64 counts on after the barrier below)
+    const uint32_t epoch = ld_volatile_u32(ctrl32 + kCtrlEpoch / 4 + bid), flag = epoch + 1u;      // (warp 3 counts on, off the critical path)
     const DCtx cx(p, c, smem, globaltimer_ns() + p.timeout_ns, epoch & 1u);
     constexpr uint32_t kEW = 4;                                       // the first of the warps that build the token tile
     const bool builder = warp >= kEW && warp < kEW + kDEpiWarps;

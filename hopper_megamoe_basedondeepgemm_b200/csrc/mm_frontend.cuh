@@ -16,7 +16,7 @@ namespace mm {
 
 struct FeParams {
     const __nv_bfloat16* hidden; const __nv_bfloat16* router_w; const float* bias;
-    float* logits; uint32_t* arrive;
+    float* logits;
     uint8_t* x; uint8_t* x_sf; long long* topk_idx; float* topk_w;
     int T, H, E, topk, score_mode, fmt, x_row_bytes, x_sf_row_bytes;
     float x_gs;
@@ -33,7 +33,10 @@ constexpr int kFeMaxFusedTokens = 256;       // tokens per rank the single-kerne
 
 // Partial logits live in the workspace as 16 B records per (token, expert): {first half, flag, second half, flag}; each
 // half is written by its warp with one 8-byte store, so a reader that finds `flag` in a half also has its value.
-// One warp per (expert, half of K, block of up to 4 tokens); `warp` of `nwarps` warps cooperate.
+// One warp per (expert, half of K, block of up to 4 tokens); `warp` of `nwarps` warps cooperate. This function and
+// `fe_select_token` serve the multi-rank kernel: its dispatching SMs select for all tokens of the rank among up to 1024
+// experts from shared memory, within that kernel's registers. The one-rank kernels and the stand-alone frontend have
+// `fe_logits_blocks` and `fe_select_token_regs`; what those would give among several ranks has not been measured.
 __device__ __forceinline__ void fe_logits_items(const FeParams& q, uint32_t warp, uint32_t nwarps, uint32_t lane, uint32_t flag) {
     const uint32_t tblocks = (q.T + 3) / 4, nchunk = q.H / 8, half = (nchunk + kFeParts - 1) / kFeParts;
     const uint32_t nitems = static_cast<uint32_t>(q.E) * kFeParts * tblocks;

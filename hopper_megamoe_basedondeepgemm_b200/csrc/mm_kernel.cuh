@@ -292,7 +292,7 @@ __device__ __forceinline__ float sf_value(uint32_t byte) {
 // ============================================================================================= weight loader
 __device__ void role_loader(const Ctx& cx) {
     const KParams& p = cx.p; Ctl& c = cx.c;
-    const uint64_t policy = l2_evict_first_policy();             // (one rank, one token through this kernel: 25.9 us a pass without, 24.3 with)
+    const uint64_t policy = l2_evict_first_policy();             // (one rank, one token through this kernel: 25.9 us a pass without, 24.2 with)
     uint32_t it = 0, s = 0, ph = 0;                              // units issued; ring stage and its phase bit
     #pragma unroll 1
     for (uint32_t ti = 0; ti < c.ntasks; ++ti) {
@@ -891,8 +891,8 @@ __device__ void role_epilogue(const Ctx& cx, uint32_t etid) {
 // space of the token staging buffers), another the records into a ring of record slots in the token region; the MMA
 // issuer waits for both copies of a unit. A task needs no token staging of its own and the token operand costs one bulk
 // copy per unit, whatever the weight flood does to small loads. A token tile has `c.tw` rows: 16, or 32 when an expert
-// has more than 16 rows (the block-scaled MMA takes the same time for 16 and 32 columns: an expert's weights stream
-// once for up to 32 rows).
+// has more than 16 rows (a weight unit's MMAs take about 200 cycles for either: an expert's weights stream once for
+// up to 32 rows).
 // The launch parameters the tile-image roles use, handed to them by value (in registers).
 struct TileP {
     uint32_t unit_bytes, wide_stage_bytes, nstage_wide, tile_capacity, token_tile_bytes, mid_tile_bytes, sm_vt, knobs, sm_rec, nrec, rec_slot_bytes;
