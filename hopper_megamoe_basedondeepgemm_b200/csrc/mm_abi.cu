@@ -24,6 +24,8 @@ int cuda_fail(cudaError_t e, const char* what) {
 
 inline int64_t align_up(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
 
+constexpr int64_t kRedBytes = 256 /* SMs */ * 2 /* phases */ * 2 /* slots */ * mm::kTileTokens * mm::kTileRows * 4;          // split-tile partial sums
+
 int sf_vec_of(int fmt) { return fmt == MM_FMT_NVFP4 ? 16 : 32; }
 
 // development knobs (mm_set_tuning): kernel feature bits, ring depth (0 = chosen from the shared-memory plan), and how
@@ -128,7 +130,7 @@ int mm_get_layout(const mm_config_t* c, mm_layout_t* out) {
     out->off_comb = take(t_max * c->num_topk * c->hidden * 4);
     const int64_t n_max = (2 * c->intermediate > c->hidden ? 2 * c->intermediate : c->hidden) / mm::kTileRows;
     out->cnt_per_phase = (out->mid_rows / mm::kTileTokens) * n_max;
-    out->off_red = take(256 /* SMs */ * 2 /* phases */ * 2 /* slots */ * mm::kTileTokens * mm::kTileRows * 4);
+    out->off_red = take(kRedBytes);
     out->off_cnt = take(2 * out->cnt_per_phase * 4);
     // partial router logits of the fused frontend: 16 B per (token, expert), flagged with the launch number
     out->off_logits = take((t_max < mm::kFeMaxFusedTokens ? t_max : mm::kFeMaxFusedTokens) * c->num_experts * 16);
@@ -157,6 +159,10 @@ int mm_get_layout(const mm_config_t* c, mm_layout_t* out) {
 // Regions of the one-rank kernels behind the arrival counters, and the expert outputs at the end of the buffer. (The outputs
 // are plain bf16: they must not share memory with the flagged words of the combine buffer, which they could imitate.)
 static int64_t batch_routes_offset(const mm_layout_t& L) { return L.off_arrive + 2 * 2 * L.tile_capacity * 4 + 2 * mm::kBCounts * 4; }
+// The decode kernel's flagged partial sums lie in the split-tile region behind the multi-rank kernel's plain ones (32 KB per SM), whose
+// words could carry any launch's number: [SM][16 rows][128] words of 8 bytes.
+static int64_t decode_parts_offset(const mm_layout_t& L, int grid) { return L.off_red + grid * (4ll * mm::kTileTokens * mm::kTileRows * 4); }
+static bool decode_parts_fit(int grid) { return grid * ((4ll * 4 + 8) * mm::kTileTokens * mm::kTileRows) <= kRedBytes; }
 static int64_t batch_out_offset(const mm_layout_t& L) { return align_up(batch_routes_offset(L) + mm::kFeMaxFusedTokens * 8 * 16, 1024); }
 
 // ----------------------------------------------------------------------------- symmetric window without torch
@@ -427,16 +433,16 @@ static bool wants_batch_kernel(const mm_launch_args_t* a, const mm::KParams& p) 
 
 // The decode kernel (mm_decode.cuh) takes the launches up to there. The token tile and, with E4M3 tokens, the widened units
 // have to leave it a ring of three weight stages; wider layers stay with the multi-rank kernel, as inputs in host memory do.
-static bool wants_decode_kernel(const mm_config_t* cfg, const mm_launch_args_t* a, const mm::KParams& p) {
+static bool wants_decode_kernel(const mm_config_t* cfg, const mm_launch_args_t* a, const mm::KParams& p, int grid) {
     if (p.R != 1 || a->input_region != nullptr || a->engine != MM_ENGINE_UMMA || p.T == 0) return false;
-    if ((p.knobs & mm::kKnobDecode) == 0u || static_cast<long long>(p.T) * p.topk > mm::kDEntries) return false;
+    if ((p.knobs & mm::kKnobDecode) == 0u || static_cast<long long>(p.T) * p.topk > mm::kDEntries || !decode_parts_fit(grid)) return false;
     const bool a8 = cfg->act_format == MM_FMT_FP8;
     const int planes = mm::kUnitK / (4 * sf_vec_of(cfg->act_format));
     const long long tiles = static_cast<long long>(p.k1_units > p.k2_units ? p.k1_units : p.k2_units) * (2048 * (a8 ? 2 : 1) + planes * 512);
     return tiles + (a8 ? 2 * mm::kXbufBytes : 0) + 3ll * p.unit_bytes <= 232448 - static_cast<long long>(sizeof(mm::DShared)) - 256 - 1024;
 }
 
-static mm::BParams one_rank_params(const mm_config_t* cfg, const mm::KParams& k) {
+static mm::BParams one_rank_params(const mm_config_t* cfg, const mm::KParams& k, int grid) {
     mm_layout_t L;
     mm_get_layout(cfg, &L);
     mm::BParams p;
@@ -451,7 +457,7 @@ static mm::BParams one_rank_params(const mm_config_t* cfg, const mm::KParams& k)
     p.buf = k.peer[k.rank]; p.w1 = k.w1; p.w2 = k.w2; p.y = k.y; p.stats = k.stats;
     p.off_ctrl = k.off_ctrl; p.off_x = k.off_x; p.off_x_sf = k.off_x_sf; p.off_topk_idx = k.off_topk_idx; p.off_topk_w = k.off_topk_w;
     p.off_rx = k.off_rx; p.off_comb = k.off_comb; p.off_token_tiles = k.off_token_tiles; p.off_mid_tiles = k.off_mid_tiles; p.off_arrive = k.off_arrive;
-    p.off_mid = k.off_mid; p.off_mid_sf = k.off_mid_sf; p.off_red = k.off_red;
+    p.off_mid = k.off_mid; p.off_mid_sf = k.off_mid_sf; p.off_parts = decode_parts_offset(L, grid);
     p.off_routes = batch_routes_offset(L); p.off_out = batch_out_offset(L);
     p.rx_region = k.rx_region; p.tile_capacity = k.tile_capacity; p.cap_rows = static_cast<uint32_t>(k.cap);
     p.fe = k.fe;
@@ -482,7 +488,7 @@ static int launch_one_rank_fmt(mm::BParams& p, bool decode, int grid, cudaStream
 
 template <bool kFe>
 static int launch_one_rank_kernel(const mm_config_t* cfg, const mm::KParams& k, bool decode, int grid, cudaStream_t s) {
-    mm::BParams p = one_rank_params(cfg, k);
+    mm::BParams p = one_rank_params(cfg, k, grid);
     return cfg->act_format == MM_FMT_FP8 ? launch_one_rank_fmt<2, kFe>(p, decode, grid, s)
          : cfg->act_format == MM_FMT_NVFP4 ? launch_one_rank_fmt<1, kFe>(p, decode, grid, s) : launch_one_rank_fmt<0, kFe>(p, decode, grid, s);
 }
@@ -497,7 +503,7 @@ int mm_mega_moe_launch(const mm_config_t* cfg, const mm_launch_args_t* a, void* 
     if (st != MM_OK) return st;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const bool umma = a->engine == MM_ENGINE_UMMA;
-    const bool decode = wants_decode_kernel(cfg, a, p);
+    const bool decode = wants_decode_kernel(cfg, a, p, grid);
     if (decode || wants_batch_kernel(a, p)) return launch_one_rank_kernel<false>(cfg, p, decode, grid, s);
     if (!dispatch_list_fits(p)) return MM_ERR_UNSUPPORTED;
     if (cfg->act_format == MM_FMT_FP8)                                     // tensor-core engine only
@@ -671,7 +677,7 @@ int mm_mega_moe_from_hidden_launch(const mm_config_t* cfg, const mm_launch_args_
     if (cfg->num_experts < cfg->num_topk) return MM_ERR_INVALID_ARGUMENT;      // fewer experts than routes per token
     if (fe->score_mode == 1 && fe->expert_bias == nullptr) return MM_ERR_INVALID_ARGUMENT;
     const bool a8 = cfg->act_format == MM_FMT_FP8;
-    const bool decode = wants_decode_kernel(cfg, a, p), one_rank = decode || wants_batch_kernel(a, p);
+    const bool decode = wants_decode_kernel(cfg, a, p, grid), one_rank = decode || wants_batch_kernel(a, p);
     if (!one_rank && (!dispatch_list_fits(p) ||
         static_cast<size_t>(cfg->num_experts) * 2 * 4 * ((mm::kThreads + (a8 ? mm::kNumExpThreads : 0)) / 32) > p.stage_region)) return MM_ERR_UNSUPPORTED;
     if (fe->num_tokens > mm::kFeMaxFusedTokens) return MM_ERR_UNSUPPORTED;
@@ -749,7 +755,7 @@ int mm_mega_moe_launch_static_scratch(const mm_config_t* cfg, const mm_static_ar
     // must start from zero (the launch counters restart with them, so every call runs as the buffer's first launch),
     // and with the counters every flagged word of the receive pool and the combine buffer
     // The multi-rank kernel always writes its split-tile partial sums between them before it reads them. The decode kernel polls
-    // its own there, flagged like the rest: [SM][row of the expert][weight row], rows below the number of routing entries.
+    // its own behind them, flagged like the rest: of every SM's 16 rows those below the number of routing entries.
     MM_CUDA(cudaMemsetAsync(scratch + L.off_ctrl, 0, L.off_x - L.off_ctrl, s));
     MM_CUDA(cudaMemsetAsync(scratch + L.off_rx, 0, L.off_red - L.off_rx, s));
     const int64_t entries = static_cast<int64_t>(a->num_tokens) * cfg->num_topk;
@@ -758,7 +764,7 @@ int mm_mega_moe_launch_static_scratch(const mm_config_t* cfg, const mm_static_ar
         st = grid_size(cfg, &grid);
         if (st != MM_OK) return st;
         constexpr size_t kRowBytes = mm::kTileRows * 8;
-        MM_CUDA(cudaMemset2DAsync(scratch + L.off_red, mm::kDEntries * kRowBytes, 0, static_cast<size_t>(entries) * kRowBytes, grid, s));
+        MM_CUDA(cudaMemset2DAsync(scratch + decode_parts_offset(L, grid), mm::kDEntries * kRowBytes, 0, static_cast<size_t>(entries) * kRowBytes, grid, s));
     }
     MM_CUDA(cudaMemsetAsync(scratch + L.off_cnt, 0, L.off_token_tiles - L.off_cnt, s));
     MM_CUDA(cudaMemsetAsync(scratch + L.off_arrive, 0, batch_out_offset(L) - L.off_arrive, s));      // (the tile images and the batch kernel's outputs need no clearing)

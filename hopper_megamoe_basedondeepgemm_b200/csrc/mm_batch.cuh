@@ -61,7 +61,7 @@ struct BParams {
     long long rx_region;
     uint32_t tile_capacity, cap_rows;              // token tiles the images, rows the receive pool and the images have room for
     long long off_routes, off_out;                 // [tokens][8] flagged routing records (launches from hidden states); [entries][H] bf16 expert outputs
-    long long off_mid, off_mid_sf, off_red;        // flagged words of the decode kernel: intermediate rows, their scale bytes, partial sums
+    long long off_mid, off_mid_sf, off_parts;      // flagged words of the decode kernel: intermediate rows, their scale bytes, partial sums
     uint32_t mid_row_bytes;
     FeParams fe;
     uint32_t smem_ring;                            // bytes of dynamic shared memory for the two rings (and the widened units)

@@ -303,10 +303,8 @@ __device__ void d_role_epilogue(const DCtx& cx, uint32_t grp, uint32_t etid, uin
         if (ti < 2u && etid == 0u) cx.sm_phase(kSmFirstMmaDone);
         if (t.parts > 1u) {
             // A part of a remainder tile: [part SM][row of the expert][weight row] flagged fp32 words; the group's first SM adds.
-            // (The multi-rank kernel leaves plain partial sums in this region. Read as a float a launch number is a denormal,
-            // which a sum of block-scaled products is only where the scales themselves have underflowed.)
             const uint32_t first = c.split_first;
-            auto part_word = [&](uint32_t sm, uint32_t i) { return p.buf + p.off_red + ((static_cast<size_t>(sm) * kDEntries + i) * kTileRows + etid) * 8u; };
+            auto part_word = [&](uint32_t sm, uint32_t i) { return p.buf + p.off_parts + ((static_cast<size_t>(sm) * kDEntries + i) * kTileRows + etid) * 8u; };
             if (blockIdx.x != first) {
                 #pragma unroll 1
                 for (uint32_t i = 0; i < nv; ++i) st_volatile_v2(part_word(blockIdx.x, i), __float_as_uint(vt_w[(c0 + i) * kBVtStride]), flag);

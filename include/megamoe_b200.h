@@ -54,7 +54,8 @@ typedef struct mm_layout {
     int64_t off_mid_sf;        /* [mid_rows][intermediate / 64] flagged words {scale bytes of 64 columns, launch flag} */
     int64_t off_comb;          /* [T_max][topk][hidden] bf16 expert outputs written back by the peers, as flagged 8-byte words
                                   {2 bf16, launch flag}: 4 bytes per element */
-    int64_t off_red;           /* [256 SMs][2 phases][2][16][128] float partial sums of weight tiles split between SMs (local) */
+    int64_t off_red;           /* [256 SMs][2 phases][2][16][128] float partial sums of weight tiles split between SMs (local); behind the
+                                  32 KB per SM of the launch's grid the one-rank decode kernel's, as flagged 8-byte words */
     int64_t off_cnt;           /* [2 phases][cnt_per_phase] uint32 contributors that have parked their part of a tile (local) */
     int64_t off_logits;        /* [min(T_max, 256)][num_experts] 16 B records {half logit, launch flag} x 2 of the fused router frontend */
     int64_t x_row_bytes, x_sf_row_bytes;

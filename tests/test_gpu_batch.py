@@ -398,3 +398,29 @@ def test_launches_with_mapped_inputs_alternate_with_the_one_rank_kernels(fmt):
         st, words = buf.device_status()
         assert st == 0 and words[1] == it + 1 and words[4] == (MULTI_RANK if mapped else (BATCH if tokens * topk > 16 else DECODE))
         assert O.rel_rmse(y.cpu(), ref.y[0]) <= REL_RMSE_TOL, (it, tokens, mapped)
+
+
+@pytest.mark.parametrize('fmt', ['mxfp4', 'nvfp4', 'fp8'])
+def test_partial_sums_of_the_multi_rank_kernel_are_not_taken_for_the_decode_kernels(fmt):
+    """The multi-rank kernel keeps plain fp32 sums in the split-tile region: 32 KB per SM, any bit pattern, the next launch's number
+    among them. The decode kernel's flagged words lie elsewhere in the region."""
+    e, hidden, inter, topk, tokens = 8, 1024, 512, 8, 1
+    w, gs1, gs2 = O.make_expert_weights(e, hidden, inter, fmt, seed=150, std=0.05)
+    l1, l2 = mm.transform_weights_for_mega_moe(*U.to_operator_weights(w, fmt, 'cuda'))
+    buf = mm.get_symm_buffer_for_mega_moe(None, e, 16, topk, hidden, inter, act_format=fmt)
+    idx, tw = U.random_routing(tokens, e, topk, 151)
+    _, inp, sfb = U.make_rank_inputs(tokens, hidden, fmt, 152, idx, tw)
+    ref = O.moe_layer_reference([inp], [w], fmt, e, clamp=None, w1_global_scale=gs1, w2_global_scale=gs2)
+    U.write_inputs(buf, inp, sfb)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    off = int(buf.layout.off_red)
+    sums = buf.buffer[off:off + sms * 32768].view(torch.int32)
+    y = torch.empty((tokens, hidden), dtype=torch.bfloat16, device='cuda')
+    call = mm.fp8_fp4_mega_moe if fmt == 'fp8' else mm.fp4_fp4_mega_moe
+    kw = dict(l1_global_scale=gs1, l2_global_scale=gs2) if fmt == 'nvfp4' else {}
+    for launch in range(1, 9):
+        sums.fill_(launch)
+        call(y, l1, l2, buf, timeout_ms=500.0, **kw)
+        st, words = buf.device_status()
+        assert st == 0 and words[4] == DECODE and words[1] == launch
+        assert bool((sums == launch).all()) and O.rel_rmse(y.cpu(), ref.y[0]) <= REL_RMSE_TOL
