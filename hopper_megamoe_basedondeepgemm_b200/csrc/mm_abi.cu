@@ -431,15 +431,15 @@ static bool wants_batch_kernel(const mm_launch_args_t* a, const mm::KParams& p) 
     return tiles <= mm::kBMaxTiles;
 }
 
-// The decode kernel (mm_decode.cuh) takes the launches up to there. The token tile and, with E4M3 tokens, the widened units
-// have to leave it a ring of three weight stages; wider layers stay with the multi-rank kernel, as inputs in host memory do.
+// The decode kernel (mm_decode.cuh) takes the launches up to there. The token tile has to leave it a
+// ring of three weight stages (four with E4M3 tokens); wider layers stay with the multi-rank kernel, as inputs in host memory do.
 static bool wants_decode_kernel(const mm_config_t* cfg, const mm_launch_args_t* a, const mm::KParams& p, int grid) {
     if (p.R != 1 || a->input_region != nullptr || a->engine != MM_ENGINE_UMMA || p.T == 0) return false;
     if ((p.knobs & mm::kKnobDecode) == 0u || static_cast<long long>(p.T) * p.topk > mm::kDEntries || !decode_parts_fit(grid)) return false;
     const bool a8 = cfg->act_format == MM_FMT_FP8;
     const int planes = mm::kUnitK / (4 * sf_vec_of(cfg->act_format));
     const long long tiles = static_cast<long long>(p.k1_units > p.k2_units ? p.k1_units : p.k2_units) * (2048 * (a8 ? 2 : 1) + planes * 512);
-    return tiles + (a8 ? 2 * mm::kXbufBytes : 0) + 3ll * p.unit_bytes <= 232448 - static_cast<long long>(sizeof(mm::DShared)) - 256 - 1024;
+    return tiles + (a8 ? 4ll : 3ll) * p.unit_bytes <= 232448 - static_cast<long long>(sizeof(mm::DShared)) - 256 - 1024;
 }
 
 static mm::BParams one_rank_params(const mm_config_t* cfg, const mm::KParams& k, int grid) {
@@ -450,7 +450,7 @@ static mm::BParams one_rank_params(const mm_config_t* cfg, const mm::KParams& k,
     p.T = k.T; p.topk = k.topk; p.E = k.e_local; p.H = k.H; p.I = k.I;
     p.n1 = k.n1_tiles; p.n2 = k.n2_tiles; p.k1 = k.k1_units; p.k2 = k.k2_units;
     p.unit_bytes = k.unit_bytes;
-    p.tile_limit = cfg->act_format == MM_FMT_FP8 ? 96u : 128u;         // (E4M3: a wider record would leave too few weight stages beside the widened units)
+    p.tile_limit = cfg->act_format == MM_FMT_FP8 ? 96u : 128u;         // (E4M3: a record has twice the bytes)
     p.x_row_bytes = k.x_row_bytes; p.x_sf_row_bytes = k.x_sf_row_bytes; p.rx_row_bytes = k.rx_row_bytes; p.mid_row_bytes = k.mid_row_bytes;
     p.has_clamp = k.has_clamp; p.fast_math = k.fast_math; p.clamp = k.clamp;
     p.l1_scale = k.l1_scale; p.l2_scale = k.l2_scale; p.mid_gs = k.mid_gs; p.mid_gs_recip = k.mid_gs >= 0x1p-40f && k.mid_gs <= 0x1p40f ? 1.0f / k.mid_gs : 0.f;

@@ -22,8 +22,8 @@
 //
 // Bound: HBM (the weights of the live experts once) up to about 40 rows per expert; beyond that the bytes an SM takes in
 // per unit (weights + token record, about 48 GB/s from the L2). 64 tokens, MXFP4, 48 experts (301 MB): 60 us a pass, of
-// which the stream is 46; the multi-rank kernel takes 88. With E4M3 tokens: the units widened in shared memory, 0.62 us
-// each (100 tokens: 91 us, 765 with the multi-rank kernel).
+// which the stream is 46; the multi-rank kernel takes 88. With E4M3 tokens the units are widened into tensor memory,
+// which keeps up with the stream (100 tokens: 67.7 us, 765 with the multi-rank kernel).
 #pragma once
 #include "mm_kernel.cuh"
 
@@ -45,6 +45,8 @@ constexpr int kBThreadsA8 = 32 * (kBServiceWarps + kBEpiWarps + kBExpWarps);
 constexpr int kBColCounters = 32;                  // column blocks of 128 (hidden <= 4096)
 constexpr int kBCounts = kBColCounters + 32;       // counters of a launch besides the tiles': the column blocks', the claimed L2 tasks
 constexpr uint32_t kBVtStride = 152;               // floats between the tokens of `vt`
+// tensor-memory columns with E4M3 tokens: scales of the weights and of the tokens (two areas of 8 each), widened units (two of 64)
+constexpr uint32_t kTmScaleW = 256, kTmScaleX = 272, kTmWide = 384;
 constexpr uint32_t kBBarEpi0 = 1, kBBarEpi1 = 2, kBBarWork = 3, kBBarTiles = 4;    // named barriers
 
 struct BParams {
@@ -64,7 +66,7 @@ struct BParams {
     long long off_mid, off_mid_sf, off_parts;      // flagged words of the decode kernel: intermediate rows, their scale bytes, partial sums
     uint32_t mid_row_bytes;
     FeParams fe;
-    uint32_t smem_ring;                            // bytes of dynamic shared memory for the two rings (and the widened units)
+    uint32_t smem_ring;                            // bytes of dynamic shared memory for the two rings
     unsigned long long timeout_ns;
 };
 
@@ -344,9 +346,9 @@ __device__ void b_role_mma(const BCtx& cx, uint32_t lane) {
     const BParams& p = cx.p; BShared& c = cx.c;
     // Everything the instructions below take as operands is broadcast from lane 0, which tells the compiler that it is the
     // same in all lanes: the operands then stay in uniform registers. (A unit of 4 MMAs, 4 scale copies and a commit goes out in
-    // 210 cycles with 16 rows and 257 with 96: the tensor pipe itself needs 199 and 256. E4M3 tokens, 16 to 32 rows: 525, the pipe 345 to 365.)
+    // 210 cycles with 16 rows and 257 with 96: the tensor pipe itself needs 199 and 256. E4M3 tokens: 206 for 16 rows, 480 for 96.)
     const uint32_t nr = b_uniform(c.nr), slot_bytes = b_uniform(c.slot_bytes), step = b_uniform(c.spu), tm = b_uniform(c.tmem_base);
-    const uint32_t rec0 = b_uniform(smem_u32(cx.smem)), ring0 = rec0 + nr * slot_bytes, x0 = ring0 + b_uniform(c.nw) * p.unit_bytes;
+    const uint32_t rec0 = b_uniform(smem_u32(cx.smem)), ring0 = rec0 + nr * slot_bytes;
     uint32_t it = 0, rs = 0, rph = 0;                                   // units consumed; record slot (without widening also weight stage), its phase bit
     BTasks tasks(cx);
     #pragma unroll 1
@@ -378,23 +380,24 @@ __device__ void b_role_mma(const BCtx& cx, uint32_t lane) {
                     for (uint32_t uu = 0; uu < (kA8 ? 1u : 2u); ++uu) {
                         if (uu < step && u0 + uu < units) {
                             const uint32_t i = it + b * step + uu;
-                            const uint32_t wsm = kA8 ? x0 + (i & 1u) * kXbufBytes : wsm0 + uu * p.unit_bytes, tok = tok0 + uu * rec;
+                            const uint32_t wsm = wsm0 + uu * p.unit_bytes, tok = tok0 + uu * rec;      // (E4M3 tokens: weights and their scales are in tensor memory)
                             const uint64_t adesc = smem_desc(wsm, 1024u, kLayoutSw128), bdesc = smem_desc(tok, 1024u, kLayoutSw128);
-                            const uint64_t asf = smem_desc(wsm + (kA8 ? 2u * kUnitWBytes : static_cast<uint32_t>(kUnitWBytes)), 128u, kLayoutNone);
+                            const uint64_t asf = smem_desc(wsm + kUnitWBytes, 128u, kLayoutNone);
                             const uint64_t bsf = smem_desc(tok + atom * F::kAtoms, 128u, kLayoutNone);
-                            const uint32_t sfa = tm + 256u + (i & 1u) * 32u, sfb = sfa + 16u;
+                            const uint32_t sfa = kA8 ? tm + kTmScaleW + (i & 1u) * 8u : tm + 256u + (i & 1u) * 32u, sfb = kA8 ? tm + kTmScaleX + (i & 1u) * 8u : sfa + 16u;
+                            const uint32_t wide = tm + kTmWide + (i & 1u) * 64u;
                             #pragma unroll
                             for (uint32_t pl = 0; pl < kPlanes; ++pl) {
-                                utccp_32x128b_warpx4(sfa + pl * 4u, asf + pl * 32u);
+                                if constexpr (!kA8) utccp_32x128b_warpx4(sfa + pl * 4u, asf + pl * 32u);
                                 utccp_32x128b_warpx4(sfb + pl * 4u, bsf + pl * 32u);
                             }
                             #pragma unroll
                             for (uint32_t ks = 0; ks < kUnitK / kStepK; ++ks) {
                                 const uint32_t pl = (ks * kStepK) / (4u * F::kVec), sf_id = ((ks * kStepK) % (4u * F::kVec)) / F::kVec;
-                                const uint64_t ad = adesc + (ks & 3u) * 2u + (kA8 ? (ks >> 2) * (kUnitWBytes >> 4) : 0u);
+                                const uint64_t ad = adesc + (ks & 3u) * 2u;
                                 const uint64_t bd = bdesc + (ks & 3u) * 2u + (kA8 ? (ks >> 2) * (atom >> 4) : 0u);
                                 const uint32_t idesc = idesc_with_sf(idesc_n, sf_id, sf_id), accum = (u0 | uu | ks) != 0u ? 1u : 0u;
-                                if constexpr (kA8) umma_mxf8f6f4(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
+                                if constexpr (kA8) umma_mxf8f6f4_ta(d, wide + ks * 8u, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
                                 else if constexpr (kFmt == 0) umma_mxf4_block32(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
                                 else umma_nvf4_block16(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
                             }
@@ -417,45 +420,61 @@ __device__ void b_role_mma(const BCtx& cx, uint32_t lane) {
 }
 
 // ============================================================================================= weight widener (E4M3 tokens)
-// kind::mxf8f6f4 reads 4-bit operands from byte-wide slots: every 16 E2M1 values (8 bytes) sit in a 16-byte slot. kThreads
-// threads turn a packed unit (128 rows x 128 B) into two atoms of 128 rows x 128 B.
-// Eight lanes read the eight chunks of a row and store the two halves of each; the lanes of the second atom store theirs in
-// the other order, so that the eight stores of a quarter-warp fall on different banks.
-template <uint32_t kThreads>
+// kind::mxf8f6f4 wants a byte per weight. Two groups of four warps take the units in turn and write them into tensor memory,
+// where the MMAs read their A operand: a thread reads the 128 packed bytes of its weight row and stores 64 columns of E2M1
+// codes in bytes, the form in which tcgen05.cp would decompress them (code in bits 2 to 5). The unit's scale planes go the same way, in
+// the layout that the scale copy would give them. Measured for one SM, cycles a unit: 313 with both groups (one group 508; codes turned into E4M3 bytes
+// by byte permutes, in order, 669; by shifts and masks 435), beside MMAs of 206 (16 rows) to 480 (96), which take 431 to 731 with A in shared
+// memory. HBM brings a unit in 790. Widened in shared memory (16 KB read, 32 KB written, those read again by
+// the tensor core, and a proxy fence) a unit took 1200: 2 tokens 37.7 -> 31.9 us a pass, 100 tokens 91.4 -> 67.7.
+// Shifts and masks alone leave the codes of the even elements in one word and those of the odd ones in the next: the token
+// images have every eight elements of a row in the same order (`even_odd`).
+constexpr uint32_t kXGroupThreads = 128;
+// eight E2M1 codes -> eight bytes with the code in bits 2..5, those of the even elements first: two shifts and two masks
+__device__ __forceinline__ void widen8(uint32_t w, uint32_t& even, uint32_t& odd) {
+    even = (w << 2) & 0x3C3C3C3Cu;
+    odd = (w >> 2) & 0x3C3C3C3Cu;
+}
+// the same order of eight consecutive E4M3 bytes
+__device__ __forceinline__ uint2 even_odd(uint32_t a, uint32_t b) { return make_uint2(__byte_perm(a, b, 0x6420u), __byte_perm(a, b, 0x7531u)); }
+__device__ __forceinline__ uint4 even_odd(const uint4& v) {
+    const uint2 a = even_odd(v.x, v.y), b = even_odd(v.z, v.w);
+    return make_uint4(a.x, a.y, b.x, b.y);
+}
 struct BWiden {
-    static constexpr uint32_t kItems = kTileRows * 8 / kThreads;
-    uint4 v[kItems], sf;
-    __device__ __forceinline__ void load(const uint8_t* wsm, uint32_t xtid) {
-        const uint32_t ch = xtid & 7u;
+    uint4 v[8], sf[2];
+    __device__ __forceinline__ void load(const uint8_t* wsm, uint32_t row) {
         #pragma unroll
-        for (uint32_t k = 0; k < kItems; ++k) {
-            const uint32_t r = k * (kThreads / 8) + (xtid >> 3);
-            v[k] = *reinterpret_cast<const uint4*>(wsm + r * 128u + ((ch ^ (r & 7u)) << 4));
-        }
-        if (xtid < 64u) sf = *reinterpret_cast<const uint4*>(wsm + kUnitWBytes + xtid * 16u);
+        for (uint32_t c = 0; c < 8; ++c) v[c] = *reinterpret_cast<const uint4*>(wsm + row * 128u + ((c ^ (row & 7u)) << 4));
+        #pragma unroll
+        for (uint32_t pl = 0; pl < 2; ++pl) sf[pl] = *reinterpret_cast<const uint4*>(wsm + kUnitWBytes + pl * 512u + (row & 31u) * 16u);
     }
-    __device__ __forceinline__ void store(uint8_t* xb, uint32_t xtid) const {
-        const uint32_t ch = xtid & 7u, at = ch >> 2, j = 2u * (ch & 3u);
+    // (`ta`, `tsf`: columns, with the first of the warp's lanes)
+    __device__ __forceinline__ void store(uint32_t ta, uint32_t tsf) const {
         #pragma unroll
-        for (uint32_t k = 0; k < kItems; ++k) {
-            const uint32_t r = k * (kThreads / 8) + (xtid >> 3);
-            uint8_t* row = xb + at * kUnitWBytes + r * 128u;
-            const uint32_t first = (j + at) ^ (r & 7u), second = (j + 1u - at) ^ (r & 7u);
-            *reinterpret_cast<uint4*>(row + (first << 4)) = at ? make_uint4(v[k].z, v[k].w, 0u, 0u) : make_uint4(v[k].x, v[k].y, 0u, 0u);
-            *reinterpret_cast<uint4*>(row + (second << 4)) = at ? make_uint4(v[k].x, v[k].y, 0u, 0u) : make_uint4(v[k].z, v[k].w, 0u, 0u);
+        for (uint32_t c = 0; c < 8; c += 2) {
+            uint32_t r[16];
+            #pragma unroll
+            for (uint32_t h = 0; h < 2; ++h) {
+                const uint4 q = v[c + h];
+                widen8(q.x, r[8 * h], r[8 * h + 1]); widen8(q.y, r[8 * h + 2], r[8 * h + 3]);
+                widen8(q.z, r[8 * h + 4], r[8 * h + 5]); widen8(q.w, r[8 * h + 6], r[8 * h + 7]);
+            }
+            tmem_st_32x32b_x16(ta + c * 8u, r);
         }
-        if (xtid < 64u) *reinterpret_cast<uint4*>(xb + 2 * kUnitWBytes + xtid * 16u) = sf;
+        tmem_st_32x32b_x8(tsf, sf[0], sf[1]);
+        tmem_st_wait();
+        tc_fence_before();
     }
 };
 
-// All eight warps on one unit after the other: the next one is read from the ring while the tensor core has this one. (Two
-// groups of four on alternate units, which the decode kernel prefers, keep more of a unit in registers here and want an even
-// ring: 100 tokens 91.8 us, this way 90.9.)
-__device__ void b_role_widen(const BCtx& cx, uint32_t xtid) {
+// The ring has an even number of stages, so that a stage always belongs to the same group: a group that skipped a stage's
+// previous use could take the older phase of its barrier for the one it wants.
+__device__ void b_role_widen(const BCtx& cx, uint32_t grp, uint32_t xtid) {
     const BParams& p = cx.p; BShared& c = cx.c;
     const uint32_t lane = xtid & 31u, nw = c.nw;
-    uint8_t* ring = cx.smem + c.nr * c.slot_bytes;
-    uint8_t* xb = ring + static_cast<size_t>(nw) * p.unit_bytes;
+    const uint8_t* ring = cx.smem + c.nr * c.slot_bytes;
+    const uint32_t tm = c.tmem_base + ((xtid & 96u) << 16), ta = tm + kTmWide + grp * 64u, tsf = tm + kTmScaleW + grp * 8u;
     uint32_t it = 0, s = 0, ph = 0;
     BTasks tasks(cx);
     #pragma unroll 1
@@ -465,17 +484,18 @@ __device__ void b_role_widen(const BCtx& cx, uint32_t xtid) {
         const uint32_t units = (t >> 28) ? p.k2 : p.k1;
         #pragma unroll 1
         for (uint32_t u = 0; u < units; ++u, ++it) {
-            if (!cx.warp_wait(&c.wfull[s], ph, kErrWaitFull)) return;
-            BWiden<32 * kBExpWarps> w;
-            w.load(ring + static_cast<size_t>(s) * p.unit_bytes, xtid);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&c.wempty[s]);        // (the unit is in registers: its stage can be refilled)
-            const uint32_t b = it & 1u;
-            if (!cx.warp_wait(&c.xempty[b], ((it >> 1) & 1u) ^ 1u, kErrWaitEmpty)) return;
-            w.store(xb + b * kXbufBytes, xtid);
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&c.xfull[b]);
+            if ((it & 1u) == grp) {
+                if (!cx.warp_wait(&c.wfull[s], ph, kErrWaitFull)) return;
+                BWiden w;
+                w.load(ring + static_cast<size_t>(s) * p.unit_bytes, xtid);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&c.wempty[s]);        // (the unit is in registers: its stage can be refilled)
+                if (!cx.warp_wait(&c.xempty[grp], ((it >> 1) & 1u) ^ 1u, kErrWaitEmpty)) return;
+                tc_fence_after();
+                w.store(ta, tsf);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&c.xfull[grp]);
+            }
             if (++s == nw) { s = 0; ph ^= 1u; }
         }
     }
@@ -638,8 +658,8 @@ __device__ void b_role_epilogue(const BCtx& cx, uint32_t grp, uint32_t etid) {
                 if (live) {
                     if constexpr (kA8) {
                         uint8_t* at = img + ((j >> 1) & 1u) * a16 * 2048u + sw128_off(n, (j & 1u) * 4u + (q >> 1)) + (q & 1u) * 8u;
-                        *reinterpret_cast<uint2*>(at) = make_uint2(cvt_e4m3x2(o[0], o[1]) | (cvt_e4m3x2(o[2], o[3]) << 16),
-                                                                   cvt_e4m3x2(o[4], o[5]) | (cvt_e4m3x2(o[6], o[7]) << 16));
+                        *reinterpret_cast<uint2*>(at) = make_uint2(cvt_e4m3x2(o[0], o[2]) | (cvt_e4m3x2(o[4], o[6]) << 16),
+                                                                   cvt_e4m3x2(o[1], o[3]) | (cvt_e4m3x2(o[5], o[7]) << 16));    // (see widen8)
                     } else {
                         uint8_t* at = img + sw128_off(n, (j & 3u) * 2u + (q >> 2)) + (q & 3u) * 4u;
                         *reinterpret_cast<uint32_t*>(at) = cvt_e2m1x2(o[0], o[1]) | (cvt_e2m1x2(o[2], o[3]) << 8) |
@@ -789,11 +809,12 @@ __device__ __forceinline__ void b_tiles(const BCtx& cx, uint32_t lane) {
         // weights stream. A stage holds two K units where four such stages fit (narrow tiles): the MMA warp's barrier waits
         // and loop cost more than its issue, and this halves them.
         const uint32_t rec = (max16 ? max16 : 1u) * 2048u * F::kAtoms + F::kPlanes * 512u;
-        const uint32_t room = p.smem_ring - (F::kA8 ? 2u * kXbufBytes : 0u), pair = p.unit_bytes + rec;
-        const uint32_t spu = pair * 8u <= room ? 2u : 1u;
+        const uint32_t room = p.smem_ring, pair = p.unit_bytes + rec;
+        const uint32_t spu = !F::kA8 && pair * 8u <= room ? 2u : 1u;
         uint32_t nr = udiv_small(room, pair * spu), nw = nr;
-        if (F::kA8) {                                        // single-unit weight stages beside two or three records at least
-            nw = udiv_small(room - (rec > 12288u ? 2u : 3u) * rec, p.unit_bytes);
+        if (F::kA8) {                                        // rings of their own; an even number of weight stages (see b_role_widen)
+            nw = udiv_small(room, pair) & ~1u;
+            nw = nw < 4u ? 4u : (nw > kBWStages ? kBWStages : nw);
             nr = udiv_small(room - nw * p.unit_bytes, rec);
         }
         nr = nr > kBRSlots ? kBRSlots : nr;
@@ -816,11 +837,11 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
     const uint32_t ww = warp - kBServiceWarps;
     // ---- what needs nothing of the launches before this one: it overlaps the end of the previous kernel in the stream
     if (warp == 2) {
-        if (lane < kBWStages) { mbar_init(&c.wfull[lane], 1); mbar_init(&c.wempty[lane], F::kA8 ? kBExpWarps : 1); }
+        if (lane < kBWStages) { mbar_init(&c.wfull[lane], 1); mbar_init(&c.wempty[lane], F::kA8 ? kBExpWarps / 2 : 1); }
         if (lane < kBRSlots) { mbar_init(&c.rfull[lane], F::kA8 ? 1 : 2); mbar_init(&c.rempty[lane], 1); }
         if (lane < 2) {
             mbar_init(&c.tmem_full[lane], 1); mbar_init(&c.tmem_empty[lane], 4);
-            mbar_init(&c.xfull[lane], kBExpWarps); mbar_init(&c.xempty[lane], 1);
+            mbar_init(&c.xfull[lane], kBExpWarps / 2); mbar_init(&c.xempty[lane], 1);
         }
         c.task[lane] = 0u; c.task[lane + 32] = 0u;
         mbar_fence_init();
@@ -1032,7 +1053,7 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
                     const uint32_t ci = lane + u * 32;
                     if (ci < xq) {
                         const uint32_t at = ci >> 3;                                          // 128 B atom of the row
-                        *reinterpret_cast<uint4*>(img + (F::kA8 ? (at >> 1) * rec + (at & 1u) * a16 * 2048u : at * rec) + sw128_off(n, ci & 7u)) = row[u];
+                        *reinterpret_cast<uint4*>(img + (F::kA8 ? (at >> 1) * rec + (at & 1u) * a16 * 2048u : at * rec) + sw128_off(n, ci & 7u)) = F::kA8 ? even_odd(row[u]) : row[u];
                     } else if (ci < per_row) {
                         const uint32_t g = (ci - xq) * 4u;                                    // scale words g .. g + 3: unit g / planes, plane g % planes
                         const uint32_t wv[4] = {row[u].x, row[u].y, row[u].z, row[u].w};
@@ -1095,7 +1116,7 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
         else if (warp >= kBServiceWarps && warp < kBServiceWarps + kBEpiWarps)
             b_role_epilogue<kFmt, kFe>(cx, (warp - kBServiceWarps) >> 2, tid - 32u * kBServiceWarps - ((warp - kBServiceWarps) >> 2) * 128u);
         else if (warp >= kBServiceWarps + kBEpiWarps) {
-            if constexpr (F::kA8) b_role_widen(cx, tid - 32u * (kBServiceWarps + kBEpiWarps));
+            if constexpr (F::kA8) { const uint32_t x = tid - 32u * (kBServiceWarps + kBEpiWarps); b_role_widen(cx, x / kXGroupThreads, x % kXGroupThreads); }
         }
     }
     if (tid == 128) { cx.stamp_max(kStampLastTasksDone); cx.sm_phase(kSmTasksDone); if (bid == 0) cx.stamp(kStampTasksDone); }

@@ -22,7 +22,6 @@ constexpr uint32_t kDEntries = 16;                 // routing entries (= rows) o
 constexpr int kDEpiWarps = 8;                      // warps 4..11: build the token tiles, two epilogue groups
 constexpr int kDThreads = 32 * (4 + kDEpiWarps);
 constexpr int kDThreadsA8 = kDThreads + 32 * kBExpWarps;     // E4M3 tokens: widening warps 12..19
-constexpr uint32_t kDWidenThreads = kBExpWarps * 16;         // of one of their two groups
 constexpr int kDStages = 12;
 constexpr uint32_t kDBarGroups = 5, kDBarRouted = 6;
 
@@ -46,6 +45,7 @@ struct DCtx : BCore {
 
 template <int kFmt> struct DFmt : BFmt<kFmt> {
     static constexpr int kThreads = BFmt<kFmt>::kA8 ? kDThreadsA8 : kDThreads;
+    static constexpr uint32_t kTmemColumns = BFmt<kFmt>::kA8 ? 512u : 128u;
     static constexpr uint32_t kRec = 2048u * BFmt<kFmt>::kAtoms + BFmt<kFmt>::kPlanes * 512u;     // one K unit of the 16-row tile
 };
 
@@ -118,7 +118,7 @@ __device__ void d_role_mma(const DCtx& cx, uint32_t lane, uint32_t nw_, uint32_t
     const BParams& p = cx.p; DShared& c = cx.c;
     // (operands broadcast from lane 0: uniform registers, see the batch kernel's issuer)
     const uint32_t nw = b_uniform(nw_), tm = b_uniform(c.tmem_base);
-    const uint32_t s0 = b_uniform(smem_u32(cx.smem)), ring0 = s0 + b_uniform(ring_off), x0 = ring0 + nw * p.unit_bytes;
+    const uint32_t s0 = b_uniform(smem_u32(cx.smem)), ring0 = s0 + b_uniform(ring_off);
     uint32_t it = 0, s = 0, ph = 0, wsm0 = ring0;
     bool have1 = false, have2 = false;
     DTasks tasks(cx);
@@ -139,23 +139,23 @@ __device__ void d_role_mma(const DCtx& cx, uint32_t lane, uint32_t nw_, uint32_t
             tc_fence_after();
             if (lane == 0 && it == 0u) cx.sm_phase(kSmFirstLanded);
             if (elect_one()) {
-                const uint32_t wsm = kA8 ? x0 + (it & 1u) * kXbufBytes : wsm0;
-                const uint64_t adesc = smem_desc(wsm, 1024u, kLayoutSw128), bdesc = smem_desc(tok, 1024u, kLayoutSw128);
-                const uint64_t asf = smem_desc(wsm + (kA8 ? 2u * kUnitWBytes : static_cast<uint32_t>(kUnitWBytes)), 128u, kLayoutNone);
+                const uint64_t adesc = smem_desc(wsm0, 1024u, kLayoutSw128), bdesc = smem_desc(tok, 1024u, kLayoutSw128);
+                const uint64_t asf = smem_desc(wsm0 + kUnitWBytes, 128u, kLayoutNone);
                 const uint64_t bsf = smem_desc(tok + 2048u * F::kAtoms, 128u, kLayoutNone);
-                const uint32_t sfa = tm + 32u + (it & 1u) * 32u, sfb = sfa + 16u;
+                const uint32_t sfa = kA8 ? tm + kTmScaleW + (it & 1u) * 8u : tm + 32u + (it & 1u) * 32u, sfb = kA8 ? tm + kTmScaleX + (it & 1u) * 8u : sfa + 16u;
+                const uint32_t wide = tm + kTmWide + (it & 1u) * 64u;
                 #pragma unroll
                 for (uint32_t pl = 0; pl < kPlanes; ++pl) {
-                    utccp_32x128b_warpx4(sfa + pl * 4u, asf + pl * 32u);
+                    if constexpr (!kA8) utccp_32x128b_warpx4(sfa + pl * 4u, asf + pl * 32u);
                     utccp_32x128b_warpx4(sfb + pl * 4u, bsf + pl * 32u);
                 }
                 #pragma unroll
                 for (uint32_t ks = 0; ks < kUnitK / kStepK; ++ks) {
                     const uint32_t pl = (ks * kStepK) / (4u * F::kVec), sf_id = ((ks * kStepK) % (4u * F::kVec)) / F::kVec;
-                    const uint64_t ad = adesc + (ks & 3u) * 2u + (kA8 ? (ks >> 2) * (kUnitWBytes >> 4) : 0u);
+                    const uint64_t ad = adesc + (ks & 3u) * 2u;
                     const uint64_t bd = bdesc + (ks & 3u) * 2u + (kA8 ? (ks >> 2) * (2048u >> 4) : 0u);
                     const uint32_t idesc = idesc_with_sf(kIdesc, sf_id, sf_id), accum = (u != ub || ks != 0u) ? 1u : 0u;
-                    if constexpr (kA8) umma_mxf8f6f4(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
+                    if constexpr (kA8) umma_mxf8f6f4_ta(d, wide + ks * 8u, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
                     else if constexpr (kFmt == 0) umma_mxf4_block32(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
                     else umma_nvf4_block16(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
                 }
@@ -171,15 +171,11 @@ __device__ void d_role_mma(const DCtx& cx, uint32_t lane, uint32_t nw_, uint32_t
     if (lane == 0 && it != 0u) cx.stamp_max(kStampLastWeight);
 }
 
-// The widening warps' loop (E4M3 tokens) over this kernel's tasks. Two groups of four warps take the units in turn, each into a
-// buffer of its own: a group's barrier waits and its proxy fence (400 cycles of a unit's 1200) lie beside the other's copying
-// (two tokens: 37.0 us a pass, 38.7 with all eight warps on one unit). A free buffer is awaited before the unit: it
-// says that the MMAs of the unit two before are over, so every earlier use of the stage (three or more units back) has landed
-// and been read. Whatever the depth of the ring, a group therefore never takes an older phase of the barrier for its own.
-__device__ void d_role_widen(const DCtx& cx, uint32_t grp, uint32_t xtid, uint32_t nw, uint8_t* ring) {
+// The widening warps' loop (E4M3 tokens, see b_role_widen) over this kernel's tasks; the ring is even here too.
+__device__ void d_role_widen(const DCtx& cx, uint32_t grp, uint32_t xtid, uint32_t nw, const uint8_t* ring) {
     const BParams& p = cx.p; DShared& c = cx.c;
     const uint32_t lane = xtid & 31u;
-    uint8_t* xb = ring + static_cast<size_t>(nw) * p.unit_bytes + grp * kXbufBytes;
+    const uint32_t tm = c.tmem_base + ((xtid & 96u) << 16), ta = tm + kTmWide + grp * 64u, tsf = tm + kTmScaleW + grp * 8u;
     uint32_t it = 0, s = 0, ph = 0;
     DTasks tasks(cx);
     #pragma unroll 1
@@ -189,14 +185,14 @@ __device__ void d_role_widen(const DCtx& cx, uint32_t grp, uint32_t xtid, uint32
         #pragma unroll 1
         for (uint32_t u = t.ub; u < t.ue; ++u, ++it) {
             if ((it & 1u) == grp) {
-                if (!cx.warp_wait(&c.xempty[grp], ((it >> 1) & 1u) ^ 1u, kErrWaitEmpty)) return;
                 if (!cx.warp_wait(&c.wfull[s], ph, kErrWaitFull)) return;
-                BWiden<kDWidenThreads> w;
+                BWiden w;
                 w.load(ring + static_cast<size_t>(s) * p.unit_bytes, xtid);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&c.wempty[s]);
-                w.store(xb, xtid);
-                fence_proxy_async_smem();
+                if (!cx.warp_wait(&c.xempty[grp], ((it >> 1) & 1u) ^ 1u, kErrWaitEmpty)) return;
+                tc_fence_after();
+                w.store(ta, tsf);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&c.xfull[grp]);
             }
@@ -237,7 +233,7 @@ __device__ __forceinline__ bool d_gather(const DCtx& cx, uint8_t* tile, uint32_t
             if (i < n) {
                 const uint32_t col = udiv_small(i, pieces), pc = i - col * pieces, ci = pc >> 1, at = ci >> 3;       // 16 B chunk, 128 B atom of the row
                 uint8_t* dst = tile + (F::kA8 ? (at >> 1) * F::kRec + (at & 1u) * 2048u : at * F::kRec) + sw128_off(col, ci & 7u) + (pc & 1u) * 8u;
-                *reinterpret_cast<uint2*>(dst) = make_uint2(v[u].x, v[u].z);
+                *reinterpret_cast<uint2*>(dst) = F::kA8 ? even_odd(v[u].x, v[u].z) : make_uint2(v[u].x, v[u].z);
             }
         }
     }
@@ -473,10 +469,10 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, bid = blockIdx.x, G = gridDim.x;
     uint32_t* ctrl32 = reinterpret_cast<uint32_t*>(p.buf + p.off_ctrl);
     const uint32_t n = static_cast<uint32_t>(p.T) * p.topk;
-    // shared memory: token tile (the intermediate rows' tile takes the place of the tokens'), weight ring, widened units
+    // shared memory: token tile (the intermediate rows' tile takes the place of the tokens'), weight ring
     const uint32_t ring_off = (p.k1 > p.k2 ? p.k1 : p.k2) * F::kRec;
-    uint32_t nw = udiv_small(p.smem_ring - ring_off - (F::kA8 ? 2u * kXbufBytes : 0u), p.unit_bytes);
-    nw = nw > kDStages ? kDStages : nw;
+    uint32_t nw = udiv_small(p.smem_ring - ring_off, p.unit_bytes);
+    nw = nw > kDStages ? kDStages : (F::kA8 ? nw & ~1u : nw);
     // ---- what needs nothing of the launches before this one: it overlaps the end of the previous kernel in the stream
     if (warp == 2) {
         if (lane < kDStages) { mbar_init(&c.wfull[lane], 1); mbar_init(&c.wempty[lane], F::kA8 ? kBExpWarps / 2 : 1); }
@@ -489,7 +485,7 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
         if (lane < kDEntries) c.exp_n[lane] = 0u;
         if (lane == 0) { c.abort_flag = 0u; c.comb_next = 0u; c.wissued = 0u; c.start_ok = 0u; }
     }
-    if (warp == 1) { tmem_alloc(&c.tmem_base, 128); tmem_relinquish(); tc_fence_before(); }
+    if (warp == 1) { tmem_alloc(&c.tmem_base, F::kTmemColumns); tmem_relinquish(); tc_fence_before(); }
     __syncthreads();
     tc_fence_after();
     grid_dependency_wait();
@@ -619,7 +615,7 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
                             const uint32_t ci = lane + u * 32;
                             if (ci < xq) {
                                 const uint32_t at = ci >> 3;
-                                *reinterpret_cast<uint4*>(smem + (F::kA8 ? (at >> 1) * F::kRec + (at & 1u) * 2048u : at * F::kRec) + sw128_off(col, ci & 7u)) = v[a][u];
+                                *reinterpret_cast<uint4*>(smem + (F::kA8 ? (at >> 1) * F::kRec + (at & 1u) * 2048u : at * F::kRec) + sw128_off(col, ci & 7u)) = F::kA8 ? even_odd(v[a][u]) : v[a][u];
                             } else if (ci < per_row) {
                                 const uint32_t g = (ci - xq) * 4u;
                                 const uint32_t wv[4] = {v[a][u].x, v[a][u].y, v[a][u].z, v[a][u].w};
@@ -634,7 +630,7 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
                         for (uint32_t u = 0; u < 16; ++u) {
                             if (u < static_cast<uint32_t>(p.k1)) {
                                 uint8_t* rec = smem + u * F::kRec;
-                                if constexpr (F::kA8) *reinterpret_cast<uint2*>(rec + (lane >> 4) * 2048u + sw128_off(col, (lane >> 1) & 7u) + (lane & 1u) * 8u) = hb[a][u];
+                                if constexpr (F::kA8) *reinterpret_cast<uint2*>(rec + (lane >> 4) * 2048u + sw128_off(col, (lane >> 1) & 7u) + (lane & 1u) * 8u) = even_odd(hb[a][u].x, hb[a][u].y);
                                 else *reinterpret_cast<uint32_t*>(rec + sw128_off(col, lane >> 2) + (lane & 3u) * 4u) = hb[a][u].x;
                                 const uint32_t blk = lane / kLanes;
                                 if (lane % kLanes == 0u)
@@ -649,7 +645,7 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
             if (lane == 0) { mbar_arrive(&c.tile_full[0]); cx.sm_phase(kSmRowsCached); }
             d_role_epilogue<kFmt>(cx, (warp - kEW) >> 2, (tid - 32u * kEW) & 127u, smem, flag);
         } else if (warp >= kEW + kDEpiWarps) {
-            if constexpr (F::kA8) { const uint32_t x = tid - 32u * (kEW + kDEpiWarps); d_role_widen(cx, x / kDWidenThreads, x % kDWidenThreads, nw, smem + ring_off); }
+            if constexpr (F::kA8) { const uint32_t x = tid - 32u * (kEW + kDEpiWarps); d_role_widen(cx, x / kXGroupThreads, x % kXGroupThreads, nw, smem + ring_off); }
         }
     }
     // ---- off the critical path: launch number, counters, stamps, and what others may inspect afterwards
@@ -692,7 +688,7 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
         for (uint32_t spin = 0; spin < 2000u; ++spin) __nanosleep(100);
     }
     __syncthreads();
-    if (warp == 1) { tc_fence_after(); tmem_dealloc(c.tmem_base, 128); }
+    if (warp == 1) { tc_fence_after(); tmem_dealloc(c.tmem_base, F::kTmemColumns); }
     if (tid == 0) { if (bid == 0) cx.stamp(kStampExit); cx.stamp_max(kStampLastExit); cx.sm_phase(kSmExit); }
 }
 

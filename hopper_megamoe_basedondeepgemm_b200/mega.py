@@ -166,7 +166,8 @@ class SymmBuffer:
         """(rows uint8 [R, mid_row_bytes], scale words uint8 [R, words, 4]) of the latest launch of the one-rank batch
         kernel (csrc/mm_batch.cuh): an expert's rows start on a 16-row boundary, experts in ascending order. An expert's
         n rows form t = ceil(n / limit) token tiles of ceil(n / t) rows (rounded up to 16); a tile's image is one record
-        per K unit: its rows (a multiple of 16) x 128 B in the 128 B swizzle (E4M3: two such atoms), then the unit's scale
+        per K unit: its rows (a multiple of 16) x 128 B in the 128 B swizzle (E4M3: two such atoms, and of every eight elements
+        first the even ones), then the unit's scale
         planes of 512 B, the word of row r at (r % 32) * 16 + (r // 32) * 4. No rows for a launch that had none or has failed."""
         L = self.layout
         counts = [0] * self.num_experts
@@ -193,7 +194,10 @@ class SymmBuffer:
                 rows_out.append(torch.gather(tok, 3, stored).permute(2, 0, 1, 3, 4).reshape(r16, row_bytes))
                 slots = recs[:, r16 * 128 * atoms:].reshape(units, planes, 32, 4, 4)[:, :, r % 32, r // 32]
                 words_out.append(slots.permute(2, 0, 1, 3).reshape(r16, units * planes, 4))
-        return torch.cat(rows_out).contiguous(), torch.cat(words_out).contiguous()
+        rows = torch.cat(rows_out)
+        if self.act_format == 'fp8':
+            rows = rows.view(-1, row_bytes // 8, 8)[:, :, [0, 4, 1, 5, 2, 6, 3, 7]].reshape(-1, row_bytes)
+        return rows.contiguous(), torch.cat(words_out).contiguous()
 
     def l2_acts_payload(self) -> torch.Tensor:
         """The intermediate rows of the latest launch without flag words or swizzle: uint8 [mid_rows, mid_row_bytes]."""
@@ -479,7 +483,7 @@ def fp8_fp4_mega_moe(y: torch.Tensor, l1_weights, l2_weights, sym_buffer: SymmBu
 
     Tokens are E4M3 with one UE8M0 scale per 32 elements, the intermediate is requantised the same way, weights are
     the MXFP4 streams of `transform_weights_for_mega_moe`. The tensor cores read 4-bit operands of an 8-bit x 4-bit
-    product from byte-wide slots, so the kernel widens each streamed weight unit in shared memory; HBM traffic is
+    product from byte-wide slots, so the kernel widens each streamed weight unit on the SM; HBM traffic is
     that of the W4A4 variant.
     """
     assert sym_buffer.act_format == 'fp8', 'buffer must be created with act_format fp8'

@@ -28,6 +28,15 @@ def test_row_counts_around_the_tile_edges(fmt, e_local, topk, tokens):
     check_against_oracle(y, stats, ref, buf, fmt, 256)
 
 
+@pytest.mark.parametrize('e_local,hidden,inter,topk,tokens', [
+    (4, 4096, 768, 2, 8), (3, 512, 256, 3, 5), (2, 1536, 1280, 2, 1),          # decode kernel: the widest token tile; units per task odd and even
+    (4, 4096, 256, 2, 170), (3, 1536, 768, 3, 31), (8, 512, 256, 2, 12),       # batch kernel: 96-row records (fewest weight stages), 32- and 16-row ones
+])
+def test_widened_units_over_ring_depths_and_odd_unit_counts(e_local, hidden, inter, topk, tokens):
+    y, stats, ref, buf, _ = run_layer('fp8', e_local, hidden, inter, topk, tokens, 'random', 'umma', seed=tokens, std=0.02)
+    check_against_oracle(y, stats, ref, buf, 'fp8', inter)
+
+
 @pytest.mark.parametrize('num_sms', [5, 0])
 @pytest.mark.parametrize('hidden,inter', [(512, 768), (1536, 256), (4096, 256)])
 def test_shapes_and_small_grids(hidden, inter, num_sms):
