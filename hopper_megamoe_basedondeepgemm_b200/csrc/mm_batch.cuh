@@ -2,8 +2,8 @@
 //
 // With one rank nothing crosses NVLink, every SM can work out the whole routing by itself and rows need no flagged words:
 //
-//   routing  : every SM ranks all routing entries per expert (warp-wide matches, one histogram per warp), so the token
-//              tiles and the task list follow without any exchange between SMs.
+//   routing  : every SM counts all routing entries per expert (one histogram per run of entries and warp), so the token
+//              tiles and the task list follow without any exchange between SMs; the list of rows is made behind the first copies.
 //   tiles    : an expert's rows form ceil(rows / tile limit) token tiles of at most 128 rows (96 with E4M3 tokens). The
 //              block-scaled MMAs of a weight unit take 199 cycles for 16 rows and 288 for 128, so wide tiles are nearly free and an
 //              expert's weights stream once per tile.
@@ -37,8 +37,8 @@ constexpr int kBWStages = 12, kBRSlots = 12;       // at most: weight ring stage
 constexpr int kBServiceWarps = 4;                  // weight loader, MMA issuer, record loader, spare
 constexpr int kBEpiWarps = 8;                      // two groups of four
 constexpr int kBCombineWarps = 4;
-constexpr int kBWorkWarps = kBEpiWarps + kBCombineWarps;    // warps 4..15 place the rows and copy them into the images
-constexpr int kBRankWarps = kBServiceWarps + kBWorkWarps;   // warps 0..15 rank the routing entries
+constexpr int kBWorkWarps = kBEpiWarps + kBCombineWarps;    // warps 4..15 copy the rows into the images and list them
+constexpr int kBRankWarps = kBServiceWarps + kBWorkWarps;   // warps 0..15 count the routing entries, a run of them each
 constexpr int kBThreads = 32 * (kBServiceWarps + kBWorkWarps);
 constexpr int kBExpWarps = 8;                      // E4M3 tokens: widening warps 12..19 (they take up the combine when their role ends)
 constexpr int kBThreadsA8 = 32 * (kBServiceWarps + kBEpiWarps + kBExpWarps);
@@ -47,7 +47,7 @@ constexpr int kBCounts = kBColCounters + 32;       // counters of a launch besid
 constexpr uint32_t kBVtStride = 152;               // floats between the tokens of `vt`
 // tensor-memory columns with E4M3 tokens: scales of the weights and of the tokens (two areas of 8 each), widened units (two of 64)
 constexpr uint32_t kTmScaleW = 256, kTmScaleX = 272, kTmWide = 384;
-constexpr uint32_t kBBarEpi0 = 1, kBBarEpi1 = 2, kBBarWork = 3, kBBarTiles = 4;    // named barriers
+constexpr uint32_t kBBarEpi0 = 1, kBBarEpi1 = 2, kBBarWork = 3, kBBarTiles = 4, kBBarPlaced = 7;    // named barriers (5, 6: the decode kernel's)
 
 struct BParams {
     int T, topk, E, H, I;
@@ -74,7 +74,7 @@ struct BShared {
     uint64_t wfull[kBWStages], wempty[kBWStages], rfull[kBRSlots], rempty[kBRSlots];
     uint64_t tmem_full[2], tmem_empty[2], xfull[2], xempty[2];
     uint32_t tmem_base, abort_flag, M, wissued, rissued, comb_next, nw, nr, slot_bytes, spu, total, start_ok;
-    uint32_t seg_shift;                            // routing entries per ranking warp: 1 << seg_shift
+    uint32_t seg_shift;                            // routing entries of a run: 1 << seg_shift
     uint32_t cnt[kMaxLocalExperts], ebase[kMaxLocalExperts];
     uint32_t tile_e[kBMaxTiles];                   // expert
     uint32_t tile_row0[kBMaxTiles];                // first row (index into `rowf`)
@@ -82,10 +82,10 @@ struct BShared {
     uint32_t tile_a16[kBMaxTiles];                 // 16-row groups of all tiles before this one
     uint32_t etile[kMaxLocalExperts];              // first tile of the expert
     uint32_t task[kBTaskRing];                     // claimed tasks: turn of the ring << 16 | L2 << 15 | tile << 8 | weight tile (0xFFFF: no more)
-    alignas(16) uint16_t wcnt[kBRankWarps][kMaxLocalExperts];  // routing entries per (ranking warp, expert), then the exclusive sums over the warps
+    alignas(16) uint16_t wcnt[kBRankWarps][kMaxLocalExperts];  // routing entries per (run, expert), then the exclusive sums over the runs
     alignas(16) uint8_t ex[kBMaxRows];             // expert of every routing entry (0xFF: masked, 0xFE: no such expert)
     union {
-        uint16_t rank[kBMaxRows];                  // rank of the entry among those of its expert in its ranking warp (until the rows are placed)
+        uint16_t run_cnt[kBRankWarps][kMaxLocalExperts];   // running counts while the list of rows is made (until then)
         float vt[2][kTileTokens * kBVtStride];     // 16 tokens' accumulators of a task, per epilogue group (see b_role_epilogue)
     };
     uint16_t ef[2][128];                           // per epilogue group: routing entry and top-k weight of the task's rows
@@ -231,6 +231,10 @@ __device__ void b_role_weights(const BCtx& cx, uint32_t lane) {
     const uint64_t policy = l2_evict_first_policy();
     uint32_t it = 0, s = 0, ph = 0;
     BTasks tasks(cx);
+    // The stream starts when this SM's rows are in the images. What an SM has asked for comes back in order: behind 100 KB and more of weights
+    // the acknowledgement of the rows' release took 2 to 3 us, and every task that wants one of them waited
+    // for it (13 tokens: 51.3 -> 50.0 us a pass, 64: 60.3 -> 58.6, 512: 80.3 -> 79.8, 6 of the small layer: 15.4 -> 15.0).
+    bar_sync(kBBarPlaced, 32u * (kBWorkWarps + 1));
     // Order of the L2 tasks: tile by tile (the first tiles' L1 outputs are complete long before the last ones'), but the last
     // tiles, kBColumnTasks tasks per SM of them, column block by column block: the combine starts on a column block when all
     // tiles have it, beside the remaining ones.
@@ -753,16 +757,55 @@ __device__ void b_role_combine(const BCtx& cx, uint32_t lane) {
 }
 
 // ============================================================================================= routing
-// Sums over the ranking warps, the experts' token tiles and the ring geometry (one warp; lane l takes the experts 2l and
+// The list of rows, for the epilogue: the run `r` of routing entries, one warp. An entry's place among the rows of its expert is the number
+// of earlier entries that name it; 32 entries are a chain of about 560 cycles, bound by the ballots' arithmetic when
+// all warps are at it. (So it is not in front of the first copy: that needs the counts alone.)
+__device__ __forceinline__ void b_list_run(const BCtx& cx, uint32_t r, uint32_t seg_shift, uint32_t nent, uint32_t lane) {
+    BShared& c = cx.c;
+    const uint32_t lo = r << seg_shift, hi = min(lo + (1u << seg_shift), nent);
+    uint16_t* cnt = c.run_cnt[r];
+    reinterpret_cast<uint32_t*>(cnt)[lane] = 0u;
+    __syncwarp();
+    #pragma unroll 1
+    for (uint32_t f0 = lo; f0 < hi; f0 += 32u) {
+        const uint32_t f = f0 + lane, e = f < hi ? c.ex[f] : 0xFFu;
+        // the lanes with the same expert: one ballot per bit (several times faster than a warp-wide match)
+        uint32_t same = __ballot_sync(0xffffffffu, e < kMaxLocalExperts);
+        #pragma unroll
+        for (uint32_t b = 0; b < 6; ++b) {
+            const uint32_t v = __ballot_sync(0xffffffffu, (e >> b) & 1u);
+            same &= (e >> b) & 1u ? v : ~v;
+        }
+        const uint32_t below = same & ((1u << lane) - 1u);
+        const uint32_t base = e < kMaxLocalExperts ? cnt[e] : 0u;
+        __syncwarp();
+        if (e < kMaxLocalExperts) {
+            c.rowf[c.ebase[e] + c.wcnt[r][e] + base + __popc(below)] = static_cast<uint16_t>(f);
+            if (below == 0u) cnt[e] = static_cast<uint16_t>(base + __popc(same));
+        }
+        __syncwarp();
+    }
+}
+// entries before entry f in its run that name the same expert e (the whole warp)
+__device__ __forceinline__ uint32_t b_rank_in_run(const BShared& c, uint32_t f, uint32_t e, uint32_t seg_shift, uint32_t lane) {
+    uint32_t k = 0u;
+    #pragma unroll 1
+    for (uint32_t i = ((f >> seg_shift) << seg_shift) + lane; i - lane < f; i += 32u) k += __popc(__ballot_sync(0xffffffffu, i < f && c.ex[i] == e));
+    return k;
+}
+
+// Sums over the runs, the experts' token tiles and the ring geometry (one warp; lane l takes the experts 2l and
 // 2l + 1). Everything the SM does waits for it and its code runs once, from a cold instruction cache: few instructions.
 template <int kFmt>
 __device__ __forceinline__ void b_tiles(const BCtx& cx, uint32_t lane) {
     using F = BFmt<kFmt>;
     const BParams& p = cx.p; BShared& c = cx.c;
     uint32_t* w32 = reinterpret_cast<uint32_t*>(&c.wcnt[0][0]) + lane;
-    uint32_t run = 0u;                                       // two 16-bit counts, at most 4096 each
-    #pragma unroll 4
-    for (uint32_t w = 0; w < kBRankWarps; ++w) { const uint32_t v = w32[w * (kMaxLocalExperts / 2)]; w32[w * (kMaxLocalExperts / 2)] = run; run += v; }
+    uint32_t run = 0u, wv[kBRankWarps];                      // two 16-bit counts, at most 4096 each
+    #pragma unroll
+    for (uint32_t w = 0; w < kBRankWarps; ++w) wv[w] = w32[w * (kMaxLocalExperts / 2)];
+    #pragma unroll
+    for (uint32_t w = 0; w < kBRankWarps; ++w) { w32[w * (kMaxLocalExperts / 2)] = run; run += wv[w]; }
     const uint32_t lim = p.tile_limit;
     uint32_t cn[2] = {run & 0xFFFFu, run >> 16}, nt[2], rpt[2];
     #pragma unroll
@@ -853,27 +896,28 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
     const unsigned long long t_first = globaltimer_ns();
     const uint32_t epoch = ld_volatile_u32(ctrl32 + kCtrlEpoch / 4 + bid);         // (tid 0 counts on after the barrier below)
     const uint32_t ntok = bid < static_cast<uint32_t>(p.T) ? udiv_small(p.T - 1u - bid, G) + 1u : 0u, nrows = ntok * p.topk;
-    const uint32_t xq = p.x_row_bytes / 16u, per_row = xq + p.x_sf_row_bytes / 16u;
-    constexpr uint32_t kChunks = F::kA8 ? 9u : 5u;               // 16 B chunks of a row per lane (hidden <= 4096)
+    // a row in a warp's registers: 16 B chunks of the packed row and words of its scale bytes (hidden <= 4096)
+    const uint32_t xq = p.x_row_bytes / 16u, nsf = p.x_sf_row_bytes / 4u;
+    constexpr uint32_t kChunks = F::kA8 ? 8u : 4u, kWords = F::kVec == 16 ? 2u : 1u;
     constexpr uint32_t kAhead = F::kA8 ? 1u : 2u;                // rows a worker warp has in flight
     uint4 v[kAhead][kChunks];
-    auto load_row = [&](uint4 (&v)[kChunks], uint32_t k) {
+    uint32_t vs[kAhead][kWords];
+    auto load_row = [&](uint4 (&v)[kChunks], uint32_t (&vs)[kWords], uint32_t k) {
         if (k >= nrows) return;
         const uint32_t tok = bid + udiv_small(k, p.topk) * G;
-        const uint8_t* xs = p.buf + p.off_x + static_cast<size_t>(tok) * p.x_row_bytes;
-        const uint8_t* sf = p.buf + p.off_x_sf + static_cast<size_t>(tok) * p.x_sf_row_bytes;
+        const uint8_t* xs = p.buf + p.off_x + static_cast<size_t>(tok) * p.x_row_bytes + lane * 16u;
+        const uint8_t* sf = p.buf + p.off_x_sf + static_cast<size_t>(tok) * p.x_sf_row_bytes + lane * 4u;
         #pragma unroll
-        for (uint32_t u = 0; u < kChunks; ++u) {
-            const uint32_t ci = lane + u * 32;
-            if (ci < per_row) v[u] = ld_cg_v4(ci < xq ? xs + ci * 16u : sf + (ci - xq) * 16u);
-        }
+        for (uint32_t u = 0; u < kChunks; ++u) if (lane + u * 32u < xq) v[u] = ld_cg_v4(xs + u * 512u);
+        #pragma unroll
+        for (uint32_t u = 0; u < kWords; ++u) if (lane + u * 32u < nsf) vs[u] = ld_cg_u32(sf + u * 128u);
     };
     const BCtx cx(p, c, smem, globaltimer_ns() + p.timeout_ns, epoch & 1u);
     if constexpr (!kFe) {
         // ---- this SM's tokens (token mod G): the first rows of every worker warp are fetched before the routing is known
         if (worker) {
             #pragma unroll
-            for (uint32_t a = 0; a < kAhead; ++a) load_row(v[a], ww + a * kBWorkWarps);
+            for (uint32_t a = 0; a < kAhead; ++a) load_row(v[a], vs[a], ww + a * kBWorkWarps);
         }
         // ---- the routing entries' experts into shared memory
         const long long* tk = reinterpret_cast<const long long*>(p.buf + p.off_topk_idx);
@@ -885,7 +929,7 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
     }
     if (tid == 0) {
         c.abort_flag = 0u; c.comb_next = 0u; c.wissued = 0u; c.rissued = 0u;
-        // a run of 32, 64, 128 or 256 routing entries per ranking warp
+        // a run of 32, 64, 128 or 256 routing entries per counting warp
         const uint32_t per = (nent + kBRankWarps - 1u) / kBRankWarps;
         c.seg_shift = per <= 32u ? 5u : 32u - __clz(per - 1u);
         reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlSmEntry)[bid] = t_first;
@@ -953,7 +997,7 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
         if (bid == 0 && tid == 0) cx.stamp(kStampFrontend);
         if (worker) {
             #pragma unroll
-            for (uint32_t a = 0; a < kAhead; ++a) load_row(v[a], ww + a * kBWorkWarps);
+            for (uint32_t a = 0; a < kAhead; ++a) load_row(v[a], vs[a], ww + a * kBWorkWarps);
         }
     }
     if (tid == 0) {
@@ -968,29 +1012,15 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
             cx.stamp(kStampPrologue);
         }
     }
-    // ---- rank of every entry among the entries of its expert in this warp's run
+    // ---- how often each run of entries names each expert
     const uint32_t seg_shift = c.seg_shift;
     if (warp < kBRankWarps) {
-        const uint32_t lo = warp << seg_shift, hi = lo + (1u << seg_shift);
-        uint16_t* cnt = c.wcnt[warp];
+        const uint32_t lo = warp << seg_shift, hi = min(lo + (1u << seg_shift), nent);
         #pragma unroll 1
-        for (uint32_t f = lo + lane; f - lane < (hi < nent ? hi : nent); f += 32u) {
-            const uint32_t e = f < nent ? c.ex[f] : 0xFFu;
-            // the lanes with the same expert: one ballot per bit (several times faster than a warp-wide match)
-            uint32_t same = __ballot_sync(0xffffffffu, e < kMaxLocalExperts);
-            #pragma unroll
-            for (uint32_t b = 0; b < 6; ++b) {
-                const uint32_t v = __ballot_sync(0xffffffffu, (e >> b) & 1u);
-                same &= (e >> b) & 1u ? v : ~v;
-            }
-            const uint32_t below = same & ((1u << lane) - 1u);
-            const uint32_t base = e < kMaxLocalExperts ? cnt[e] : 0u;
-            __syncwarp();
-            if (e < kMaxLocalExperts) {
-                c.rank[f] = static_cast<uint16_t>(base + __popc(below));
-                if (below == 0u) cnt[e] = static_cast<uint16_t>(base + __popc(same));
-            } else if (e == 0xFEu) cx.fail(kErrWaitCombineFlag, 0xFFFFu);       // a route to an expert that does not exist
-            __syncwarp();
+        for (uint32_t f = lo + lane; f < hi; f += 32u) {
+            const uint32_t e = c.ex[f];
+            if (e < kMaxLocalExperts) atomicAdd(reinterpret_cast<uint32_t*>(c.wcnt[warp]) + (e >> 1), 1u << (16u * (e & 1u)));
+            else if (e == 0xFEu) cx.fail(kErrWaitCombineFlag, 0xFFFFu);       // a route to an expert that does not exist
         }
     }
     __syncthreads();
@@ -1034,33 +1064,38 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
             const uint32_t kt = udiv_small(k, p.topk), tok = bid + kt * G, f = tok * p.topk + k - kt * p.topk;
             const uint32_t e = c.ex[f];
             uint4 row[kChunks];
+            uint32_t word[kWords];
             #pragma unroll
             for (uint32_t u = 0; u < kChunks; ++u) {
                 row[u] = v[0][u];
                 #pragma unroll
                 for (uint32_t a = 1; a < kAhead; ++a) v[a - 1][u] = v[a][u];
             }
-            load_row(v[kAhead - 1u], k + kAhead * kBWorkWarps);
+            #pragma unroll
+            for (uint32_t u = 0; u < kWords; ++u) {
+                word[u] = vs[0][u];
+                #pragma unroll
+                for (uint32_t a = 1; a < kAhead; ++a) vs[a - 1][u] = vs[a][u];
+            }
+            load_row(v[kAhead - 1u], vs[kAhead - 1u], k + kAhead * kBWorkWarps);
             if (e < kMaxLocalExperts) {
                 // the expert's tile with this row
-                const uint32_t pos = c.wcnt[f >> seg_shift][e] + c.rank[f], eb = c.ebase[e];
+                const uint32_t pos = c.wcnt[f >> seg_shift][e] + b_rank_in_run(c, f, e, seg_shift, lane), eb = c.ebase[e];
                 uint32_t m = c.etile[e];
                 while (pos >= c.tile_row0[m] - eb + c.tile_rows[m]) ++m;
                 const uint32_t n = pos - (c.tile_row0[m] - eb), a16 = (c.tile_rows[m] + 15u) >> 4, rec = F::rec(a16);
                 uint8_t* img = p.buf + p.off_token_tiles + F::image(p.k1, c.tile_a16[m], m);
+                // chunk u of a lane: 512 B further along the row, four 128 B atoms (with E4M3 two units of two atoms each, otherwise four units)
+                const uint32_t at = lane >> 3;
+                uint8_t* dst = img + (F::kA8 ? (at >> 1) * rec + (at & 1u) * a16 * 2048u : at * rec) + sw128_off(n, lane & 7u);
                 #pragma unroll
-                for (uint32_t u = 0; u < kChunks; ++u) {
-                    const uint32_t ci = lane + u * 32;
-                    if (ci < xq) {
-                        const uint32_t at = ci >> 3;                                          // 128 B atom of the row
-                        *reinterpret_cast<uint4*>(img + (F::kA8 ? (at >> 1) * rec + (at & 1u) * a16 * 2048u : at * rec) + sw128_off(n, ci & 7u)) = F::kA8 ? even_odd(row[u]) : row[u];
-                    } else if (ci < per_row) {
-                        const uint32_t g = (ci - xq) * 4u;                                    // scale words g .. g + 3: unit g / planes, plane g % planes
-                        const uint32_t wv[4] = {row[u].x, row[u].y, row[u].z, row[u].w};
-                        #pragma unroll
-                        for (uint32_t q = 0; q < 4; ++q)
-                            *reinterpret_cast<uint32_t*>(img + ((g + q) / F::kPlanes) * rec + a16 * 2048u * F::kAtoms + ((g + q) % F::kPlanes) * 512u + plane_off(n)) = wv[q];
-                    }
+                for (uint32_t u = 0; u < kChunks; ++u)
+                    if (lane + u * 32u < xq) *reinterpret_cast<uint4*>(dst + u * (F::kA8 ? 2u : 4u) * rec) = F::kA8 ? even_odd(row[u]) : row[u];
+                // scale word g: unit g / planes, plane g % planes
+                #pragma unroll
+                for (uint32_t u = 0; u < kWords; ++u) {
+                    const uint32_t g = lane + u * 32u;
+                    if (g < nsf) *reinterpret_cast<uint32_t*>(img + (g / F::kPlanes) * rec + a16 * 2048u * F::kAtoms + (g % F::kPlanes) * 512u + plane_off(n)) = word[u];
                 }
                 #pragma unroll
                 for (uint32_t q = 0; q < 4; ++q) if (q == ndone) done_m[q] = m;
@@ -1076,13 +1111,11 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
                 ndone = 0u;
             }
         }
+        bar_arrive(kBBarPlaced, 32u * (kBWorkWarps + 1));        // (the weight loader)
         if (lane == 0) cx.sm_phase(kSmRowsCached);
         // ---- the list of rows, for the epilogue
         #pragma unroll 1
-        for (uint32_t f = tid - 32u * kBServiceWarps; f < nent; f += kBWorkWarps * 32u) {
-            const uint32_t e = c.ex[f];
-            if (e < kMaxLocalExperts) c.rowf[c.ebase[e] + c.wcnt[f >> seg_shift][e] + c.rank[f]] = static_cast<uint16_t>(f);
-        }
+        for (uint32_t r = ww; r < kBRankWarps; r += kBWorkWarps) b_list_run(cx, r, seg_shift, nent, lane);
         bar_sync(kBBarWork, kBWorkWarps * 32u);
         // ---- off the critical path: the rows' records in the receive pool (a row's place: the live entries before it), for
         //      whoever inspects the pool afterwards
