@@ -45,6 +45,7 @@ struct DCtx : BCore {
 
 template <int kFmt> struct DFmt : BFmt<kFmt> {
     static constexpr int kThreads = BFmt<kFmt>::kA8 ? kDThreadsA8 : kDThreads;
+    static constexpr uint32_t kBuilders = BFmt<kFmt>::kA8 ? kDEpiWarps + kBExpWarps : kDEpiWarps;    // warps from 4 on that build the first token tile
     static constexpr uint32_t kTmemColumns = BFmt<kFmt>::kA8 ? 512u : 128u;
     static constexpr uint32_t kRec = 2048u * BFmt<kFmt>::kAtoms + BFmt<kFmt>::kPlanes * 512u;     // one K unit of the 16-row tile
 };
@@ -79,7 +80,9 @@ struct DTasks {
     }
 };
 
-__device__ void d_role_weights(const DCtx& cx, uint32_t nw, uint8_t* ring) {
+// `routed` is called once, when the first unit has been asked for.
+template <typename Routed>
+__device__ __forceinline__ void d_role_weights(const DCtx& cx, uint32_t nw, uint8_t* ring, Routed routed) {
     const BParams& p = cx.p; DShared& c = cx.c;
     const uint64_t policy = l2_evict_first_policy();
     uint32_t it = 0, s = 0, ph = 0;
@@ -97,15 +100,13 @@ __device__ void d_role_weights(const DCtx& cx, uint32_t nw, uint8_t* ring) {
                 mbar_arrive_expect_tx(&c.wfull[s], p.unit_bytes);
                 bulk_g2s_hint(ring + static_cast<size_t>(s) * p.unit_bytes, src, p.unit_bytes, &c.wfull[s], policy);
                 c.wissued = it + 1u;
-                if (it == 0u) {
-                    reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlSmWFirst)[blockIdx.x] = globaltimer_ns();
-                    cx.sm_phase(kSmFirstIssue);
-                }
             }
             __syncwarp();
+            if (it == 0u) routed();
             if (++s == nw) { s = 0; ph ^= 1u; }
         }
     }
+    if (it == 0u) routed();
 }
 
 template <int kFmt>
@@ -119,7 +120,7 @@ __device__ void d_role_mma(const DCtx& cx, uint32_t lane, uint32_t nw_, uint32_t
     // (operands broadcast from lane 0: uniform registers, see the batch kernel's issuer)
     const uint32_t nw = b_uniform(nw_), tm = b_uniform(c.tmem_base);
     const uint32_t s0 = b_uniform(smem_u32(cx.smem)), ring0 = s0 + b_uniform(ring_off);
-    uint32_t it = 0, s = 0, ph = 0, wsm0 = ring0;
+    uint32_t it = 0, s = 0, ph = 0;
     bool have1 = false, have2 = false;
     DTasks tasks(cx);
     #pragma unroll 1
@@ -132,38 +133,50 @@ __device__ void d_role_mma(const DCtx& cx, uint32_t lane, uint32_t nw_, uint32_t
         if (layer == 0u && !have1) { if (!cx.warp_wait(&c.tile_full[0], 0u, kErrWaitActsFull)) return; have1 = true; }
         if (layer != 0u && !have2) { if (!cx.warp_wait(&c.tile_full[1], 0u, kErrWaitL1Done)) return; have2 = true; }
         tc_fence_after();
-        uint32_t tok = s0 + ub * F::kRec;
+        // A stage that is there already goes out in the same turn: a turn is a barrier wait, a fence, an election and a reconvergence beside
+        // the issue, 540 to 640 cycles for a unit that the tensor pipe has in 200 (one token 20.6 -> 20.4 us a pass, two 27.2
+        // -> 26.7; four stages a turn no better). With E4M3 tokens the second is seldom there yet.
+        constexpr uint32_t kTurn = kA8 ? 1u : 2u;
         #pragma unroll 1
-        for (uint32_t u = ub; u < ue; ++u, ++it, tok += F::kRec) {
+        for (uint32_t u = ub; u < ue;) {
             if (!cx.warp_wait(kA8 ? &c.xfull[it & 1u] : &c.wfull[s], kA8 ? (it >> 1) & 1u : ph, kErrWaitFull)) return;
+            uint32_t n = 1u;
+            if constexpr (kTurn == 2u) {
+                const uint32_t s1 = s + 1u == nw ? 0u : s + 1u;
+                if (__all_sync(0xffffffffu, u + 1u < ue && mbar_test(&c.wfull[s1], s1 == 0u ? ph ^ 1u : ph))) n = 2u;
+            }
             tc_fence_after();
             if (lane == 0 && it == 0u) cx.sm_phase(kSmFirstLanded);
             if (elect_one()) {
-                const uint64_t adesc = smem_desc(wsm0, 1024u, kLayoutSw128), bdesc = smem_desc(tok, 1024u, kLayoutSw128);
-                const uint64_t asf = smem_desc(wsm0 + kUnitWBytes, 128u, kLayoutNone);
-                const uint64_t bsf = smem_desc(tok + 2048u * F::kAtoms, 128u, kLayoutNone);
-                const uint32_t sfa = kA8 ? tm + kTmScaleW + (it & 1u) * 8u : tm + 32u + (it & 1u) * 32u, sfb = kA8 ? tm + kTmScaleX + (it & 1u) * 8u : sfa + 16u;
-                const uint32_t wide = tm + kTmWide + (it & 1u) * 64u;
-                #pragma unroll
-                for (uint32_t pl = 0; pl < kPlanes; ++pl) {
-                    if constexpr (!kA8) utccp_32x128b_warpx4(sfa + pl * 4u, asf + pl * 32u);
-                    utccp_32x128b_warpx4(sfb + pl * 4u, bsf + pl * 32u);
+                #pragma unroll 1
+                for (uint32_t b = 0; b < n; ++b) {
+                    const uint32_t slot = b == 0u ? s : (s + 1u == nw ? 0u : s + 1u), i = it + b, wsm = ring0 + slot * p.unit_bytes, tok = s0 + (u + b) * F::kRec;
+                    const uint64_t adesc = smem_desc(wsm, 1024u, kLayoutSw128), bdesc = smem_desc(tok, 1024u, kLayoutSw128);
+                    const uint64_t asf = smem_desc(wsm + kUnitWBytes, 128u, kLayoutNone);
+                    const uint64_t bsf = smem_desc(tok + 2048u * F::kAtoms, 128u, kLayoutNone);
+                    const uint32_t sfa = kA8 ? tm + kTmScaleW + (i & 1u) * 8u : tm + 32u + (i & 1u) * 32u, sfb = kA8 ? tm + kTmScaleX + (i & 1u) * 8u : sfa + 16u;
+                    const uint32_t wide = tm + kTmWide + (i & 1u) * 64u;
+                    #pragma unroll
+                    for (uint32_t pl = 0; pl < kPlanes; ++pl) {
+                        if constexpr (!kA8) utccp_32x128b_warpx4(sfa + pl * 4u, asf + pl * 32u);
+                        utccp_32x128b_warpx4(sfb + pl * 4u, bsf + pl * 32u);
+                    }
+                    #pragma unroll
+                    for (uint32_t ks = 0; ks < kUnitK / kStepK; ++ks) {
+                        const uint32_t pl = (ks * kStepK) / (4u * F::kVec), sf_id = ((ks * kStepK) % (4u * F::kVec)) / F::kVec;
+                        const uint64_t ad = adesc + (ks & 3u) * 2u;
+                        const uint64_t bd = bdesc + (ks & 3u) * 2u + (kA8 ? (ks >> 2) * (2048u >> 4) : 0u);
+                        const uint32_t idesc = idesc_with_sf(kIdesc, sf_id, sf_id), accum = (u + b != ub || ks != 0u) ? 1u : 0u;
+                        if constexpr (kA8) umma_mxf8f6f4_ta(d, wide + ks * 8u, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
+                        else if constexpr (kFmt == 0) umma_mxf4_block32(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
+                        else umma_nvf4_block16(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
+                    }
+                    tc_commit(kA8 ? &c.xempty[i & 1u] : &c.wempty[slot]);
                 }
-                #pragma unroll
-                for (uint32_t ks = 0; ks < kUnitK / kStepK; ++ks) {
-                    const uint32_t pl = (ks * kStepK) / (4u * F::kVec), sf_id = ((ks * kStepK) % (4u * F::kVec)) / F::kVec;
-                    const uint64_t ad = adesc + (ks & 3u) * 2u;
-                    const uint64_t bd = bdesc + (ks & 3u) * 2u + (kA8 ? (ks >> 2) * (2048u >> 4) : 0u);
-                    const uint32_t idesc = idesc_with_sf(kIdesc, sf_id, sf_id), accum = (u != ub || ks != 0u) ? 1u : 0u;
-                    if constexpr (kA8) umma_mxf8f6f4_ta(d, wide + ks * 8u, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
-                    else if constexpr (kFmt == 0) umma_mxf4_block32(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
-                    else umma_nvf4_block16(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
-                }
-                tc_commit(kA8 ? &c.xempty[it & 1u] : &c.wempty[s]);
             }
             __syncwarp();
-            wsm0 += p.unit_bytes;
-            if (++s == nw) { s = 0; ph ^= 1u; wsm0 = ring0; }
+            u += n; it += n; s += n;
+            if (s >= nw) { s -= nw; ph ^= 1u; }
         }
         if (elect_one()) tc_commit(&c.tmem_full[acc]);
         __syncwarp();
@@ -214,17 +227,19 @@ __device__ __forceinline__ bool d_gather(const DCtx& cx, uint8_t* tile, uint32_t
     for (uint32_t i0 = gtid; i0 < n; i0 += kThreads * kFly) {
         uint4 v[kFly];
         bool ok;
-        do {
+        const uint8_t* src[kFly];
+        #pragma unroll
+        for (uint32_t u = 0; u < kFly; ++u) {
+            const uint32_t i = i0 + u * kThreads, col = udiv_small(i < n ? i : 0u, pieces), pc = (i < n ? i : 0u) - col * pieces;
+            src[u] = p.buf + p.off_mid + static_cast<size_t>(c.col_mid[col]) * 2u * p.mid_row_bytes + pc * 16u;
+            v[u] = make_uint4(0u, flag ^ 1u, 0u, flag ^ 1u);
+        }
+        do {                                             // (only the missing ones again: polls of all of them slowed the last L1 tasks and the stream, 21.4 -> 20.6 us for one token)
+            #pragma unroll
+            for (uint32_t u = 0; u < kFly; ++u) if (i0 + u * kThreads < n && (v[u].y != flag || v[u].w != flag)) v[u] = ld_volatile_v4(src[u]);
             ok = true;
             #pragma unroll
-            for (uint32_t u = 0; u < kFly; ++u) {
-                const uint32_t i = i0 + u * kThreads;
-                if (i < n) {
-                    const uint32_t col = udiv_small(i, pieces), pc = i - col * pieces;
-                    v[u] = ld_volatile_v4(p.buf + p.off_mid + static_cast<size_t>(c.col_mid[col]) * 2u * p.mid_row_bytes + pc * 16u);
-                    ok = ok && v[u].y == flag && v[u].w == flag;
-                }
-            }
+            for (uint32_t u = 0; u < kFly; ++u) ok = ok && (i0 + u * kThreads >= n || (v[u].y == flag && v[u].w == flag));
             if (!ok && cx.give_up(spins, kErrWaitL1Done, 0u)) return false;
         } while (!ok);
         #pragma unroll
@@ -479,7 +494,7 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
         if (lane < 2) {
             mbar_init(&c.tmem_full[lane], 1); mbar_init(&c.tmem_empty[lane], 4);
             mbar_init(&c.xfull[lane], kBExpWarps / 2); mbar_init(&c.xempty[lane], 1);
-            mbar_init(&c.tile_full[lane], kDEpiWarps);
+            mbar_init(&c.tile_full[lane], lane == 0 ? F::kBuilders : kDEpiWarps);
         }
         mbar_fence_init();
         if (lane < kDEntries) c.exp_n[lane] = 0u;
@@ -494,9 +509,9 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
     const uint32_t epoch = ld_volatile_u32(ctrl32 + kCtrlEpoch / 4 + bid), flag = epoch + 1u;      // (warp 3 counts on, off the critical path)
     const DCtx cx(p, c, smem, globaltimer_ns() + p.timeout_ns, epoch & 1u);
     constexpr uint32_t kEW = 4;                                       // the first of the warps that build the token tile
-    const bool builder = warp >= kEW && warp < kEW + kDEpiWarps;
-    constexpr uint32_t kPerWarp = kDEntries / kDEpiWarps;             // entries a builder warp writes: 2
-    // Rows of entries bw and bw + 8 in registers before the routing is known: the 16 B chunks of the packed row and its scale
+    const bool builder = warp >= kEW && warp < kEW + F::kBuilders;
+    constexpr uint32_t kPerWarp = kDEntries / F::kBuilders;           // entries a builder warp writes: 2, with E4M3 tokens 1
+    // Rows of entries bw (and bw + 8) in registers before the routing is known: the 16 B chunks of the packed row and its scale
     // bytes (lane, lane + 32, ...), or, from hidden states, the quantised pieces of this lane (8 elements of every unit).
     constexpr uint32_t kChunks = F::kA8 ? 9u : 5u;
     const uint32_t xq = p.x_row_bytes / 16u, per_row = xq + p.x_sf_row_bytes / 16u;
@@ -514,7 +529,7 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
         if (builder) {
             #pragma unroll
             for (uint32_t a = 0; a < kPerWarp; ++a) {
-                const uint32_t f = warp - kEW + a * kDEpiWarps;
+                const uint32_t f = warp - kEW + a * F::kBuilders;
                 if (f < n) {
                     const uint32_t tok = udiv_small(f, p.topk);
                     const uint8_t* xs = p.buf + p.off_x + static_cast<size_t>(tok) * p.x_row_bytes;
@@ -533,7 +548,7 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
         if (builder) {
             #pragma unroll
             for (uint32_t a = 0; a < kPerWarp; ++a) {
-                const uint32_t f = warp - kEW + a * kDEpiWarps;
+                const uint32_t f = warp - kEW + a * F::kBuilders;
                 if (f < n) {
                     const uint32_t tok = f >> 3;                      // (eight routes per token)
                     const uint4* xrow = reinterpret_cast<const uint4*>(p.fe.hidden + static_cast<size_t>(tok) * p.H);
@@ -593,20 +608,30 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
         if (lane == 0) c.start_ok = cx.aborted() ? 0u : flag;        // (decided once: every warp takes the same way from here)
         __threadfence_block();
         __syncwarp();
-        bar_arrive(kDBarRouted, F::kThreads);
-        if (lane == 0) { cx.sm_phase(kSmScheduled); cx.stamp_max(kStampLastScheduled); if (bid == 0) cx.stamp(kStampScheduled); }
+        // The others hear of the routing when the stream has begun, so that their first instructions, which come from the L2, do not hold up the
+        // loader's (one token 22.0 -> 21.4 us a pass, two 28.2 -> 27.6). With E4M3 tokens the tile takes longer than
+        // the first unit, and the others start first (two tokens 31.7 us, the other way round 32.9).
+        auto routed = [&] {
+            bar_arrive(kDBarRouted, F::kThreads);
+            if (lane == 0) {
+                cx.sm_phase(kSmScheduled); cx.stamp_max(kStampLastScheduled); if (bid == 0) cx.stamp(kStampScheduled);
+                reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlSmWFirst)[bid] = globaltimer_ns();
+                cx.sm_phase(kSmFirstIssue);
+            }
+        };
+        const bool go = *reinterpret_cast<volatile uint32_t*>(&c.start_ok) != 0u;
+        if (F::kA8 || !go) routed();
+        if (go) d_role_weights(cx, nw, smem + ring_off, [&] { if constexpr (!F::kA8) routed(); });
     } else bar_sync(kDBarRouted, F::kThreads);
     const bool start = *reinterpret_cast<volatile uint32_t*>(&c.start_ok) != 0u;
     if (start) {
-        if (warp == 0) {
-            d_role_weights(cx, nw, smem + ring_off);
-        } else if (warp == 1) {
+        if (warp == 1) {
             d_role_mma<kFmt>(cx, lane, nw, ring_off);
         } else if (builder) {
             // ---- the token tile
             #pragma unroll
             for (uint32_t a = 0; a < kPerWarp; ++a) {
-                const uint32_t f = warp - kEW + a * kDEpiWarps;
+                const uint32_t f = warp - kEW + a * F::kBuilders;
                 if (f < n && ((c.live_mask >> f) & 1u) != 0u) {
                     const uint32_t col = c.ent_col[f];
                     if constexpr (!kFe) {
@@ -643,9 +668,8 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) { mbar_arrive(&c.tile_full[0]); cx.sm_phase(kSmRowsCached); }
-            d_role_epilogue<kFmt>(cx, (warp - kEW) >> 2, (tid - 32u * kEW) & 127u, smem, flag);
-        } else if (warp >= kEW + kDEpiWarps) {
-            if constexpr (F::kA8) { const uint32_t x = tid - 32u * (kEW + kDEpiWarps); d_role_widen(cx, x / kXGroupThreads, x % kXGroupThreads, nw, smem + ring_off); }
+            if (warp < kEW + kDEpiWarps) d_role_epilogue<kFmt>(cx, (warp - kEW) >> 2, (tid - 32u * kEW) & 127u, smem, flag);
+            else if constexpr (F::kA8) { const uint32_t x = tid - 32u * (kEW + kDEpiWarps); d_role_widen(cx, x / kXGroupThreads, x % kXGroupThreads, nw, smem + ring_off); }
         }
     }
     // ---- off the critical path: launch number, counters, stamps, and what others may inspect afterwards
@@ -678,6 +702,9 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
         }
     }
     if (tid == 128) { cx.stamp_max(kStampLastTasksDone); cx.sm_phase(kSmTasksDone); if (bid == 0) cx.stamp(kStampTasksDone); }
+    // (two warps have nothing else to do: they begin when this SM has all intermediate rows, until then their polls would only take from what the stream
+    // and the hand-over can get)
+    if (start && (warp == 2 || warp == 3)) cx.warp_wait(&c.tile_full[1], 0u, kErrWaitL1Done);
     if (start) d_role_combine(cx, flag);
     // ---- exit: an aborted SM lets the copies in flight land (bounded waits) before its shared memory goes away
     if (cx.aborted() && warp == 0) {
