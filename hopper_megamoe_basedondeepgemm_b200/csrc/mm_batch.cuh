@@ -30,7 +30,6 @@
 namespace mm {
 
 constexpr int kBMaxRows = 4096;                    // routed rows of one launch
-constexpr int kBMaxTiles = 128;                    // token tiles of one launch (64 experts + rows beyond the tile limit)
 constexpr uint32_t kBColumnTasks = 4;              // L2 tasks per SM that are claimed column block by column block
 constexpr int kBTaskRing = 64;                     // claimed tasks of one SM that some role has still to see, at most
 constexpr int kBWStages = 12, kBRSlots = 12;       // at most: weight ring stages, token record slots
@@ -42,8 +41,6 @@ constexpr int kBRankWarps = kBServiceWarps + kBWorkWarps;   // warps 0..15 count
 constexpr int kBThreads = 32 * (kBServiceWarps + kBWorkWarps);
 constexpr int kBExpWarps = 8;                      // E4M3 tokens: widening warps 12..19 (they take up the combine when their role ends)
 constexpr int kBThreadsA8 = 32 * (kBServiceWarps + kBEpiWarps + kBExpWarps);
-constexpr int kBColCounters = 32;                  // column blocks of 128 (hidden <= 4096)
-constexpr int kBCounts = kBColCounters + 32;       // counters of a launch besides the tiles': the column blocks', the claimed L2 tasks
 constexpr uint32_t kBVtStride = 152;               // floats between the tokens of `vt`
 // tensor-memory columns with E4M3 tokens: scales of the weights and of the tokens (two areas of 8 each), widened units (two of 64)
 constexpr uint32_t kTmScaleW = 256, kTmScaleX = 272, kTmWide = 384;
@@ -73,7 +70,7 @@ struct BParams {
 struct BShared {
     uint64_t wfull[kBWStages], wempty[kBWStages], rfull[kBRSlots], rempty[kBRSlots];
     uint64_t tmem_full[2], tmem_empty[2], xfull[2], xempty[2];
-    uint32_t tmem_base, abort_flag, M, wissued, rissued, comb_next, nw, nr, slot_bytes, spu, total, start_ok;
+    uint32_t tmem_base, abort_flag, M, wissued, rissued, comb_next, comb_open, nw, nr, slot_bytes, spu, total, start_ok;
     uint32_t seg_shift;                            // routing entries of a run: 1 << seg_shift
     uint32_t cnt[kMaxLocalExperts], ebase[kMaxLocalExperts];
     uint32_t tile_e[kBMaxTiles];                   // expert
@@ -143,7 +140,8 @@ struct BCore {
     // a count in global memory reaches `need` (one lane polls for its warp)
     __device__ __forceinline__ bool wait_count(const uint32_t* cnt, uint32_t need, uint32_t code, uint32_t detail) const {
         uint32_t it = 0;
-        while (ld_acquire_gpu(cnt) < need) {
+        for (uint32_t v; (v = ld_acquire_gpu(cnt)) < need;) {
+            if (need - v > 2u) __nanosleep(min(8u * (need - v), 300u));      // (a poll takes from what the others' counts and weights can get)
             if ((++it & 0x1Fu) == 0u) {
                 if (aborted()) return false;
                 if (expired()) { fail(code, detail); return false; }
@@ -160,9 +158,17 @@ struct BCore {
     __device__ __forceinline__ void stamp_max(int slot) const {
         atomicMax(reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlStamps) + slot, globaltimer_ns());
     }
-    __device__ __forceinline__ uint32_t* arrive_set() const { return reinterpret_cast<uint32_t*>(p.buf + p.off_arrive) + par * 2u * p.tile_capacity; }
-    __device__ __forceinline__ uint32_t* col_counts(uint32_t parity) const {
-        return reinterpret_cast<uint32_t*>(p.buf + p.off_arrive) + 4u * p.tile_capacity + parity * kBCounts;
+    // counters, `kBCountStride` words apart: `i` is a column block, kBCountClaims, or kBCountTiles + (layer - 1) * kBMaxTiles + tile
+    __device__ __forceinline__ uint32_t* counter(uint32_t parity, uint32_t i) const {
+        return reinterpret_cast<uint32_t*>(p.buf + p.off_arrive) + 4u * p.tile_capacity + parity * kBCounts + i * kBCountStride;
+    }
+    // clears the sets of the other parity, the multi-rank kernel's arrival counts among them (one warp of every SM)
+    __device__ __forceinline__ void clear_other(uint32_t lane) const {
+        uint32_t* other = reinterpret_cast<uint32_t*>(p.buf + p.off_arrive) + (par ^ 1u) * 2u * p.tile_capacity;
+        #pragma unroll 1
+        for (uint32_t i = blockIdx.x * 32u + lane; i < 2u * p.tile_capacity; i += gridDim.x * 32u) other[i] = 0u;
+        #pragma unroll 1
+        for (uint32_t i = blockIdx.x * 32u + lane; i < static_cast<uint32_t>(kBCounters); i += gridDim.x * 32u) *counter(par ^ 1u, i) = 0u;
     }
 };
 struct BCtx : BCore {
@@ -239,7 +245,7 @@ __device__ void b_role_weights(const BCtx& cx, uint32_t lane) {
     // tiles, kBColumnTasks tasks per SM of them, column block by column block: the combine starts on a column block when all
     // tiles have it, beside the remaining ones.
     const uint32_t NT1 = M * n1, NT2 = M * n2, tail = udiv_small(kBColumnTasks * G + n2 - 1u, n2), mA = tail < M ? M - tail : 0u, NA = mA * n2;
-    uint32_t* claims = cx.col_counts(cx.par) + kBColCounters;
+    uint32_t* claims = cx.counter(cx.par, kBCountClaims);
     uint32_t next = 0u;
     if (tasks.my1 == 0u && lane == 0) next = atomicAdd(claims, 1u);
     #pragma unroll 1
@@ -254,11 +260,12 @@ __device__ void b_role_weights(const BCtx& cx, uint32_t lane) {
                 q -= NT1;
                 t = 0xFFFFu;
                 if (q < NA) { const uint32_t m = udiv_small(q, n2); t = 0x8000u | (m << 8) | (q - m * n2); }
-                else if (q < NT2) { const uint32_t j = udiv_small(q - NA, M - mA); t = 0x8000u | ((mA + q - NA - j * (M - mA)) << 8) | j; }
+                else if (q < NT2) { const uint32_t j = udiv_small(q - NA, M - mA); *reinterpret_cast<volatile uint32_t*>(&c.comb_open) = 1u; t = 0x8000u | ((mA + q - NA - j * (M - mA)) << 8) | j; }
             }
             if (lane == 0) *reinterpret_cast<volatile uint32_t*>(&c.task[k % kBTaskRing]) = ((k / kBTaskRing + 1u) << 16) | t;
             if (t == 0xFFFFu) {                              // (the epilogue groups look at every second task: both of the next two end there)
                 if (lane == 0) *reinterpret_cast<volatile uint32_t*>(&c.task[(k + 1u) % kBTaskRing]) = (((k + 1u) / kBTaskRing + 1u) << 16) | t;
+                *reinterpret_cast<volatile uint32_t*>(&c.comb_open) = 1u;
                 break;
             }
             t = ((t & 0x8000u) << 13) | (t & 0x7FFFu);
@@ -292,7 +299,6 @@ __device__ void b_role_records(const BCtx& cx) {
     using F = BFmt<kFmt>;
     const BParams& p = cx.p; BShared& c = cx.c;
     const uint32_t lane = threadIdx.x & 31u, nr = b_uniform(c.nr), slot_bytes = b_uniform(c.slot_bytes), step = b_uniform(c.spu);
-    const uint32_t* arrive = cx.arrive_set();
     uint32_t it = 0, s = 0, ph = 0;
     uint32_t ready = 0u, seen = ~0u;
     bool seen_l2 = false;
@@ -307,12 +313,14 @@ __device__ void b_role_records(const BCtx& cx) {
         const uint32_t window = (m >> 5) | (layer << 8);
         if (window != seen || ((ready >> (m & 31u)) & 1u) == 0u) {
             uint32_t spins = 0;
+            const uint32_t mm_ = (m & ~31u) + lane;
+            const uint32_t* count = cx.counter(cx.par, kBCountTiles + layer * kBMaxTiles + mm_);
+            bool r = false;
             for (;;) {
-                const uint32_t mm_ = (m & ~31u) + lane;
-                const bool r = mm_ < c.M && ld_acquire_gpu(arrive + layer * p.tile_capacity + mm_) >= (layer ? static_cast<uint32_t>(p.n1) : c.tile_rows[mm_]);
+                if (mm_ < c.M && (spins == 0u || mm_ == m)) r = ld_acquire_gpu(count) >= (layer ? static_cast<uint32_t>(p.n1) : c.tile_rows[mm_]);
                 ready = __ballot_sync(0xffffffffu, r);
                 if ((ready >> (m & 31u)) & 1u) break;
-                if ((++spins & 0xFu) == 0u) {
+                if ((++spins & 0xFu) == 0u) {                 // (the others' answers are asked for once, this tile's until it is complete)
                     if (cx.aborted()) return;
                     if (cx.expired()) { cx.fail(layer ? kErrWaitL1Done : kErrWaitDispatchFlag, c.tile_e[m]); return; }
                 }
@@ -689,10 +697,10 @@ __device__ void b_role_epilogue(const BCtx& cx, uint32_t grp, uint32_t etid) {
         if (etid == 96u) {
             if (ti < 2u) cx.sm_phase(kSmFirstEpilogue);
             if (layer == 0u) {
-                red_release_gpu_add(cx.arrive_set() + p.tile_capacity + m, 1u);
+                red_release_gpu_add(cx.counter(cx.par, kBCountTiles + kBMaxTiles + m), 1u);
                 cx.sm_phase(kSmLastL1Epilogue);
             } else {
-                red_release_gpu_add(cx.col_counts(cx.par) + j, 1u);
+                red_release_gpu_add(cx.counter(cx.par, j), 1u);
             }
         }
     }
@@ -704,9 +712,14 @@ __device__ void b_role_epilogue(const BCtx& cx, uint32_t grp, uint32_t etid) {
 __device__ void b_role_combine(const BCtx& cx, uint32_t lane) {
     const BParams& p = cx.p; BShared& c = cx.c;
     const uint32_t G = gridDim.x, nitems = static_cast<uint32_t>(p.T) * p.n2, half = lane >> 4, l16 = lane & 15u;
-    const uint32_t* cols = cx.col_counts(cx.par);
     const uint32_t M = c.M;
     uint32_t known = 0xFFFFFFFFu;                            // the column block this half-warp saw complete last
+    // nothing is complete before this SM, like the others, has come to the tasks that go column block by column block
+    for (uint32_t spins = 0; *reinterpret_cast<volatile uint32_t*>(&c.comb_open) == 0u;) {
+        __nanosleep(200);
+        if (cx.give_up(spins, kErrWaitCombineFlag, 0u)) break;
+    }
+    __syncwarp();
     #pragma unroll 1
     for (;;) {
         uint32_t k = 0u;
@@ -721,7 +734,7 @@ __device__ void b_role_combine(const BCtx& cx, uint32_t lane) {
         #pragma unroll 1
         for (int sl = 0; sl < p.topk; ++sl) mask |= (c.ex[tok * p.topk + sl] < kMaxLocalExperts ? 1u : 0u) << sl;
         bool ok = true;
-        if (col != known && l16 == 0u) ok = cx.wait_count(cols + col, M, kErrWaitCombineFlag, tok);
+        if (col != known && l16 == 0u) ok = cx.wait_count(cx.counter(cx.par, col), M, kErrWaitCombineFlag, tok);
         known = col;
         if (!__all_sync(0xffffffffu, ok)) return;
         __syncwarp();
@@ -928,7 +941,7 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
         }
     }
     if (tid == 0) {
-        c.abort_flag = 0u; c.comb_next = 0u; c.wissued = 0u; c.rissued = 0u;
+        c.abort_flag = 0u; c.comb_next = 0u; c.comb_open = 0u; c.wissued = 0u; c.rissued = 0u;
         // a run of 32, 64, 128 or 256 routing entries per counting warp
         const uint32_t per = (nent + kBRankWarps - 1u) / kBRankWarps;
         c.seg_shift = per <= 32u ? 5u : 32u - __clz(per - 1u);
@@ -1041,12 +1054,8 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
     if (warp == 3) {
         // the arrival counts of this launch's parity were cleared by the launch before it; clear the other set for the next one
         // (also when this launch has failed: the set holds the counts of the launch before)
-        uint32_t* other = reinterpret_cast<uint32_t*>(p.buf + p.off_arrive) + (cx.par ^ 1u) * 2u * p.tile_capacity;
-        #pragma unroll 1
-        for (uint32_t i = bid * 32u + lane; i < 2u * p.tile_capacity; i += G * 32u) other[i] = 0u;
+        cx.clear_other(lane);
         if (bid == 0) {
-            cx.col_counts(cx.par ^ 1u)[lane] = 0u;
-            cx.col_counts(cx.par ^ 1u)[lane + 32] = 0u;
             if (start) {
                 #pragma unroll 1
                 for (uint32_t e = lane; e < static_cast<uint32_t>(p.E) && p.stats != nullptr; e += 32) p.stats[e] += static_cast<int>(c.cnt[e]);
@@ -1106,7 +1115,7 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
                 if (lane == 0) {
                     fence_acq_rel_gpu();             // (the reader's proxy fence after its acquire orders these stores with its bulk copies)
                     #pragma unroll
-                    for (uint32_t q = 0; q < 4; ++q) if (q < ndone) atomicAdd(cx.arrive_set() + done_m[q], 1u);
+                    for (uint32_t q = 0; q < 4; ++q) if (q < ndone) atomicAdd(cx.counter(cx.par, kBCountTiles + done_m[q]), 1u);
                 }
                 ndone = 0u;
             }

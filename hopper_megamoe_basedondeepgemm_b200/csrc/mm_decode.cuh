@@ -686,10 +686,7 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
             }
         }
         // the batch kernel's arrival counts of the other parity (also when this launch has failed)
-        uint32_t* other = reinterpret_cast<uint32_t*>(p.buf + p.off_arrive) + (cx.par ^ 1u) * 2u * p.tile_capacity;
-        #pragma unroll 1
-        for (uint32_t i = bid * 32u + lane; i < 2u * p.tile_capacity; i += G * 32u) other[i] = 0u;
-        if (bid == 0) { cx.col_counts(cx.par ^ 1u)[lane] = 0u; cx.col_counts(cx.par ^ 1u)[lane + 32] = 0u; }
+        cx.clear_other(lane);
         if (bid == 0 && start) {
             if (p.stats != nullptr && lane < c.M) p.stats[c.exp_e[lane]] += static_cast<int>(c.exp_n[lane]);
             uint8_t* region = p.buf + p.off_rx + static_cast<size_t>(cx.par) * p.rx_region;
