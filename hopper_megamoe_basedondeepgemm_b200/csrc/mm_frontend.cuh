@@ -482,10 +482,9 @@ __global__ void __launch_bounds__(kFeThreads, 1) frontend_logits_kernel(const __
 template <int kPer>
 __global__ void __launch_bounds__(32) frontend_select_kernel(const __grid_constant__ FeParams q) {
     const uint32_t lane = threadIdx.x, t = blockIdx.x;
-    // (the hidden states are there: the logits kernel let this one start when its own wait for the kernels before it was over)
-    const bool nonzero = fe_row_nonzero(q.hidden + static_cast<size_t>(t) * q.H, q.H, lane);
     grid_dependency_wait();
     grid_launch_dependents();
+    const bool nonzero = fe_row_nonzero(q.hidden + static_cast<size_t>(t) * q.H, q.H, lane);
     fe_select_token_regs<kPer>(q, t, nonzero, lane, 0u, nullptr, [] { return false; });
 }
 
