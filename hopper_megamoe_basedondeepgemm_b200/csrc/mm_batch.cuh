@@ -21,7 +21,7 @@
 //   combine  : per (token, 128-column block) behind a count per column block; routes added in slot order in fp32.
 //
 // Bound: HBM (the weights of the live experts once) up to about 40 rows per expert; beyond that the bytes an SM takes in
-// per unit (weights + token record, about 48 GB/s from the L2). 64 tokens, MXFP4, 48 experts (301 MB): 60 us a pass, of
+// per unit (weights + token record, about 48 GB/s from the L2). 64 tokens, MXFP4, 48 experts (301 MB): 53.5 us a pass, of
 // which the stream is 46; the multi-rank kernel takes 88. With E4M3 tokens the units are widened into tensor memory,
 // which keeps up with the stream (100 tokens: 67.7 us, 765 with the multi-rank kernel).
 #pragma once
