@@ -146,9 +146,10 @@ int mm_get_layout(const mm_config_t* c, mm_layout_t* out) {
         out->token_tile_bytes = mm::kWideTokens * 16 + (c->hidden / mm::kUnitK) * rec32;
         out->mid_tile_bytes = (c->intermediate / mm::kUnitK) * rec32;
     }
+    take(mm::kBCountBytes);                                                      // the one-rank batch kernel's counters
     out->off_token_tiles = take(out->tile_capacity * out->token_tile_bytes);
     out->off_mid_tiles = take(out->tile_capacity * out->mid_tile_bytes);
-    out->off_arrive = take(2 * 2 * out->tile_capacity * 4 + 2 * mm::kBCounts * 4 + mm::kFeMaxFusedTokens * 8 * 16);   // (then the one-rank batch kernel's counts and routing records)
+    out->off_arrive = take(2 * 2 * out->tile_capacity * 4 + mm::kRoutesGap + mm::kFeMaxFusedTokens * 8 * 16);   // (then the one-rank batch kernel's counts and routing records)
     // the same kernel's expert outputs, of as many routing entries as it takes (`batch_out_offset`)
     const int64_t out_rows = t_max * c->num_topk < mm::kBMaxRows ? t_max * c->num_topk : mm::kBMaxRows;
     take(c->num_ranks == 1 ? out_rows * c->hidden * 2 : 0);
@@ -158,7 +159,7 @@ int mm_get_layout(const mm_config_t* c, mm_layout_t* out) {
 
 // Regions of the one-rank kernels behind the arrival counters, and the expert outputs at the end of the buffer. (The outputs
 // are plain bf16: they must not share memory with the flagged words of the combine buffer, which they could imitate.)
-static int64_t batch_routes_offset(const mm_layout_t& L) { return L.off_arrive + 2 * 2 * L.tile_capacity * 4 + 2 * mm::kBCounts * 4; }
+static int64_t batch_routes_offset(const mm_layout_t& L) { return L.off_arrive + 2 * 2 * L.tile_capacity * 4 + mm::kRoutesGap; }
 // The decode kernel's flagged partial sums lie in the split-tile region behind the multi-rank kernel's plain ones (32 KB per SM), whose
 // words could carry any launch's number: [SM][16 rows][128] words of 8 bytes.
 static int64_t decode_parts_offset(const mm_layout_t& L, int grid) { return L.off_red + grid * (4ll * mm::kTileTokens * mm::kTileRows * 4); }

@@ -160,7 +160,7 @@ struct BCore {
     }
     // counters, `kBCountStride` words apart: `i` is a column block, kBCountClaims, or kBCountTiles + (layer - 1) * kBMaxTiles + tile
     __device__ __forceinline__ uint32_t* counter(uint32_t parity, uint32_t i) const {
-        return reinterpret_cast<uint32_t*>(p.buf + p.off_arrive) + 4u * p.tile_capacity + parity * kBCounts + i * kBCountStride;
+        return reinterpret_cast<uint32_t*>(p.buf + p.off_token_tiles - kBCountBytes) + parity * kBCounts + i * kBCountStride;
     }
     // clears the sets of the other parity, the multi-rank kernel's arrival counts among them (one warp of every SM)
     __device__ __forceinline__ void clear_other(uint32_t lane) const {

@@ -122,6 +122,9 @@ constexpr int kBColCounters = 32;                  // (hidden <= 4096)
 constexpr int kBCountClaims = kBColCounters, kBCountTiles = kBColCounters + 32, kBCounters = kBCountTiles + 2 * kBMaxTiles;
 constexpr int kBCountStride = 32;                  // words from one counter to the next
 constexpr int kBCounts = kBCounters * kBCountStride;
+constexpr int kBCountBytes = 2 * kBCounts * 4;      // of both sets, which end where the token images begin
+constexpr int kRoutesGap = 512;                     // bytes between the arrival counts and the routing records
+static_assert(kBCountBytes % 1024 == 0, "no gap in front of the token images");
 
 struct RowMeta { int32_t src, token, slot; float weight; };
 
@@ -1852,7 +1855,7 @@ __global__ void __launch_bounds__(kA8 ? kThreads + kNumExpThreads : kThreads, 1)
         // (and the counts of the one-rank batch kernel, which shares the buffer and the launch numbering)
         #pragma unroll 1
         for (uint32_t i = bid * kO + tid; i < static_cast<uint32_t>(kBCounters); i += G * kO)
-            reinterpret_cast<uint32_t*>(buf + p.off_arrive)[4u * p.tile_capacity + (par ^ 1u) * kBCounts + i * kBCountStride] = 0u;
+            reinterpret_cast<uint32_t*>(buf + p.off_token_tiles - kBCountBytes)[(par ^ 1u) * kBCounts + i * kBCountStride] = 0u;
     }
     // The rows of this rank's own tokens never travel when `own_ok`: every SM lists them from topk_idx and reads their
     // tokens where the caller put them. The SM that would have dispatched them only leaves their header line and records
