@@ -59,7 +59,7 @@ class MMStaticArgs(ctypes.Structure):
         ('timeout_ms', ctypes.c_float), ('device_status_out', ctypes.c_void_p)]
 
 
-STATIC_SCRATCH_BYTES = 24 * 1024 * 1024
+STATIC_SCRATCH_BYTES = 24 * 1024 * 1024 + 128 * 1024
 TUNE = {'knobs': 0, 'stages': 1, 'prefetch_w1_experts': 2, 'prefetch_w2_experts': 3, 'row_cache': 4}
 KNOB_PREFETCH, KNOB_OWN_ROWS, KNOB_EARLY_COMBINE = 1, 2, 4
 WINDOW_HANDLE_BYTES = 64

@@ -718,6 +718,7 @@ int mm_mega_moe_from_hidden_launch(const mm_config_t* cfg, const mm_launch_args_
 // the process exits. In host code the symbol below is only a handle; the device address comes from
 // cudaGetSymbolAddress (looked up once per device, with that device current) and that address is what the kernel gets.
 static __device__ __align__(256) unsigned char g_static_scratch[MM_STATIC_SCRATCH_BYTES];
+static_assert(MM_STATIC_SCRATCH_BYTES >= 24 * 1024 * 1024 + mm::kBCountBytes, "what fitted 24 MiB before there were counters still fits");
 
 namespace {
 constexpr int kMaxDevices = 64;

@@ -206,8 +206,9 @@ enum mm_tuning_key { MM_TUNE_KNOBS = 0, MM_TUNE_STAGES = 1 /* ring depth, 0 = de
 int mm_set_tuning(int32_t key, int32_t value);
 int32_t mm_get_tuning(int32_t key);
 
-/* Bytes of the library's built-in working memory (one array per GPU, resident from library load to process exit). */
-#define MM_STATIC_SCRATCH_BYTES (24ll * 1024 * 1024)
+/* Bytes of the library's built-in working memory (one array per GPU, resident from library load to process exit): 24 MiB, and room
+ * for the one-rank batch kernel's counters, which every configuration has beside what it needed without them. */
+#define MM_STATIC_SCRATCH_BYTES (24ll * 1024 * 1024 + 128 * 1024)
 
 typedef struct mm_static_args {
     const void* x;                   /* packed tokens [num_tokens][hidden / 2] (device) */

@@ -428,3 +428,25 @@ def test_tile_images_of_e4m3_tokens_take_the_room_their_one_user_needs():
         assert st == 0 and L.tile_capacity >= groups and L.tile_capacity <= 4096 // 16 + experts
         assert L.tile_capacity * L.token_tile_bytes >= 12 * (groups * 2 * 2048 + tiles * 2 * 512)
         assert L.tile_capacity * L.mid_tile_bytes >= 5 * (groups * 2 * 2048 + tiles * 2 * 512)
+
+
+def _counter_bytes(L, tmax, experts):
+    """What lies between the router logits and the tile images: the one-rank batch kernel's counters."""
+    return L.off_token_tiles - (L.off_logits + (min(tmax, 256) * experts * 16 + 1023) // 1024 * 1024)
+
+
+def test_the_static_scratch_has_room_for_the_counters_beside_24_mib():
+    """Configurations that need 24 MiB or less without the batch kernel's counters are served by the launch without any allocation."""
+    lib, near = _lib.load(), 0
+    header = open(os.path.join(ROOT, 'include', 'megamoe_b200.h')).read()
+    expr = re.search(r'#define MM_STATIC_SCRATCH_BYTES (.*)', header).group(1).replace('ll', '')
+    assert eval(expr) == _lib.STATIC_SCRATCH_BYTES
+    shapes = [(fmt, e, h, i, k, t) for fmt in ('mxfp4', 'nvfp4', 'fp8') for e in (1, 2, 8, 20, 32, 48, 64) for h in range(512, 4097, 512)
+              for i in range(256, 4097, 256) for k in (1, 2, 4, 6, 8, 16) for t in (1, 8, 16, 32, 64, 128, 256, 512)]
+    for fmt, e, h, i, k, t in [('mxfp4', 8, 1536, 512, 8, 128), ('mxfp4', 32, 4096, 2048, 2, 128)] + shapes:
+        cfg, L = _lib.MMConfig(1, 0, e, t, k, h, i, _lib.FMT[fmt], 148), _lib.MMLayout()
+        assert lib.mm_get_layout(ctypes.byref(cfg), ctypes.byref(L)) == 0
+        if L.total_bytes - _counter_bytes(L, t, e) <= 24 * 1024 * 1024:
+            near += L.total_bytes > 24 * 1024 * 1024
+            assert L.total_bytes <= _lib.STATIC_SCRATCH_BYTES, (fmt, e, h, i, k, t, L.total_bytes)
+    assert near >= 2

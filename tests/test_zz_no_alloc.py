@@ -88,6 +88,26 @@ def test_static_scratch_decode_launches_in_a_row(fmt, e_local, topk, sizes):
         assert O.rel_rmse(y.cpu(), ref.y[0]) <= 3e-3, (call, O.rel_rmse(y.cpu(), ref.y[0]))
 
 
+@pytest.mark.parametrize('tokens', [128, 1])                    # the batch kernel, whose outputs end where the array does, and the decode kernel
+def test_static_scratch_serves_a_configuration_of_24_mib_and_the_counters(tokens):
+    lib, (fmt, e_local, hidden, inter, topk, t_max) = _lib.load(), ('mxfp4', 8, 1536, 512, 8, 128)
+    cfg, L = _lib.MMConfig(1, 0, e_local, t_max, topk, hidden, inter, _lib.FMT[fmt], 0), _lib.MMLayout()
+    assert lib.mm_get_layout(ctypes.byref(cfg), ctypes.byref(L)) == 0 and 24 * 1024 * 1024 < L.total_bytes <= _lib.STATIC_SCRATCH_BYTES
+    w, _, _ = O.make_expert_weights(e_local, hidden, inter, fmt, seed=73, std=0.05)
+    l1, l2 = mm.transform_weights_for_mega_moe(*U.to_operator_weights(w, fmt, 'cuda'))
+    idx, tw = U.random_routing(tokens, e_local, topk, 74)
+    _, inp, sfb = U.make_rank_inputs(tokens, hidden, fmt, 75, idx, tw)
+    ref = O.moe_layer_reference([inp], [w], fmt, e_local, clamp=10.0)
+    x_d, sf_d, idx_d, tw_d = inp.x_q.view(torch.int8).cuda(), sfb.contiguous().cuda(), idx.cuda(), tw.cuda()
+    y, status = torch.empty((tokens, hidden), dtype=torch.bfloat16, device='cuda'), torch.full((16,), 0xFFFF, dtype=torch.int32, device='cuda')
+    args = _lib.MMStaticArgs(x_d.data_ptr(), sf_d.data_ptr(), idx_d.data_ptr(), tw_d.data_ptr(), l1[0].data_ptr(), l2[0].data_ptr(),
+                             y.data_ptr(), tokens, 1, None, 10.0, 1.0, 1.0, 1.0, 1.0, 500.0, status.data_ptr())
+    for _ in range(2):
+        assert lib.mm_mega_moe_launch_static_scratch(ctypes.byref(cfg), ctypes.byref(args), torch.cuda.current_stream().cuda_stream) == 0
+        torch.cuda.synchronize()
+        assert int(status[0]) == 0 and O.rel_rmse(y.cpu(), ref.y[0]) <= 3e-3
+
+
 def test_static_scratch_entry_rejects_what_it_cannot_hold():
     lib = _lib.load()
     stream = torch.cuda.current_stream().cuda_stream
