@@ -149,14 +149,14 @@ struct BCore {
         }
         return true;
     }
-    __device__ __forceinline__ void sm_phase(int slot) const {
-        reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlSmPhase)[blockIdx.x * kSmPhaseSlots + slot] = globaltimer_ns();
+    __device__ __forceinline__ void sm_phase(int slot, unsigned long long t = globaltimer_ns()) const {
+        reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlSmPhase)[blockIdx.x * kSmPhaseSlots + slot] = t;
     }
-    __device__ __forceinline__ void stamp(int slot) const {
-        reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlStamps)[slot] = globaltimer_ns();
+    __device__ __forceinline__ void stamp(int slot, unsigned long long t = globaltimer_ns()) const {
+        reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlStamps)[slot] = t;
     }
-    __device__ __forceinline__ void stamp_max(int slot) const {
-        atomicMax(reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlStamps) + slot, globaltimer_ns());
+    __device__ __forceinline__ void stamp_max(int slot, unsigned long long t = globaltimer_ns()) const {
+        atomicMax(reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlStamps) + slot, t);
     }
     // counters, `kBCountStride` words apart: `i` is a column block, kBCountClaims, or kBCountTiles + (layer - 1) * kBMaxTiles + tile
     __device__ __forceinline__ uint32_t* counter(uint32_t parity, uint32_t i) const {

@@ -80,9 +80,9 @@ struct DTasks {
     }
 };
 
-// `routed` is called once, when the first unit has been asked for.
-template <typename Routed>
-__device__ __forceinline__ void d_role_weights(const DCtx& cx, uint32_t nw, uint8_t* ring, Routed routed) {
+// `first` is called once: when the first unit has been asked for, or (false) on an SM without any.
+template <typename First>
+__device__ __forceinline__ void d_role_weights(const DCtx& cx, uint32_t nw, uint8_t* ring, First first) {
     const BParams& p = cx.p; DShared& c = cx.c;
     const uint64_t policy = l2_evict_first_policy();
     uint32_t it = 0, s = 0, ph = 0;
@@ -102,11 +102,11 @@ __device__ __forceinline__ void d_role_weights(const DCtx& cx, uint32_t nw, uint
                 c.wissued = it + 1u;
             }
             __syncwarp();
-            if (it == 0u) routed();
+            if (it == 0u) first(true);
             if (++s == nw) { s = 0; ph ^= 1u; }
         }
     }
-    if (it == 0u) routed();
+    if (it == 0u) first(false);
 }
 
 template <int kFmt>
@@ -611,17 +611,20 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
         // The others hear of the routing when the stream has begun, so that their first instructions, which come from the L2, do not hold up the
         // loader's (one token 22.0 -> 21.4 us a pass, two 28.2 -> 27.6). With E4M3 tokens the tile takes longer than
         // the first unit, and the others start first (two tokens 31.7 us, the other way round 32.9).
-        auto routed = [&] {
-            bar_arrive(kDBarRouted, F::kThreads);
-            if (lane == 0) {
-                cx.sm_phase(kSmScheduled); cx.stamp_max(kStampLastScheduled); if (bid == 0) cx.stamp(kStampScheduled);
-                reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlSmWFirst)[bid] = globaltimer_ns();
-                cx.sm_phase(kSmFirstIssue);
-            }
-        };
+        // (The times go to memory when the whole stream has been asked for.)
         const bool go = *reinterpret_cast<volatile uint32_t*>(&c.start_ok) != 0u;
-        if (F::kA8 || !go) routed();
-        if (go) d_role_weights(cx, nw, smem + ring_off, [&] { if constexpr (!F::kA8) routed(); });
+        unsigned long long t_routed = 0ull, t_first = ~0ull;          // (~0: no weights on this SM)
+        if (F::kA8 || !go) { t_routed = globaltimer_ns(); bar_arrive(kDBarRouted, F::kThreads); }
+        if (go) d_role_weights(cx, nw, smem + ring_off, [&](bool any) {
+            const unsigned long long t = globaltimer_ns();
+            if (any) t_first = t;
+            if constexpr (!F::kA8) { t_routed = t; bar_arrive(kDBarRouted, F::kThreads); }
+        });
+        if (lane == 0) {
+            cx.sm_phase(kSmScheduled, t_routed); cx.stamp_max(kStampLastScheduled, t_routed); if (bid == 0) cx.stamp(kStampScheduled, t_routed);
+            reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlSmWFirst)[bid] = t_first;
+            if (t_first != ~0ull) cx.sm_phase(kSmFirstIssue, t_first);
+        }
     } else bar_sync(kDBarRouted, F::kThreads);
     const bool start = *reinterpret_cast<volatile uint32_t*>(&c.start_ok) != 0u;
     if (start) {

@@ -433,3 +433,40 @@ def test_partial_sums_of_the_multi_rank_kernel_are_not_taken_for_the_decode_kern
         st, words = buf.device_status()
         assert st == 0 and words[4] == DECODE and words[1] == launch
         assert bool((sums == launch).all()) and O.rel_rmse(y.cpu(), ref.y[0]) <= REL_RMSE_TOL
+
+
+@pytest.mark.parametrize('fmt', ['mxfp4', 'nvfp4', 'fp8'])
+def test_first_weight_request_of_the_decode_kernel(fmt):
+    """Slot 13 of the stamps and slot 5 of an SM's record are the times of a weight request, not of the routing: an SM that asks for no
+    weights has none, whatever the launch before it left there, nor has a launch that fails at routing."""
+    e, hidden, inter, topk = 8, 512, 256, 2
+    w, _, _ = O.make_expert_weights(e, hidden, inter, fmt, seed=170, std=0.05)
+    l1, l2 = mm.transform_weights_for_mega_moe(*U.to_operator_weights(w, fmt, 'cuda'))
+    buf = mm.get_symm_buffer_for_mega_moe(None, e, 16, topk, hidden, inter, act_format=fmt)
+    call = mm.fp8_fp4_mega_moe if fmt == 'fp8' else mm.fp4_fp4_mega_moe
+    y = torch.empty((1, hidden), dtype=torch.bfloat16, device='cuda')
+    idx, tw = U.random_routing(1, e, topk, 171)
+    _, inp, sfb = U.make_rank_inputs(1, hidden, fmt, 172, idx, tw)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+
+    def launch(route):
+        U.write_inputs(buf, inp, sfb)
+        if route is not None:
+            buf.topk_idx[:1] = route
+        call(y, l1, l2, buf, timeout_ms=500.0)
+        st, words = buf.device_status()
+        assert words[4] == DECODE
+        return st, buf.phase_stamps(), buf.sm_phases()[:sms]
+
+    st, s, ph = launch(-1)                                          # no unit on any SM
+    assert st == 0 and s[13] == 0 and bool((ph[:, 5] == 0).all())
+    st, s, ph = launch(None)                                        # eight L1 tiles of two units, eight L2 tiles of one: part of the SMs
+    on = ph[:, 5] != 0
+    assert st == 0 and 0 < int(on.sum()) < sms and int(ph[on, 5].min()) == s[13]
+    assert bool((ph[on, 4] <= ph[on, 5]).all()) and bool((ph[on, 5] <= ph[on, 6]).all())       # scheduled, requested, landed
+    assert s[12] <= s[13] <= s[14] <= s[8]
+    st, s, _ = launch(-1)
+    assert st == 0 and s[13] == 0
+    launch(None)
+    st, s, _ = launch(e)                                            # no such expert
+    assert st == 4 and s[13] == 0
