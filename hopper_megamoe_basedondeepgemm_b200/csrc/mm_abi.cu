@@ -146,10 +146,10 @@ int mm_get_layout(const mm_config_t* c, mm_layout_t* out) {
         out->token_tile_bytes = mm::kWideTokens * 16 + (c->hidden / mm::kUnitK) * rec32;
         out->mid_tile_bytes = (c->intermediate / mm::kUnitK) * rec32;
     }
-    take(mm::kBCountBytes);                                                      // the one-rank batch kernel's counters
+    take(c->num_ranks == 1 ? mm::kBCountBytes : 0);                              // the one-rank batch kernel's counters
     out->off_token_tiles = take(out->tile_capacity * out->token_tile_bytes);
     out->off_mid_tiles = take(out->tile_capacity * out->mid_tile_bytes);
-    out->off_arrive = take(2 * 2 * out->tile_capacity * 4 + mm::kRoutesGap + mm::kFeMaxFusedTokens * 8 * 16);   // (then the one-rank batch kernel's counts and routing records)
+    out->off_arrive = take(2 * 2 * out->tile_capacity * 4 + (c->num_ranks == 1 ? mm::kRoutesGap + mm::kFeMaxFusedTokens * 8 * 16 : 0));   // (then the one-rank batch kernel's routing records)
     // the same kernel's expert outputs, of as many routing entries as it takes (`batch_out_offset`)
     const int64_t out_rows = t_max * c->num_topk < mm::kBMaxRows ? t_max * c->num_topk : mm::kBMaxRows;
     take(c->num_ranks == 1 ? out_rows * c->hidden * 2 : 0);

@@ -1852,10 +1852,12 @@ __global__ void __launch_bounds__(kA8 ? kThreads + kNumExpThreads : kThreads, 1)
         uint32_t* other = reinterpret_cast<uint32_t*>(buf + p.off_arrive) + (par ^ 1u) * 2u * p.tile_capacity;
         #pragma unroll 1
         for (uint32_t i = bid * kO + tid; i < 2u * p.tile_capacity; i += G * kO) other[i] = 0u;
-        // (and the counts of the one-rank batch kernel, which shares the buffer and the launch numbering)
-        #pragma unroll 1
-        for (uint32_t i = bid * kO + tid; i < static_cast<uint32_t>(kBCounters); i += G * kO)
-            reinterpret_cast<uint32_t*>(buf + p.off_token_tiles - kBCountBytes)[(par ^ 1u) * kBCounts + i * kBCountStride] = 0u;
+        // (and, on one rank, the counts of the batch kernel, which shares the buffer and the launch numbering)
+        if (p.R == 1) {
+            #pragma unroll 1
+            for (uint32_t i = bid * kO + tid; i < static_cast<uint32_t>(kBCounters); i += G * kO)
+                reinterpret_cast<uint32_t*>(buf + p.off_token_tiles - kBCountBytes)[(par ^ 1u) * kBCounts + i * kBCountStride] = 0u;
+        }
     }
     // The rows of this rank's own tokens never travel when `own_ok`: every SM lists them from topk_idx and reads their
     // tokens where the caller put them. The SM that would have dispatched them only leaves their header line and records

@@ -57,7 +57,9 @@ typedef struct mm_layout {
     int64_t off_red;           /* [256 SMs][2 phases][2][16][128] float partial sums of weight tiles split between SMs (local); behind the
                                   32 KB per SM of the launch's grid the one-rank decode kernel's, as flagged 8-byte words */
     int64_t off_cnt;           /* [2 phases][cnt_per_phase] uint32 contributors that have parked their part of a tile (local) */
-    int64_t off_logits;        /* [min(T_max, 256)][num_experts] 16 B records {half logit, launch flag} x 2 of the fused router frontend */
+    int64_t off_logits;        /* [min(T_max, 256)][num_experts] 16 B records {half logit, launch flag} x 2 of the fused router frontend;
+                                  on one rank the batch kernel's counters follow, which end where the token tiles begin: [2 parities] of a
+                                  128 B line per column block and per token tile and layer (csrc/mm_batch.cuh) */
     int64_t x_row_bytes, x_sf_row_bytes;
     int64_t rx_row_bytes, rx_cap_rows;
     int64_t mid_rows, mid_row_bytes, mid_sf_row_bytes;
@@ -70,7 +72,8 @@ typedef struct mm_layout {
                                   records of 16 B {source rank, token, slot, weight}, then per streamed K unit the unit's 128 B of every
                                   row in the tensor core's shared-memory order (128 B swizzle) and the unit's scale-word slots */
     int64_t off_mid_tiles;     /* [tile_capacity][mid_tile_bytes] the same, without the row records, for the requantised SwiGLU output */
-    int64_t off_arrive;        /* [2 parities][2][tile_capacity] uint32: rows of a token tile written / L1 weight tiles of a mid tile written */
+    int64_t off_arrive;        /* [2 parities][2][tile_capacity] uint32: rows of a token tile written / L1 weight tiles of a mid tile written;
+                                  on one rank the batch kernel's routing records and expert outputs follow */
     int64_t tile_capacity, token_tile_bytes, mid_tile_bytes;
 } mm_layout_t;
 
