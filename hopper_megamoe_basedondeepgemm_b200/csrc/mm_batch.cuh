@@ -481,7 +481,8 @@ struct BWiden {
 };
 
 // The ring has an even number of stages, so that a stage always belongs to the same group: a group that skipped a stage's
-// previous use could take the older phase of its barrier for the one it wants.
+// previous use could take the older phase of its barrier for the one it wants. The decode kernel's ring too: `fit` stages have room.
+__device__ __forceinline__ uint32_t even_stages(uint32_t fit, uint32_t most) { return (fit < most ? fit : most) & ~1u; }
 __device__ void b_role_widen(const BCtx& cx, uint32_t grp, uint32_t xtid) {
     const BParams& p = cx.p; BShared& c = cx.c;
     const uint32_t lane = xtid & 31u, nw = c.nw;
@@ -869,8 +870,8 @@ __device__ __forceinline__ void b_tiles(const BCtx& cx, uint32_t lane) {
         const uint32_t spu = !F::kA8 && pair * 8u <= room ? 2u : 1u;
         uint32_t nr = udiv_small(room, pair * spu), nw = nr;
         if (F::kA8) {                                        // rings of their own; an even number of weight stages (see b_role_widen)
-            nw = udiv_small(room, pair) & ~1u;
-            nw = nw < 4u ? 4u : (nw > kBWStages ? kBWStages : nw);
+            nw = even_stages(udiv_small(room, pair), kBWStages);
+            nw = nw < 4u ? 4u : nw;
             nr = udiv_small(room - nw * p.unit_bytes, rec);
         }
         nr = nr > kBRSlots ? kBRSlots : nr;

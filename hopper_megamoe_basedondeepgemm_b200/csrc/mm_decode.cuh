@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
     // shared memory: token tile (the intermediate rows' tile takes the place of the tokens'), weight ring
     const uint32_t ring_off = (p.k1 > p.k2 ? p.k1 : p.k2) * F::kRec;
     uint32_t nw = udiv_small(p.smem_ring - ring_off, p.unit_bytes);
-    nw = nw > kDStages ? kDStages : (F::kA8 ? nw & ~1u : nw);
+    nw = F::kA8 ? even_stages(nw, kDStages) : (nw > kDStages ? kDStages : nw);
     // ---- what needs nothing of the launches before this one: it overlaps the end of the previous kernel in the stream
     if (warp == 2) {
         if (lane < kDStages) { mbar_init(&c.wfull[lane], 1); mbar_init(&c.wempty[lane], F::kA8 ? kBExpWarps / 2 : 1); }
