@@ -119,12 +119,11 @@ enum SmPhase : int {
 // in a shared line the L2 takes them one after the other (64 tokens: 55.7 -> 53.6 us a pass, 96 skewed from hidden states 70.6 -> 69.3).
 constexpr int kBMaxTiles = 128;                    // token tiles of one launch (64 experts + rows beyond the tile limit)
 constexpr int kBColCounters = 32;                  // (hidden <= 4096)
-constexpr int kBCountClaims = kBColCounters, kBCountTiles = kBCountClaims + 1;
-constexpr int kBCounters = (kBCountTiles + 2 * kBMaxTiles + 3) / 4 * 4;            // (two sets of whole 512 B: the token images start on 1 KB)
+constexpr int kBCountClaims = kBColCounters, kBCountTiles = kBColCounters + 32, kBCounters = kBCountTiles + 2 * kBMaxTiles;
 constexpr int kBCountStride = 32;                  // words from one counter to the next
 constexpr int kBCounts = kBCounters * kBCountStride;
 constexpr int kBCountBytes = 2 * kBCounts * 4;      // of both sets, which end where the token images begin
-constexpr int kRoutesGap = 512;                     // bytes between the arrival counts and the routing records, which nothing uses: a buffer's end stays as long as it was
+constexpr int kRoutesGap = 512;                     // bytes between the arrival counts and the routing records
 static_assert(kBCountBytes % 1024 == 0, "no gap in front of the token images");
 
 struct RowMeta { int32_t src, token, slot; float weight; };

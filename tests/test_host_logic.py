@@ -438,10 +438,10 @@ def _counter_bytes(L, tmax, experts):
 @pytest.mark.parametrize('fmt', ['mxfp4', 'fp8'])
 @pytest.mark.parametrize('experts,tmax', [(8, 1), (48, 128), (64, 512), (64, 32768)])
 def test_counters_of_the_batch_kernel_are_in_the_buffers_of_one_rank_only(fmt, experts, tmax):
-    """Two sets of 128 B lines, one per column block (hidden / 128 <= 32), one of the claims and two per token tile (at most 128), between the router logits
+    """Two sets of 128 B lines, one per column block (hidden / 128 <= 32) and two per token tile (at most 128), between the router logits
     and the token tiles. Several ranks have no such kernel: nothing lies there or behind the arrival counts."""
     st, L = _layout(ranks=1, experts=experts, tmax=tmax, fmt=fmt)
-    assert st == 0 and 0 <= _counter_bytes(L, tmax, experts) - 2 * (32 + 1 + 2 * 128) * 128 < 1024 and L.off_token_tiles % 1024 == 0
+    assert st == 0 and 2 * (32 + 2 * 128) * 128 <= _counter_bytes(L, tmax, experts) <= 80 * 1024 and L.off_token_tiles % 1024 == 0
     for ranks in (2, 8):
         st, L = _layout(ranks=ranks, experts=experts * ranks, tmax=tmax, fmt=fmt)
         assert st == 0 and _counter_bytes(L, tmax, experts * ranks) == 0
