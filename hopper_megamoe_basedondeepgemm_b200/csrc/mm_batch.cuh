@@ -16,14 +16,14 @@
 //   order    : the L1 tasks dealt round-robin, but the last one to two rounds of them and all L2 tasks claimed one by one
 //              (no tile is split along K, a slow SM takes fewer). L2 goes tile by tile, its last four tasks per SM column
 //              block by column block. The weight ring runs ahead over the L1 -> L2 hand-over, so that the stream does not
-//              stop there. (All L1 tasks dealt and L2 column by column: 59.2, 67.2 and 102 us where this order takes 57.2,
-//              64.9 and 100, for 13 and 64 tokens over 48 experts and 96 skewed ones.)
+//              stop there. (When this order came in: 59.2, 67.2 and 102 us with all L1 tasks dealt and L2 column by column, 57.2,
+//              64.9 and 100 with it, for 13 and 64 tokens over 48 experts and 96 skewed ones from hidden states.)
 //   combine  : per (token, 128-column block) behind a count per column block; routes added in slot order in fp32.
 //
 // Bound: HBM (the weights of the live experts once) up to about 40 rows per expert; beyond that the bytes an SM takes in
-// per unit (weights + token record, about 48 GB/s from the L2). 64 tokens, MXFP4, 48 experts (301 MB): 53.5 us a pass, of
+// per unit (weights + token record, about 48 GB/s from the L2). 64 tokens, MXFP4, 48 experts (301 MB): 54.3 us a pass, of
 // which the stream is 46; the multi-rank kernel takes 88. With E4M3 tokens the units are widened into tensor memory,
-// which keeps up with the stream (100 tokens: 67.7 us, 765 with the multi-rank kernel).
+// which keeps up with the stream (100 tokens: 70.0 us, 765 with the multi-rank kernel).
 #pragma once
 #include "mm_kernel.cuh"
 
@@ -158,7 +158,8 @@ struct BCore {
     __device__ __forceinline__ void stamp_max(int slot, unsigned long long t = globaltimer_ns()) const {
         atomicMax(reinterpret_cast<unsigned long long*>(p.buf + p.off_ctrl + kCtrlStamps) + slot, t);
     }
-    // counters, `kBCountStride` words apart: `i` is a column block, kBCountClaims, or kBCountTiles + (layer - 1) * kBMaxTiles + tile
+    // counters, `kBCountStride` words apart: `i` is a column block, kBCountClaims, or kBCountTiles + layer * kBMaxTiles + tile (layer 0:
+    // rows in the token image, layer 1: L1 tasks done)
     __device__ __forceinline__ uint32_t* counter(uint32_t parity, uint32_t i) const {
         return reinterpret_cast<uint32_t*>(p.buf + p.off_token_tiles - kBCountBytes) + parity * kBCounts + i * kBCountStride;
     }
@@ -709,14 +710,15 @@ __device__ void b_role_epilogue(const BCtx& cx, uint32_t grp, uint32_t etid) {
 
 // ============================================================================================= combine
 // Item i = column block * T + token: a half-warp adds the token's routes over 128 columns. SM b has the items b, b + G, ...;
-// its warps take them two by two in that order: the combine warps from the start, the others when their role has ended.
+// its warps take them two by two in that order: the combine warps when the SM has come to its first column task, the others
+// when their role has ended.
 __device__ void b_role_combine(const BCtx& cx, uint32_t lane) {
     const BParams& p = cx.p; BShared& c = cx.c;
     const uint32_t G = gridDim.x, nitems = static_cast<uint32_t>(p.T) * p.n2, half = lane >> 4, l16 = lane & 15u;
     const uint32_t M = c.M;
     uint32_t known = 0xFFFFFFFFu;                            // the column block this half-warp saw complete last
     // nothing is complete before this SM, like the others, has come to the tasks that go column block by column block (without live rows
-    // there is nothing to wait for: 200 tokens, every slot masked, 9.62 us a pass behind the gate, 9.25 so)
+    // there is nothing to wait for: 200 tokens, every slot masked, 9.66 us a pass behind the gate, 9.27 so)
     for (uint32_t spins = 0; M != 0u && *reinterpret_cast<volatile uint32_t*>(&c.comb_open) == 0u;) {
         __nanosleep(200);
         if (cx.give_up(spins, kErrWaitCombineFlag, 0u)) break;
@@ -1039,7 +1041,7 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
         }
     }
     __syncthreads();
-    // ---- tiles. The warp that works them out is the weight loader: it starts the weight stream without waiting for the others
+    // ---- tiles. The warp that works them out is the weight loader (its stream starts when the worker warps have placed the SM's rows)
     if (warp == 0) {
         if (lane == 0) cx.sm_phase(kSmCountsKnown);
         b_tiles<kFmt>(cx, lane);
@@ -1068,7 +1070,7 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
     }
     if (worker && start) {
         // ---- copy the rows of this SM's tokens into the tiles' images, one warp per row; a warp's stores are released four
-        //      rows at a time (under the weight stream a release takes microseconds)
+        //      rows at a time (a release waits for the stores before it: this SM's own weight stream begins behind them)
         uint32_t done_m[4], ndone = 0;
         #pragma unroll 1
         for (uint32_t k = ww; k < nrows; k += kBWorkWarps) {
@@ -1128,8 +1130,9 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
         #pragma unroll 1
         for (uint32_t r = ww; r < kBRankWarps; r += kBWorkWarps) b_list_run(cx, r, seg_shift, nent, lane);
         bar_sync(kBBarWork, kBWorkWarps * 32u);
-        // ---- off the critical path: the rows' records in the receive pool (a row's place: the live entries before it), for
-        //      whoever inspects the pool afterwards
+        // ---- the rows' records in the receive pool (a row's place: the live entries before it), for whoever inspects the pool
+        //      afterwards. With 4-bit tokens these warps only wait for the combine; with E4M3 tokens they are the widening group of
+        //      the first unit, which waits for the records.
         if (warp >= kBServiceWarps + kBEpiWarps) {
             #pragma unroll 1
             for (uint32_t k = ww - kBEpiWarps; k < nrows; k += kBWorkWarps - kBEpiWarps) {

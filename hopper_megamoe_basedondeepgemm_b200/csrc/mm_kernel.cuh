@@ -119,11 +119,13 @@ enum SmPhase : int {
 // in a shared line the L2 takes them one after the other (64 tokens: 55.7 -> 53.6 us a pass, 96 skewed from hidden states 70.6 -> 69.3).
 constexpr int kBMaxTiles = 128;                    // token tiles of one launch (64 experts + rows beyond the tile limit)
 constexpr int kBColCounters = 32;                  // (hidden <= 4096)
+// (31 lines between the claims and the tiles are unused. With the tiles next to the claims 200 tokens with 95 % of their slots masked took
+// 45.4 us instead of 44.9, 64 tokens 51.7 instead of 51.5, the small layer 14.79 instead of 14.89.)
 constexpr int kBCountClaims = kBColCounters, kBCountTiles = kBColCounters + 32, kBCounters = kBCountTiles + 2 * kBMaxTiles;
 constexpr int kBCountStride = 32;                  // words from one counter to the next
 constexpr int kBCounts = kBCounters * kBCountStride;
 constexpr int kBCountBytes = 2 * kBCounts * 4;      // of both sets, which end where the token images begin
-constexpr int kRoutesGap = 512;                     // bytes between the arrival counts and the routing records
+constexpr int kRoutesGap = 512;                     // bytes between the arrival counts and the routing records, unused (with the claims there: small layer 14.68 -> 14.73 us)
 static_assert(kBCountBytes % 1024 == 0, "no gap in front of the token images");
 
 struct RowMeta { int32_t src, token, slot; float weight; };

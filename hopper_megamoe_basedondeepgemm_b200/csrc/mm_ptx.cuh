@@ -211,7 +211,7 @@ __device__ __forceinline__ void umma_mxf8f6f4(uint32_t d_tmem, uint64_t adesc, u
         "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
         ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa_tmem), "r"(sfb_tmem) : "memory");
 }
-// The same with A in tensor memory, one weight row per lane and four E4M3 values per column (K = 32: eight columns)
+// The same with A in tensor memory: one weight row per lane, four E2M1 codes per column, each in bits 2 to 5 of a byte (K = 32: eight columns)
 __device__ __forceinline__ void umma_mxf8f6f4_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
                                                  uint32_t sfa_tmem, uint32_t sfb_tmem, uint32_t accumulate) {
     asm volatile(
