@@ -965,20 +965,14 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
             if (cx.expired()) { cx.fail(kErrWaitFrontend); return true; }
             return false;
         };
-        // the upper warps, which have the fewest logits to work out, quantise this SM's tokens first
-        const uint32_t half_warps = kBRankWarps / 2;
-        if (warp >= half_warps && warp < kBRankWarps) {
-            #pragma unroll 1
-            for (uint32_t k = warp - half_warps; k < ntok; k += half_warps) {
-                const uint32_t tok = bid + k * G;
-                fe_quant_token(p.fe.hidden + static_cast<size_t>(tok) * p.H, p.H, kFmt, p.fe.x_gs, p.buf + p.off_x + static_cast<size_t>(tok) * p.x_row_bytes,
-                               p.buf + p.off_x_sf + static_cast<size_t>(tok) * p.x_sf_row_bytes, lane);
-            }
-        }
-        const uint32_t eb = fe_expert_block(p.fe, G);
-        if (eb == 1u) fe_logits_blocks<1, 3>(p.fe, gw, nw, lane, flag);
-        else if (F::kA8 || eb == 2u) fe_logits_blocks<2, 2>(p.fe, gw, nw, lane, flag);
-        else fe_logits_blocks<4, 2>(p.fe, gw, nw, lane, flag);
+        // Items of one token where every warp gets one at most: all its loads are in flight at once (two round trips less than with
+        // items of four tokens; 3 tokens 37.2 -> 35.3 us a pass, 24: 57.5 -> 55.3). Up to 24 items of four tokens per SM, one expert to an
+        // item (150 tokens 72.0 -> 70.7); beyond, where the bytes count, blocks of experts (256: 79.2 -> 76.8 all in all). Two
+        // more block sizes in between gained nothing: the launch pays for code that it jumps over.
+        const uint32_t half_warps = kBRankWarps / 2, per = static_cast<uint32_t>(p.E) * kFeParts;
+        if (per * p.T <= 16u * G) fe_logits_blocks<1, 6, 1>(p.fe, gw, nw, lane, flag);
+        else if (per * ((p.T + 3u) / 4u) <= 24u * G) fe_logits_blocks<1, 3>(p.fe, gw, nw, lane, flag);
+        else fe_logits_blocks<F::kA8 ? 2 : 4, 2>(p.fe, gw, nw, lane, flag);
         if (warp < half_warps) {
             #pragma unroll 1
             for (uint32_t k = warp; k < ntok; k += half_warps) {
@@ -986,6 +980,16 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
                 // later (96 tokens of 3072, 128 experts: 77.3 -> 75.7 us a pass)
                 const bool nz = fe_row_nonzero(p.fe.hidden + static_cast<size_t>(bid + k * G) * p.H, p.H, lane);
                 if (!fe_select_token_regs<2>(p.fe, bid + k * G, nz, lane, flag, p.buf + p.off_routes, give_up)) break;
+            }
+        } else {
+            // The other warps quantise this SM's tokens, a slice of 256 elements at a time. (A warp takes 5 to 7 us for a whole token, most of it divisions;
+            // before its logits, as it once was, the records of its items came that much later: 256 tokens 86.0 -> 81.8 us, NVFP4.)
+            const uint32_t nslice = static_cast<uint32_t>(p.H) / 256u, nq = F::kThreadsAll / 32 - half_warps;
+            #pragma unroll 2
+            for (uint32_t i = warp - half_warps; i < ntok * nslice; i += nq) {
+                const uint32_t k = udiv_small(i, nslice), tok = bid + k * G;
+                fe_quant_slice(p.fe.hidden + static_cast<size_t>(tok) * p.H, kFmt, p.fe.x_gs, p.buf + p.off_x + static_cast<size_t>(tok) * p.x_row_bytes,
+                               p.buf + p.off_x_sf + static_cast<size_t>(tok) * p.x_sf_row_bytes, i - k * nslice, lane);
             }
         }
         #pragma unroll 1

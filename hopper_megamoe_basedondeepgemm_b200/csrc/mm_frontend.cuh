@@ -90,31 +90,34 @@ __device__ __forceinline__ void fe_logits_items(const FeParams& q, uint32_t warp
     }
 }
 
-// The same partial logits (the same sums in the same order) with blocks of kEb experts x 4 tokens per warp and kAhead chunks
+// The same partial logits (the same sums in the same order) with blocks of kEb experts x kTb tokens per warp and kAhead chunks
 // per lane in flight: per multiply-add a block of 4 x 4 reads 0.5 operand chunks instead of 1.25. The loads run at what an
 // SM takes in from the L2 (about 50 GB/s), so that is the time of a large batch; a small one needs every (expert, half) as
-// an item of its own to have enough of them. `fe_expert_block` draws the line at four items per SM.
-template <int kEb, int kAhead>
+// an item of its own to have enough of them. `fe_expert_block` draws the stand-alone frontend's line at four items per SM.
+template <int kEb, int kAhead, int kTb = 4>
 __device__ __forceinline__ void fe_logits_blocks(const FeParams& q, uint32_t warp, uint32_t nwarps, uint32_t lane, uint32_t flag) {
-    const uint32_t tblocks = (q.T + 3) / 4, eblocks = (q.E + kEb - 1) / kEb, nchunk = q.H / 8, half = (nchunk + kFeParts - 1) / kFeParts;
+    const uint32_t tblocks = (q.T + kTb - 1) / kTb, eblocks = (q.E + kEb - 1) / kEb, nchunk = q.H / 8, half = (nchunk + kFeParts - 1) / kFeParts;
     const uint32_t nitems = eblocks * kFeParts * tblocks;
     #pragma unroll 1
     for (uint32_t item = warp; item < nitems; item += nwarps) {
-        const uint32_t part = item % kFeParts, r = item / kFeParts, tb = udiv_small(r, eblocks), e0 = (r - tb * eblocks) * kEb, t0 = tb * 4u;
-        const uint32_t nt = min(4u, static_cast<uint32_t>(q.T) - t0), ne = min(static_cast<uint32_t>(kEb), static_cast<uint32_t>(q.E) - e0);
+        const uint32_t part = item % kFeParts, r = item / kFeParts, tb = udiv_small(r, eblocks), e0 = (r - tb * eblocks) * kEb, t0 = tb * kTb;
+        const uint32_t nt = min(static_cast<uint32_t>(kTb), static_cast<uint32_t>(q.T) - t0), ne = min(static_cast<uint32_t>(kEb), static_cast<uint32_t>(q.E) - e0);
         const uint32_t c_lo = part * half, c_hi = min(nchunk, c_lo + half);
-        float acc[kEb][4];
+        float acc[kEb][kTb];
         #pragma unroll
-        for (int e = 0; e < kEb; ++e) { acc[e][0] = 0.f; acc[e][1] = 0.f; acc[e][2] = 0.f; acc[e][3] = 0.f; }
+        for (int e = 0; e < kEb; ++e) {
+            #pragma unroll
+            for (int t = 0; t < kTb; ++t) acc[e][t] = 0.f;
+        }
         // (rows beyond the last expert or token repeat the last one: their sums are not stored)
-        const uint4 *wrow[kEb], *xrow[4];
+        const uint4 *wrow[kEb], *xrow[kTb];
         #pragma unroll
         for (uint32_t e = 0; e < kEb; ++e) wrow[e] = reinterpret_cast<const uint4*>(q.router_w + static_cast<size_t>(e0 + (e < ne ? e : ne - 1u)) * q.H);
         #pragma unroll
-        for (uint32_t t = 0; t < 4; ++t) xrow[t] = reinterpret_cast<const uint4*>(q.hidden + static_cast<size_t>(t0 + (t < nt ? t : nt - 1u)) * q.H);
+        for (uint32_t t = 0; t < kTb; ++t) xrow[t] = reinterpret_cast<const uint4*>(q.hidden + static_cast<size_t>(t0 + (t < nt ? t : nt - 1u)) * q.H);
         #pragma unroll 1
         for (uint32_t ch0 = c_lo + lane; ch0 < c_hi; ch0 += 32 * kAhead) {
-            uint4 wq[kEb][kAhead], xq[4][kAhead];
+            uint4 wq[kEb][kAhead], xq[kTb][kAhead];
             #pragma unroll
             for (uint32_t b = 0; b < kAhead; ++b) {
                 const uint32_t ch = ch0 + 32 * b;
@@ -122,14 +125,14 @@ __device__ __forceinline__ void fe_logits_blocks(const FeParams& q, uint32_t war
                     #pragma unroll
                     for (uint32_t e = 0; e < kEb; ++e) wq[e][b] = __ldg(wrow[e] + ch);
                     #pragma unroll
-                    for (uint32_t t = 0; t < 4; ++t) if (t < nt) xq[t][b] = __ldg(xrow[t] + ch);
+                    for (uint32_t t = 0; t < kTb; ++t) if (t < nt) xq[t][b] = __ldg(xrow[t] + ch);
                 }
             }
             #pragma unroll
             for (uint32_t b = 0; b < kAhead; ++b) {
                 if (ch0 + 32 * b < c_hi) {
                     #pragma unroll
-                    for (uint32_t t = 0; t < 4; ++t) {
+                    for (uint32_t t = 0; t < kTb; ++t) {
                         if (t < nt) {
                             float x[8];
                             unpack_bf16x8(xq[t][b], x);
@@ -148,7 +151,7 @@ __device__ __forceinline__ void fe_logits_blocks(const FeParams& q, uint32_t war
         #pragma unroll
         for (uint32_t e = 0; e < kEb; ++e) {
             #pragma unroll
-            for (uint32_t t = 0; t < 4; ++t) {
+            for (uint32_t t = 0; t < kTb; ++t) {
                 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) acc[e][t] += __shfl_xor_sync(0xffffffffu, acc[e][t], o);
                 if (lane == 0 && t < nt && e < ne)
@@ -269,6 +272,17 @@ __device__ __forceinline__ bool fe_quant_token(const __nv_bfloat16* xrow, int H,
         }
     }
     return __any_sync(0xffffffffu, nonzero);
+}
+
+// One warp quantises the 256 elements `slice` of a token row.
+__device__ __forceinline__ void fe_quant_slice(const __nv_bfloat16* xrow, int fmt, float x_gs, uint8_t* qrow, uint8_t* sfrow, uint32_t slice, uint32_t lane) {
+    const uint32_t k0 = slice * 256u + lane * 8u, vec = fmt == 1 ? 16u : 32u;
+    bool nonzero = false;
+    uint32_t sf_byte;
+    const uint2 bytes = fe_quant8(*reinterpret_cast<const uint4*>(xrow + k0), fmt, x_gs, nonzero, sf_byte);
+    if (lane % (vec / 8u) == 0u) sfrow[k0 / vec] = static_cast<uint8_t>(sf_byte);
+    if (fmt == 2) *reinterpret_cast<uint2*>(qrow + k0) = bytes;
+    else *reinterpret_cast<uint32_t*>(qrow + k0 / 2u) = bytes.x;
 }
 
 // One warp: is any element of the bf16 row non-zero?

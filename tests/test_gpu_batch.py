@@ -353,6 +353,37 @@ def test_from_hidden_states_on_one_or_two_sms_fills_every_view(fmt, num_sms, tok
         assert torch.equal(a, v[:tokens].view(torch.uint8))
 
 
+@pytest.mark.parametrize('fmt', ['mxfp4', 'nvfp4', 'fp8'])
+@pytest.mark.parametrize('tokens,e,hidden', [
+    (1, 16, 4096), (2, 48, 512), (3, 48, 4096),                       # one token to an item: rows of one and of eight chunks a lane, more than are in flight
+    (24, 48, 512), (25, 48, 1536), (148, 48, 512), (149, 48, 1024),   # both sides of the lines between the item sizes (on 148 SMs)
+    (256, 16, 512), (256, 64, 1024),
+])
+def test_frontend_of_the_one_rank_kernels_matches_the_stand_alone_one(fmt, tokens, e, hidden):
+    """Routing and quantised tokens, bit for bit, whatever the items the partial logits are cut into."""
+    g = torch.Generator().manual_seed(190 + tokens)
+    x = torch.randn((tokens, hidden), generator=g).to(torch.bfloat16)
+    x[tokens // 2] = 0
+    x = x.cuda()
+    wr = (torch.randn((e, hidden), generator=g) / hidden ** 0.5).to(torch.bfloat16).cuda()
+    inter = 256
+    stream = lambda n, k: (torch.zeros((e, n // 128, k // 256, 18432 if fmt == 'nvfp4' else 17408), dtype=torch.uint8, device='cuda'),      # noqa: E731
+                           torch.tensor([n, k, 16 if fmt == 'nvfp4' else 32]))
+    buf = mm.get_symm_buffer_for_mega_moe(None, e, tokens, 8, hidden, inter, act_format=fmt)
+    ws = torch.zeros(mm.fe_workspace_bytes(buf), dtype=torch.uint8, device='cuda')
+    y = torch.empty((tokens, hidden), dtype=torch.bfloat16, device='cuda')
+    kw = dict(x_global_scale=1.0 / 64.0) if fmt == 'nvfp4' else {}
+    views = (buf.x, buf.x_sf, buf.topk_idx, buf.topk_weights)
+    for v in views:
+        v.view(torch.uint8).fill_(0x55)
+    mm.mega_moe_from_hidden(y, x, wr, stream(2 * inter, hidden), stream(hidden, inter), buf, ws, timeout_ms=500.0, **kw)
+    assert buf.device_status()[0] == 0
+    got = [v[:tokens].view(torch.uint8).clone() for v in views]
+    mm.fe_forward_into_buffer(x, wr, buf, ws, **kw)
+    for a, v in zip(got, views):
+        assert torch.equal(a, v[:tokens].view(torch.uint8))
+
+
 MULTI_RANK, BATCH, DECODE = 1, 2, 3             # status word 4
 
 
