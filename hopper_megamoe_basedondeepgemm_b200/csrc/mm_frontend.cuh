@@ -274,15 +274,20 @@ __device__ __forceinline__ bool fe_quant_token(const __nv_bfloat16* xrow, int H,
     return __any_sync(0xffffffffu, nonzero);
 }
 
-// One warp quantises the 256 elements `slice` of a token row.
-__device__ __forceinline__ void fe_quant_slice(const __nv_bfloat16* xrow, int fmt, float x_gs, uint8_t* qrow, uint8_t* sfrow, uint32_t slice, uint32_t lane) {
+// One warp quantises the 256 elements `slice` of a token row; with `also` the bytes go to a second row too.
+__device__ __forceinline__ void fe_quant_slice(const __nv_bfloat16* xrow, int fmt, float x_gs, uint8_t* qrow, uint8_t* sfrow, uint32_t slice, uint32_t lane,
+                                               bool also = false, uint8_t* qrow2 = nullptr, uint8_t* sfrow2 = nullptr) {
     const uint32_t k0 = slice * 256u + lane * 8u, vec = fmt == 1 ? 16u : 32u;
     bool nonzero = false;
     uint32_t sf_byte;
     const uint2 bytes = fe_quant8(*reinterpret_cast<const uint4*>(xrow + k0), fmt, x_gs, nonzero, sf_byte);
-    if (lane % (vec / 8u) == 0u) sfrow[k0 / vec] = static_cast<uint8_t>(sf_byte);
-    if (fmt == 2) *reinterpret_cast<uint2*>(qrow + k0) = bytes;
-    else *reinterpret_cast<uint32_t*>(qrow + k0 / 2u) = bytes.x;
+    auto put = [&](uint8_t* q, uint8_t* sf) {
+        if (lane % (vec / 8u) == 0u) sf[k0 / vec] = static_cast<uint8_t>(sf_byte);
+        if (fmt == 2) *reinterpret_cast<uint2*>(q + k0) = bytes;
+        else *reinterpret_cast<uint32_t*>(q + k0 / 2u) = bytes.x;
+    };
+    put(qrow, sfrow);
+    if (also) put(qrow2, sfrow2);
 }
 
 // One warp: is any element of the bf16 row non-zero?
