@@ -24,10 +24,14 @@ constexpr int kDThreads = 32 * (4 + kDEpiWarps);
 constexpr int kDThreadsA8 = kDThreads + 32 * kBExpWarps;     // E4M3 tokens: widening warps 12..19
 constexpr int kDStages = 12;
 constexpr uint32_t kDBarGroups = 5, kDBarRouted = 6;
+// tensor-memory columns with E4M3 tokens: behind the two accumulators the scales of the weights and of the tokens (8 each) and the widened units (64 each).
+// Four units: the widening runs ahead of the MMAs, which take two at a turn (two tokens 28.3 -> 27.9 us a pass against two units, one at a turn).
+// In the batch kernel, whose accumulators leave room for four too, that gained nothing (100 tokens 68.4, 69.1).
+constexpr uint32_t kDWide = 4, kDTmScaleW = 64, kDTmScaleX = kDTmScaleW + kDWide * 8, kDTmWide = 128;
 
 struct DShared {
     uint64_t wfull[kDStages], wempty[kDStages];
-    uint64_t tmem_full[2], tmem_empty[2], xfull[2], xempty[2], tile_full[2];
+    uint64_t tmem_full[2], tmem_empty[2], xfull[kDWide], xempty[kDWide], tile_full[2];
     uint32_t tmem_base, abort_flag, comb_next, wissued, M, nlive, live_mask, start_ok;
     uint32_t split_t, split_range, split_first, split_parts;      // this SM's part of a remainder tile: tile, first unit | end unit << 8, first SM of the group, parts (0: none)
     uint32_t exp_e[kDEntries], exp_c0[kDEntries], exp_n[kDEntries];    // active experts, ascending: id, first column, rows
@@ -135,27 +139,24 @@ __device__ void d_role_mma(const DCtx& cx, uint32_t lane, uint32_t nw_, uint32_t
         tc_fence_after();
         // A stage that is there already goes out in the same turn: a turn is a barrier wait, a fence, an election and a reconvergence beside
         // the issue, 540 to 640 cycles for a unit that the tensor pipe has in 200 (one token 20.6 -> 20.4 us a pass, two 27.2
-        // -> 26.7; four stages a turn no better). With E4M3 tokens the second is seldom there yet.
-        constexpr uint32_t kTurn = kA8 ? 1u : 2u;
+        // -> 26.7; four stages a turn no better).
         #pragma unroll 1
         for (uint32_t u = ub; u < ue;) {
-            if (!cx.warp_wait(kA8 ? &c.xfull[it & 1u] : &c.wfull[s], kA8 ? (it >> 1) & 1u : ph, kErrWaitFull)) return;
-            uint32_t n = 1u;
-            if constexpr (kTurn == 2u) {
-                const uint32_t s1 = s + 1u == nw ? 0u : s + 1u;
-                if (__all_sync(0xffffffffu, u + 1u < ue && mbar_test(&c.wfull[s1], s1 == 0u ? ph ^ 1u : ph))) n = 2u;
-            }
+            if (!cx.warp_wait(kA8 ? &c.xfull[it % kDWide] : &c.wfull[s], kA8 ? (it / kDWide) & 1u : ph, kErrWaitFull)) return;
+            const uint32_t s1 = s + 1u == nw ? 0u : s + 1u;
+            const bool next = u + 1u < ue && (kA8 ? mbar_test(&c.xfull[(it + 1u) % kDWide], ((it + 1u) / kDWide) & 1u) : mbar_test(&c.wfull[s1], s1 == 0u ? ph ^ 1u : ph));
+            const uint32_t n = __all_sync(0xffffffffu, next) ? 2u : 1u;
             tc_fence_after();
             if (lane == 0 && it == 0u) cx.sm_phase(kSmFirstLanded);
             if (elect_one()) {
                 #pragma unroll 1
                 for (uint32_t b = 0; b < n; ++b) {
-                    const uint32_t slot = b == 0u ? s : (s + 1u == nw ? 0u : s + 1u), i = it + b, wsm = ring0 + slot * p.unit_bytes, tok = s0 + (u + b) * F::kRec;
+                    const uint32_t slot = b == 0u ? s : s1, i = it + b, wsm = ring0 + slot * p.unit_bytes, tok = s0 + (u + b) * F::kRec;
                     const uint64_t adesc = smem_desc(wsm, 1024u, kLayoutSw128), bdesc = smem_desc(tok, 1024u, kLayoutSw128);
                     const uint64_t asf = smem_desc(wsm + kUnitWBytes, 128u, kLayoutNone);
                     const uint64_t bsf = smem_desc(tok + 2048u * F::kAtoms, 128u, kLayoutNone);
-                    const uint32_t sfa = kA8 ? tm + kTmScaleW + (i & 1u) * 8u : tm + 32u + (i & 1u) * 32u, sfb = kA8 ? tm + kTmScaleX + (i & 1u) * 8u : sfa + 16u;
-                    const uint32_t wide = tm + kTmWide + (i & 1u) * 64u;
+                    const uint32_t sfa = kA8 ? tm + kDTmScaleW + (i % kDWide) * 8u : tm + 32u + (i & 1u) * 32u, sfb = kA8 ? tm + kDTmScaleX + (i % kDWide) * 8u : sfa + 16u;
+                    const uint32_t wide = tm + kDTmWide + (i % kDWide) * 64u;
                     #pragma unroll
                     for (uint32_t pl = 0; pl < kPlanes; ++pl) {
                         if constexpr (!kA8) utccp_32x128b_warpx4(sfa + pl * 4u, asf + pl * 32u);
@@ -171,7 +172,7 @@ __device__ void d_role_mma(const DCtx& cx, uint32_t lane, uint32_t nw_, uint32_t
                         else if constexpr (kFmt == 0) umma_mxf4_block32(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
                         else umma_nvf4_block16(d, ad, bd, idesc, sfa + pl * 4u, sfb + pl * 4u, accum);
                     }
-                    tc_commit(kA8 ? &c.xempty[i & 1u] : &c.wempty[slot]);
+                    tc_commit(kA8 ? &c.xempty[i % kDWide] : &c.wempty[slot]);
                 }
             }
             __syncwarp();
@@ -188,7 +189,7 @@ __device__ void d_role_mma(const DCtx& cx, uint32_t lane, uint32_t nw_, uint32_t
 __device__ void d_role_widen(const DCtx& cx, uint32_t grp, uint32_t xtid, uint32_t nw, const uint8_t* ring) {
     const BParams& p = cx.p; DShared& c = cx.c;
     const uint32_t lane = xtid & 31u;
-    const uint32_t tm = c.tmem_base + ((xtid & 96u) << 16), ta = tm + kTmWide + grp * 64u, tsf = tm + kTmScaleW + grp * 8u;
+    const uint32_t tm = c.tmem_base + ((xtid & 96u) << 16);
     uint32_t it = 0, s = 0, ph = 0;
     DTasks tasks(cx);
     #pragma unroll 1
@@ -203,11 +204,12 @@ __device__ void d_role_widen(const DCtx& cx, uint32_t grp, uint32_t xtid, uint32
                 w.load(ring + static_cast<size_t>(s) * p.unit_bytes, xtid);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&c.wempty[s]);
-                if (!cx.warp_wait(&c.xempty[grp], ((it >> 1) & 1u) ^ 1u, kErrWaitEmpty)) return;
+                const uint32_t x = it % kDWide;                  // (always one of this group's)
+                if (!cx.warp_wait(&c.xempty[x], ((it / kDWide) & 1u) ^ 1u, kErrWaitEmpty)) return;
                 tc_fence_after();
-                w.store(ta, tsf);
+                w.store(tm + kDTmWide + x * 64u, tm + kDTmScaleW + x * 8u);
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&c.xfull[grp]);
+                if (lane == 0) mbar_arrive(&c.xfull[x]);
             }
             if (++s == nw) { s = 0; ph ^= 1u; }
         }
@@ -508,9 +510,9 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
         if (lane < kDStages) { mbar_init(&c.wfull[lane], 1); mbar_init(&c.wempty[lane], F::kA8 ? kBExpWarps / 2 : 1); }
         if (lane < 2) {
             mbar_init(&c.tmem_full[lane], 1); mbar_init(&c.tmem_empty[lane], 4);
-            mbar_init(&c.xfull[lane], kBExpWarps / 2); mbar_init(&c.xempty[lane], 1);
             mbar_init(&c.tile_full[lane], lane == 0 ? F::kBuilders : kDEpiWarps);
         }
+        if (lane < kDWide) { mbar_init(&c.xfull[lane], kBExpWarps / 2); mbar_init(&c.xempty[lane], 1); }
         mbar_fence_init();
         if (lane == 0) { c.abort_flag = 0u; c.comb_next = 0u; c.wissued = 0u; c.start_ok = 0u; }
     }
