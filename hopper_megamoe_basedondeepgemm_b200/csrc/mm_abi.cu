@@ -258,13 +258,15 @@ int mm_read_phase_stamps(const mm_config_t* cfg, const void* buffer, uint64_t ou
 // prologue disappear behind the end of the previous kernel (one token of hidden 3072, 8 experts, back to back: 26.9 us a pass
 // without, 25.5 with; 6 tokens of a small layer: 18.4 and 16.1).
 template <typename P>
-static int launch_early(void (*kern)(P), unsigned grid, unsigned threads, size_t smem_bytes, cudaStream_t stream, const P& params) {
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
+static int launch_early(void (*kern)(P), unsigned grid, unsigned threads, size_t smem_bytes, cudaStream_t stream, const P& params, unsigned cluster = 1) {
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem_bytes; cfg.stream = stream;
-    cfg.attrs = &attr; cfg.numAttrs = 1;
+    cfg.attrs = attr; cfg.numAttrs = cluster > 1 ? 2 : 1;
     MM_CUDA(cudaLaunchKernelEx(&cfg, kern, params));
     return MM_OK;
 }
@@ -396,9 +398,45 @@ static bool wants_tile_images(const mm::KParams& p) {
     return (p.knobs & mm::kKnobTileImages) != 0u && p.nstage_wide >= 3u && p.nrec >= 2u && static_cast<long long>(p.T) * p.topk > mm::kTileTokens;
 }
 
-// logits + quantisation, then the selection with as many experts per lane as the expert count needs
-static int launch_frontend(const mm::FeParams& q, int grid, cudaStream_t s) {
-    const int st = launch_early<mm::FeParams>(mm::frontend_logits_kernel, grid, mm::kFeThreads, 0, s, q);
+// The stand-alone frontend for a few tokens: one launch of clusters of 16 CTAs (`frontend_cluster_kernel`), all on the GPU at once. A cluster per token is the
+// faster way wherever the clusters fit (seven on a B200: us, two launches against one, 7 tokens: 48 experts of 3072 7.1 and 6.3, 384 of 3072 9.8 and
+// 7.7, 384 of 4096 11.3 and 10.2), two tokens to a cluster from 256 experts on, if a warp has all its experts in flight
+// (8 tokens of 3072: 384 experts 10.2 and 9.1, 256 9.0 and 8.7, 128 7.9 and 8.4; 384 of 4096 11.6 and 12.5). A call from
+// Python takes 1.5 us less of the host too. False: two launches (or the GPU holds no such cluster).
+static bool launch_frontend_cluster(mm::FeParams& q, int grid, cudaStream_t s, int* status) {
+    using Kernel = void (*)(mm::FeParams);
+    static const Kernel kernels[2][3] = {{mm::frontend_cluster_kernel<2, 6, 3>, mm::frontend_cluster_kernel<8, 6, 3>, mm::frontend_cluster_kernel<12, 6, 3>},
+                                         {mm::frontend_cluster_kernel<2, 8, 2>, mm::frontend_cluster_kernel<8, 8, 2>, mm::frontend_cluster_kernel<12, 8, 2>}};
+    static int resident[64][2][3] = {};                 // clusters the device holds at a time, + 1 (0: not asked yet)
+    int dev = 0;
+    if (q.E > 384 || q.H > 4096 || q.T > 32 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    const int wide = q.H > 3072 ? 1 : 0, per = q.E <= 64 ? 0 : (q.E <= 256 ? 1 : 2);
+    const Kernel kern = kernels[wide][per];
+    if (resident[dev][wide][per] == 0) {
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = mm::kFcCluster; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(mm::kFcCluster); cfg.blockDim = dim3(mm::kFcThreads); cfg.attrs = &attr; cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) { n = 0; (void)cudaGetLastError(); }
+        resident[dev][wide][per] = n + 1;
+    }
+    const int n = resident[dev][wide][per] - 1;
+    if (q.T > n && (q.T > 2 * n || q.E < 256 || q.E > mm::kFcCluster * 8 * (wide ? 2 : 3))) return false;
+    q.cluster_tokens = q.T > n ? 2 : 1;
+    const int ctas = mm::kFcCluster * ((q.T + q.cluster_tokens - 1) / q.cluster_tokens);
+    if (ctas > grid) return false;                      // (the caller's limit)
+    *status = launch_early<mm::FeParams>(kern, ctas, mm::kFcThreads, 0, s, q, mm::kFcCluster);
+    return true;
+}
+
+// Otherwise two launches: logits + quantisation, then the selection. Either with as many experts per lane of the selecting warp as the expert count needs.
+static int launch_frontend(mm::FeParams q, int grid, cudaStream_t s) {
+    int st = MM_OK;
+    if (launch_frontend_cluster(q, grid, s, &st)) return st;
+    st = launch_early<mm::FeParams>(mm::frontend_logits_kernel, grid, mm::kFeThreads, 0, s, q);
     if (st != MM_OK) return st;
     auto select = q.E <= 64 ? mm::frontend_select_kernel<2> : (q.E <= 256 ? mm::frontend_select_kernel<8> : (q.E <= 384 ? mm::frontend_select_kernel<12> : mm::frontend_select_kernel<32>));
     return launch_early<mm::FeParams>(select, q.T, 32, 0, s, q);
@@ -637,7 +675,7 @@ int32_t mm_fe_router_ctas(int32_t m, int32_t h, int32_t e, int32_t topk) {
     (void)m; (void)h; (void)e; (void)topk;
     int dev = 0, g = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&g, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -1;
-    return g;                              // the logits kernel runs one CTA per SM whatever the shape
+    return g;                              // one CTA per SM (a few tokens: fewer, in clusters), whatever the shape
 }
 
 int mm_fe_forward(const void* hidden, const void* router_weight, void* x, void* x_sf, void* topk_idx, void* topk_weights,

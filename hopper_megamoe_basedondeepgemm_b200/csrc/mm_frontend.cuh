@@ -20,6 +20,7 @@ struct FeParams {
     uint8_t* x; uint8_t* x_sf; long long* topk_idx; float* topk_w;
     int T, H, E, topk, score_mode, fmt, x_row_bytes, x_sf_row_bytes;
     float x_gs;
+    int cluster_tokens;                      // tokens of a cluster (`frontend_cluster_kernel` alone)
 };
 
 __device__ __forceinline__ void unpack_bf16x8(const uint4& v, float (&f)[8]) {
@@ -166,6 +167,8 @@ __device__ __forceinline__ uint32_t fe_expert_block(const FeParams& q, uint32_t 
     return per >= 16u * grid ? 4u : (per >= 8u * grid ? 2u : 1u);
 }
 
+// the logit from its two halves
+__device__ __forceinline__ float fe_logit(float first, float second) { return bf16_round(first + second) + 0.0f; }
 // logit of (token t, expert e) from its two halves; `flag` != 0: poll until both halves carry it (`ok` = false if `give_up`
 // says so first)
 template <typename GiveUp>
@@ -174,7 +177,7 @@ __device__ __forceinline__ float fe_read_logit(const FeParams& q, uint32_t t, ui
     uint32_t spins = 0;
     for (;;) {
         const uint4 v = ld_volatile_v4(src);
-        if (flag == 0u || (v.y == flag && v.w == flag)) return bf16_round(__uint_as_float(v.x) + __uint_as_float(v.z)) + 0.0f;
+        if (flag == 0u || (v.y == flag && v.w == flag)) return fe_logit(__uint_as_float(v.x), __uint_as_float(v.z));
         if ((++spins & 0x3Fu) == 0u && give_up()) { ok = false; return 0.f; }
     }
 }
@@ -182,6 +185,11 @@ __device__ __forceinline__ float fe_read_logit(const FeParams& q, uint32_t t, ui
 __device__ __forceinline__ uint32_t orderable_f32(float v) {
     const uint32_t b = __float_as_uint(v);
     return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+// orderable score of an expert, 0: not selectable
+__device__ __forceinline__ uint32_t fe_key(const FeParams& q, float v, float bias) {
+    const float s = (q.score_mode == 1 ? (1.0f / (1.0f + expf(-v))) + bias : v) + 0.0f;
+    return s != -INFINITY ? orderable_f32(s) : 0u;
 }
 __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v) {
     #pragma unroll
@@ -381,47 +389,10 @@ __device__ __forceinline__ bool fe_select_token(const FeParams& q, uint32_t t, f
     return true;
 }
 
-// One warp selects the top-8 of token t among at most 32 kPer experts, kPer per lane, in registers: the same keys, weights
-// and order of additions as `fe_select_token` (maximum of the scores, then the smallest expert with it, eight times); a lane
-// keeps its best score at hand, so that a round is two warp reductions and a rescan by one lane. The routing goes into
-// topk_idx / topk_weights and, with `records`, as flagged 16 B records {expert (~0: none), flag, weight, flag} to where the
-// launch's other SMs poll it; `e_out` / `w_out` get lane k's route k (`publish` false: only those). `flag` 0: the logits are complete. Returns false if `give_up` ended a poll.
-template <int kPer, typename GiveUp>
-__device__ __forceinline__ bool fe_select_token_regs(const FeParams& q, uint32_t t, bool nonzero, uint32_t lane, uint32_t flag, uint8_t* records, GiveUp give_up,
-                                                     bool publish = true, uint32_t* e_out = nullptr, float* w_out = nullptr) {
-    bool ok = true;
-    float lg[kPer];
-    uint32_t key[kPer];                                           // orderable score, 0: not selectable
-    constexpr int kFly = kPer < 8 ? kPer : 4;                     // records in flight
-    float bias[kPer];                                             // (fetched before the records are awaited: the load may come from HBM)
-    #pragma unroll
-    for (int h = 0; h < kPer; ++h) {
-        const uint32_t e = lane + 32u * h;
-        bias[h] = q.score_mode == 1 && e < static_cast<uint32_t>(q.E) ? __ldg(q.bias + e) : 0.f;
-    }
-    #pragma unroll
-    for (int h0 = 0; h0 < kPer; h0 += kFly) {
-        uint4 rec[kFly];
-        #pragma unroll
-        for (int h = 0; h < kFly; ++h) {
-            const uint32_t e = lane + 32u * (h0 + h);
-            if (e < static_cast<uint32_t>(q.E)) rec[h] = ld_volatile_v4(reinterpret_cast<const uint8_t*>(q.logits) + (static_cast<size_t>(t) * q.E + e) * 16u);
-        }
-        #pragma unroll
-        for (int h = 0; h < kFly; ++h) {
-            const uint32_t e = lane + 32u * (h0 + h);
-            lg[h0 + h] = 0.f; key[h0 + h] = 0u;
-            if (e < static_cast<uint32_t>(q.E)) {
-                float v;
-                if (flag == 0u || (rec[h].y == flag && rec[h].w == flag)) v = bf16_round(__uint_as_float(rec[h].x) + __uint_as_float(rec[h].z)) + 0.0f;
-                else v = fe_read_logit(q, t, e, flag, ok, give_up);
-                const float s = (q.score_mode == 1 ? (1.0f / (1.0f + expf(-v))) + bias[h0 + h] : v) + 0.0f;
-                lg[h0 + h] = v;
-                if (s != -INFINITY) key[h0 + h] = orderable_f32(s);
-            }
-        }
-    }
-    if (!__all_sync(0xffffffffu, ok)) return false;
+// The top-8 of one token from its logits and score keys, kPer experts per lane (lane, lane + 32, ...): see `fe_select_token_regs`.
+template <int kPer>
+__device__ __forceinline__ void fe_choose(const FeParams& q, uint32_t t, bool nonzero, uint32_t lane, uint32_t flag, uint8_t* records, const float (&lg)[kPer],
+                                          uint32_t (&key)[kPer], bool publish = true, uint32_t* e_out = nullptr, float* w_out = nullptr) {
     uint32_t top = 0u, top_h = 0u;                                // this lane's best score and the first of its experts that has it
     float top_v = 0.f;
     auto rescan = [&]() {
@@ -477,6 +448,49 @@ __device__ __forceinline__ bool fe_select_token_regs(const FeParams& q, uint32_t
             q.topk_w[static_cast<size_t>(t) * 8 + lane] = w;
         }
     }
+}
+
+// One warp selects the top-8 of token t among at most 32 kPer experts, kPer per lane, in registers: the same keys, weights
+// and order of additions as `fe_select_token` (maximum of the scores, then the smallest expert with it, eight times); a lane
+// keeps its best score at hand, so that a round is two warp reductions and a rescan by one lane. The routing goes into
+// topk_idx / topk_weights and, with `records`, as flagged 16 B records {expert (~0: none), flag, weight, flag} to where the
+// launch's other SMs poll it; `e_out` / `w_out` get lane k's route k (`publish` false: only those). `flag` 0: the logits are complete. Returns false if `give_up` ended a poll.
+template <int kPer, typename GiveUp>
+__device__ __forceinline__ bool fe_select_token_regs(const FeParams& q, uint32_t t, bool nonzero, uint32_t lane, uint32_t flag, uint8_t* records, GiveUp give_up,
+                                                     bool publish = true, uint32_t* e_out = nullptr, float* w_out = nullptr) {
+    bool ok = true;
+    float lg[kPer];
+    uint32_t key[kPer];                                           // orderable score, 0: not selectable
+    constexpr int kFly = kPer < 8 ? kPer : 4;                     // records in flight
+    float bias[kPer];                                             // (fetched before the records are awaited: the load may come from HBM)
+    #pragma unroll
+    for (int h = 0; h < kPer; ++h) {
+        const uint32_t e = lane + 32u * h;
+        bias[h] = q.score_mode == 1 && e < static_cast<uint32_t>(q.E) ? __ldg(q.bias + e) : 0.f;
+    }
+    #pragma unroll
+    for (int h0 = 0; h0 < kPer; h0 += kFly) {
+        uint4 rec[kFly];
+        #pragma unroll
+        for (int h = 0; h < kFly; ++h) {
+            const uint32_t e = lane + 32u * (h0 + h);
+            if (e < static_cast<uint32_t>(q.E)) rec[h] = ld_volatile_v4(reinterpret_cast<const uint8_t*>(q.logits) + (static_cast<size_t>(t) * q.E + e) * 16u);
+        }
+        #pragma unroll
+        for (int h = 0; h < kFly; ++h) {
+            const uint32_t e = lane + 32u * (h0 + h);
+            lg[h0 + h] = 0.f; key[h0 + h] = 0u;
+            if (e < static_cast<uint32_t>(q.E)) {
+                float v;
+                if (flag == 0u || (rec[h].y == flag && rec[h].w == flag)) v = fe_logit(__uint_as_float(rec[h].x), __uint_as_float(rec[h].z));
+                else v = fe_read_logit(q, t, e, flag, ok, give_up);
+                lg[h0 + h] = v;
+                key[h0 + h] = fe_key(q, v, bias[h0 + h]);
+            }
+        }
+    }
+    if (!__all_sync(0xffffffffu, ok)) return false;
+    fe_choose<kPer>(q, t, nonzero, lane, flag, records, lg, key, publish, e_out, w_out);
     return true;
 }
 
@@ -505,6 +519,108 @@ __global__ void __launch_bounds__(32) frontend_select_kernel(const __grid_consta
     grid_launch_dependents();
     const bool nonzero = fe_row_nonzero(q.hidden + static_cast<size_t>(t) * q.H, q.H, lane);
     fe_select_token_regs<kPer>(q, t, nonzero, lane, 0u, nullptr, [] { return false; });
+}
+
+// The same for a few tokens, in one launch. A cluster of CTAs takes one or two tokens through all three steps, so that the partial
+// logits meet in shared memory instead of in a second launch: CTA r works out the experts [r E / C, (r + 1) E / C) and sends each
+// sum to the CTA that selects for the token (token i of the cluster: CTA i), which also quantises it; behind one cluster
+// barrier those select. The sums are those of `fe_logits_blocks`, in the same order, and go to the workspace too, for whoever inspects it.
+// Bound: latency, of the weights' trip (147 KB to a CTA with 384 experts of 3072) and of the selection.
+constexpr int kFcThreads = 512;
+constexpr int kFcTokens = 2;                 // tokens of a cluster at most
+constexpr int kFcCluster = 16;               // CTAs of a cluster (of 8, 8 tokens over 384 experts: 9.4 us, of 16 9.1)
+
+// kPer: experts per lane of the selecting warp; kChunks: 16 B chunks of half a row per lane (hidden <= 512 kChunks); kExperts: experts of a warp in flight
+template <int kPer, int kChunks, int kExperts>
+__global__ void __launch_bounds__(kFcThreads, 1) frontend_cluster_kernel(const __grid_constant__ FeParams q) {
+    __shared__ uint4 xs[kFcTokens][kChunks * 64];
+    __shared__ float parts[kFeParts][kPer * 32];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, rank = cluster_rank(), C = cluster_size();
+    const uint32_t t0 = udiv_small(blockIdx.x, C) * q.cluster_tokens, nt = min(static_cast<uint32_t>(q.cluster_tokens), static_cast<uint32_t>(q.T) - t0);
+    cluster_arrive();                        // (nobody writes into a CTA that has not started)
+    grid_dependency_wait();
+    grid_launch_dependents();
+    const uint32_t nchunk = q.H / 8, half = (nchunk + kFeParts - 1) / kFeParts, part = warp & 1u;
+    const uint32_t c_lo = part * half + lane, c_hi = min(nchunk, part * half + half);
+    const uint32_t e_lo = udiv_small(rank * q.E, C) + (warp >> 1), e_hi = udiv_small((rank + 1u) * q.E, C);
+    constexpr uint32_t kStride = kFcThreads / 32 / kFeParts;
+    #pragma unroll 1
+    for (uint32_t e0 = e_lo;; e0 += kStride * kExperts) {
+        uint4 w[kExperts][kChunks];
+        #pragma unroll
+        for (uint32_t k = 0; k < kExperts; ++k) {
+            #pragma unroll
+            for (uint32_t b = 0; b < kChunks; ++b) {
+                const uint32_t e = e0 + k * kStride, ch = c_lo + 32u * b;
+                if (e < e_hi && ch < c_hi) w[k][b] = __ldg(reinterpret_cast<const uint4*>(q.router_w + static_cast<size_t>(e) * q.H) + ch);
+            }
+        }
+        if (e0 == e_lo) {                    // the tokens, behind the first weights' requests
+            const uint4* src = reinterpret_cast<const uint4*>(q.hidden + static_cast<size_t>(t0) * q.H);
+            for (uint32_t t = 0; t < nt; ++t)
+                for (uint32_t i = tid; i < nchunk; i += kFcThreads) xs[t][i] = __ldg(src + t * nchunk + i);
+            __syncthreads();
+            cluster_wait();
+        }
+        if (e0 >= e_hi) break;
+        #pragma unroll 1
+        for (uint32_t t = 0; t < nt; ++t) {
+            float acc[kExperts];
+            #pragma unroll
+            for (uint32_t k = 0; k < kExperts; ++k) acc[k] = 0.f;
+            #pragma unroll
+            for (uint32_t b = 0; b < kChunks; ++b) {
+                if (c_lo + 32u * b < c_hi) {
+                    float x[8];
+                    unpack_bf16x8(xs[t][c_lo + 32u * b], x);
+                    #pragma unroll
+                    for (uint32_t k = 0; k < kExperts; ++k) {
+                        float f[8];
+                        unpack_bf16x8(w[k][b], f);       // (an expert beyond the last one: whatever was there, its sum is not stored)
+                        #pragma unroll
+                        for (int i = 0; i < 8; ++i) acc[k] = fmaf(x[i], f[i], acc[k]);
+                    }
+                }
+            }
+            #pragma unroll
+            for (uint32_t k = 0; k < kExperts; ++k) {
+                #pragma unroll
+                for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+            }
+            #pragma unroll
+            for (uint32_t k = 0; k < kExperts; ++k) {
+                const uint32_t e = e0 + k * kStride;
+                if (lane == k && e < e_hi) {
+                    st_cluster_f32(&parts[part][e], t, acc[k]);
+                    st_volatile_v2(reinterpret_cast<uint8_t*>(q.logits) + (static_cast<size_t>(t0 + t) * q.E + e) * 16u + part * 8u, __float_as_uint(acc[k]), 1u);
+                }
+            }
+        }
+    }
+    __syncwarp();
+    cluster_arrive();
+    const uint32_t t = t0 + rank;
+    const __nv_bfloat16* row = reinterpret_cast<const __nv_bfloat16*>(xs[rank < nt ? rank : 0u]);
+    bool nz = false;
+    if (rank < nt && warp == 0u) nz = fe_row_nonzero(row, q.H, lane);
+    if (rank < nt && warp == 1u)
+        fe_quant_token(row, q.H, q.fmt, q.x_gs, q.x + static_cast<size_t>(t) * q.x_row_bytes, q.x_sf + static_cast<size_t>(t) * q.x_sf_row_bytes, lane);
+    __syncwarp();
+    cluster_wait();                          // (the last access to another CTA's shared memory lies before it)
+    if (rank < nt && warp == 0u) {
+        float lg[kPer];
+        uint32_t key[kPer];
+        #pragma unroll
+        for (uint32_t h = 0; h < kPer; ++h) {
+            const uint32_t e = lane + 32u * h;
+            lg[h] = 0.f; key[h] = 0u;
+            if (e < static_cast<uint32_t>(q.E)) {
+                lg[h] = fe_logit(parts[0][e], parts[1][e]);
+                key[h] = fe_key(q, lg[h], q.score_mode == 1 ? __ldg(q.bias + e) : 0.f);
+            }
+        }
+        fe_choose<kPer>(q, t, nz, lane, 0u, nullptr, lg, key);
+    }
 }
 
 }  // namespace mm

@@ -31,6 +31,17 @@ __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepco
 // this grid no longer holds back the start of the next one in its stream (which waits for this grid's end by itself)
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// ----------------------------------------------------------------------------- thread-block cluster
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ uint32_t cluster_size() { uint32_t n; asm volatile("mov.u32 %0, %cluster_nctarank;" : "=r"(n)); return n; }
+// the two halves of the barrier over all threads of the cluster (release, acquire)
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
+// to this CTA's shared-memory address in the CTA `rank` of the cluster
+__device__ __forceinline__ void st_cluster_f32(const float* p, uint32_t rank, float v) {
+    asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tst.shared::cluster.f32 [a], %2;\n\t}" ::"r"(smem_u32(p)), "r"(rank), "f"(v) : "memory");
+}
+
 // ----------------------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));

@@ -92,6 +92,41 @@ def test_frontend_matches_oracle(fmt, score_mode):
     assert torch.equal(got_sf, sfb)
 
 
+@pytest.mark.parametrize('mode', [2, 3, 4])
+@pytest.mark.parametrize('tokens,num_experts,hidden', [
+    (1, 8, 256), (2, 17, 768), (7, 64, 1024), (7, 65, 3072), (3, 48, 3328), (7, 384, 4096),      # a cluster of CTAs per token
+    (8, 256, 1280), (13, 384, 3072), (14, 256, 4096),                                            # two tokens to a cluster, the last cluster full and not
+    (8, 255, 512), (15, 384, 1024), (9, 384, 4096), (5, 385, 512),                               # the other side of the lines: two launches
+])
+def test_forward_of_a_few_tokens_is_bit_exact(mode, tokens, num_experts, hidden):
+    """Logits, routing and quantised tokens of the one-launch frontend and beyond its lines, with a row of zeros and tied experts."""
+    fmt = {2: 'fp8', 3: 'mxfp4', 4: 'nvfp4'}[mode]
+    g = torch.Generator().manual_seed(300 + tokens + num_experts)
+    x = torch.randn((tokens, hidden), generator=g).to(torch.bfloat16)
+    wr = (torch.randn((num_experts, hidden), generator=g) / hidden ** 0.5).to(torch.bfloat16)
+    wr[num_experts - 1] = wr[0]
+    wr[5] = wr[2]
+    if tokens > 1:
+        x[1] = 0
+    vec = 16 if fmt == 'nvfp4' else 32
+    q_out = torch.zeros((tokens, hidden if mode == 2 else hidden // 2), dtype=torch.float8_e4m3fn if mode == 2 else torch.int8, device='cuda')
+    sf_out = torch.zeros((tokens, hidden // (4 * vec)), dtype=torch.int32, device='cuda')
+    idx_out = torch.full((tokens, 8), -7, dtype=torch.int64, device='cuda')
+    w_out = torch.full((tokens, 8), -7.0, dtype=torch.float32, device='cuda')
+    ws = torch.full((mm.fe_workspace_bytes(num_experts),), 0x5A, dtype=torch.uint8, device='cuda')
+    for _ in range(2):
+        mm.fe_forward(x.cuda(), wr.cuda(), q_out, sf_out, idx_out, w_out, ws, mode)
+    parts = ws[256:256 + tokens * num_experts * 16].view(torch.float32).view(tokens, num_experts, 4).cpu()
+    logits = O.router_logits_device_order(x, wr)
+    assert torch.equal((parts[..., 0] + parts[..., 2]).to(torch.bfloat16).float() + 0.0, logits.float())
+    idx, w = O.route_from_logits(logits, x, 8)
+    assert torch.equal(idx_out.cpu(), idx)
+    assert torch.allclose(w_out.cpu(), w, rtol=2e-6, atol=1e-7)
+    q, sf, sfb = O.quantise_tokens(x, fmt, rounding='rne', sf_rule='mul', global_scale=1.0)
+    assert torch.equal(_canon(q_out.cpu(), fmt), _canon(q, fmt))
+    assert torch.equal(sf_out.cpu().view(torch.uint8).view(tokens, -1), sfb)
+
+
 def test_frontend_then_layer_matches_oracle():
     fmt, tokens, e_local, hidden, inter = 'mxfp4', 6, 48, 3072, 1280
     g = torch.Generator().manual_seed(11)
