@@ -14,23 +14,26 @@
 //              turns 16 tokens at a time through shared memory, so that all 128 threads of a group work whatever the row
 //              count and a thread holds eight gate and eight up values of one token. Two groups take the tasks in turn.
 //   order    : the L1 tasks dealt round-robin, but the last one to two rounds of them and all L2 tasks claimed one by one
-//              (no tile is split along K, a slow SM takes fewer). L2 goes tile by tile, its last four tasks per SM column
+//              (no tile is split along K, a slow SM takes fewer). L2 goes tile by tile, its last two tasks per SM column
 //              block by column block. The weight ring runs ahead over the L1 -> L2 hand-over, so that the stream does not
 //              stop there. (When this order came in: 59.2, 67.2 and 102 us with all L1 tasks dealt and L2 column by column, 57.2,
 //              64.9 and 100 with it, for 13 and 64 tokens over 48 experts and 96 skewed ones from hidden states.)
 //   combine  : per (token, 128-column block) behind a count per column block; routes added in slot order in fp32.
 //
-// Bound: HBM (the weights of the live experts once) up to about 40 rows per expert; beyond that the bytes an SM takes in
-// per unit (weights + token record, about 48 GB/s from the L2). 64 tokens, MXFP4, 48 experts (301 MB): 54.3 us a pass, of
-// which the stream is 46; the multi-rank kernel takes 88. With E4M3 tokens the units are widened into tensor memory,
-// which keeps up with the stream (100 tokens: 70.0 us, 765 with the multi-rank kernel).
+// Bound: HBM (the weights of the live experts once) up to about 40 rows per expert. 64 tokens, MXFP4, 48 experts (301 MB): 51.9 us a
+// pass, of which the stream is 42 at 7.1 TB/s; with weights from the L2 the same launch takes 40. The multi-rank kernel takes 88. Beyond, no single thing: 512
+// tokens 75.9 us, 67 with the weights from the L2, 70 without the epilogue's arithmetic, 71 with a quarter of the MMAs, 72 with short
+// records, and the power limit takes a tenth of the clock. With E4M3 tokens the units are widened into tensor memory
+// (100 tokens: 68 us, 765 with the multi-rank kernel), and the clock is 5 % lower.
 #pragma once
 #include "mm_kernel.cuh"
 
 namespace mm {
 
 constexpr int kBMaxRows = 4096;                    // routed rows of one launch
-constexpr uint32_t kBColumnTasks = 4;              // L2 tasks per SM that are claimed column block by column block
+constexpr uint32_t kBColumnTasks = 2;              // L2 tasks per SM that are claimed column block by column block (four: 200 tokens over 24 experts, NVFP4, 29.9 us instead of 28.7, 96 skewed 67.8, 67.3)
+constexpr uint32_t kBAhead = 4;                    // K units that are asked into the L2 ahead, twice at the start of a launch
+constexpr uint32_t kBAheadEntries = 2048;          // of at most so many routing entries (512 tokens of 8: 78.1 us without, 78.7 with; 256 76.9, 76.4)
 constexpr int kBTaskRing = 64;                     // claimed tasks of one SM that some role has still to see, at most
 constexpr int kBWStages = 12, kBRSlots = 12;       // at most: weight ring stages, token record slots
 constexpr int kBServiceWarps = 4;                  // weight loader, MMA issuer, record loader, spare
@@ -278,6 +281,19 @@ __device__ void b_role_weights(const BCtx& cx, uint32_t lane) {
         #pragma unroll 1
         for (uint32_t u = 0; u < units; u += step, ++it, src += stage_bytes) {
             uint64_t* full = kA8 ? &c.wfull[s] : &c.rfull[s];
+            if (!kA8 && it == nw && static_cast<uint32_t>(p.T) * p.topk <= kBAheadEntries) {
+                // the ring is full for the first time: the units behind it into the L2, while the MMAs wait for the first records
+                if (lane == 0) {
+                    const uint32_t here = kBAhead < units - u ? kBAhead : units - u, there = kBAhead - here;
+                    bulk_prefetch_l2(src, here * p.unit_bytes);
+                    if (there != 0u && ti + 1u < tasks.my1) {
+                        const uint32_t next_t = tasks.l1(blockIdx.x + (ti + 1u) * G);
+                        bulk_prefetch_l2(p.w1 + (static_cast<size_t>(c.tile_e[next_t >> 8]) * n1 + (next_t & 0xFFu)) * p.k1 * p.unit_bytes,
+                                         (there < static_cast<uint32_t>(p.k1) ? there : p.k1) * p.unit_bytes);
+                    }
+                }
+                __syncwarp();
+            }
             if (!cx.warp_wait(kA8 ? &c.wempty[s] : &c.rempty[s], ph ^ 1u, kErrWaitEmpty)) return;
             if (elect_one()) {
                 const uint32_t bytes = (units - u < step ? units - u : step) * p.unit_bytes;
@@ -1020,6 +1036,24 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
             #pragma unroll
             for (uint32_t a = 0; a < kAhead; ++a) load_row(v[a], vs[a], ww + a * kBWorkWarps);
         }
+    }
+    // The HBM has nothing to do until the rows are placed. Beside that, warp 3 asks the first units of the weight tile `bid` into the L2, if one of the first
+    // 128 entries names its expert: some SM's first task, this one's if no expert is empty. The loader adds as many when its ring is full. (us a pass
+    // without and with both: 4 tokens 33.0, 32.0; 13 48.1, 47.3; 64 52.8, 51.9; 100 over 32 experts of 4096 x 512 32.6, 31.7. Longer reaches hold up the
+    // small loads of the start: 12 units here, 64 tokens 52.3 -> 53.0. All entries looked through: 200 tokens, every slot masked, 9.3 -> 11.6. With E4M3
+    // tokens 100 tokens lose 1 % and 12 over 64 experts gain 3: not there. Nor where an
+    // SM has less than two tiles: its ring holds them. Every slot masked costs 0.15 us.)
+    if (!F::kA8 && nent <= kBAheadEntries && warp == 3 && static_cast<uint32_t>(p.E) * p.n1 >= 2u * G) {
+        const uint32_t e = udiv_small(bid, p.n1);
+        bool has = false;
+        #pragma unroll 1
+        for (uint32_t i = 0; i < nent && i < 128u; i += 32u) {
+            const uint32_t x = i + lane < nent ? c.ex[i + lane] : 0xFFu;
+            has = __any_sync(0xffffffffu, x == e);
+            if (has || !__any_sync(0xffffffffu, x < kMaxLocalExperts)) break;        // (found, or 32 masked ones)
+        }
+        if (has && lane == 0u)
+            bulk_prefetch_l2(p.w1 + static_cast<size_t>(bid) * p.k1 * p.unit_bytes, (p.k1 < static_cast<int>(kBAhead) ? p.k1 : kBAhead) * p.unit_bytes);
     }
     if (tid == 0) {
         ctrl32[kCtrlEpoch / 4 + bid] = epoch + 1u;
