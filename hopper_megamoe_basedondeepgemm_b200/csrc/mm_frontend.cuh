@@ -92,9 +92,8 @@ __device__ __forceinline__ void fe_logits_items(const FeParams& q, uint32_t warp
 }
 
 // The same partial logits (the same sums in the same order) with blocks of kEb experts x kTb tokens per warp and kAhead chunks
-// per lane in flight: per multiply-add a block of 4 x 4 reads 0.5 operand chunks instead of 1.25. The loads run at what an
-// SM takes in from the L2 (about 50 GB/s), so that is the time of a large batch; a small one needs every (expert, half) as
-// an item of its own to have enough of them. `fe_expert_block` draws the stand-alone frontend's line at four items per SM.
+// per lane in flight: per multiply-add a block of 4 x 4 reads 0.5 operand chunks instead of 1.25, which is the time of a large
+// batch; a small one needs every (expert, half) as an item of its own to have enough of them. `fe_expert_block` draws the stand-alone frontend's line at four items per SM.
 template <int kEb, int kAhead, int kTb = 4>
 __device__ __forceinline__ void fe_logits_blocks(const FeParams& q, uint32_t warp, uint32_t nwarps, uint32_t lane, uint32_t flag) {
     const uint32_t tblocks = (q.T + kTb - 1) / kTb, eblocks = (q.E + kEb - 1) / kEb, nchunk = q.H / 8, half = (nchunk + kFeParts - 1) / kFeParts;
