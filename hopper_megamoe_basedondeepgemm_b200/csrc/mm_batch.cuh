@@ -33,7 +33,7 @@ namespace mm {
 constexpr int kBMaxRows = 4096;                    // routed rows of one launch
 constexpr uint32_t kBColumnTasks = 2;              // L2 tasks per SM that are claimed column block by column block (four: 200 tokens over 24 experts, NVFP4, 29.9 us instead of 28.7, 96 skewed 67.8, 67.3)
 constexpr uint32_t kBAhead = 4;                    // K units that are asked into the L2 ahead, twice at the start of a launch
-constexpr uint32_t kBAheadEntries = 2048;          // of at most so many routing entries (512 tokens of 8: 78.1 us without, 78.7 with; 256 76.9, 76.4)
+constexpr int kBAheadEntries = 2048;               // of at most so many routing entries (512 tokens of 8: 78.1 us without, 78.7 with; 256 57.2, 56.9)
 constexpr int kBTaskRing = 64;                     // claimed tasks of one SM that some role has still to see, at most
 constexpr int kBWStages = 12, kBRSlots = 12;       // at most: weight ring stages, token record slots
 constexpr int kBServiceWarps = 4;                  // weight loader, MMA issuer, record loader, spare
@@ -233,7 +233,7 @@ struct BTasks {
 };
 
 // ============================================================================================= loaders
-template <bool kA8>
+template <bool kA8, bool kAsk>
 __device__ void b_role_weights(const BCtx& cx, uint32_t lane) {
     const BParams& p = cx.p; BShared& c = cx.c;
     const uint32_t nw = b_uniform(c.nw), step = kA8 ? 1u : b_uniform(c.spu), stage_bytes = step * p.unit_bytes, G = gridDim.x, n1 = p.n1, n2 = p.n2, M = b_uniform(c.M);
@@ -281,7 +281,7 @@ __device__ void b_role_weights(const BCtx& cx, uint32_t lane) {
         #pragma unroll 1
         for (uint32_t u = 0; u < units; u += step, ++it, src += stage_bytes) {
             uint64_t* full = kA8 ? &c.wfull[s] : &c.rfull[s];
-            if (!kA8 && it == nw && static_cast<uint32_t>(p.T) * p.topk <= kBAheadEntries) {
+            if (kAsk && it == nw) {
                 // the ring is full for the first time: the units behind it into the L2, while the MMAs wait for the first records
                 if (lane == 0) {
                     const uint32_t here = kBAhead < units - u ? kBAhead : units - u, there = kBAhead - here;
@@ -900,7 +900,7 @@ __device__ __forceinline__ void b_tiles(const BCtx& cx, uint32_t lane) {
 }
 
 // ============================================================================================= the kernel
-template <int kFmt, bool kFe>
+template <int kFmt, bool kFe, bool kAsk>
 __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(const __grid_constant__ BParams p) {
     using F = BFmt<kFmt>;
     extern __shared__ uint8_t smem_raw[];
@@ -1037,24 +1037,6 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
             for (uint32_t a = 0; a < kAhead; ++a) load_row(v[a], vs[a], ww + a * kBWorkWarps);
         }
     }
-    // The HBM has nothing to do until the rows are placed. Beside that, warp 3 asks the first units of the weight tile `bid` into the L2, if one of the first
-    // 128 entries names its expert: some SM's first task, this one's if no expert is empty. The loader adds as many when its ring is full. (us a pass
-    // without and with both: 4 tokens 33.0, 32.0; 13 48.1, 47.3; 64 52.8, 51.9; 100 over 32 experts of 4096 x 512 32.6, 31.7. Longer reaches hold up the
-    // small loads of the start: 12 units here, 64 tokens 52.3 -> 53.0. All entries looked through: 200 tokens, every slot masked, 9.3 -> 11.6. With E4M3
-    // tokens 100 tokens lose 1 % and 12 over 64 experts gain 3: not there. Nor where an
-    // SM has less than two tiles: its ring holds them. Every slot masked costs 0.15 us.)
-    if (!F::kA8 && nent <= kBAheadEntries && warp == 3 && static_cast<uint32_t>(p.E) * p.n1 >= 2u * G) {
-        const uint32_t e = udiv_small(bid, p.n1);
-        bool has = false;
-        #pragma unroll 1
-        for (uint32_t i = 0; i < nent && i < 128u; i += 32u) {
-            const uint32_t x = i + lane < nent ? c.ex[i + lane] : 0xFFu;
-            has = __any_sync(0xffffffffu, x == e);
-            if (has || !__any_sync(0xffffffffu, x < kMaxLocalExperts)) break;        // (found, or 32 masked ones)
-        }
-        if (has && lane == 0u)
-            bulk_prefetch_l2(p.w1 + static_cast<size_t>(bid) * p.k1 * p.unit_bytes, (p.k1 < static_cast<int>(kBAhead) ? p.k1 : kBAhead) * p.unit_bytes);
-    }
     if (tid == 0) {
         ctrl32[kCtrlEpoch / 4 + bid] = epoch + 1u;
         cx.sm_phase(kSmPrologue);
@@ -1088,6 +1070,18 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
         bar_arrive(kBBarTiles, F::kThreadsAll);
         if (lane == 0) { cx.sm_phase(kSmScheduled); if (bid == 0) cx.stamp(kStampScheduled); }
     } else {
+        // The HBM has nothing to do until the rows are placed. While the tiles are worked out, warp 3 asks the first units of the weight tile `bid` into
+        // the L2, if one of the first 128 entries names its expert: some SM's first task, this one's if no expert is empty. The loader adds as many when its
+        // ring is full. (us a pass without and with both: 4 tokens 32.7, 31.6; 13 46.9, 45.6; 64 51.5, 50.5; 40 over 64 experts of 2048 x 1024 39.6, 37.5; 96
+        // NVFP4 from hidden states, skewed, level. In front of the counting 64 take 50.6 and 200 tokens with every slot masked 9.3 instead of 9.2 (9.1
+        // without). Longer reaches hold up the small loads of the start: 12 units here, 64 tokens 52.3 -> 53.0. Nor is there anything to gain where an SM has
+        // less than two tiles: its ring holds them.)
+        if (kAsk && warp == 3 && static_cast<uint32_t>(p.E) * p.n1 >= 2u * G) {
+            const uint32_t e = udiv_small(bid, p.n1), left = 4u * lane < nent ? nent - 4u * lane : 0u;
+            const uint32_t hit = __vcmpeq4(*reinterpret_cast<const uint32_t*>(c.ex + 4u * lane), e * 0x01010101u) & (left < 4u ? (1u << (8u * left)) - 1u : ~0u);
+            if (__any_sync(0xffffffffu, hit != 0u) && lane == 0u)
+                bulk_prefetch_l2(p.w1 + static_cast<size_t>(bid) * p.k1 * p.unit_bytes, (p.k1 < static_cast<int>(kBAhead) ? p.k1 : kBAhead) * p.unit_bytes);
+        }
         bar_sync(kBBarTiles, F::kThreadsAll);
         if (tid == 96) cx.stamp_max(kStampLastScheduled);
     }
@@ -1195,7 +1189,7 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
 
     // ---- roles
     if (start) {
-        if (warp == 0) b_role_weights<F::kA8>(cx, lane);
+        if (warp == 0) b_role_weights<F::kA8, kAsk>(cx, lane);
         else if (warp == 1) b_role_mma<kFmt>(cx, lane);
         else if (warp == 2) b_role_records<kFmt>(cx);
         else if (warp >= kBServiceWarps && warp < kBServiceWarps + kBEpiWarps)

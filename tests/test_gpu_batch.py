@@ -47,6 +47,20 @@ def test_shapes_and_small_grids(hidden, inter, num_sms):
     check_against_oracle(y, stats, ref, buf, 'mxfp4', inter)
 
 
+@pytest.mark.parametrize('fmt', ['mxfp4', 'nvfp4'])
+@pytest.mark.parametrize('num_sms,e_local,hidden,inter,topk,tokens', [
+    (8, 2, 512, 512, 2, 9), (7, 2, 512, 512, 2, 9),           # 48 units of weights: six per SM, the ring's own, and more; first units of a tile per SM and the loader's
+    (5, 2, 1024, 256, 2, 9),                                  # less than two tiles per SM: the loader's alone
+    (2, 3, 512, 256, 3, 9), (1, 3, 4096, 256, 3, 9),          # tiles of two units, and of sixteen
+    (2, 24, 512, 256, 1, 40),                                 # experts without rows among those whose weights may be asked for
+    (20, 16, 512, 256, 16, 128), (20, 16, 512, 256, 16, 129),         # 2048 routing entries, and more
+])
+@pytest.mark.parametrize('masked', [0.0, 0.4])
+def test_weights_asked_ahead_on_both_sides_of_the_lines(fmt, num_sms, e_local, hidden, inter, topk, tokens, masked):
+    y, stats, ref, buf, _ = run_layer(fmt, e_local, hidden, inter, topk, tokens, 'random', 'umma', seed=tokens, std=0.02, num_sms=num_sms, masked_ratio=masked)
+    check_against_oracle(y, stats, ref, buf, fmt, inter)
+
+
 def _small_layer(fmt, e, hidden, inter, topk, tokens, seed, masked=0.0):
     w, _, _ = O.make_expert_weights(e, hidden, inter, fmt, seed=seed, std=0.05)
     l1, l2 = mm.transform_weights_for_mega_moe(*U.to_operator_weights(w, fmt, 'cuda'))
