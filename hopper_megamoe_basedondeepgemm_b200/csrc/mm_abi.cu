@@ -523,10 +523,10 @@ static int launch_one_rank(void (*kern)(mm::BParams), int threads, mm::BParams& 
 
 // The batch kernel asks weights into the L2 ahead of its stream (`kAsk`) in a build of its own: the code alone, jumped over, costs the other launches 0.1 to
 // 0.5 us (6 tokens of a small NVFP4 layer 14.9 us a pass with it, 14.7 without; 402 tokens 65.0, 64.6; 512 70.2, 69.8). It is for 4-bit tokens (E4M3: 100
-// tokens lose 1 %, 12 over 64 experts gain 3), up to 2048 routing entries, and layers that fill an SM's ring, of six units and more, before they
-// end (89 tokens over 8 experts of 1024 x 2048, 10 units per SM: 24.3 with it, 25.1 without).
+// tokens lose 1 %, 12 over 64 experts gain 3), up to 2048 routing entries, and layers of more than eight units per SM, which
+// fill its ring well before they end (10.4 units, 89 tokens over 8 experts of 1024 x 2048: 24.3 with it, 25.1 without; 7.8, 250 over 32 of 1536 x 256: 26.4, 26.0).
 static bool asks_ahead(const mm::BParams& p, int grid) {
-    return static_cast<long long>(p.T) * p.topk <= mm::kBAheadEntries && p.E * (p.n1 * p.k1 + p.n2 * p.k2) > 6 * grid;
+    return static_cast<long long>(p.T) * p.topk <= mm::kBAheadEntries && p.E * (p.n1 * p.k1 + p.n2 * p.k2) > 8 * grid;
 }
 
 template <int kFmt, bool kFe>

@@ -49,7 +49,7 @@ def test_shapes_and_small_grids(hidden, inter, num_sms):
 
 @pytest.mark.parametrize('fmt', ['mxfp4', 'nvfp4'])
 @pytest.mark.parametrize('num_sms,e_local,hidden,inter,topk,tokens', [
-    (8, 2, 512, 512, 2, 9), (7, 2, 512, 512, 2, 9),           # 48 units of weights: six per SM, the ring's own, and more; first units of a tile per SM and the loader's
+    (6, 2, 512, 512, 2, 9), (5, 2, 512, 512, 2, 9),           # 48 units of weights: eight per SM, and more; first units of a tile per SM and the loader's
     (5, 2, 1024, 256, 2, 9),                                  # less than two tiles per SM: the loader's alone
     (2, 3, 512, 256, 3, 9), (1, 3, 4096, 256, 3, 9),          # tiles of two units, and of sixteen
     (2, 24, 512, 256, 1, 40),                                 # experts without rows among those whose weights may be asked for
