@@ -31,7 +31,7 @@
 namespace mm {
 
 constexpr int kBMaxRows = 4096;                    // routed rows of one launch
-constexpr uint32_t kBColumnTasks = 2;              // L2 tasks per SM that are claimed column block by column block (four: 200 tokens over 24 experts, NVFP4, 29.9 us instead of 28.7, 96 skewed 67.8, 67.3)
+constexpr uint32_t kBColumnTasks = 2;              // L2 tasks per SM that are claimed column block by column block, at least (`column_tasks`)
 constexpr uint32_t kBAhead = 4;                    // K units that are asked into the L2 ahead, twice at the start of a launch
 constexpr int kBAheadEntries = 2048;               // of at most so many routing entries (512 tokens of 8: 78.1 us without, 78.7 with; 256 57.2, 56.9)
 constexpr int kBTaskRing = 64;                     // claimed tasks of one SM that some role has still to see, at most
@@ -67,6 +67,7 @@ struct BParams {
     uint32_t mid_row_bytes;
     FeParams fe;
     uint32_t smem_ring;                            // bytes of dynamic shared memory for the two rings
+    uint32_t column_tasks;                         // L2 tasks per SM that are claimed column block by column block (batch kernel), if there is time for them
     unsigned long long timeout_ns;
 };
 
@@ -246,9 +247,11 @@ __device__ void b_role_weights(const BCtx& cx, uint32_t lane) {
     // for it (13 tokens: 51.3 -> 50.0 us a pass, 64: 60.3 -> 58.6, 512: 80.3 -> 79.8, 6 of the small layer: 15.4 -> 15.0).
     bar_sync(kBBarPlaced, 32u * (kBWorkWarps + 1));
     // Order of the L2 tasks: tile by tile (the first tiles' L1 outputs are complete long before the last ones'), but the last
-    // tiles, kBColumnTasks tasks per SM of them, column block by column block: the combine starts on a column block when all
-    // tiles have it, beside the remaining ones.
-    const uint32_t NT1 = M * n1, NT2 = M * n2, tail = udiv_small(kBColumnTasks * G + n2 - 1u, n2), mA = tail < M ? M - tail : 0u, NA = mA * n2;
+    // tiles, two or four tasks per SM of them, column block by column block: the combine starts on a column block when all
+    // tiles have it, beside the remaining ones. Four where the launch asks for them (`column_tasks`) and the tiles in front keep an SM busy for
+    // ten units: the last tiles have just had their L1 tasks, and the first column block wants all of them (300 E4M3 tokens over 32 experts of
+    // 4096 x 512, six units: 57.2 us a pass with four, 53.9 with two).
+    const uint32_t NT1 = M * n1, NT2 = M * n2, tail = udiv_small((NT2 * p.k2 >= (4u * p.k2 + 10u) * G ? p.column_tasks : kBColumnTasks) * G + n2 - 1u, n2), mA = tail < M ? M - tail : 0u, NA = mA * n2;
     uint32_t* claims = cx.counter(cx.par, kBCountClaims);
     uint32_t next = 0u;
     if (tasks.my1 == 0u && lane == 0) next = atomicAdd(claims, 1u);

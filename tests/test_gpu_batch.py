@@ -61,6 +61,17 @@ def test_weights_asked_ahead_on_both_sides_of_the_lines(fmt, num_sms, e_local, h
     check_against_oracle(y, stats, ref, buf, fmt, inter)
 
 
+@pytest.mark.parametrize('fmt', ['mxfp4', 'nvfp4', 'fp8'])
+@pytest.mark.parametrize('num_sms,e_local,inter,topk,tokens', [
+    (1, 8, 256, 4, 10), (1, 8, 256, 4, 11),        # 40 and 44 rows of 512 columns on one SM: 40 KB, and more
+    (4, 14, 256, 2, 100), (4, 13, 256, 2, 100),    # 14 tasks of one unit per SM, the least that leaves ten in front of four, and 13
+    (3, 4, 512, 3, 90), (1, 2, 256, 2, 40),        # two units to a task; fewer tiles than would go column block by column block
+])
+def test_column_tasks_on_both_sides_of_the_lines(fmt, num_sms, e_local, inter, topk, tokens):
+    y, stats, ref, buf, _ = run_layer(fmt, e_local, 512, inter, topk, tokens, 'random', 'umma', seed=tokens, std=0.02, num_sms=num_sms)
+    check_against_oracle(y, stats, ref, buf, fmt, inter)
+
+
 def _small_layer(fmt, e, hidden, inter, topk, tokens, seed, masked=0.0):
     w, _, _ = O.make_expert_weights(e, hidden, inter, fmt, seed=seed, std=0.05)
     l1, l2 = mm.transform_weights_for_mega_moe(*U.to_operator_weights(w, fmt, 'cuda'))
