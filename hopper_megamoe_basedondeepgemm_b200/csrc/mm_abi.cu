@@ -399,10 +399,12 @@ static bool wants_tile_images(const mm::KParams& p) {
 }
 
 // The stand-alone frontend for a few tokens: one launch of clusters of 16 CTAs (`frontend_cluster_kernel`), all on the GPU at once. A cluster per token is the
-// faster way wherever the clusters fit (seven on a B200: us, two launches against one, 7 tokens: 48 experts of 3072 7.1 and 6.3, 384 of 3072 9.8 and
-// 7.7, 384 of 4096 11.3 and 10.2), two tokens to a cluster from 256 experts on, if a warp has all its experts in flight
-// (8 tokens of 3072: 384 experts 10.2 and 9.1, 256 9.0 and 8.7, 128 7.9 and 8.4; 384 of 4096 11.6 and 12.5). A call from
-// Python takes 1.5 us less of the host too. False: two launches (or the GPU holds no such cluster).
+// faster way wherever the clusters fit (seven on a B200: us in a graph, two launches against one, 7 tokens: 48 experts of 3072 7.1 and 4.7, NVFP4 9.1
+// and 4.8, 384 of 3072 10.0 and 7.7, of 4096 11.1 and 9.0; only one or two tokens of hidden 512 over 128 to 256 experts lose, 0.1 to 0.3).
+// Two tokens to a cluster are where two launches take longer than a cluster's second token: from hidden 2048 on (8 tokens: 48 experts 5.9 and
+// 5.3, 128 6.8 and 6.8, 256 7.5 and 7.3; of 1536 6.5 and 6.8 with 128) and beyond 256 experts (of 512 7.6 and 7.1; 256 6.0 and 6.3), and with two more tokens
+// than clusters also from hidden 1536 on (9 tokens: 128 experts 0.4 less) and beyond 192 experts (224 of 512 0.7 less; 192 of 512 level, 128 of 1024
+// 0.1 more). A call from Python takes 1.5 us less of the host too. False: two launches (or the GPU holds no such cluster).
 static bool launch_frontend_cluster(mm::FeParams& q, int grid, cudaStream_t s, int* status) {
     using Kernel = void (*)(mm::FeParams);
     static const Kernel kernels[2][3] = {{mm::frontend_cluster_kernel<2, 6, 3>, mm::frontend_cluster_kernel<8, 6, 3>, mm::frontend_cluster_kernel<12, 6, 3>},
@@ -424,7 +426,7 @@ static bool launch_frontend_cluster(mm::FeParams& q, int grid, cudaStream_t s, i
         resident[dev][wide][per] = n + 1;
     }
     const int n = resident[dev][wide][per] - 1;
-    if (q.T > n && (q.T > 2 * n || q.E < 256 || q.E > mm::kFcCluster * 8 * (wide ? 2 : 3))) return false;
+    if (q.T > n && (q.T > 2 * n || !(q.H >= 2048 || q.E > 256 || (q.T > n + 1 && (q.H >= 1536 || q.E > 192))))) return false;
     q.cluster_tokens = q.T > n ? 2 : 1;
     const int ctas = mm::kFcCluster * ((q.T + q.cluster_tokens - 1) / q.cluster_tokens);
     if (ctas > grid) return false;                      // (the caller's limit)

@@ -95,8 +95,9 @@ def test_frontend_matches_oracle(fmt, score_mode):
 @pytest.mark.parametrize('mode', [2, 3, 4])
 @pytest.mark.parametrize('tokens,num_experts,hidden', [
     (1, 8, 256), (2, 17, 768), (7, 64, 1024), (7, 65, 3072), (3, 48, 3328), (7, 384, 4096),      # a cluster of CTAs per token
-    (8, 256, 1280), (13, 384, 3072), (14, 256, 4096),                                            # two tokens to a cluster, the last cluster full and not
-    (8, 255, 512), (15, 384, 1024), (9, 384, 4096), (5, 385, 512),                               # the other side of the lines: two launches
+    (9, 256, 1280), (13, 384, 3072), (14, 256, 4096), (9, 384, 4096),                            # two tokens to a cluster, the last cluster full and not
+    (8, 16, 2048), (8, 257, 512), (9, 48, 1536), (9, 193, 512),                                  # ... at the lines
+    (8, 256, 1280), (8, 255, 512), (15, 384, 1024), (5, 385, 512), (8, 48, 1792), (9, 192, 1280),         # the other side of them: two launches
 ])
 def test_forward_of_a_few_tokens_is_bit_exact(mode, tokens, num_experts, hidden):
     """Logits, routing and quantised tokens of the one-launch frontend and beyond its lines, with a row of zeros and tied experts."""
