@@ -258,7 +258,7 @@ int mm_read_phase_stamps(const mm_config_t* cfg, const void* buffer, uint64_t ou
 // prologue disappear behind the end of the previous kernel (one token of hidden 3072, 8 experts, back to back: 26.9 us a pass
 // without, 25.5 with; 6 tokens of a small layer: 18.4 and 16.1).
 template <typename P>
-static int launch_early(void (*kern)(P), unsigned grid, unsigned threads, size_t smem_bytes, cudaStream_t stream, const P& params, unsigned cluster = 1) {
+static cudaError_t launch_early_error(void (*kern)(P), unsigned grid, unsigned threads, size_t smem_bytes, cudaStream_t stream, const P& params, unsigned cluster = 1) {
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -267,7 +267,11 @@ static int launch_early(void (*kern)(P), unsigned grid, unsigned threads, size_t
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem_bytes; cfg.stream = stream;
     cfg.attrs = attr; cfg.numAttrs = cluster > 1 ? 2 : 1;
-    MM_CUDA(cudaLaunchKernelEx(&cfg, kern, params));
+    return cudaLaunchKernelEx(&cfg, kern, params);
+}
+template <typename P>
+static int launch_early(void (*kern)(P), unsigned grid, unsigned threads, size_t smem_bytes, cudaStream_t stream, const P& params) {
+    MM_CUDA(launch_early_error(kern, grid, threads, smem_bytes, stream, params));
     return MM_OK;
 }
 
@@ -398,50 +402,55 @@ static bool wants_tile_images(const mm::KParams& p) {
     return (p.knobs & mm::kKnobTileImages) != 0u && p.nstage_wide >= 3u && p.nrec >= 2u && static_cast<long long>(p.T) * p.topk > mm::kTileTokens;
 }
 
-// The stand-alone frontend for a few tokens: one launch of clusters of 16 CTAs (`frontend_cluster_kernel`), all on the GPU at once. A cluster per token is the
-// faster way wherever the clusters fit (seven on a B200: us in a graph, two launches against one, 7 tokens: 48 experts of 3072 7.1 and 4.7, NVFP4 9.1
-// and 4.8, 384 of 3072 10.0 and 7.7, of 4096 11.1 and 9.0; only one or two tokens of hidden 512 over 128 to 256 experts lose, 0.1 to 0.3).
-// Two tokens to a cluster are where two launches take longer than a cluster's second token: from hidden 2048 on (8 tokens: 48 experts 5.9 and
-// 5.3, 128 6.8 and 6.8, 256 7.5 and 7.3; of 1536 6.5 and 6.8 with 128) and beyond 256 experts (of 512 7.6 and 7.1; 256 6.0 and 6.3), and with two more tokens
-// than clusters also from hidden 1536 on (9 tokens: 128 experts 0.4 less) and beyond 192 experts (224 of 512 0.7 less; 192 of 512 level, 128 of 1024
-// 0.1 more). A call from Python takes 1.5 us less of the host too. False: two launches (or the GPU holds no such cluster).
-static bool launch_frontend_cluster(mm::FeParams& q, int grid, cudaStream_t s, int* status) {
+// The stand-alone frontend: one launch of clusters of 16 CTAs (`frontend_cluster_kernel`), all on the GPU at once, or logits + quantisation and
+// then the selection. Either with as many experts per lane of the selecting warp as the expert count needs.
+namespace {
+struct FrontendLaunch {
     using Kernel = void (*)(mm::FeParams);
-    static const Kernel kernels[2][3] = {{mm::frontend_cluster_kernel<2, 6, 3>, mm::frontend_cluster_kernel<8, 6, 3>, mm::frontend_cluster_kernel<12, 6, 3>},
-                                         {mm::frontend_cluster_kernel<2, 8, 2>, mm::frontend_cluster_kernel<8, 8, 2>, mm::frontend_cluster_kernel<12, 8, 2>}};
-    static int resident[64][2][3] = {};                 // clusters the device holds at a time, + 1 (0: not asked yet)
-    int dev = 0;
-    if (q.E > 384 || q.H > 4096 || q.T > 32 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
-    const int wide = q.H > 3072 ? 1 : 0, per = q.E <= 64 ? 0 : (q.E <= 256 ? 1 : 2);
-    const Kernel kern = kernels[wide][per];
-    if (resident[dev][wide][per] == 0) {
-        cudaLaunchAttribute attr;
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = mm::kFcCluster; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(mm::kFcCluster); cfg.blockDim = dim3(mm::kFcThreads); cfg.attrs = &attr; cfg.numAttrs = 1;
-        int n = 0;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) { n = 0; (void)cudaGetLastError(); }
-        resident[dev][wide][per] = n + 1;
+    mm::FeParams q;
+    int grid;
+    cudaStream_t stream;
+    int variant() const { return (q.H > 3072 ? 3 : 0) + (q.E <= 64 ? 0 : (q.E <= 256 ? 1 : 2)); }
+    Kernel cluster_kernel() const {
+        static const Kernel kernels[6] = {mm::frontend_cluster_kernel<2, 6, 3>, mm::frontend_cluster_kernel<8, 6, 3>, mm::frontend_cluster_kernel<12, 6, 3>,
+                                          mm::frontend_cluster_kernel<2, 8, 2>, mm::frontend_cluster_kernel<8, 8, 2>, mm::frontend_cluster_kernel<12, 8, 2>};
+        return kernels[variant()];
     }
-    const int n = resident[dev][wide][per] - 1;
-    if (q.T > n && (q.T > 2 * n || !(q.H >= 2048 || q.E > 256 || (q.T > n + 1 && (q.H >= 1536 || q.E > 192))))) return false;
-    q.cluster_tokens = q.T > n ? 2 : 1;
-    const int ctas = mm::kFcCluster * ((q.T + q.cluster_tokens - 1) / q.cluster_tokens);
-    if (ctas > grid) return false;                      // (the caller's limit)
-    *status = launch_early<mm::FeParams>(kern, ctas, mm::kFcThreads, 0, s, q, mm::kFcCluster);
-    return true;
-}
+    bool error_pending() const { return cudaPeekAtLastError() != cudaSuccess; }
+    void clear_error() const { (void)cudaGetLastError(); }
+    bool clusters(int* n) const {
+        static mm::KnownClusters known[64][6];
+        int dev = 0;
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaStreamIsCapturing(stream, &capture) != cudaSuccess) return false;
+        const bool in_table = dev >= 0 && dev < 64;
+        return known[in_table ? dev : 0][variant()].get(in_table && capture == cudaStreamCaptureStatusNone, n, [&](int* out) {
+            cudaLaunchAttribute attr;
+            attr.id = cudaLaunchAttributeClusterDimension;
+            attr.val.clusterDim.x = mm::kFcCluster; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(mm::kFcCluster); cfg.blockDim = dim3(mm::kFcThreads); cfg.stream = stream; cfg.attrs = &attr; cfg.numAttrs = 1;
+            return cudaFuncSetAttribute(cluster_kernel(), cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                   cudaOccupancyMaxActiveClusters(out, cluster_kernel(), &cfg) == cudaSuccess;
+        });
+    }
+    bool one_launch(int tokens_per_cluster) {
+        q.cluster_tokens = tokens_per_cluster;
+        const int ctas = mm::kFcCluster * ((q.T + tokens_per_cluster - 1) / tokens_per_cluster);
+        return launch_early_error<mm::FeParams>(cluster_kernel(), ctas, mm::kFcThreads, 0, stream, q, mm::kFcCluster) == cudaSuccess;
+    }
+    int two_launches() const {
+        const int st = launch_early<mm::FeParams>(mm::frontend_logits_kernel, grid, mm::kFeThreads, 0, stream, q);
+        if (st != MM_OK) return st;
+        const Kernel select = q.E <= 64 ? mm::frontend_select_kernel<2> : (q.E <= 256 ? mm::frontend_select_kernel<8> : (q.E <= 384 ? mm::frontend_select_kernel<12> : mm::frontend_select_kernel<32>));
+        return launch_early<mm::FeParams>(select, q.T, 32, 0, stream, q);
+    }
+};
+}  // namespace
 
-// Otherwise two launches: logits + quantisation, then the selection. Either with as many experts per lane of the selecting warp as the expert count needs.
-static int launch_frontend(mm::FeParams q, int grid, cudaStream_t s) {
-    int st = MM_OK;
-    if (launch_frontend_cluster(q, grid, s, &st)) return st;
-    st = launch_early<mm::FeParams>(mm::frontend_logits_kernel, grid, mm::kFeThreads, 0, s, q);
-    if (st != MM_OK) return st;
-    auto select = q.E <= 64 ? mm::frontend_select_kernel<2> : (q.E <= 256 ? mm::frontend_select_kernel<8> : (q.E <= 384 ? mm::frontend_select_kernel<12> : mm::frontend_select_kernel<32>));
-    return launch_early<mm::FeParams>(select, q.T, 32, 0, s, q);
+static int launch_frontend(const mm::FeParams& q, int grid, cudaStream_t s) {
+    FrontendLaunch launch{q, grid, s};
+    return mm::launch_frontend_by_size(launch, q.T, q.H, q.E, grid);
 }
 
 template <int kVec, bool kUmma, bool kFe = false, bool kA8 = false, bool kTiles = false>

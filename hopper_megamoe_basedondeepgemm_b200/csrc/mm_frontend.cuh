@@ -11,6 +11,7 @@
 #include <cuda_bf16.h>
 #include <cstdint>
 #include "mm_ptx.cuh"
+#include "mm_frontend_route.h"
 
 namespace mm {
 
@@ -527,7 +528,6 @@ __global__ void __launch_bounds__(32) frontend_select_kernel(const __grid_consta
 // Bound: latency, of the weights' trip (147 KB to a CTA with 384 experts of 3072) and of the selection. 1 token over 48 experts of 3072 4.2 us, 8 over 384 9.1.
 constexpr int kFcThreads = 512;
 constexpr int kFcTokens = 2;                 // tokens of a cluster at most
-constexpr int kFcCluster = 16;               // CTAs of a cluster (of 8, 8 tokens over 384 experts: 9.4 us, of 16 9.1)
 
 // kPer: experts per lane of the selecting warp; kChunks: 16 B chunks of half a row per lane (hidden <= 512 kChunks); kExperts: experts of a warp in flight
 template <int kPer, int kChunks, int kExperts>

@@ -128,6 +128,106 @@ def test_forward_of_a_few_tokens_is_bit_exact(mode, tokens, num_experts, hidden)
     assert torch.equal(sf_out.cpu().view(torch.uint8).view(tokens, -1), sfb)
 
 
+def _kernels_of(graph):
+    """(name, CTAs) of a captured graph's kernel launches."""
+    d = pytest.importorskip('cuda.bindings.driver')
+    g = d.CUgraph(graph.raw_cuda_graph())
+    _, _, n = d.cuGraphGetNodes(g)
+    _, nodes, n = d.cuGraphGetNodes(g, n)
+    out = []
+    for node in nodes[:n]:
+        if d.cuGraphNodeGetType(node)[1] != d.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            continue
+        err, p = d.cuGraphKernelNodeGetParams(node)
+        assert err == d.CUresult.CUDA_SUCCESS
+        err, name = d.cuFuncGetName(p.func) if int(p.func) != 0 else d.cuKernelGetName(p.kern)
+        assert err == d.CUresult.CUDA_SUCCESS
+        out.append((name.decode(), int(p.gridDimX)))
+    return out
+
+
+@pytest.mark.parametrize('fmt', ['mxfp4', 'nvfp4', 'fp8'])
+@pytest.mark.parametrize('tokens,num_experts,hidden,num_sms,per', [
+    (3, 64, 1024, 0, 1), (7, 128, 1536, 0, 1), (5, 256, 3584, 0, 1), (2, 384, 4096, 0, 1),      # a cluster per token: 64, 256, 384 experts, both widths
+    (9, 48, 2048, 0, 2), (8, 256, 2048, 0, 2), (13, 384, 3072, 0, 2),                           # two tokens to a cluster
+    (3, 64, 1024, 48, 1), (3, 64, 1024, 47, 0), (9, 48, 2048, 80, 2), (9, 48, 2048, 79, 0), (1, 48, 512, 15, 0),       # the buffer's CTAs, too few for the clusters
+])
+def test_bias_scales_and_the_buffers_ctas_in_one_launch_and_in_two(fmt, tokens, num_experts, hidden, num_sms, per):
+    """Sigmoid scores with an expert bias and a global scale through the C entry, and which way the call takes. The routing views start from
+    other values than the frontend writes."""
+    import ctypes
+    from hopper_megamoe_basedondeepgemm_b200 import _lib
+    lib = _lib.load()
+    g = torch.Generator().manual_seed(500 + tokens + num_experts)
+    x = torch.randn((tokens, hidden), generator=g).to(torch.bfloat16)
+    if tokens > 1:
+        x[1] = 0
+    wr = (torch.randn((num_experts, hidden), generator=g) / hidden ** 0.5).to(torch.bfloat16)
+    bias = 0.3 * torch.rand(num_experts, generator=g)
+    x_gs = 1.0 / 64.0 if fmt == 'nvfp4' else 1.0
+    cfg = _lib.MMConfig(8, 0, num_experts, 16, 8, hidden, 1280, _lib.FMT[fmt], num_sms)
+    L = _lib.MMLayout()
+    assert lib.mm_get_layout(ctypes.byref(cfg), ctypes.byref(L)) == 0
+    buf = torch.full((int(L.total_bytes),), 0x55, dtype=torch.uint8, device='cuda')
+    ws = torch.full((int(lib.mm_frontend_workspace_bytes(ctypes.byref(cfg))),), 0x5A, dtype=torch.uint8, device='cuda')
+    xd, wd, bd = x.cuda(), wr.cuda(), bias.cuda()
+    args = _lib.MMFrontendArgs(xd.data_ptr(), wd.data_ptr(), bd.data_ptr(), tokens, 1, ws.data_ptr(), x_gs)
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        assert lib.mm_frontend_launch(ctypes.byref(cfg), buf.data_ptr(), ctypes.byref(args), torch.cuda.current_stream().cuda_stream) == 0
+    ran = _kernels_of(graph)
+    if per:
+        assert len(ran) == 1 and 'frontend_cluster_kernel' in ran[0][0] and ran[0][1] == 16 * -(-tokens // per)
+    else:
+        assert len(ran) == 2 and not any('cluster' in name for name, _ in ran)
+    graph.instantiate()
+    graph.replay()
+    torch.cuda.synchronize()
+    idx, w = O.route_from_logits(O.router_logits_device_order(x, wr), x, 8, 'sigmoid_bias', bias)
+    view = lambda off, n, t: buf[off:off + n].view(t).cpu()          # noqa: E731
+    assert torch.equal(view(L.off_topk_idx, tokens * 64, torch.int64).view(tokens, 8), idx)
+    assert torch.allclose(view(L.off_topk_weights, tokens * 32, torch.float32).view(tokens, 8), w, rtol=2e-6, atol=1e-7)
+    q, sf, sfb = O.quantise_tokens(x, fmt, rounding='rne', sf_rule='mul', global_scale=x_gs)
+    got = view(L.off_x, tokens * int(L.x_row_bytes), torch.uint8).view(tokens, -1)
+    assert torch.equal(_canon(got, fmt), _canon(q, fmt))
+    assert torch.equal(view(L.off_x_sf, tokens * int(L.x_sf_row_bytes), torch.uint8).view(tokens, -1), sfb)
+
+
+_FIRST_CALL = r"""
+import torch
+import hopper_megamoe_basedondeepgemm_b200 as mm
+g = torch.Generator().manual_seed(7)
+tokens, experts, hidden = 5, 48, 1024
+x = torch.randn((tokens, hidden), generator=g).to(torch.bfloat16).cuda()
+wr = (torch.randn((experts, hidden), generator=g) / 32).to(torch.bfloat16).cuda()
+new = lambda: (torch.full((tokens, hidden // 2), 0x55, dtype=torch.int8, device='cuda'), torch.full((tokens, hidden // 128), 0x55, dtype=torch.int32, device='cuda'),
+               torch.full((tokens, 8), -7, dtype=torch.int64, device='cuda'), torch.full((tokens, 8), -7.0, device='cuda'))
+ws = torch.zeros(mm.fe_workspace_bytes(experts), dtype=torch.uint8, device='cuda')
+a, b = new(), new()
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    mm.fe_forward(x, wr, *a, ws, 3)
+graph.replay()
+torch.cuda.synchronize()
+assert int(a[2].min()) >= 0
+mm.fe_forward(x, wr, *b, ws, 3)
+torch.cuda.synchronize()
+assert all(torch.equal(p, q) for p, q in zip(a, b))
+print('captured first')
+"""
+
+
+def test_first_call_of_a_process_may_be_captured():
+    """The frontend asks the device about clusters in its first call; under capture that has to work as later."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, '-c', _FIRST_CALL], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and 'captured first' in r.stdout, r.stderr[-2000:]
+
+
 def test_frontend_then_layer_matches_oracle():
     fmt, tokens, e_local, hidden, inter = 'mxfp4', 6, 48, 3072, 1280
     g = torch.Generator().manual_seed(11)

@@ -463,3 +463,112 @@ def test_the_static_scratch_has_room_for_the_counters_beside_24_mib():
             near += L.total_bytes > 24 * 1024 * 1024
             assert L.total_bytes <= _lib.STATIC_SCRATCH_BYTES, (fmt, e, h, i, k, t, L.total_bytes)
     assert near >= 2
+
+
+_ROUTE_PROGRAM = r"""
+#include <cstdio>
+#include <cstdlib>
+#include <thread>
+#include <vector>
+#include "mm_frontend_route.h"
+static int known_clusters() {                    // failures are asked again, answers kept unless not to be, by threads in any order
+    mm::KnownClusters k;
+    int n = -1, asked = 0;
+    auto fails = [&](int*) { ++asked; return false; };
+    auto seven = [&](int* out) { ++asked; *out = 7; return true; };
+    if (k.get(true, &n, fails) || k.get(true, &n, fails) || asked != 2) return 1;
+    if (!k.get(false, &n, seven) || n != 7 || asked != 3) return 2;
+    if (k.get(true, &n, fails) || asked != 4) return 3;
+    if (!k.get(true, &n, seven) || !k.get(true, &n, fails) || n != 7 || asked != 5) return 4;
+    if (k.get(false, &n, fails) || asked != 6) return 5;
+    mm::KnownClusters none;
+    auto zero = [&](int* out) { *out = 0; return true; };
+    if (!none.get(true, &n, zero) || !none.get(true, &n, seven) || n != 0 || asked != 6) return 6;
+    mm::KnownClusters shared;
+    static int attribute;                        // set before the answer is kept: who finds it kept sees it set
+    std::atomic<int> bad{0};
+    std::vector<std::thread> threads;
+    for (int t = 0; t < 8; ++t)
+        threads.emplace_back([&] {
+            for (int i = 0; i < 1000; ++i) {
+                int m = 0;
+                if (!shared.get(true, &m, [&](int* out) { __atomic_store_n(&attribute, 1, __ATOMIC_RELAXED); *out = 7; return true; }) || m != 7) ++bad;
+                if (__atomic_load_n(&attribute, __ATOMIC_RELAXED) != 1) ++bad;
+            }
+        });
+    for (auto& t : threads) t.join();
+    return bad.load() == 0 ? 0 : 7;
+}
+struct Fake {                                    // a GPU whose answers are made up; `log`: what was done
+    int clusters_; bool query_ok, launch_ok, error = false; char log[64] = {}; int n = 0;
+    void put(char c) { log[n++] = c; }
+    bool error_pending() { return error; }
+    void clear_error() { error = false; put('c'); }
+    bool clusters(int* out) { put('q'); if (!query_ok) { error = true; return false; } *out = clusters_; return true; }
+    bool one_launch(int per) { put(static_cast<char>('0' + per)); if (!launch_ok) error = true; return launch_ok; }
+    int two_launches() { put('T'); return 42; }
+};
+int main(int argc, char** argv) {                // clusters query_ok launch_ok pending tokens hidden experts grid
+    if (argc == 1) return known_clusters();
+    int a[8];
+    for (int i = 0; i < 8; ++i) a[i] = atoi(argv[i + 1]);
+    Fake f{a[0], a[1] != 0, a[2] != 0, a[3] != 0};
+    const int st = mm::launch_frontend_by_size(f, a[4], a[5], a[6], a[7]);
+    printf("%s %d %d\n", f.log, st, f.error ? 1 : 0);
+    return 0;
+}
+"""
+
+
+@pytest.fixture(scope='module')
+def frontend_route(tmp_path_factory):
+    import shutil
+    import subprocess
+    if shutil.which('g++') is None:
+        pytest.skip('no C++ compiler')
+    d = tmp_path_factory.mktemp('route')
+    (d / 'route.cpp').write_text(_ROUTE_PROGRAM)
+    csrc = os.path.join(ROOT, 'hopper_megamoe_basedondeepgemm_b200', 'csrc')
+    cmd = ['g++', '-std=c++17', '-O1', '-pthread', '-Wall', '-Werror', '-I', csrc, '-o', str(d / 'route'), str(d / 'route.cpp')]
+    for sanitizer in (['-fsanitize=thread'], []):                 # (without it where it is not installed or cannot run)
+        if subprocess.run(cmd + sanitizer, capture_output=bool(sanitizer)).returncode == 0:
+            if not sanitizer or 'FATAL: ThreadSanitizer' not in subprocess.run([str(d / 'route')], capture_output=True, text=True).stderr:
+                break
+
+    def run(tokens, hidden=3072, experts=48, grid=148, clusters=7, query_ok=True, launch_ok=True, pending=False):
+        args = [clusters, int(query_ok), int(launch_ok), int(pending), tokens, hidden, experts, grid]
+        if tokens is None:
+            return subprocess.run([str(d / 'route')], capture_output=True, text=True)
+        done, status, error = subprocess.run([str(d / 'route')] + [str(v) for v in args], check=True, capture_output=True, text=True).stdout.split()
+        return done, int(status), bool(int(error))
+    return run
+
+
+def test_frontend_takes_two_launches_where_the_clusters_are_refused(frontend_route):
+    """What the GPU refuses, a query or a launch, leaves the two launches and their status, and no error of its own; one that the
+    caller had pending is not taken away."""
+    assert frontend_route(1) == ('q1', 0, False)
+    assert frontend_route(1, launch_ok=False) == ('q1cT', 42, False)
+    assert frontend_route(9, launch_ok=False) == ('q2cT', 42, False)
+    assert frontend_route(1, query_ok=False) == ('qcT', 42, False)
+    assert frontend_route(1, launch_ok=False, pending=True) == ('q1T', 42, True)
+    assert frontend_route(1, query_ok=False, pending=True) == ('qT', 42, True)
+    assert frontend_route(1, pending=True) == ('q1', 0, True)
+    assert frontend_route(1, clusters=0) == ('qT', 42, False)
+    assert frontend_route(33) == frontend_route(1, hidden=4352) == frontend_route(1, experts=385) == ('T', 42, False)
+
+
+def test_known_clusters_are_kept_only_when_the_query_succeeded(frontend_route):
+    """Under the thread sanitizer, where there is one: the table that threads share has no data race."""
+    r = frontend_route(None)
+    assert r.returncode == 0, (r.returncode, r.stderr[-2000:])
+
+
+@pytest.mark.parametrize('tokens,hidden,experts,grid,per', [
+    (7, 256, 8, 148, 1), (7, 4096, 384, 148, 1), (14, 2048, 8, 148, 2), (15, 4096, 384, 148, 0),                  # as many tokens as clusters, twice as many
+    (8, 2048, 8, 148, 2), (8, 1792, 256, 148, 0), (8, 256, 257, 148, 2),                                          # one token more
+    (9, 1536, 8, 148, 2), (9, 1280, 192, 148, 0), (9, 256, 193, 148, 2),
+    (1, 3072, 48, 16, 1), (1, 3072, 48, 15, 0), (7, 3072, 48, 112, 1), (7, 3072, 48, 111, 0), (9, 3072, 48, 80, 2), (9, 3072, 48, 79, 0),        # the caller's CTAs
+])
+def test_frontend_lines_between_one_and_two_launches(frontend_route, tokens, hidden, experts, grid, per):
+    assert frontend_route(tokens, hidden, experts, grid) == (('q%d' % per, 0, False) if per else ('qT', 42, False))
