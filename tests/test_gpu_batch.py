@@ -8,6 +8,7 @@ import hopper_megamoe_basedondeepgemm_b200 as mm
 from hopper_megamoe_basedondeepgemm_b200 import _lib
 from oracle import megamoe_oracle as O
 from tests import util_moe as U
+from tests.test_gpu_frontend import _canon
 from tests.test_gpu_layer import REL_RMSE_TOL, check_against_oracle, run_layer
 
 pytestmark = pytest.mark.gpu
@@ -223,6 +224,8 @@ def test_from_hidden_states_in_the_decode_and_batch_kernels(fmt, tokens, score_m
     idx, tw = O.route_from_logits(O.router_logits_device_order(x, wr), x, 8, 'sigmoid_bias' if score_mode else 'softmax', bias)
     assert torch.equal(buf.topk_idx[:tokens].cpu(), idx) and torch.allclose(buf.topk_weights[:tokens].cpu(), tw, rtol=2e-6, atol=1e-7)
     fused = [t[:tokens].view(torch.uint8).clone() for t in (buf.x, buf.x_sf, buf.topk_weights)]
+    for t in (buf.x, buf.x_sf, buf.topk_weights):                 # (what the second call left out would be the first one's)
+        t.view(torch.uint8).fill_(0xAA)
     mm.fe_forward_into_buffer(x.cuda(), wr.cuda(), buf, ws, score_mode=score_mode, expert_bias=bias_d, x_global_scale=x_gs)
     assert all(torch.equal(a, t[:tokens].view(torch.uint8)) for a, t in zip(fused, (buf.x, buf.x_sf, buf.topk_weights)))
     q, sf, _ = O.quantise_tokens(x, fmt, rounding='rne', sf_rule='mul', global_scale=x_gs)
@@ -373,6 +376,8 @@ def test_from_hidden_states_on_one_or_two_sms_fills_every_view(fmt, num_sms, tok
     mm.mega_moe_from_hidden(y, x, wr, l1, l2, buf, ws, timeout_ms=500.0)
     assert buf.device_status()[0] == 0
     got = [v[:tokens].view(torch.uint8).clone() for v in views]
+    for v in views:
+        v.view(torch.uint8).fill_(0xAA)
     mm.fe_forward_into_buffer(x, wr, buf, ws)
     for a, v in zip(got, views):
         assert torch.equal(a, v[:tokens].view(torch.uint8))
@@ -385,7 +390,7 @@ def test_from_hidden_states_on_one_or_two_sms_fills_every_view(fmt, num_sms, tok
     (256, 16, 512), (256, 64, 1024),
 ])
 def test_frontend_of_the_one_rank_kernels_matches_the_stand_alone_one(fmt, tokens, e, hidden):
-    """Routing and quantised tokens, bit for bit, whatever the items the partial logits are cut into."""
+    """Routing and quantised tokens, bit for bit, whatever the items the partial logits are cut into; routing and quantised tokens of the oracle."""
     g = torch.Generator().manual_seed(190 + tokens)
     x = torch.randn((tokens, hidden), generator=g).to(torch.bfloat16)
     x[tokens // 2] = 0
@@ -404,6 +409,12 @@ def test_frontend_of_the_one_rank_kernels_matches_the_stand_alone_one(fmt, token
     mm.mega_moe_from_hidden(y, x, wr, stream(2 * inter, hidden), stream(hidden, inter), buf, ws, timeout_ms=500.0, **kw)
     assert buf.device_status()[0] == 0
     got = [v[:tokens].view(torch.uint8).clone() for v in views]
+    idx, _ = O.route_from_logits(O.router_logits_device_order(x.cpu(), wr.cpu()), x.cpu(), 8)
+    assert torch.equal(buf.topk_idx[:tokens].cpu(), idx)
+    q, _, sfb = O.quantise_tokens(x.cpu(), fmt, rounding='rne', sf_rule='mul', global_scale=kw.get('x_global_scale', 1.0))
+    assert torch.equal(_canon(got[0].cpu(), fmt), _canon(q, fmt)) and torch.equal(got[1].cpu().view(tokens, -1), sfb)
+    for v in views:
+        v.view(torch.uint8).fill_(0xAA)
     mm.fe_forward_into_buffer(x, wr, buf, ws, **kw)
     for a, v in zip(got, views):
         assert torch.equal(a, v[:tokens].view(torch.uint8))
