@@ -30,8 +30,8 @@ int sf_vec_of(int fmt) { return fmt == MM_FMT_NVFP4 ? 16 : 32; }
 
 // development knobs (mm_set_tuning): kernel feature bits, ring depth (0 = chosen from the shared-memory plan), and how
 // many experts' W1 / W2 the scout may prefetch into the L2 in one launch
-// (the L2 prefetch of live experts' weights is off by default: measured, it does not shorten the weight stream - bulk
-// copies from the L2 are barely faster than from HBM here - and its traffic delays the launch's small critical loads)
+// (the L2 prefetch of live experts' weights is off by default: measured, it does not shorten the weight stream, whose
+// bytes have to come from HBM all the same, and its traffic delays the launch's small critical loads)
 int g_tuning[MM_TUNE_COUNT] = {mm::kKnobOwnRows | mm::kKnobEarlyCombine | mm::kKnobTileImages | mm::kKnobDecode, 0, 14, 14, 1};
 
 int check_config(const mm_config_t* c) {
@@ -502,7 +502,7 @@ static mm::BParams one_rank_params(const mm_config_t* cfg, const mm::KParams& k,
     p.unit_bytes = k.unit_bytes;
     // (96 rows of E4M3 tokens: set when the units were widened in 66 KB of shared memory, beside which records of 128 rows left too few stages. With
     // the units in tensor memory 128 rows measure better where an expert has more than 96: 300 tokens over 24 experts 81.1 -> 74.5 us, 512
-    // over 48 124.3 -> 119.8, 100 over 48 level. The limit is the older one.)
+    // over 48 124.3 -> 119.8, 100 over 48 level; four stages and three records would fit. Not raised so far.)
     p.tile_limit = cfg->act_format == MM_FMT_FP8 ? 96u : 128u;
     p.x_row_bytes = k.x_row_bytes; p.x_sf_row_bytes = k.x_sf_row_bytes; p.rx_row_bytes = k.rx_row_bytes; p.mid_row_bytes = k.mid_row_bytes;
     p.has_clamp = k.has_clamp; p.fast_math = k.fast_math; p.clamp = k.clamp;

@@ -14,17 +14,17 @@
 //              turns 16 tokens at a time through shared memory, so that all 128 threads of a group work whatever the row
 //              count and a thread holds eight gate and eight up values of one token. Two groups take the tasks in turn.
 //   order    : the L1 tasks dealt round-robin, but the last one to two rounds of them and all L2 tasks claimed one by one
-//              (no tile is split along K, a slow SM takes fewer). L2 goes tile by tile, its last two tasks per SM column
-//              block by column block. The weight ring runs ahead over the L1 -> L2 hand-over, so that the stream does not
+//              (no tile is split along K, a slow SM takes fewer). L2 goes tile by tile, its last two or four tasks per SM
+//              column block by column block. The weight ring runs ahead over the L1 -> L2 hand-over, so that the stream does not
 //              stop there. (When this order came in: 59.2, 67.2 and 102 us with all L1 tasks dealt and L2 column by column, 57.2,
 //              64.9 and 100 with it, for 13 and 64 tokens over 48 experts and 96 skewed ones from hidden states.)
 //   combine  : per (token, 128-column block) behind a count per column block; routes added in slot order in fp32.
 //
-// Bound: HBM (the weights of the live experts once) up to about 40 rows per expert. 64 tokens, MXFP4, 48 experts (301 MB): 51.9 us a
-// pass, of which the stream is 42 at 7.1 TB/s; with weights from the L2 the same launch takes 40. The multi-rank kernel takes 88. Beyond, no single thing: 512
-// tokens 75.9 us, 67 with the weights from the L2, 70 without the epilogue's arithmetic, 71 with a quarter of the MMAs, 72 with short
-// records, and the power limit takes a tenth of the clock. With E4M3 tokens the units are widened into tensor memory
-// (100 tokens: 68 us, 765 with the multi-rank kernel), and the clock is 5 % lower.
+// Bound: HBM (the weights of the live experts once) up to about 40 rows per expert. 64 tokens, MXFP4, 48 experts (301 MB): 52 to 53.5 us a
+// pass on different B200s, of which the stream is 42 at 7.1 TB/s; with four experts' weights in the place of all 48, which stay in the L2, 40. The
+// multi-rank kernel takes 88. Beyond, no single thing: 512 tokens 76 to 79 us; 67 with weights from the L2 in the same way, 70 without the epilogue's
+// arithmetic, 71 with a quarter of the MMAs, 72 with short records (76 without any of it, on the same GPU), and the power limit takes a tenth of
+// the clock. With E4M3 tokens the units are widened into tensor memory (100 tokens: 67 to 70 us, 765 with the multi-rank kernel), and the clock is 5 % lower.
 #pragma once
 #include "mm_kernel.cuh"
 
@@ -984,8 +984,8 @@ __global__ void __launch_bounds__(BFmt<kFmt>::kThreadsAll, 1) batch_moe_kernel(c
             if (cx.expired()) { cx.fail(kErrWaitFrontend); return true; }
             return false;
         };
-        // Items of one token where every warp gets one at most: all its loads are in flight at once (two round trips less than with
-        // items of four tokens; 3 tokens 37.2 -> 35.3 us a pass, 24: 57.5 -> 55.3). Up to 24 items of four tokens per SM, one expert to an
+        // Items of one token where every warp gets one at most: all its loads are in flight at once up to hidden 3072, in two trips beyond (two
+        // round trips less than with items of four tokens; 3 tokens 37.2 -> 35.3 us a pass, 24: 57.5 -> 55.3). Up to 24 items of four tokens per SM, one expert to an
         // item (150 tokens 72.0 -> 70.7); beyond, where the bytes count, blocks of experts (256: 79.2 -> 76.8 all in all). Two
         // more block sizes in between gained nothing: the launch pays for code that it jumps over.
         const uint32_t half_warps = kBRankWarps / 2, per = static_cast<uint32_t>(p.E) * kFeParts;

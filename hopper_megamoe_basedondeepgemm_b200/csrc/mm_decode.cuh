@@ -561,7 +561,7 @@ __global__ void __launch_bounds__(DFmt<kFmt>::kThreads, 1) decode_moe_kernel(con
         }
     } else {
         // ---- router frontend: partial logits spread over the SMs; selection and quantisation on every SM. An item is one token's, with all its
-        //      loads in flight (one token 27.2 -> 26.2 us a pass against items of four tokens in two trips, two with E4M3 38.9 -> 36.8)
+        //      loads in flight up to hidden 3072, in two trips beyond (one token 27.2 -> 26.2 us a pass against items of four tokens in two trips, two with E4M3 38.9 -> 36.8)
         fe_logits_blocks<1, 6, 1>(p.fe, warp * G + bid, G * (F::kThreads / 32), lane, flag);
         if (builder) {
             // A slice of 256 elements to a warp at a time, two in flight. (Every warp used to quantise the tokens of its entries, the same token in eight

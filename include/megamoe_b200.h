@@ -114,8 +114,8 @@ typedef struct mm_frontend_args {
     const float* expert_bias;        /* optional float [num_experts] (score_mode 1) */
     int32_t num_tokens;
     int32_t score_mode;              /* 0: softmax over the selected logits; 1: sigmoid + bias selection, renormalised */
-    void* workspace;                 /* mm_frontend_workspace_bytes() bytes of device memory (partial logits of the two-kernel frontend;
-                                        the single-kernel path keeps its own inside the buffer and only requires it non-NULL) */
+    void* workspace;                 /* mm_frontend_workspace_bytes() bytes of device memory (partial logits of the stand-alone frontend;
+                                        the launch that runs router and layer keeps its own inside the buffer and only requires it non-NULL) */
     float x_global_scale;
 } mm_frontend_args_t;
 
