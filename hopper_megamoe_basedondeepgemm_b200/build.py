@@ -9,7 +9,7 @@ LIB_PATH = os.path.join(PKG_DIR, LIB_NAME)
 # test build: the same library plus the CUDA-core cross-check engine (`engine='check'`), loaded by the tests only
 CHECK_LIB_PATH = os.path.join(PKG_DIR, 'libmegamoe_b200_check.so')
 SOURCES = ['mm_abi.cu']
-HEADERS = ['mm_kernel.cuh', 'mm_frontend.cuh', 'mm_frontend_route.h', 'mm_ptx.cuh', 'mm_prep.cuh', 'mm_batch.cuh', 'mm_decode.cuh', os.path.join('..', '..', 'include', 'megamoe_b200.h')]
+HEADERS = ['mm_kernel.cuh', 'mm_frontend.cuh', 'mm_frontend_route.h', 'mm_device_attribute.h', 'mm_ptx.cuh', 'mm_prep.cuh', 'mm_batch.cuh', 'mm_decode.cuh', os.path.join('..', '..', 'include', 'megamoe_b200.h')]
 
 
 def _stale(path: str) -> bool:

@@ -11,6 +11,7 @@
 #include "mm_prep.cuh"
 #include "mm_batch.cuh"
 #include "mm_decode.cuh"
+#include "mm_device_attribute.h"
 
 namespace {
 
@@ -457,13 +458,11 @@ template <int kVec, bool kUmma, bool kFe = false, bool kA8 = false, bool kTiles 
 static int launch_variant(const mm::KParams& p, int grid, size_t smem_bytes, cudaStream_t stream) {
     auto kern = mm::mega_moe_kernel<kVec, kUmma, kFe, kA8, kTiles>;
     // the opt-in shared-memory size is a per-device function attribute: set once per (variant, device), raised on demand
-    static int attr_bytes[64] = {};
+    static mm::DeviceAttribute attribute;
     int dev = 0;
     MM_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || attr_bytes[dev] < static_cast<int>(smem_bytes)) {
-        MM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_bytes)));
-        if (dev >= 0 && dev < 64) attr_bytes[dev] = static_cast<int>(smem_bytes);
-    }
+    const int bytes = static_cast<int>(smem_bytes);
+    MM_CUDA(attribute.raise(dev, bytes, [&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); }));
     return launch_early<mm::KParams>(kern, grid, kA8 ? mm::kThreads + mm::kNumExpThreads : mm::kThreads, smem_bytes, stream, p);
 }
 
@@ -520,15 +519,12 @@ static mm::BParams one_rank_params(const mm_config_t* cfg, const mm::KParams& k,
 
 // shared memory: all an SM has, less the kernel's static part
 template <typename Shared>
-static int launch_one_rank(void (*kern)(mm::BParams), int threads, mm::BParams& p, int grid, bool (&attr_set)[64], cudaStream_t stream) {
+static int launch_one_rank(void (*kern)(mm::BParams), int threads, mm::BParams& p, int grid, mm::DeviceAttribute& attribute, cudaStream_t stream) {
     const int dyn = 232448 - static_cast<int>((sizeof(Shared) + 255) / 256 * 256);
     p.smem_ring = static_cast<uint32_t>(dyn - 1024);
     int dev = 0;
     MM_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-        MM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
-        if (dev >= 0 && dev < 64) attr_set[dev] = true;
-    }
+    MM_CUDA(attribute.raise(dev, dyn, [&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn); }));
     return launch_early<mm::BParams>(kern, grid, threads, dyn, stream, p);
 }
 
@@ -550,7 +546,7 @@ static uint32_t column_tasks(const mm::BParams& p, int grid) {
 
 template <int kFmt, bool kFe>
 static int launch_one_rank_fmt(mm::BParams& p, bool decode, int grid, cudaStream_t stream) {
-    static bool batch_attr[64] = {}, ask_attr[64] = {}, decode_attr[64] = {};
+    static mm::DeviceAttribute batch_attr, ask_attr, decode_attr;
     if (decode) return launch_one_rank<mm::DShared>(mm::decode_moe_kernel<kFmt, kFe>, mm::DFmt<kFmt>::kThreads, p, grid, decode_attr, stream);
     p.column_tasks = column_tasks(p, grid);
     constexpr bool kMayAsk = kFmt != 2;

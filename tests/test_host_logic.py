@@ -471,6 +471,7 @@ _ROUTE_PROGRAM = r"""
 #include <thread>
 #include <vector>
 #include "mm_frontend_route.h"
+#include "mm_device_attribute.h"
 static int known_clusters() {                    // failures are asked again, answers kept unless not to be, by threads in any order
     mm::KnownClusters k;
     int n = -1, asked = 0;
@@ -499,6 +500,30 @@ static int known_clusters() {                    // failures are asked again, an
     for (auto& t : threads) t.join();
     return bad.load() == 0 ? 0 : 7;
 }
+static int device_attribute() {                  // raised by threads in any order, never below what one of them needs
+    mm::DeviceAttribute a;
+    int sets = 0;
+    auto fails = [&] { ++sets; return 7; };
+    auto sets_it = [&] { ++sets; return 0; };
+    if (a.raise(1, 100, fails) != 7 || a.raise(1, 100, sets_it) != 0 || a.raise(1, 90, fails) != 0 || sets != 2) return 1;
+    if (a.raise(2, 90, sets_it) != 0 || a.raise(1, 101, sets_it) != 0 || sets != 4) return 2;
+    if (a.raise(-1, 1, fails) != 7 || a.raise(64, 1, sets_it) != 0 || a.raise(64, 1, fails) != 7 || sets != 7) return 3;
+    std::atomic<int> bad{0};
+    for (int round = 0; round < 200; ++round) {
+        mm::DeviceAttribute shared;
+        std::atomic<int> now{0};                 // the attribute
+        std::vector<std::thread> threads;
+        for (int t = 1; t <= 4; ++t)
+            threads.emplace_back([&, t] {
+                for (int bytes = t; bytes < 40; bytes += 4) {
+                    shared.raise(0, bytes, [&] { std::this_thread::yield(); now = bytes; return 0; });
+                    if (now < bytes) ++bad;      // (a launch that needs `bytes` would be refused)
+                }
+            });
+        for (auto& t : threads) t.join();
+    }
+    return bad.load() == 0 ? 0 : 4;
+}
 struct Fake {                                    // a GPU whose answers are made up; `log`: what was done
     int clusters_; bool query_ok, launch_ok, error = false; char log[64] = {}; int n = 0;
     void put(char c) { log[n++] = c; }
@@ -510,6 +535,7 @@ struct Fake {                                    // a GPU whose answers are made
 };
 int main(int argc, char** argv) {                // clusters query_ok launch_ok pending tokens hidden experts grid
     if (argc == 1) return known_clusters();
+    if (argc == 2) return device_attribute();
     int a[8];
     for (int i = 0; i < 8; ++i) a[i] = atoi(argv[i + 1]);
     Fake f{a[0], a[1] != 0, a[2] != 0, a[3] != 0};
@@ -537,8 +563,8 @@ def frontend_route(tmp_path_factory):
 
     def run(tokens, hidden=3072, experts=48, grid=148, clusters=7, query_ok=True, launch_ok=True, pending=False):
         args = [clusters, int(query_ok), int(launch_ok), int(pending), tokens, hidden, experts, grid]
-        if tokens is None:
-            return subprocess.run([str(d / 'route')], capture_output=True, text=True)
+        if isinstance(tokens, list):
+            return subprocess.run([str(d / 'route')] + tokens, capture_output=True, text=True)
         done, status, error = subprocess.run([str(d / 'route')] + [str(v) for v in args], check=True, capture_output=True, text=True).stdout.split()
         return done, int(status), bool(int(error))
     return run
@@ -560,7 +586,13 @@ def test_frontend_takes_two_launches_where_the_clusters_are_refused(frontend_rou
 
 def test_known_clusters_are_kept_only_when_the_query_succeeded(frontend_route):
     """Under the thread sanitizer, where there is one: the table that threads share has no data race."""
-    r = frontend_route(None)
+    r = frontend_route([])
+    assert r.returncode == 0, (r.returncode, r.stderr[-2000:])
+
+
+def test_kernel_attributes_of_a_device_are_only_raised(frontend_route):
+    """Threads that launch a kernel with different shared memory sizes for the first time: none finds the attribute below its own."""
+    r = frontend_route(['attribute'])
     assert r.returncode == 0, (r.returncode, r.stderr[-2000:])
 
 
