@@ -536,19 +536,24 @@ static bool asks_ahead(const mm::BParams& p, int grid) {
     return static_cast<long long>(p.T) * p.topk <= mm::kBAheadEntries && p.E * (p.n1 * p.k1 + p.n2 * p.k2) > 8 * grid;
 }
 
-// L2 tasks per SM that go column block by column block, beside which the combine runs: two, or four where it takes longer than two, that is where
-// it reads more than 40 KB per SM and K unit of a task. (us a pass with two, four: 400 tokens over 64 experts of 3072 x 512, 66 KB, 49.0, 48.2, NVFP4
+// Tiles whose L2 tasks go column block by column block, so that the combine runs beside them: two tasks per SM, or four where it takes longer than two, that
+// is where it reads more than 40 KB per SM and K unit of a task (us a pass with two, four: 400 tokens over 64 experts of 3072 x 512, 66 KB, 49.0, 48.2, NVFP4
 // 52.2, 50.9, E4M3 61.4, 60.9; 512 over 16 of 4096 x 768, 76 KB, 59.0, 58.3; 250 over 48 of 3072 x 1280, 17 KB, 57.2, 58.3; 128 over 16 of
-// 4096 x 768, 19 KB, 32.7, 34.5; 512 over 64 of 1536 x 1536, 14 KB, 56.0, 57.3.)
-static uint32_t column_tasks(const mm::BParams& p, int grid) {
-    return static_cast<long long>(p.T) * p.topk * p.H * 2 > 40960ll * p.k2 * grid ? 2u * mm::kBColumnTasks : mm::kBColumnTasks;
+// 4096 x 768, 19 KB, 32.7, 34.5; 512 over 64 of 1536 x 1536, 14 KB, 56.0, 57.3), and where the tiles in front of them keep an SM busy for ten units: the last
+// tiles have just had their L1 tasks, and the first column block wants all of them (300 E4M3 tokens over 32 experts of 4096 x 512, six units: 53.9, 57.2).
+// How many tiles a launch has is known on the device only; it gets both numbers.
+static void set_column_tiles(mm::BParams& p, int grid) {
+    const bool long_combine = static_cast<long long>(p.T) * p.topk * p.H * 2 > 40960ll * p.k2 * grid;
+    p.column_tiles = (mm::kBColumnTasks * grid + p.n2 - 1) / p.n2;
+    p.column_tiles_long = (2 * mm::kBColumnTasks * grid + p.n2 - 1) / p.n2;
+    p.column_long_from = long_combine ? ((2 * mm::kBColumnTasks * p.k2 + 10) * grid + p.n2 * p.k2 - 1) / (p.n2 * p.k2) : ~0u;
 }
 
 template <int kFmt, bool kFe>
 static int launch_one_rank_fmt(mm::BParams& p, bool decode, int grid, cudaStream_t stream) {
     static mm::DeviceAttribute batch_attr, ask_attr, decode_attr;
     if (decode) return launch_one_rank<mm::DShared>(mm::decode_moe_kernel<kFmt, kFe>, mm::DFmt<kFmt>::kThreads, p, grid, decode_attr, stream);
-    p.column_tasks = column_tasks(p, grid);
+    set_column_tiles(p, grid);
     constexpr bool kMayAsk = kFmt != 2;
     if (kMayAsk && asks_ahead(p, grid))
         return launch_one_rank<mm::BShared>(mm::batch_moe_kernel<kFmt, kFe, kMayAsk>, mm::BFmt<kFmt>::kThreadsAll, p, grid, ask_attr, stream);

@@ -31,7 +31,7 @@
 namespace mm {
 
 constexpr int kBMaxRows = 4096;                    // routed rows of one launch
-constexpr uint32_t kBColumnTasks = 2;              // L2 tasks per SM that are claimed column block by column block, at least (`column_tasks`)
+constexpr uint32_t kBColumnTasks = 2;              // L2 tasks per SM that are claimed column block by column block, at least (`set_column_tiles`)
 constexpr uint32_t kBAhead = 4;                    // K units that are asked into the L2 ahead, twice at the start of a launch
 constexpr int kBAheadEntries = 2048;               // of at most so many routing entries (512 tokens of 8: 78.1 us without, 78.7 with; 256 57.2, 56.9)
 constexpr int kBTaskRing = 64;                     // claimed tasks of one SM that some role has still to see, at most
@@ -67,7 +67,7 @@ struct BParams {
     uint32_t mid_row_bytes;
     FeParams fe;
     uint32_t smem_ring;                            // bytes of dynamic shared memory for the two rings
-    uint32_t column_tasks;                         // L2 tasks per SM that are claimed column block by column block (batch kernel), if there is time for them
+    uint32_t column_tiles, column_tiles_long, column_long_from;    // tiles whose L2 tasks go column block by column block (batch kernel); the larger number from so many tiles on
     unsigned long long timeout_ns;
 };
 
@@ -242,16 +242,13 @@ __device__ void b_role_weights(const BCtx& cx, uint32_t lane) {
     const uint64_t policy = l2_evict_first_policy();
     uint32_t it = 0, s = 0, ph = 0;
     BTasks tasks(cx);
+    // Order of the L2 tasks: tile by tile (the first tiles' L1 outputs are complete long before the last ones'), but the last
+    // tiles column block by column block: the combine starts on a column block when all tiles have it, beside the remaining ones. How many: `set_column_tiles`.
+    const uint32_t NT1 = M * n1, NT2 = M * n2, tail = M >= p.column_long_from ? p.column_tiles_long : p.column_tiles, mA = tail < M ? M - tail : 0u, NA = mA * n2;
     // The stream starts when this SM's rows are in the images. What an SM has asked for comes back in order: behind 100 KB and more of weights
     // the acknowledgement of the rows' release took 2 to 3 us, and every task that wants one of them waited
     // for it (13 tokens: 51.3 -> 50.0 us a pass, 64: 60.3 -> 58.6, 512: 80.3 -> 79.8, 6 of the small layer: 15.4 -> 15.0).
     bar_sync(kBBarPlaced, 32u * (kBWorkWarps + 1));
-    // Order of the L2 tasks: tile by tile (the first tiles' L1 outputs are complete long before the last ones'), but the last
-    // tiles, two or four tasks per SM of them, column block by column block: the combine starts on a column block when all
-    // tiles have it, beside the remaining ones. Four where the launch asks for them (`column_tasks`) and the tiles in front keep an SM busy for
-    // ten units: the last tiles have just had their L1 tasks, and the first column block wants all of them (300 E4M3 tokens over 32 experts of
-    // 4096 x 512, six units: 57.2 us a pass with four, 53.9 with two).
-    const uint32_t NT1 = M * n1, NT2 = M * n2, tail = udiv_small((NT2 * p.k2 >= (4u * p.k2 + 10u) * G ? p.column_tasks : kBColumnTasks) * G + n2 - 1u, n2), mA = tail < M ? M - tail : 0u, NA = mA * n2;
     uint32_t* claims = cx.counter(cx.par, kBCountClaims);
     uint32_t next = 0u;
     if (tasks.my1 == 0u && lane == 0) next = atomicAdd(claims, 1u);
